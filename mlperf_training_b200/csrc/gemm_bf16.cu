@@ -219,7 +219,8 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
 // One CTA pair per 256 x BN tile (gemm_core.cuh).
 template <int BN>
 static int run_pair(const void* a, const void* b, void* d, int M, int N, int K, long long lda, long long ldb,
-                    long long ldd, int a_mn_major, int b_mn_major, const gemmcore::EpiArgs& epi, cudaStream_t stream) {
+                    long long ldd, int a_mn_major, int b_mn_major, const gemmcore::EpiArgs& epi, void* ws, long long ws_bytes,
+                    cudaStream_t stream) {
   using namespace gemmcore;
   CUtensorMap tmA, tmB, tmD;
   int r;
@@ -238,16 +239,27 @@ static int run_pair(const void* a, const void* b, void* d, int M, int N, int K, 
   p.group_m = raster_group_m() > 1 ? raster_group_m() / 2 : 1;
   p.epi = epi;
   p.status = b200::status_ptr();
-  return launch_pair<KIND_BF16, BN, 1>(tmA, tmB, tmA, tmB, tmD, tmDt, p, stream, "gemm_bf16(pair)");
+  return launch_pair<KIND_BF16, BN, 1, 1>(tmA, tmB, tmA, tmB, tmD, tmDt, p, stream, "gemm_bf16(pair)", nullptr, (float*)ws,
+                                       ws_bytes, d, ldd);
+}
+
+// Workspace (bytes, 16-byte aligned) with which b200_gemm_bf16 splits the last wave of an M x N x K problem along K
+// (gemm_core.cuh: SplitArgs); 0 where that does not pay.  The call accepts none, too.
+B200_API long long b200_gemm_bf16_workspace(int M, int N, int K) {
+  using namespace gemmcore;
+  if (M <= 128 || N <= 0 || K <= 0 || !pair_enabled()) return 0;
+  int rc = 0;
+  return N > 128 ? split_bytes<256>(pair_split<KIND_BF16, 256, 1>(M, N, K, rc)) : split_bytes<128>(pair_split<KIND_BF16, 128, 1>(M, N, K, rc));
 }
 
 // D[M,N] (=|+=) alpha * A * B^T (+ bias) (+ residual)
 //   a: K-major [M, lda] (a_mn_major = 0) or MN-major [K, lda] (a_mn_major = 1); same for b with N.
 //   lda / ldb / ldd / ldr are row pitches in elements.  out_f32 selects fp32 D.  accumulate != 0 adds into D.
+//   workspace: null, or b200_gemm_bf16_workspace(M, N, K) bytes that nothing else uses until this call's work is done.
 B200_API int b200_gemm_bf16(const void* a, const void* b, void* d, int M, int N, int K, long long lda,
                             long long ldb, long long ldd, int a_mn_major, int b_mn_major, int out_f32,
                             int accumulate, const void* bias, const void* residual, long long ldr, float alpha,
-                            void* stream) {
+                            void* workspace, long long workspace_bytes, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return b200::fail(210, "gemm_bf16: empty problem %d x %d x %d", M, N, K);
   const int BN = (N > 128) ? 256 : 128;
   gemmcore::EpiArgs epi = {};
@@ -259,9 +271,9 @@ B200_API int b200_gemm_bf16(const void* a, const void* b, void* d, int M, int N,
   epi.alpha = alpha;
   if (M > 128 && gemmcore::pair_enabled()) {
     if (BN == 256) return run_pair<256>(a, b, d, M, N, K, lda, ldb, ldd, a_mn_major ? 1 : 0, b_mn_major ? 1 : 0, epi,
-                                        (cudaStream_t)stream);
+                                        workspace, workspace_bytes, (cudaStream_t)stream);
     return run_pair<128>(a, b, d, M, N, K, lda, ldb, ldd, a_mn_major ? 1 : 0, b_mn_major ? 1 : 0, epi,
-                         (cudaStream_t)stream);
+                         workspace, workspace_bytes, (cudaStream_t)stream);
   }
   CUtensorMap tmA, tmB, tmD, tmDt;
   int r;

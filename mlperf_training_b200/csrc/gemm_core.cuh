@@ -32,6 +32,7 @@
 //
 // Tile schedulers on the same mainloop (tile_info):
 //   * dense            grouped raster over (row tile, column tile)
+//   * SplitArgs        dense, with the tiles of the last, partly filled wave cut along K over the idle pairs
 //   * GroupArgs        MoE: rows grouped by expert with the stacked expert weights as B (forward, dgrad), or one
 //                      contraction range per expert (weight gradients)
 //   * TpGather         all-gather -> GEMM: the first CTA pairs of the launch copy the ranks' row blocks over NVLink
@@ -340,8 +341,40 @@ struct GroupArgs {
 
 struct TileInfo {
   int mb, nb, e, kb0, nkb;
+  int part;                       // >= 0: index of the partial tile in the split workspace
   bool valid;
 };
+
+// The last wave of a persistent launch.  `tiles` tiles on P pairs take ceil(tiles / P) waves, so a launch of 96 tiles
+// on 74 pairs spends half its time with 52 pairs idle, and a weight gradient of 16 tiles leaves 58 idle for all of its
+// (long) contraction.  The first `first` tiles (whole waves) run as they are; each of the `rem` tiles left is cut along K
+// into S slices of `per` k stages, which write fp32 partial tiles to a workspace ([rem * S][256][BN], dense) that
+// split_finish_kernel adds up in slice order (no atomics: runs are bit-reproducible) and takes through the epilogue.
+struct SplitArgs {
+  int first, rem, S, per;         // rem = 0: no split
+};
+
+// Chooses S for `tiles` tiles of `num_kb` k stages of `stage_us` microseconds on P pairs; partial tiles of `tile_bytes`.
+// Estimated time of the last wave: rounds of slices, plus the partial tiles written and read once (6 TB/s, out of L2)
+// and 5 us for the second launch; the split is taken when that is 5 % less than the unsplit wave.  Measured on 74
+// pairs, L2 flushed, without -> with the split (M x N x K):
+//   bf16   2048 x 512 x 92160 456 -> 144 us;  512 x 1536 x 92160 457 -> 112;  2048 x 3072 x 12288 131 -> 105;
+//          4011 x 4096 x 14336 341 -> 290;  256 x 3072 x 12288 68 -> 38;  2000 x 5120 x 2880 68 -> 54
+//   MXFP8  2048 x 4096 x 14336 123 -> 103 us;  256 x 3072 x 14336 51 -> 34;  4096 x 4096 x 8192 121 -> 116
+// No problem that the rule splits was slower in a sweep of 256..8192 x 512..6144 x 1024..14336.
+inline SplitArgs split_plan(int tiles, int num_kb, double stage_us, double tile_bytes, int P) {
+  SplitArgs best = {tiles, 0, 1, num_kb};
+  const int first = tiles / P * P, rem = tiles - first;
+  if (rem == 0) return best;
+  double best_us = num_kb * stage_us;
+  for (int S = 2; S <= 16 && num_kb / S >= 4; ++S) {
+    const int per = (num_kb + S - 1) / S;
+    if ((S - 1) * per >= num_kb) continue;             // every slice needs work: its partial tile is read
+    const double us = (double)((rem * S + P - 1) / P) * per * stage_us + 2.0 * rem * S * tile_bytes / 6e6 + 5.0;
+    if (us < 0.95 * best_us) { best_us = us; best = {first, rem, S, per}; }
+  }
+  return best;
+}
 
 // All-gather -> GEMM inside one launch (tensor parallelism, sequence-parallel activations): the rows of A are
 // gathered over W ranks.  Rank c's block is the byte range [c * chunk_bytes, (c + 1) * chunk_bytes) of a buffer
@@ -395,6 +428,7 @@ struct OwnerMaps { CUtensorMap m[NOWN]; };
 
 struct PairParams {
   GroupArgs grp;
+  SplitArgs split;
   int M, N, K;                    // K in elements (bf16) or bytes (e4m3); mode 2: M, N per expert, K = all rows
   int a_mn_major, b_mn_major;     // bf16 only
   int a_fmt, b_fmt;               // FP8 only: 0 = e4m3, 1 = e5m2
@@ -409,7 +443,16 @@ struct PairParams {
 // elements per stage).
 B200_DEVICE TileInfo tile_info(int t, int num_m, int num_n, int num_kb, int kb_elems, const PairParams& p) {
   TileInfo ti;
-  ti.e = 0; ti.kb0 = 0; ti.nkb = num_kb; ti.valid = true;
+  ti.e = 0; ti.kb0 = 0; ti.nkb = num_kb; ti.valid = true; ti.part = -1;
+  if (p.split.rem > 0 && t >= p.split.first) {
+    // neighbouring pairs take the same slice of neighbouring tiles (their operand panels are shared in L2)
+    const int r = t - p.split.first, slice = r / p.split.rem, i = r - slice * p.split.rem;
+    ti.kb0 = slice * p.split.per;
+    ti.nkb = min(p.split.per, num_kb - ti.kb0);
+    ti.part = i * p.split.S + slice;
+    tile_coords(p.split.first + i, num_m, num_n, p.group_m, ti.mb, ti.nb);
+    return ti;
+  }
   if (p.grp.mode == 2) {
     const int per = num_m * num_n;
     ti.e = t / per;
@@ -446,6 +489,7 @@ __global__ void __launch_bounds__(PairCfg<KIND, BN, KSUB>::THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmSFA, const __grid_constant__ CUtensorMap tmSFB,
                  const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmDt,
+                 const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmWt,
                  const __grid_constant__ PairParams p, const __grid_constant__ OwnerMaps<NOWN> om) {
   using C = PairCfg<KIND, BN, KSUB>;
   constexpr bool MX = C::MX;
@@ -481,7 +525,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int num_pairs = (int)(gridDim.x >> 1) - n_aux;
   const int num_m = (p.M + 255) / 256;
   const int num_n = (p.N + BN - 1) / BN;
-  const int num_tiles = (p.grp.mode == 2 ? p.grp.E : 1) * num_m * num_n;
+  // work units: whole tiles, then the slices of the split tiles
+  const int num_tiles = p.split.rem > 0 ? p.split.first + p.split.rem * p.split.S
+                                        : (p.grp.mode == 2 ? p.grp.E : 1) * num_m * num_n;
   const int num_kb = (p.K + KB_ELEMS * KSUB - 1) / (KB_ELEMS * KSUB);
   const int num_kb128 = (p.K + KB_ELEMS - 1) / KB_ELEMS;   // 128-byte K blocks (scale groups of the MX layout)
 
@@ -667,7 +713,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           tpcopy::red_release_sys_add(p.rs.flag_peer[owner] + (m0 - owner * p.rs.rows_per) / 128, 1);
         }
       } else {
-        epilogue_drain<BN, (BN % 64 == 0)>(&tmD, &tmDt, p.epi, t_row, ti.mb * 256 + (int)rank * 128 + q * 32, ti.nb * BN, stg, buf,
+        const bool part = ti.part >= 0;             // a slice of a split tile: fp32 accumulators, as they are
+        EpiArgs e = p.epi;
+        if (part) {
+          e = EpiArgs{};
+          e.M = 0x7fffffff; e.N = BN; e.out_f32 = 1; e.alpha = 1.f;
+        }
+        epilogue_drain<BN, (BN % 64 == 0)>(part ? &tmW : &tmD, part ? &tmWt : &tmDt, e, t_row,
+                                           (part ? ti.part : ti.mb) * 256 + (int)rank * 128 + q * 32, part ? 0 : ti.nb * BN, stg, buf,
                                            lane, p.grp.mode == 2 ? ti.e * p.M : 0);
       }
       // all TMEM reads of this accumulator are complete (tcgen05.wait::ld inside): hand it back to the leader
@@ -736,23 +789,75 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
-// Launches gemm_pair_kernel on as many CTA pairs as can be resident at once (a persistent grid must
-// not exceed that: a pair that waits for SMs would start only after a resident pair finished all its
-// tiles).  Returns 0, or a failure code with message.
-template <int KIND, int BN, int KSUB, int NOWN = 1>
-int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmSFA, const CUtensorMap& tmSFB,
-                const CUtensorMap& tmD, const CUtensorMap& tmDt, const PairParams& p, cudaStream_t stream,
-                const char* what, const OwnerMaps<NOWN>* owners = nullptr) {
+// Adds up the S partial tiles of every split tile in slice order and finishes them as the epilogue would (alpha, bias,
+// residual, store or add).  A thread owns 8 columns of a row: 2 x S 16-byte loads in flight, one or two 16-byte stores.
+template <int BN>
+__global__ void __launch_bounds__(256)
+split_finish_kernel(const float* __restrict__ ws, SplitArgs sp, int num_m, int num_n, int group_m, EpiArgs e, void* d, long long ldd) {
+  constexpr int VPR = BN / 8;
+  float alpha = e.alpha;
+  if (e.alpha_a != nullptr) alpha *= *e.alpha_a;
+  if (e.alpha_b != nullptr) alpha *= *e.alpha_b;
+  const int i = blockIdx.y;
+  int mb, nb;
+  tile_coords(sp.first + i, num_m, num_n, group_m, mb, nb);
+  for (int u = blockIdx.x * 256 + threadIdx.x; u < 256 * VPR; u += gridDim.x * 256) {
+    const int r = u / VPR, c = (u - r * VPR) * 8;
+    const int row = mb * 256 + r, col = nb * BN + c;
+    if (row >= e.M || col >= e.N) continue;
+    const float* src = ws + ((long long)i * sp.S * 256 + r) * BN + c;
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int s = 0; s < sp.S; ++s) {
+      const float4 a = *reinterpret_cast<const float4*>(src + (long long)s * 256 * BN);
+      const float4 b = *reinterpret_cast<const float4*>(src + (long long)s * 256 * BN + 4);
+      v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w; v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+    }
+    const int n = min(8, e.N - col);                 // (N may end inside the vector)
+    const __nv_bfloat16* res = e.residual != nullptr ? e.residual + (long long)row * e.ldr + col : nullptr;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] *= alpha;
+      if (j < n) {
+        if (e.bias != nullptr) v[j] += __bfloat162float(e.bias[col + j]);
+        if (res != nullptr) v[j] += __bfloat162float(res[j]);
+      }
+    }
+    // (D rows are 16-byte aligned and col is a multiple of 8)
+    if (e.out_f32) {
+      float* o = reinterpret_cast<float*>(d) + (long long)row * ldd + col;
+      if (n == 8) {
+        float4 lo = make_float4(v[0], v[1], v[2], v[3]), hi = make_float4(v[4], v[5], v[6], v[7]);
+        if (e.accumulate) {
+          const float4 a = *reinterpret_cast<float4*>(o), b = *reinterpret_cast<float4*>(o + 4);
+          lo = make_float4(lo.x + a.x, lo.y + a.y, lo.z + a.z, lo.w + a.w);
+          hi = make_float4(hi.x + b.x, hi.y + b.y, hi.z + b.z, hi.w + b.w);
+        }
+        *reinterpret_cast<float4*>(o) = lo;
+        *reinterpret_cast<float4*>(o + 4) = hi;
+      } else {
+        for (int j = 0; j < n; ++j) o[j] = e.accumulate ? o[j] + v[j] : v[j];
+      }
+    } else {
+      __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(d) + (long long)row * ldd + col;
+      if (n == 8) {
+        if (e.accumulate) {
+          const uint4 old = *reinterpret_cast<uint4*>(o);
+          const float2 a = unpack_bf16x2(old.x), b = unpack_bf16x2(old.y), g = unpack_bf16x2(old.z), h = unpack_bf16x2(old.w);
+          v[0] += a.x; v[1] += a.y; v[2] += b.x; v[3] += b.y; v[4] += g.x; v[5] += g.y; v[6] += h.x; v[7] += h.y;
+        }
+        *reinterpret_cast<uint4*>(o) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                                                  pack_bf16x2(v[6], v[7]));
+      } else {
+        for (int j = 0; j < n; ++j) o[j] = __float2bfloat16_rn(e.accumulate ? __bfloat162float(o[j]) + v[j] : v[j]);
+      }
+    }
+  }
+}
+
+template <int KIND, int BN, int KSUB>
+void pair_launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, cudaStream_t stream) {
   using C = PairCfg<KIND, BN, KSUB>;
-  static int max_pairs[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  dev &= 63;
-  auto kern = gemm_pair_kernel<KIND, BN, KSUB, NOWN>;
-  static const OwnerMaps<NOWN> no_owners = {};
-  const OwnerMaps<NOWN>& om = owners != nullptr ? *owners : no_owners;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.blockDim = dim3(C::THREADS, 1, 1);
@@ -760,36 +865,105 @@ int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMa
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+}
+
+// CTA pairs of this kernel that can be resident at once on the current device (cached); 0 or a failure code in `rc`.
+template <int KIND, int BN, int KSUB, int NOWN = 1>
+int pair_capacity(const char* what, int& rc) {
+  using C = PairCfg<KIND, BN, KSUB>;
+  static int max_pairs[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  dev &= 63;
+  rc = 0;
   if (max_pairs[dev] == 0) {
+    auto kern = gemm_pair_kernel<KIND, BN, KSUB, NOWN>;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    pair_launch_config<KIND, BN, KSUB>(cfg, attr, nullptr);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
     if (e != cudaSuccess) {
       cudaGetLastError();
-      return b200::fail(821, "%s: cannot set %d bytes of shared memory: %s", what, C::SMEM, cudaGetErrorString(e));
+      rc = b200::fail(821, "%s: cannot set %d bytes of shared memory: %s", what, C::SMEM, cudaGetErrorString(e));
+      return 0;
     }
     cfg.gridDim = dim3(2 * (b200::sm_count() / 2), 1, 1);
     int n = 0;
     e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);
     if (e != cudaSuccess || n <= 0) {
       cudaGetLastError();
-      return b200::fail(822, "%s: no resident CTA pair possible (%s)", what, cudaGetErrorString(e));
+      rc = b200::fail(822, "%s: no resident CTA pair possible (%s)", what, cudaGetErrorString(e));
+      return 0;
     }
     max_pairs[dev] = n;
   }
+  return max_pairs[dev];
+}
+
+// Split of a dense M x N x K problem of this kernel (K in elements, or bytes of e4m3), and the workspace it needs.
+// Time of one k stage of a full pair at the measured rate of the kernel (bf16: 256 x 256 x 64 at 1.4 PFLOP/s over 74
+// pairs = 0.44 us; block-scaled: 256 x 208 x 256 at 2.5 PFLOP/s = 0.8 us).
+template <int KIND, int BN, int KSUB>
+SplitArgs pair_split(int M, int N, int K, int& rc) {
+  const int P = pair_capacity<KIND, BN, KSUB>("split", rc);
+  const int tiles = ((M + 255) / 256) * ((N + BN - 1) / BN);
+  const int kb = (KIND == KIND_BF16 ? 64 : 128) * KSUB, num_kb = (K + kb - 1) / kb;
+  if (rc || P <= 0) return {tiles, 0, 1, num_kb};
+  const double stage_us = 256.0 * BN * kb * 2 / (KIND == KIND_BF16 ? 19.0e6 : 34.0e6);
+  return split_plan(tiles, num_kb, stage_us, 256.0 * BN * 4, P);
+}
+template <int BN>
+long long split_bytes(const SplitArgs& s) { return (long long)s.rem * (s.rem > 0 ? s.S : 0) * 256 * BN * 4; }
+
+// Launches gemm_pair_kernel on as many CTA pairs as can be resident at once (a persistent grid must
+// not exceed that: a pair that waits for SMs would start only after a resident pair finished all its
+// tiles).  With a workspace that is large enough (pair_split, split_bytes) the last wave is split along K; `d`, `ldd`:
+// the output the second launch finishes.  Returns 0, or a failure code with message.
+template <int KIND, int BN, int KSUB, int NOWN = 1>
+int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmSFA, const CUtensorMap& tmSFB,
+                const CUtensorMap& tmD, const CUtensorMap& tmDt, const PairParams& p_in, cudaStream_t stream,
+                const char* what, const OwnerMaps<NOWN>* owners = nullptr, float* ws = nullptr, long long ws_bytes = 0,
+                void* d = nullptr, long long ldd = 0) {
+  PairParams p = p_in;
+  auto kern = gemm_pair_kernel<KIND, BN, KSUB, NOWN>;
+  static const OwnerMaps<NOWN> no_owners = {};
+  const OwnerMaps<NOWN>& om = owners != nullptr ? *owners : no_owners;
+  int rc = 0;
+  const int max_pairs = pair_capacity<KIND, BN, KSUB, NOWN>(what, rc);
+  if (rc) return rc;
   const int num_m = (p.M + 255) / 256, num_n = (p.N + BN - 1) / BN;
   const int tiles = (p.grp.mode == 2 ? p.grp.E : 1) * num_m * num_n;
+  p.split = SplitArgs{tiles, 0, 1, 0};
+  CUtensorMap tmW = tmD, tmWt = tmDt;
+  if (ws != nullptr && d != nullptr && p.grp.mode == 0 && !p.tp.on && !p.rs.on) {
+    const SplitArgs sp = pair_split<KIND, BN, KSUB>(p.M, p.N, p.K, rc);
+    if (rc) return rc;
+    if (sp.rem > 0 && ws_bytes >= split_bytes<BN>(sp)) {
+      p.split = sp;
+      if ((rc = make_out_tmap<BN>(&tmW, &tmWt, ws, sp.rem * sp.S * 256, BN, BN, 1))) return rc;
+    }
+  }
+  const int units = p.split.rem > 0 ? p.split.first + p.split.rem * p.split.S : tiles;
   // every CTA of a gathering launch must be resident at once: its GEMM pairs wait for its copy pairs
   const int n_aux = p.tp.on ? p.tp.n_aux : (p.rs.on ? p.rs.n_aux : 0);
-  if (n_aux >= max_pairs[dev]) return b200::fail(823, "%s: %d copy pairs leave no SM for the GEMM", what, n_aux);
-  const int room = max_pairs[dev] - n_aux;
-  const int pairs = (tiles < room ? tiles : room) + n_aux;
+  if (n_aux >= max_pairs) return b200::fail(823, "%s: %d copy pairs leave no SM for the GEMM", what, n_aux);
+  const int room = max_pairs - n_aux;
+  const int pairs = (units < room ? units : room) + n_aux;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  pair_launch_config<KIND, BN, KSUB>(cfg, attr, stream);
   cfg.gridDim = dim3(2 * pairs, 1, 1);
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmSFA, tmSFB, tmD, tmDt, p, om);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmSFA, tmSFB, tmD, tmDt, tmW, tmWt, p, om);
   b200::count_launch();
   if (e != cudaSuccess) {
     cudaGetLastError();
     return b200::fail(200, "%s: launch failed: %s", what, cudaGetErrorString(e));
   }
-  return b200::check_launch(what);
+  if ((rc = b200::check_launch(what)) || p.split.rem == 0) return rc;
+  // 256 x BN / 8 vectors per tile: enough CTAs for the whole chip whatever the number of tiles
+  split_finish_kernel<BN><<<dim3(BN / 8, p.split.rem), 256, 0, stream>>>(ws, p.split, num_m, num_n, p.group_m, p.epi, d, ldd);
+  b200::count_launch();
+  return b200::check_launch("split_finish");
 }
 
 // CTA pairs are the default for every problem taller than one 128-row tile; B200_GEMM_PAIR=0 keeps

@@ -252,17 +252,33 @@ static int pick_bn(int N) {
 }
 B200_API int b200_gemm_mxfp8_bn(int N) { return pick_bn(N); }
 
-// One CTA pair per 256 x BN tile (gemm_core.cuh); KSUB = 128-byte K blocks per pipeline stage
-// (B200_MXFP8_KSUB=1|2).
-template <int BN>
-static int run_pair(const void* a_q, const void* sfa, const void* b_q, const void* sfb, void* d, int M, int N, int K,
-                    long long lda, long long ldb, long long ldd, const gemmcore::EpiArgs& epi, cudaStream_t stream) {
-  using namespace gemmcore;
+// KSUB = 128-byte K blocks per pipeline stage (B200_MXFP8_KSUB=1|2).
+static int pair_ksub() {
   static int ksub = -1;
   if (ksub < 0) {
     const char* e = getenv("B200_MXFP8_KSUB");
     ksub = (e && atoi(e) == 1) ? 1 : 2;
   }
+  return ksub;
+}
+
+// Workspace (bytes, 16-byte aligned) with which b200_gemm_mxfp8 splits the last wave of an M x N x K problem along K
+// (gemm_core.cuh: SplitArgs); 0 where that does not pay.  The call accepts none, too.
+B200_API long long b200_gemm_mxfp8_workspace(int M, int N, int K) {
+  using namespace gemmcore;
+  if (M <= 128 || N <= 0 || K <= 0 || !pair_enabled() || pair_ksub() != 2) return 0;
+  int rc = 0;
+  return pick_bn(N) == 208 ? split_bytes<208>(pair_split<KIND_MXFP8, 208, 2>(M, N, K, rc))
+                           : split_bytes<128>(pair_split<KIND_MXFP8, 128, 2>(M, N, K, rc));
+}
+
+// One CTA pair per 256 x BN tile (gemm_core.cuh).
+template <int BN>
+static int run_pair(const void* a_q, const void* sfa, const void* b_q, const void* sfb, void* d, int M, int N, int K,
+                    long long lda, long long ldb, long long ldd, const gemmcore::EpiArgs& epi, void* ws, long long ws_bytes,
+                    cudaStream_t stream) {
+  using namespace gemmcore;
+  const int ksub = pair_ksub();
   CUtensorMap tmA, tmB, tmSFA, tmSFB, tmD;
   int r;
   if ((r = b200::make_tmap_2d(&tmA, b200::DT_U8, a_q, K, M, lda, 128, 128, b200::SWZ_128))) return r;
@@ -282,15 +298,19 @@ static int run_pair(const void* a_q, const void* sfa, const void* b_q, const voi
   p.group_m = raster_group_m() > 1 ? raster_group_m() / 2 : 1;
   p.epi = epi;
   p.status = b200::status_ptr();
-  if (ksub == 2) return launch_pair<KIND_MXFP8, BN, 2>(tmA, tmB, tmSFA, tmSFB, tmD, tmDt, p, stream, "gemm_mxfp8(pair)");
+  if (ksub == 2)
+    return launch_pair<KIND_MXFP8, BN, 2, 1>(tmA, tmB, tmSFA, tmSFB, tmD, tmDt, p, stream, "gemm_mxfp8(pair)", nullptr, (float*)ws,
+                                          ws_bytes, d, ldd);
   return launch_pair<KIND_MXFP8, BN, 1>(tmA, tmB, tmSFA, tmSFB, tmD, tmDt, p, stream, "gemm_mxfp8(pair)");
 }
 
 // a_q [M, K] / b_q [N, K] e4m3 (row pitches lda / ldb in bytes), sfa / sfb scale atoms
-// (tile rows 128 for A, b200_gemm_mxfp8_bn(N) for B).  K must be a multiple of 128.
+// (tile rows 128 for A, b200_gemm_mxfp8_bn(N) for B).  K must be a multiple of 128.  workspace: null, or
+// b200_gemm_mxfp8_workspace(M, N, K) bytes that nothing else uses until this call's work is done.
 B200_API int b200_gemm_mxfp8(const void* a_q, const void* sfa, const void* b_q, const void* sfb, void* d, int M, int N,
                              int K, long long lda, long long ldb, long long ldd, int out_f32, int accumulate,
-                             const void* bias, const void* residual, long long ldr, float alpha, void* stream) {
+                             const void* bias, const void* residual, long long ldr, float alpha, void* workspace,
+                             long long workspace_bytes, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return b200::fail(810, "gemm_mxfp8: empty problem %d x %d x %d", M, N, K);
   if (K % BK != 0) return b200::fail(811, "gemm_mxfp8: K=%d must be a multiple of %d", K, BK);
   const int BN = pick_bn(N);
@@ -302,8 +322,8 @@ B200_API int b200_gemm_mxfp8(const void* a_q, const void* sfa, const void* b_q, 
   epi.ldr = ldr;
   epi.alpha = alpha;
   if (M > 128 && gemmcore::pair_enabled()) {
-    if (BN == 208) return run_pair<208>(a_q, sfa, b_q, sfb, d, M, N, K, lda, ldb, ldd, epi, (cudaStream_t)stream);
-    return run_pair<128>(a_q, sfa, b_q, sfb, d, M, N, K, lda, ldb, ldd, epi, (cudaStream_t)stream);
+    if (BN == 208) return run_pair<208>(a_q, sfa, b_q, sfb, d, M, N, K, lda, ldb, ldd, epi, workspace, workspace_bytes, (cudaStream_t)stream);
+    return run_pair<128>(a_q, sfa, b_q, sfb, d, M, N, K, lda, ldb, ldd, epi, workspace, workspace_bytes, (cudaStream_t)stream);
   }
   CUtensorMap tmA, tmB, tmD, tmDt;
   int r;

@@ -12,6 +12,7 @@ loaded, so GPU runs never fall back silently to eager PyTorch.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 from pathlib import Path
@@ -40,7 +41,7 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.b200_sm_count.restype = c_int
     P, I, L, F = c_void_p, c_int, c_ll, c_float
     sigs = {
-        "b200_gemm_bf16": [P, P, P, I, I, I, L, L, L, I, I, I, I, P, P, L, F, P],
+        "b200_gemm_bf16": [P, P, P, I, I, I, L, L, L, I, I, I, I, P, P, L, F, P, L, P],
         "b200_norm_fwd": [I, P, P, P, P, P, P, P, P, I, I, F, I, P],
         "b200_norm_bwd": [I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P],
         "b200_rope": [P, P, P, P, L, I, L, I, I, I, I, P],
@@ -58,7 +59,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_adamw_bf16m": [P, I, P, P, I, P, P, L, F, F, F, F, F, I, F, P, F, I, P],
         "b200_attn_fwd": [P, P, P, P, P, P, I, I, I, I, I, I, L, L, L, L, L, L, L, L, F, I, I, P],
         "b200_quant_mxfp8": [P, L, I, I, P, P, I, P, P, I, P],
-        "b200_gemm_mxfp8": [P, P, P, P, P, I, I, I, L, L, L, I, I, P, P, L, F, P],
+        "b200_gemm_mxfp8": [P, P, P, P, P, I, I, I, L, L, L, I, I, P, P, L, F, P, L, P],
         "b200_router_topk": [P, I, I, I, P, P, P, P],
         "b200_router_plan": [P, P, I, I, I, P, P, I, P, P],
         "b200_permute_rows": [P, P, I, I, I, P, P, P, P],
@@ -128,6 +129,10 @@ def _declare(lib: ctypes.CDLL) -> None:
     if hasattr(lib, "b200_gemm_grouped_mx_bn"):
         lib.b200_gemm_grouped_mx_bn.argtypes = [I]
         lib.b200_gemm_grouped_mx_bn.restype = c_int
+    for name in ("b200_gemm_bf16_workspace", "b200_gemm_mxfp8_workspace"):
+        if hasattr(lib, name):
+            getattr(lib, name).argtypes = [I, I, I]
+            getattr(lib, name).restype = c_ll
     if hasattr(lib, "b200_zero_grid"):
         lib.b200_zero_grid.restype = c_int
 
@@ -203,6 +208,19 @@ def call(name: str, *args) -> None:
     if rc != 0:
         msg = lib.b200_last_error().decode(errors="replace")
         raise RuntimeError(f"{name} failed with code {rc}: {msg}")
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemm_workspace_bytes(entry: str, M: int, N: int, K: int, device: int) -> int:
+    with torch.cuda.device(device):
+        return int(getattr(load(), entry)(M, N, K))
+
+
+def gemm_workspace(entry: str, M: int, N: int, K: int, device: torch.device) -> torch.Tensor | None:
+    """Scratch for the split last wave of a GEMM (None: the problem is not split).  It comes from torch's allocator on the
+    calling stream, so it is given back when the call returns and reused in stream order."""
+    n = _gemm_workspace_bytes(entry, M, N, K, device.index if device.index is not None else torch.cuda.current_device())
+    return torch.empty(n, dtype=torch.uint8, device=device) if n else None
 
 
 def launch_count() -> int:

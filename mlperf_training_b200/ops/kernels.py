@@ -94,9 +94,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
         if residual.dtype != BF16 or residual.stride(1) != 1:
             residual = residual.to(BF16).contiguous()
         ldr = residual.stride(0)
+    ws = _lib.gemm_workspace("b200_gemm_bf16_workspace", M, N, K, a.device)
     call("b200_gemm_bf16", ptr(a), ptr(b), ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
          int(a_mn_major), int(b_mn_major), int(out.dtype == torch.float32), int(accumulate), ptr(bias),
-         ptr(residual), ldr, float(alpha), stream_ptr())
+         ptr(residual), ldr, float(alpha), ptr(ws), 0 if ws is None else ws.numel(), stream_ptr())
     return out
 
 

@@ -270,7 +270,8 @@ def gemm(a: MXOperand, b: MXOperand, *, out: torch.Tensor | None = None, out_dty
         if residual.dtype != torch.bfloat16 or residual.stride(1) != 1:
             residual = residual.to(torch.bfloat16).contiguous()
         ldr = residual.stride(0)
+    ws = _lib.gemm_workspace("b200_gemm_mxfp8_workspace", M, N, Kd, a.q.device)
     call("b200_gemm_mxfp8", ptr(a.q), ptr(a.sf), ptr(b.q), ptr(b.sf), ptr(out), M, N, Kd, a.q.stride(0),
          b.q.stride(0), out.stride(0), int(out.dtype == torch.float32), int(accumulate), ptr(bias), ptr(residual),
-         ldr, float(alpha), stream_ptr())
+         ldr, float(alpha), ptr(ws), 0 if ws is None else ws.numel(), stream_ptr())
     return out

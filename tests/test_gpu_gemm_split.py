@@ -1,0 +1,70 @@
+"""Dense GEMMs whose last wave is cut along K: ragged tiles, every epilogue option, both operand kinds."""
+import pytest
+import torch
+
+from mlperf_training_b200.ops import _lib, kernels as K, mxfp8 as MX
+
+pytestmark = pytest.mark.gpu
+
+# one tile; ragged rows, columns and K; one full wave and a rest; N of one 128-wide tile
+SHAPES = [(256, 256, 4096), (300, 520, 2056), (2048, 512, 8200), (1333, 3400, 8200), (5000, 1000, 2048), (4096, 120, 8192)]
+
+
+def _rand(*shape):
+    return torch.randn(*shape, device="cuda").bfloat16()
+
+
+def _check(got, want, K_):
+    # fp32 accumulation in another order, then one rounding to the output type
+    eps = 2 ** -8 if got.dtype == torch.bfloat16 else 2 ** -24 * K_ ** 0.5 * 4
+    assert (got.double() - want).abs().max() <= eps * want.abs().max() + 1e-6
+
+
+@pytest.mark.parametrize("M,N,Kd", SHAPES)
+@pytest.mark.parametrize("mode", ["plain", "bias_residual", "f32_accumulate", "bf16_accumulate", "wgrad", "dgrad"])
+def test_bf16(M, N, Kd, mode):
+    torch.manual_seed(M + N)
+    assert _lib.gemm_workspace("b200_gemm_bf16_workspace", M, N, Kd, torch.device("cuda")) is not None
+    kw, a, b = {}, _rand(M, Kd), _rand(N, Kd)
+    want = a.double() @ b.double().t()
+    if mode == "bias_residual":
+        kw = dict(bias=_rand(N), residual=_rand(M, N), alpha=0.5)
+        want = 0.5 * want + kw["bias"].double() + kw["residual"].double()
+    elif mode == "f32_accumulate":
+        kw = dict(out=torch.randn(M, N, device="cuda"), accumulate=True)
+        want = want + kw["out"].double()
+    elif mode == "bf16_accumulate":
+        kw = dict(out=_rand(M, N), accumulate=True)
+        want = want + kw["out"].double()
+    elif mode == "wgrad":
+        M8 = M // 8 * 8
+        a, want, kw = a[:M8].t().contiguous(), want[:M8], dict(a_mn_major=True, b_mn_major=True, out_dtype=torch.float32)
+        b = b.t().contiguous()
+    elif mode == "dgrad":
+        b, kw = b.t().contiguous(), dict(b_mn_major=True)
+    first = K.gemm(a, b, **kw)
+    if mode == "bf16_accumulate":      # whole tiles round the product before they add it: one more rounding
+        assert (first.double() - want).abs().max() <= 2 ** -7 * want.abs().max()
+    else:
+        _check(first, want, Kd)
+    if "accumulate" not in mode:
+        assert torch.equal(first, K.gemm(a, b, **kw))      # no atomics: the same bits
+    _lib.check_status("split gemm")
+
+
+@pytest.mark.parametrize("M,N,Kd", [(256, 384, 4096), (1152, 512, 8192), (4096, 4096, 8192), (640, 128, 8192), (2176, 1920, 8320)])
+@pytest.mark.parametrize("mode", ["bf16", "f32_accumulate"])
+def test_mxfp8(M, N, Kd, mode):
+    torch.manual_seed(M + N)
+    assert _lib.gemm_workspace("b200_gemm_mxfp8_workspace", M, N, Kd, torch.device("cuda")) is not None
+    qa, _ = MX.quantize(_rand(M, Kd), row_tile=MX.A_TILE)
+    qb, _ = MX.quantize(_rand(N, Kd), row_tile=MX.b_tile(N))
+    want = MX.dequantize(qa).double() @ MX.dequantize(qb).double().t()
+    if mode == "bf16":
+        res = _rand(M, N)
+        _check(MX.gemm(qa, qb, residual=res), want + res.double(), Kd)
+    else:
+        out = torch.randn(M, N, device="cuda")
+        want = want + out.double()
+        _check(MX.gemm(qa, qb, out=out, accumulate=True), want, Kd)
+    _lib.check_status("split gemm")

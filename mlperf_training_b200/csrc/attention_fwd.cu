@@ -5,18 +5,30 @@
 //   logits (an extra softmax column without a value), head_dim 64 or 128, bf16 in / bf16 out,
 //   fp32 log-sum-exp saved for the backward pass.
 //
-// One CTA per (batch, head, pair of 128-query tiles); 320 threads:
-//   warp 8      TMA producer (both Q tiles once, K/V double buffered, shared by the two tiles)
+// Persistent CTAs, one per SM; a work item is a (batch, head, pair of 128-query tiles).  384 threads:
+//   warp 8      TMA producer (both Q tiles of an item, K/V double buffered, shared by the two tiles)
 //   warp 9      MMA issuer, ping-pong over the two query tiles:
 //                 S0(0) S1(0) | PV0(n) S0(n+1) PV1(n) S1(n+1) | ...
-//               so the tensor core works on one tile while the other tile's softmax runs
-//   warps 0-3   softmax of tile 0 (one query row per thread)
-//   warps 4-7   softmax of tile 1
+//               so the tensor core works on one tile while the other tile's softmax runs; the next
+//               item's Q, K and first S are fetched and computed under this item's epilogue
+//   warps 0-3   softmax of tile 0 (one query row per thread), warps 4-7 softmax of tile 1
+//   (warps 10, 11 only complete the third warpgroup, which hands its registers to the softmax warps)
 // TMEM (512 columns): S0 | S1 | O0 | O1.  The bf16 probabilities P overwrite the first half of
 // their own S columns (tcgen05.st) and feed the second GEMM straight from TMEM (A operand in
 // TMEM), so P never touches shared memory.  O is rescaled lazily: only when the running row
 // maximum grew by more than 2^8.  A quarter of the exponentials run as a polynomial on the FMA
 // pipe to relieve the MUFU unit.
+//
+// What bounds it: a pair of 128 x 128 tiles costs 4 x 512 tensor-core cycles.  The MMA issuer was the limit before: one
+// lane of a divergent warp that rebuilt its descriptors needed about 130 cycles per instruction of 64 (clock64 in the
+// roles), so the two tiles took 4900 cycles.  Now the warp stays converged, one elected lane issues, and descriptors
+// advance by an addition.  Beside that, whatever the MMAs do not wait for has left the path from S to P: they start on
+// the first 96 keys of P while the last 32 are still being exponentiated, the row sum is taken after P has been handed
+// over, and the softmax warps hold 200 registers (all 128 scores in flight, no spills).  Items are handed out longest
+// first over all heads (head after head left 14 % of the SM cycles idle at the end of a causal launch), in snake order
+// over the rounds so that no CTA gets the longest of each.
+// Measured (causal unless noted), before -> now: 8192 x 32 heads of 128 622 -> 528 us (1.04 PFLOP/s); 4 x 2048 218 -> 181;
+// 3 x 1337 107 -> 90; 8192 x 64 heads of 64, window 128 200 -> 158; 2000 x 64 of 64 114 -> 87; 8 x 512 x 24, full 56 -> 47.
 //
 // Stands in for the attention kernels the reference selects by config: Primus-Turbo / AITER /
 // CK flash attention (small_llm_pretraining/primus/conf/llama3.1_8B-pretrain-fp4.yaml:117,125)
@@ -33,7 +45,10 @@ namespace {
 constexpr int POLY = B200_ATTN_FWD_POLY;  // pairs with (i & POLY) == POLY take the FMA-pipe polynomial: 3 = a quarter, 1 = half
 constexpr int BQ = 128;   // query rows per tile (two tiles per CTA)
 constexpr int BKV = 128;  // keys per tile
-constexpr int NTHREADS = 320;  // warps 0-3 / 4-7: softmax of tile 0 / 1; warp 8: TMA; warp 9: MMA
+constexpr int NTHREADS = 384;  // warps 0-3 / 4-7: softmax of tile 0 / 1; warp 8: TMA; warp 9: MMA
+constexpr int PV_EARLY = 96;   // keys of P the second GEMM starts on
+// 3 x 128 threads launch with 168 registers each (504 per triple): 104 + 2 x 200 (56 or 72 for the other warps spilled)
+constexpr int REGS_SOFTMAX = 200, REGS_OTHER = 104;
 
 struct FwdParams {
   int B, Hq, Hkv, Sq, Skv;
@@ -43,7 +58,51 @@ struct FwdParams {
   const float* sink;  // [Hq] learned sink logits (natural-log domain, unscaled) or null
   float* lse;         // [B, Hq, Sq] natural-log log-sum-exp of the scaled scores
   int* status;
+  int bh_group;       // (batch, head) rows whose K / V stay in L2 together: items are ordered longest first inside a group
+  int items;
 };
+
+// Work item u of the launch, and the key tiles its two query tiles look at.
+struct Item {
+  int b, h, q0, j_lo;
+  int lo0, lo1, hi0, hi1;   // per query tile: key tiles j_lo + [lo, hi)
+  int n_max;
+  B200_DEVICE int lo(int t) const { return t ? lo1 : lo0; }
+  B200_DEVICE int hi(int t) const { return t ? hi1 : hi0; }
+};
+B200_DEVICE Item make_item(int u, const FwdParams& p) {
+  Item it;
+  const int num_pairs = (p.Sq + 2 * BQ - 1) / (2 * BQ);
+  const int g = u / (p.bh_group * num_pairs), r = u - g * p.bh_group * num_pairs;
+  const int gsz = min(p.bh_group, p.B * p.Hq - g * p.bh_group);
+  const int pair = num_pairs - 1 - r / gsz;          // longest (latest) query tiles first
+  const int bh = g * p.bh_group + r % gsz;
+  it.b = bh / p.Hq;
+  it.h = bh - it.b * p.Hq;
+  it.q0 = pair * 2 * BQ;
+  const int off = p.Skv - p.Sq;                      // causal diagonal offset (0 for self-attention)
+  const int j_max = (p.Skv + BKV - 1) / BKV - 1;
+  it.j_lo = 0;
+  if (p.window > 0) it.j_lo = max(0, it.q0 + off - p.window + 1) / BKV;
+  const int hi0 = p.causal ? min(j_max, (it.q0 + BQ - 1 + off) / BKV) : j_max;
+  const int hi1 = p.causal ? min(j_max, (it.q0 + 2 * BQ - 1 + off) / BKV) : j_max;
+  it.lo0 = 0;
+  it.lo1 = p.window > 0 ? max(0, it.q0 + BQ + off - p.window + 1) / BKV - it.j_lo : 0;
+  it.hi0 = max(hi0 - it.j_lo + 1, 0);
+  it.hi1 = it.q0 + BQ < p.Sq ? max(hi1 - it.j_lo + 1, it.lo1) : it.lo1;
+  it.n_max = it.hi1 > it.lo1 ? max(it.hi0, it.hi1) : it.hi0;
+  return it;
+}
+// Items of CTA blockIdx.x: one per round of gridDim.x items, in alternating direction.
+B200_DEVICE int item_of_round(int r) {
+  return r * (int)gridDim.x + ((r & 1) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
+}
+
+B200_DEVICE float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 
 B200_DEVICE void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
   asm volatile(
@@ -61,7 +120,8 @@ template <int HD>
 struct Smem {
   static constexpr int Q_TILE = BQ * HD * 2;
   static constexpr int KV_BYTES = BKV * HD * 2;
-  static constexpr int TOTAL = 2 * Q_TILE + 4 * KV_BYTES + 1024 + 256;
+  static constexpr int STAGE_O = 32 * 128;            // per softmax warp: 32 rows x 64 output columns
+  static constexpr int TOTAL = 2 * Q_TILE + 4 * KV_BYTES + 8 * STAGE_O + 1024 + 256;
 };
 
 template <int HD>
@@ -76,52 +136,33 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint8_t* sQ = smem;                       // two tiles
   uint8_t* sK = sQ + 2 * SM::Q_TILE;        // two stages
   uint8_t* sV = sK + 2 * SM::KV_BYTES;      // two stages
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * SM::KV_BYTES);
+  uint8_t* sO = sV + 2 * SM::KV_BYTES;      // eight warps' output staging
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sO + 8 * SM::STAGE_O);
   uint64_t* q_full = bars;          // 1
-  uint64_t* k_full = bars + 1;      // 2
-  uint64_t* k_empty = bars + 3;     // 2
-  uint64_t* v_full = bars + 5;      // 2
-  uint64_t* v_empty = bars + 7;     // 2
-  uint64_t* s_full = bars + 9;      // 2 (per query tile)
-  uint64_t* p_full = bars + 11;     // 2 (per query tile, 4 arrivals)
-  uint64_t* o_done = bars + 13;     // 2 (per query tile)
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* q_empty = bars + 1;     // 1: every S of the item has been computed
+  uint64_t* k_full = bars + 2;      // 2
+  uint64_t* k_empty = bars + 4;     // 2
+  uint64_t* v_full = bars + 6;      // 2
+  uint64_t* v_empty = bars + 8;     // 2
+  uint64_t* s_full = bars + 10;     // 2 (per query tile): once per key tile
+  uint64_t* p_early = bars + 12;    // 2 (4 arrivals): the first PV_EARLY keys of P are in TMEM
+  uint64_t* p_full = bars + 14;     // 2 (4 arrivals): all of P
+  uint64_t* o_done = bars + 16;     // 2: once per item, O complete
+  uint64_t* o_free = bars + 18;     // 2 (4 arrivals): once per item, O read out of TMEM
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int num_pairs = (p.Sq + 2 * BQ - 1) / (2 * BQ);
-  const int pair = num_pairs - 1 - (int)blockIdx.x;  // heaviest (latest) query tiles first
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int hk = h / (p.Hq / p.Hkv);
-  const int q0 = pair * 2 * BQ;
-  const int off = p.Skv - p.Sq;  // causal diagonal offset (0 for self-attention)
-
-  // key-tile range: a common first tile, a per-query-tile last tile
-  const int j_max = (p.Skv + BKV - 1) / BKV - 1;
-  int j_lo = 0;
-  if (p.window > 0) {
-    const int first = q0 + off - p.window + 1;
-    if (first > 0) j_lo = first / BKV;
-  }
-  int n_t[2];
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int qt0 = q0 + t * BQ;
-    int j_hi = j_max;
-    if (p.causal) {
-      const int last = (qt0 + BQ - 1 + off) / BKV;
-      if (last < j_hi) j_hi = last;
-    }
-    n_t[t] = (qt0 < p.Sq && j_hi >= j_lo) ? (j_hi - j_lo + 1) : 0;
-  }
-  const int n_max = n_t[0] > n_t[1] ? n_t[0] : n_t[1];
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int off = p.Skv - p.Sq;
+  const int rounds = (p.items + (int)gridDim.x - 1) / (int)gridDim.x;
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
+    mbar_init(q_full, 1); mbar_init(q_empty, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
       mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_done[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&p_early[i], 4); mbar_init(&p_full[i], 4);
+      mbar_init(&o_done[i], 1); mbar_init(&o_free[i], 4);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -132,225 +173,287 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
 
-
-  if (warp == 8) {
-    // ------------------------------ TMA producer ------------------------------
-    if (lane == 0 && n_max > 0) {
+  if (warp >= 8) {
+    reg_dealloc<REGS_OTHER>();
+    if (warp == 8 && lane == 0) {
+      // ------------------------------ TMA producer ------------------------------
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
-      mbar_expect_tx(q_full, 2 * SM::Q_TILE);
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-#pragma unroll
-        for (int i = 0; i < NB; ++i)
-          tma_load_4d(sQ + t * SM::Q_TILE + i * (BQ * 128), &tmQ, q_full, i * 64, h, q0 + t * BQ, b);
       bool ok = true;
-      for (int n = 0; n < n_max && ok; ++n) {
-        const int j = j_lo + n, st = n & 1;
-        const uint32_t ph = (n >> 1) & 1;
-        if (!mbar_wait(&k_empty[st], ph ^ 1, abort_flag, p.status, 40)) { ok = false; break; }
-        mbar_expect_tx(&k_full[st], SM::KV_BYTES);
+      int kv = 0, nq = 0;                    // key tiles and items so far: stage and phase of the barriers
+      for (int r = 0; r < rounds && ok; ++r) {
+        const int u = item_of_round(r);
+        if (u >= p.items) continue;
+        const Item it = make_item(u, p);
+        if (it.n_max == 0) continue;
+        const int hk = it.h / (p.Hq / p.Hkv);
+        if (!mbar_wait(q_empty, (nq & 1) ^ 1, abort_flag, p.status, 39)) { ok = false; break; }
+        ++nq;
+        mbar_expect_tx(q_full, 2 * SM::Q_TILE);
 #pragma unroll
-        for (int i = 0; i < NB; ++i)
-          tma_load_4d(sK + st * SM::KV_BYTES + i * (BKV * 128), &tmK, &k_full[st], i * 64, hk, j * BKV, b);
-        if (!mbar_wait(&v_empty[st], ph ^ 1, abort_flag, p.status, 41)) { ok = false; break; }
-        mbar_expect_tx(&v_full[st], SM::KV_BYTES);
+        for (int t = 0; t < 2; ++t)
 #pragma unroll
-        for (int i = 0; i < NB; ++i)
-          tma_load_4d(sV + st * SM::KV_BYTES + i * (BKV * 128), &tmV, &v_full[st], i * 64, hk, j * BKV, b);
+          for (int i = 0; i < NB; ++i)
+            tma_load_4d(sQ + t * SM::Q_TILE + i * (BQ * 128), &tmQ, q_full, i * 64, it.h, it.q0 + t * BQ, it.b);
+        for (int n = 0; n < it.n_max; ++n, ++kv) {
+          const int j = it.j_lo + n, st = kv & 1;
+          const uint32_t ph = (kv >> 1) & 1;
+          if (!mbar_wait(&k_empty[st], ph ^ 1, abort_flag, p.status, 40)) { ok = false; break; }
+          mbar_expect_tx(&k_full[st], SM::KV_BYTES);
+#pragma unroll
+          for (int i = 0; i < NB; ++i)
+            tma_load_4d(sK + st * SM::KV_BYTES + i * (BKV * 128), &tmK, &k_full[st], i * 64, hk, j * BKV, it.b);
+          if (!mbar_wait(&v_empty[st], ph ^ 1, abort_flag, p.status, 41)) { ok = false; break; }
+          mbar_expect_tx(&v_full[st], SM::KV_BYTES);
+#pragma unroll
+          for (int i = 0; i < NB; ++i)
+            tma_load_4d(sV + st * SM::KV_BYTES + i * (BKV * 128), &tmV, &v_full[st], i * 64, hk, j * BKV, it.b);
+        }
       }
-    }
-  } else if (warp == 9) {
-    // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0 && n_max > 0) {
+    } else if (warp == 9) {
+      // ------------------------------ MMA issuer ------------------------------
+      // The whole warp walks the schedule and one elected lane issues: the operands of the instructions then stay in
+      // uniform registers (descriptors advance by an addition).
       const uint32_t idesc_s = umma_idesc(1, 1, 0, 0, BQ, BKV);  // Q (K-major) x K (K-major)
       const uint32_t idesc_o = umma_idesc(1, 1, 0, 1, BQ, HD);   // P (TMEM)    x V (MN-major)
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.status, 50);
-      int k_ready = -1, v_ready = -1;  // last key tile index whose full barrier has been observed
-      // S_t(n) = Q_t K(n)^T into the S columns of tile t
-      auto issue_s = [&](int t, int n) -> bool {
-        const int st = n & 1;
-        if (k_ready < n) {
-          if (!mbar_wait(&k_full[st], (n >> 1) & 1, abort_flag, p.status, 51)) return false;
-          k_ready = n;
-        }
-        tc_fence_after();
-        const uint32_t qa = smem_u32(sQ + t * SM::Q_TILE), ka = smem_u32(sK + st * SM::KV_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t o = (kk / 4) * (BQ * 128) + (kk % 4) * 32;
-          tc_mma_f16_ss(tmem_base + t * 128, umma_desc_sw128(qa + o, 16, 1024), umma_desc_sw128(ka + o, 16, 1024),
-                        idesc_s, kk > 0 ? 1u : 0u);
-        }
-        tc_commit(&s_full[t]);
-        // the last tile that reads K(n) frees its stage
-        const bool last_user = (t == 1) || !(n < n_t[1]);
-        if (last_user) tc_commit(&k_empty[st]);
-        return true;
-      };
-      for (int t = 0; t < 2 && ok; ++t)
-        if (n_t[t] > 0) ok = issue_s(t, 0);
-      for (int n = 0; n < n_max && ok; ++n) {
-        const int st = n & 1;
-        for (int t = 0; t < 2 && ok; ++t) {
-          if (n >= n_t[t]) continue;
-          if (!mbar_wait(&p_full[t], n & 1, abort_flag, p.status, 53)) { ok = false; break; }
-          if (v_ready < n) {
-            if (!mbar_wait(&v_full[st], (n >> 1) & 1, abort_flag, p.status, 54)) { ok = false; break; }
-            v_ready = n;
+      const uint64_t dQ = umma_desc_sw128(smem_u32(sQ), 16, 1024), dK = umma_desc_sw128(smem_u32(sK), 16, 1024);
+      const uint64_t dV = umma_desc_sw128(smem_u32(sV), BKV * 128, 1024);
+      bool ok = true;
+      int kv = 0, nq = 0;
+      int np[2] = {0, 0}, no[2] = {0, 0};    // P tiles consumed / items finished per query tile
+      for (int r = 0; r < rounds && ok; ++r) {
+        const int u = item_of_round(r);
+        if (u >= p.items) continue;
+        const Item it = make_item(u, p);
+        if (it.n_max == 0) continue;
+        if (!mbar_wait_spin(q_full, nq & 1, abort_flag, p.status, 50)) { ok = false; break; }
+        ++nq;
+        int k_ready = -1, v_ready = -1;      // last key tile of the item whose full barrier has been observed
+        int s_left = (it.hi0 - it.lo0) + (it.hi1 - it.lo1);
+        // S_t(n) = Q_t K(n)^T into the S columns of tile t
+        auto issue_s = [&](int t, int n) -> bool {
+          const int st = (kv + n) & 1;
+          while (k_ready < n) {
+            ++k_ready;
+            if (!mbar_wait_spin(&k_full[(kv + k_ready) & 1], ((kv + k_ready) >> 1) & 1, abort_flag, p.status, 51)) return false;
           }
+          // the last S that reads K(n) frees its stage: S_t(n) is issued in step n - 1 (its first one before step 0)
+          const int o = 1 - t;
+          const bool both = n >= it.lo(o) && n < it.hi(o);
+          const int mine = n == it.lo(t) ? -1 : n - 1, theirs = n == it.lo(o) ? -1 : n - 1;
+          const bool free_k = !both || mine > theirs || (mine == theirs && t == 1);
+          const bool free_q = --s_left == 0;
           tc_fence_after();
-          const uint32_t va = smem_u32(sV + st * SM::KV_BYTES);
+          if (elect_one()) {
+            const uint64_t ad = dQ + (t * SM::Q_TILE >> 4), bd = dK + (st * SM::KV_BYTES >> 4);
 #pragma unroll
-          for (int kk = 0; kk < BKV / 16; ++kk) {
-            // A = P_t in TMEM: 16 bf16 keys = 8 columns per step; B = V: 16 key rows of 128 bytes
-            tc_mma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8,
-                          umma_desc_sw128(va + kk * (16 * 128), BKV * 128, 1024), idesc_o, (n > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < HD / 16; ++kk) {
+              const uint32_t o4 = ((kk / 4) * (BQ * 128) + (kk % 4) * 32) >> 4;
+              tc_mma_f16_ss(tmem_base + t * 128, ad + o4, bd + o4, idesc_s, kk > 0 ? 1u : 0u);
+            }
+            tc_commit(&s_full[t]);
+            if (free_k) tc_commit(&k_empty[st]);
+            if (free_q) tc_commit(q_empty);
           }
-          tc_commit(&o_done[t]);
-          const bool last_user = (t == 1) || !(n < n_t[1]);
-          if (last_user) tc_commit(&v_empty[st]);
-          if (n + 1 < n_t[t]) ok = issue_s(t, n + 1);
+          __syncwarp();
+          return true;
+        };
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+          if (ok && it.hi(t) > it.lo(t)) ok = issue_s(t, it.lo(t));
+        for (int n = 0; n < it.n_max && ok; ++n) {
+          const int st = (kv + n) & 1;
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (!ok || n < it.lo(t) || n >= it.hi(t)) continue;
+            const bool first = n == it.lo(t), last = n == it.hi(t) - 1;
+            // O of the previous item has left TMEM
+            if (first && !mbar_wait_spin(&o_free[t], (no[t] & 1) ^ 1, abort_flag, p.status, 52)) { ok = false; continue; }
+            while (ok && v_ready < n) {
+              ++v_ready;
+              ok = mbar_wait_spin(&v_full[(kv + v_ready) & 1], ((kv + v_ready) >> 1) & 1, abort_flag, p.status, 54);
+            }
+            ok = ok && mbar_wait_spin(&p_early[t], np[t] & 1, abort_flag, p.status, 53);
+            if (!ok) continue;
+            tc_fence_after();
+            // A = P_t in TMEM: 16 bf16 keys = 8 columns per step; B = V: 16 key rows of 128 bytes
+            const uint64_t bd = dV + (st * SM::KV_BYTES >> 4);
+            if (elect_one()) {
+#pragma unroll
+              for (int kk = 0; kk < PV_EARLY / 16; ++kk)
+                tc_mma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8, bd + (kk * (16 * 128) >> 4), idesc_o,
+                              (!first || kk > 0) ? 1u : 0u);
+            }
+            __syncwarp();
+            ok = mbar_wait_spin(&p_full[t], np[t] & 1, abort_flag, p.status, 55);
+            if (!ok) continue;
+            tc_fence_after();
+            const bool free_v = (t == 1) || !(n >= it.lo1 && n < it.hi1);
+            if (elect_one()) {
+#pragma unroll
+              for (int kk = PV_EARLY / 16; kk < BKV / 16; ++kk)
+                tc_mma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8, bd + (kk * (16 * 128) >> 4), idesc_o, 1u);
+              if (last) tc_commit(&o_done[t]);
+              if (free_v) tc_commit(&v_empty[st]);
+            }
+            __syncwarp();
+            ++np[t];
+            if (last) ++no[t];
+            else ok = issue_s(t, n + 1);
+          }
         }
+        kv += it.n_max;
       }
     }
-  } else if (warp < 8) {
+  } else {
     // ------------------------------ softmax + epilogue (one warpgroup per query tile) --------------
+    reg_alloc<REGS_SOFTMAX>();
     const int t = warp >> 2;
     const int q = warp & 3;
     const int r = q * 32 + lane;           // row inside the query tile
-    const int qt0 = q0 + t * BQ;
-    const int q_pos = qt0 + r;
     const uint32_t lane_base = uint32_t(q * 32) << 16;
     const uint32_t ts = tmem_base + lane_base + t * 128;        // S / P columns of this tile
     const uint32_t to = tmem_base + lane_base + 256 + t * 128;  // O columns of this tile
-    const int my_n = n_t[t];
-    float m_ref = -INFINITY, l = 0.f;
+    uint8_t* stage = sO + warp * SM::STAGE_O;
+    int ns = 0, no = 0;                    // S tiles and items so far
     bool ok = true;
-    for (int n = 0; n < my_n && ok; ++n) {
-      const int kv0 = (j_lo + n) * BKV;
-      if (!mbar_wait(&s_full[t], n & 1, abort_flag, p.status, 60)) { ok = false; break; }
-      tc_fence_after();
-      const bool need_mask = (kv0 + BKV > p.Skv) || (p.causal && kv0 + BKV - 1 > qt0 + off) ||
-                             (p.window > 0 && kv0 < qt0 + BQ - 1 + off - p.window + 1);
+    for (int round = 0; round < rounds && ok; ++round) {
+      const int u = item_of_round(round);
+      if (u >= p.items) continue;
+      const Item it = make_item(u, p);
+      if (it.hi(t) <= it.lo(t)) continue;
+      const int qt0 = it.q0 + t * BQ;
+      const int q_pos = qt0 + r;
       const int hi = p.causal ? min(q_pos + off, p.Skv - 1) : p.Skv - 1;         // last visible key
       const int lo = p.window > 0 ? q_pos + off - p.window + 1 : 0;              // first visible key
-      // the whole score row (128 fp32) comes into registers with one TMEM round trip
-      uint32_t v[BKV];
+      float m_ref = -INFINITY, l = 0.f;
+      for (int n = it.lo(t); n < it.hi(t); ++n, ++ns) {
+        const int kv0 = (it.j_lo + n) * BKV;
+        if (!mbar_wait(&s_full[t], ns & 1, abort_flag, p.status, 60)) { ok = false; break; }
+        tc_fence_after();
+        const bool need_mask = (kv0 + BKV > p.Skv) || (p.causal && kv0 + BKV - 1 > qt0 + off) ||
+                               (p.window > 0 && kv0 < qt0 + BQ - 1 + off - p.window + 1);
+        // the whole score row (128 fp32) comes into registers with one TMEM round trip
+        uint32_t v[BKV];
 #pragma unroll
-      for (int c = 0; c < BKV / 32; ++c) tmem_ld_32x32b_x32(ts + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&v[c * 32]));
-      tc_wait_ld();
-      if (need_mask) {
+        for (int c = 0; c < BKV / 32; ++c) tmem_ld_32x32b_x32(ts + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&v[c * 32]));
+        tc_wait_ld();
+        if (need_mask) {
 #pragma unroll
-        for (int i = 0; i < BKV; ++i) {
-          const int kp = kv0 + i;
-          if (kp > hi || kp < lo) v[i] = 0xff800000u;  // -inf
-        }
-      }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int i = 0; i < BKV; i += 4) {
-        mx4[0] = fmaxf(mx4[0], __uint_as_float(v[i]));
-        mx4[1] = fmaxf(mx4[1], __uint_as_float(v[i + 1]));
-        mx4[2] = fmaxf(mx4[2], __uint_as_float(v[i + 2]));
-        mx4[3] = fmaxf(mx4[3], __uint_as_float(v[i + 3]));
-      }
-      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      mx *= p.scale_log2;  // -inf stays -inf (scale > 0)
-      // lazy rescale: move the reference maximum only when it grew by more than 2^8
-      const bool grow = (mx > m_ref + 8.f) || (m_ref == -INFINITY && mx > -INFINITY);
-      if (__any_sync(0xffffffffu, grow)) {
-        const float m_new = fmaxf(m_ref, mx);
-        const float alpha = (m_ref == -INFINITY) ? 0.f : ex2_approx(m_ref - m_new);
-        m_ref = m_new;
-        l *= alpha;
-        if (n > 0) {
-          // O_t must be complete (P V of the previous key tile) before it is rescaled
-          if (!mbar_wait(&o_done[t], (n - 1) & 1, abort_flag, p.status, 61)) { ok = false; break; }
-          tc_fence_after();
-#pragma unroll 1
-          for (int c = 0; c < HD / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld_32x32b_x32(to + c * 32, o);
-            tc_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x32b_x32(to + c * 32, o);
+          for (int i = 0; i < BKV; ++i) {
+            const int kp = kv0 + i;
+            if (kp > hi || kp < lo) v[i] = 0xff800000u;  // -inf
           }
-          tc_wait_st();
         }
-      }
-      const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
-      // P = exp2(S * scale - m) as bf16 pairs over the first half of the S columns; every fourth
-      // pair takes the polynomial path (FMA pipe), the rest the MUFU path; -inf gives 0 on both
-      float2 rs2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-      const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
-      const float2 nm2 = make_float2(-m_use, -m_use);
+        float mx4[4];
 #pragma unroll
-      for (int c = 0; c < BKV / 32; ++c) {
-        uint32_t pk[16];
+        for (int c = 0; c < 4; ++c) mx4[c] = fmaxf(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1]));
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int e = c * 32 + 2 * i;
-          const float2 a = ffma2(make_float2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), sc2, nm2);
-          float2 x;
-          if ((i & POLY) == POLY) x = ex2_poly2(a);
-          else x = make_float2(ex2_approx(a.x), ex2_approx(a.y));
-          rs2[i & 1] = fadd2(rs2[i & 1], x);
-          pk[i] = pack_bf16x2(x.x, x.y);
+        for (int i = 8; i < BKV; i += 8)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) mx4[c] = max3(mx4[c], __uint_as_float(v[i + 2 * c]), __uint_as_float(v[i + 2 * c + 1]));
+        float mx = fmaxf(max3(mx4[0], mx4[1], mx4[2]), mx4[3]);
+        mx *= p.scale_log2;  // -inf stays -inf (scale > 0)
+        // lazy rescale: move the reference maximum only when it grew by more than 2^8
+        const bool grow = (mx > m_ref + 8.f) || (m_ref == -INFINITY && mx > -INFINITY);
+        if (__any_sync(0xffffffffu, grow)) {
+          const float m_new = fmaxf(m_ref, mx);
+          const float alpha = (m_ref == -INFINITY) ? 0.f : ex2_approx(m_ref - m_new);
+          m_ref = m_new;
+          l *= alpha;
+          if (n > it.lo(t)) {
+            // (S of this key tile was issued after P V of the one before it and completes after it: O is complete)
+#pragma unroll 1
+            for (int c = 0; c < HD / 32; ++c) {
+              uint32_t o[32];
+              tmem_ld_32x32b_x32(to + c * 32, o);
+              tc_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              tmem_st_32x32b_x32(to + c * 32, o);
+            }
+            tc_wait_st();
+          }
         }
-        tmem_st_32x32b_x16(ts + c * 16, pk);
+        const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
+        // P = exp2(S * scale - m) as bf16 pairs over the first half of the S columns; every fourth
+        // pair takes the polynomial path (FMA pipe), the rest the MUFU path; -inf gives 0 on both
+        const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
+        const float2 nm2 = make_float2(-m_use, -m_use);
+#pragma unroll
+        for (int c = 0; c < BKV / 32; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int e = c * 32 + 2 * i;
+            const float2 a = ffma2(make_float2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), sc2, nm2);
+            float2 x;
+            if ((i & POLY) == POLY) x = ex2_poly2(a);
+            else x = make_float2(ex2_approx(a.x), ex2_approx(a.y));
+            v[e] = __float_as_uint(x.x); v[e + 1] = __float_as_uint(x.y);
+            pk[i] = pack_bf16x2(x.x, x.y);
+          }
+          tmem_st_32x32b_x16(ts + c * 16, pk);
+          if (c == PV_EARLY / 32 - 1 || c == BKV / 32 - 1) {
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(c == BKV / 32 - 1 ? &p_full[t] : &p_early[t]);
+          }
+        }
+        // the row sum, off the path of the MMAs
+        float2 rs2[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+        for (int i = 0; i < BKV / 2; ++i)
+          rs2[i & 3] = fadd2(rs2[i & 3], make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+        const float2 ra = fadd2(rs2[0], rs2[1]), rb = fadd2(rs2[2], rs2[3]);
+        l += (ra.x + ra.y) + (rb.x + rb.y);
       }
-      const float rs = (rs2[0].x + rs2[0].y) + (rs2[1].x + rs2[1].y);
-      l += rs;
-      tc_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[t]);
-    }
-    // ------------------------------ epilogue ------------------------------
-    if (ok && my_n > 0) ok = mbar_wait(&o_done[t], (my_n - 1) & 1, abort_flag, p.status, 62);
-    if (ok && my_n > 0) {
+      // ------------------------------ epilogue ------------------------------
+      if (!ok || !mbar_wait(&o_done[t], no & 1, abort_flag, p.status, 62)) { ok = false; break; }
+      ++no;
       tc_fence_after();
       if (p.sink != nullptr) {
-        const float sk = p.sink[h] * 1.4426950408889634f;
+        const float sk = p.sink[it.h] * 1.4426950408889634f;
         if (m_ref == -INFINITY) { m_ref = sk; l = 1.f; }
         else l += ex2_approx(sk - m_ref);
       }
       const float inv = l > 0.f ? 1.f / l : 0.f;
-      uint8_t* stage = sQ + t * SM::Q_TILE;  // the Q tile is dead after the last S MMA: reuse as O staging
-      uint8_t* orow = stage + r * 128;
-#pragma unroll 1
-      for (int c = 0; c < HD / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(to + c * 32, v);
-        tc_wait_ld();
-        uint8_t* blk = orow + (c / 2) * (BQ * 128);
+      if (q_pos < p.Sq && p.lse != nullptr)
+        p.lse[((long long)it.b * p.Hq + it.h) * p.Sq + q_pos] =
+            (l > 0.f) ? (m_ref + log2f(l)) * 0.6931471805599453f : -INFINITY;
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const int chunk = (c & 1) * 4 + g;
-          uint4 u = make_uint4(
-              pack_bf16x2(__uint_as_float(v[8 * g]) * inv, __uint_as_float(v[8 * g + 1]) * inv),
-              pack_bf16x2(__uint_as_float(v[8 * g + 2]) * inv, __uint_as_float(v[8 * g + 3]) * inv),
-              pack_bf16x2(__uint_as_float(v[8 * g + 4]) * inv, __uint_as_float(v[8 * g + 5]) * inv),
-              pack_bf16x2(__uint_as_float(v[8 * g + 6]) * inv, __uint_as_float(v[8 * g + 7]) * inv));
-          *reinterpret_cast<uint4*>(blk + ((chunk ^ (r & 7)) << 4)) = u;
+      for (int i = 0; i < NB; ++i) {
+        uint32_t v[64];
+        tmem_ld_32x32b_x32(to + i * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+        tmem_ld_32x32b_x32(to + i * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+        tc_wait_ld();
+        if (i == NB - 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&o_free[t]);
+        }
+        if (lane == 0) tma_store_wait_read<0>();     // the previous block has left the staging buffer
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          uint32_t w[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            w[j] = pack_bf16x2(__uint_as_float(v[8 * g + 2 * j]) * inv, __uint_as_float(v[8 * g + 2 * j + 1]) * inv);
+          *reinterpret_cast<uint4*>(stage + lane * 128 + ((g ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          if (qt0 + q * 32 < p.Sq) tma_store_4d(&tmO, stage, i * 64, it.h, qt0 + q * 32, it.b);
+          tma_store_commit();
         }
       }
-      if (q_pos < p.Sq && p.lse != nullptr)
-        p.lse[((long long)b * p.Hq + h) * p.Sq + q_pos] =
-            (l > 0.f) ? (m_ref + log2f(l)) * 0.6931471805599453f : -INFINITY;
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0 && qt0 + q * 32 < p.Sq) {
-#pragma unroll
-        for (int i = 0; i < NB; ++i)
-          tma_store_4d(&tmO, stage + i * (BQ * 128) + q * 32 * 128, i * 64, h, qt0 + q * 32, b);
-        tma_store_commit();
-        tma_store_wait_all<0>();
-      }
     }
+    if (lane == 0) tma_store_wait_all<0>();
   }
 
+  __syncwarp();
   if (*abort_flag) {
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
@@ -381,7 +484,7 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
                                             cudaGetErrorString(e));
     configured[dev & 63] = true;
   }
-  dim3 grid((p.Sq + 2 * BQ - 1) / (2 * BQ), p.Hq, p.B);
+  const int grid = p.items < b200::sm_count() ? p.items : b200::sm_count();
   attn_fwd_kernel<HD><<<grid, NTHREADS, SM::TOTAL, stream>>>(tq, tk, tv, to, p);
   b200::count_launch();
   return b200::check_launch("attn_fwd");
@@ -411,6 +514,13 @@ B200_API int b200_attn_fwd(const void* q, const void* k, const void* v, void* o,
   p.scale_log2 = scale * 1.4426950408889634f;
   p.sink = sink; p.lse = lse;
   p.status = b200::status_ptr();
+  const long long items = (long long)((Sq + 2 * BQ - 1) / (2 * BQ)) * Hq * B;
+  if (items <= 0 || items > 0x3fffffff) return b200::fail(600, "attn_fwd: %lld query tile pairs", items);
+  p.items = (int)items;
+  // K and V of a group of heads: half of the 126 MB L2, so that the next group's fit beside them
+  const long long per_kv_head = (long long)Skv * HD * 4, fit = (64ll << 20) / per_kv_head;
+  const long long group = (fit > 0 ? fit : 1) * (Hq / Hkv);
+  p.bh_group = (int)(group < (long long)B * Hq ? group : (long long)B * Hq);
   if (HD == 128) return launch_fwd<128>(tq, tk, tv, to, p, (cudaStream_t)stream);
   return launch_fwd<64>(tq, tk, tv, to, p, (cudaStream_t)stream);
 }

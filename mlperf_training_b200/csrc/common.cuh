@@ -394,7 +394,7 @@ B200_DEVICE float2 fmul2(float2 a, float2 b) {
 }
 B200_DEVICE float ex2_approx(float x) {
   float y;
-  asm volatile("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 // 2^x for a pair of values without the MUFU unit and without float<->int conversions (which also

@@ -1,0 +1,24 @@
+"""Attention forward at the edges of its work schedule: odd tile counts, more and fewer items than CTAs, windows that skip
+a pair's first key tile, more keys than queries, several L2 groups' worth of head order."""
+import pytest
+import torch
+
+from mlperf_training_b200.ops import _lib, kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,Sq,Skv,Hq,Hkv,D,causal,window,sink", [
+    (1, 1, 1, 1, 1, 128, True, 0, False), (1, 129, 129, 2, 1, 64, True, 1, True), (2, 257, 257, 4, 2, 128, True, 128, False),
+    (1, 640, 640, 8, 8, 64, True, 200, True), (3, 384, 511, 4, 1, 128, True, 0, False), (2, 300, 1000, 6, 3, 64, False, 0, False),
+    (5, 513, 513, 8, 2, 128, True, 0, True), (1, 200, 1500, 4, 4, 128, True, 100, False)])
+def test_forward(B, Sq, Skv, Hq, Hkv, D, causal, window, sink):
+    torch.manual_seed(Sq)
+    q, k, v = (torch.randn(B, s, h, D, device="cuda").bfloat16() for s, h in ((Sq, Hq), (Skv, Hkv), (Skv, Hkv)))
+    sk = torch.randn(Hq, device="cuda") if sink else None
+    out, lse = K.attention_fwd(q, k, v, causal=causal, window=window, sink=sk)
+    ref, ref_lse = K.attention_reference(q, k, v, scale=D ** -0.5, causal=causal, window=window, sink=sk)
+    # bf16 probabilities and output: 2^-9 each per term, at most 2^-7 of the largest value
+    assert (out.float() - ref).abs().max() <= 2 ** -7 * ref.abs().max()
+    assert (lse - ref_lse).abs().max() <= 2e-3       # a quarter of the exponentials carry up to 7e-4
+    _lib.check_status("attention_fwd")

@@ -515,7 +515,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
   volatile int* work_slot = abort_flag + 1;       // reduce-scatter: the work item the epilogue warps share
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // (uniform: the roles below stay converged)
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();        // 0 = leader of the pair
   // leading CTA pairs that only move gathered blocks / only reduce
@@ -625,15 +625,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA only) ------------------------------
-    if (lane == 0 && rank == 0) {
+    // The whole warp walks the schedule and one elected lane issues: the operands of the instructions then stay in
+    // uniform registers and the descriptors advance by an addition.  (One lane of a divergent warp that rebuilt them
+    // needed more cycles per instruction than a block-scaled one runs.)
+    if (rank == 0) {
       const uint32_t idesc0 = MX ? umma_idesc_mx(0, 0, 0, 0, 256, BN)
                               : F8 ? umma_idesc(p.a_fmt, p.b_fmt, 0, 0, 256, BN)
                                    : umma_idesc(1, 1, p.a_mn_major, p.b_mn_major, 256, BN);
       const bool a_mn = !MX && !F8 && p.a_mn_major, b_mn = !MX && !F8 && p.b_mn_major;
-      const uint32_t a_lbo = a_mn ? 8192 : 16, b_lbo = b_mn ? 8192 : 16;
       // K advance per MMA: 32 bytes along a K-major row, or 16 rows of 128 bytes in an MN-major tile
-      const uint32_t a_kstep = a_mn ? 16 * 128 : UMMA_K_BYTES;
-      const uint32_t b_kstep = b_mn ? 16 * 128 : UMMA_K_BYTES;
+      const uint32_t a_kstep = (a_mn ? 16 * 128 : UMMA_K_BYTES) >> 4;
+      const uint32_t b_kstep = (b_mn ? 16 * 128 : UMMA_K_BYTES) >> 4;
+      const uint64_t ad0 = umma_desc_sw128(smem_u32(sA), a_mn ? 8192 : 16, 1024);
+      const uint64_t bd0 = umma_desc_sw128(smem_u32(sB), b_mn ? 8192 : 16, 1024);
       int stage = 0; uint32_t phase = 0;
       int it = 0;
       bool ok = true;
@@ -650,34 +654,32 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (!mbar_wait_spin(&full[stage], phase, abort_flag, p.status, 321)) { ok = false; break; }
           if (MX && !mbar_wait_spin(&sfrdy[stage], phase, abort_flag, p.status, 322)) { ok = false; break; }
           tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int s = 0; s < KSUB; ++s) {
-            const uint32_t a_addr = smem_u32(sA + (stage * KSUB + s) * C::A_SUB);
-            const uint32_t b_addr = smem_u32(sB + (stage * KSUB + s) * C::B_SUB);
-            uint32_t t_sfa = 0, t_sfb = 0;
-            if (MX) {
-              t_sfa = tmem_base + C::SF_COL + (uint32_t)(stage * KSUB + s) * C::SF_SET_COLS;
-              t_sfb = t_sfa + 4;
-            }
+            for (int s = 0; s < KSUB; ++s) {
+              const uint64_t ad = ad0 + ((stage * KSUB + s) * C::A_SUB >> 4);
+              const uint64_t bd = bd0 + ((stage * KSUB + s) * C::B_SUB >> 4);
+              const uint32_t t_sfa = tmem_base + C::SF_COL + (uint32_t)(stage * KSUB + s) * C::SF_SET_COLS;   // MX only
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-              const uint64_t ad = umma_desc_sw128(a_addr + kk * a_kstep, a_lbo, 1024);
-              const uint64_t bd = umma_desc_sw128(b_addr + kk * b_kstep, b_lbo, 1024);
-              const uint32_t accum = (kb > 0 || s > 0 || kk > 0) ? 1u : 0u;
-              if (MX) {
-                // scale byte kk of every 32-bit scale column: a_sf_id bits [29,31), b_sf_id bits [4,6)
-                tc_mma_mxf8_ss_pair(d_tmem, ad, bd, idesc0 | ((uint32_t)kk << 29) | ((uint32_t)kk << 4), accum, t_sfa, t_sfb);
-              } else if (F8) {
-                tc_mma_f8_ss_pair(d_tmem, ad, bd, idesc0, accum);
-              } else {
-                tc_mma_f16_ss_pair(d_tmem, ad, bd, idesc0, accum);
+              for (int kk = 0; kk < 4; ++kk) {
+                const uint32_t accum = (kb > 0 || s > 0 || kk > 0) ? 1u : 0u;
+                if (MX) {
+                  // scale byte kk of every 32-bit scale column: a_sf_id bits [29,31), b_sf_id bits [4,6)
+                  tc_mma_mxf8_ss_pair(d_tmem, ad + kk * a_kstep, bd + kk * b_kstep, idesc0 | ((uint32_t)kk << 29) | ((uint32_t)kk << 4),
+                                      accum, t_sfa, t_sfa + 4);
+                } else if (F8) {
+                  tc_mma_f8_ss_pair(d_tmem, ad + kk * a_kstep, bd + kk * b_kstep, idesc0, accum);
+                } else {
+                  tc_mma_f16_ss_pair(d_tmem, ad + kk * a_kstep, bd + kk * b_kstep, idesc0, accum);
+                }
               }
             }
+            tc_commit_pair(&empty[stage], 3);     // both CTAs may refill the stage once these MMAs have read it
+            if (kb == ti.nkb - 1) tc_commit_pair(&tfull[acc], 3);   // accumulator complete in both CTAs' TMEM
           }
-          tc_commit_pair(&empty[stage], 3);       // both CTAs may refill the stage once these MMAs have read it
+          __syncwarp();
           if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
         }
-        if (ok) tc_commit_pair(&tfull[acc], 3);   // accumulator complete in both CTAs' TMEM
       }
     }
   } else if (warp < 2 + EPI_WARPS) {

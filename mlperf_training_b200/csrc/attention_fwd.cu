@@ -401,12 +401,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           }
         }
         // the row sum, off the path of the MMAs
-        float2 rs2[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        float2 rs2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
         for (int i = 0; i < BKV / 2; ++i)
-          rs2[i & 3] = fadd2(rs2[i & 3], make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
-        const float2 ra = fadd2(rs2[0], rs2[1]), rb = fadd2(rs2[2], rs2[3]);
-        l += (ra.x + ra.y) + (rb.x + rb.y);
+          rs2[i & 1] = fadd2(rs2[i & 1], make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+        l += (rs2[0].x + rs2[0].y) + (rs2[1].x + rs2[1].y);
       }
       // ------------------------------ epilogue ------------------------------
       if (!ok || !mbar_wait(&o_done[t], no & 1, abort_flag, p.status, 62)) { ok = false; break; }

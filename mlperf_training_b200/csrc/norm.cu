@@ -15,7 +15,7 @@
 // Measured (bf16 in and out, L2 flushed, launch included), one warp or CTA per row -> this split:
 //   98304 x 128   forward 276 -> 16 us   backward 722 -> 30 us
 //   92160 x 512   LayerNorm 116 -> 46 us, backward 198 -> 75 us
-//    8192 x 2880  52 -> 31 us, 149 -> 67 us;   4011 x 4096  28 -> 21 us, 62 -> 50 us;   4096 x 8192  50 -> 38 us, 163 -> 87 us
+//    8192 x 2880  52 -> 31 us, 149 -> 67 us;   4096 x 8192  50 -> 38 us, 163 -> 87 us
 // Four rows of a 512-thread CTA instead of two of a 256-thread one lost 5 to 15 % at widths 2880 and 4096; above
 // 4096 the backward takes 512 threads (with 256 its accumulators leave one CTA of 8 warps per SM: 97 us).
 //
@@ -193,6 +193,87 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
   }
 }
 
+// Forward of widths that are whole vectors of a warp up to 4096: a warp per row, up to 16 vectors per lane, summed lane
+// by lane in column order.  The CTA-per-row split is up to 20 % faster at 4096 (27 -> 22 us for 4011 rows), but adds the
+// squares in another order, and with block-scaled linears behind it one flipped bf16 bit in 90000 grew to 3 % of the
+// attention gradients over three quantisers.
+constexpr int WMAXV = 16;
+template <int MODE>
+__global__ void __launch_bounds__(256)
+norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
+                     const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
+                     __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out, float* __restrict__ mean_out,
+                     float* __restrict__ rstd_out, int T, int D, float eps, int act) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nv = D >> 8;  // vectors per lane
+  for (int row = blockIdx.x * 8 + warp; row < T; row += gridDim.x * 8) {
+    const long long base = (long long)row * D;
+    uint4 xv[WMAXV];
+#pragma unroll
+    for (int i = 0; i < WMAXV; ++i)
+      if (i < nv) xv[i] = *reinterpret_cast<const uint4*>(x + base + (lane + 32 * i) * 8);
+    if (res != nullptr) {
+#pragma unroll
+      for (int i = 0; i < WMAXV; ++i)
+        if (i < nv) {
+          float a[8], r[8];
+          unpack8(xv[i], a);
+          unpack8(ld16(res + base + (lane + 32 * i) * 8), r);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) a[j] += r[j];
+          xv[i] = make_uint4(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]), pack_bf16x2(a[4], a[5]), pack_bf16x2(a[6], a[7]));
+          if (h_out != nullptr) *reinterpret_cast<uint4*>(h_out + base + (lane + 32 * i) * 8) = xv[i];
+        }
+    }
+    float s = 0.f, ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < WMAXV; ++i)
+      if (i < nv) {
+        float a[8];
+        unpack8(xv[i], a);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { s += a[j]; ss += a[j] * a[j]; }
+      }
+    float mean = 0.f, rstd;
+    if (MODE == 1) {
+      mean = warp_sum(s) / D;
+      float var = 0.f;
+#pragma unroll
+      for (int i = 0; i < WMAXV; ++i)
+        if (i < nv) {
+          float a[8];
+          unpack8(xv[i], a);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) { const float d = a[j] - mean; var += d * d; }
+        }
+      rstd = rsqrtf(warp_sum(var) / D + eps);
+    } else {
+      rstd = rsqrtf(warp_sum(ss) / D + eps);
+    }
+    if (lane == 0) {
+      if (rstd_out) rstd_out[row] = rstd;
+      if (MODE == 1 && mean_out) mean_out[row] = mean;
+    }
+#pragma unroll
+    for (int i = 0; i < WMAXV; ++i)
+      if (i < nv) {
+        const int c = (lane + 32 * i) * 8;
+        float a[8], w8[8], b8[8], o[8];
+        unpack8(xv[i], a);
+        if (w != nullptr) unpack8(ld16(w + c), w8);
+        if (b != nullptr) unpack8(ld16(b + c), b8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float n = (a[j] - mean) * rstd;
+          if (w != nullptr) n *= w8[j];
+          if (b != nullptr) n += b8[j];
+          o[j] = act ? a[j] * (1.f / (1.f + __expf(-n))) : n;
+        }
+        st16(y + base + c, pack8(o));
+      }
+  }
+}
+
 // dx for every row, plus per-CTA partial sums of dw (and db) in `partial` laid out [gridDim.x][2][D].
 template <int MODE, int ACT, int G, int V, int ROWS, int MAXT = NT>
 __global__ void __launch_bounds__(MAXT)
@@ -350,6 +431,128 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
   }
 }
 
+// Backward of the same widths, with the row sums in the same lane order (dx of the CTA-per-row split differs in the last
+// bit of 4 elements in a million; that split took 50 instead of 62 us for 4011 x 4096): dx per row; dw / db accumulated per warp in shared memory (fixed lane -> column mapping, no
+// atomics), summed over the CTA's warps in order and written as one partial row per CTA.
+template <int MODE, int ACT>
+__global__ void __launch_bounds__(256)
+norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                     const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
+                     const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
+                     const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+                     float* __restrict__ partial, int T, int D, int nwarps) {
+  extern __shared__ float acc[];  // [nwarps][(MODE == 1 || ACT) ? 2 : 1][D]
+  constexpr int NACC = (MODE == 1 || ACT) ? 2 : 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nv = D >> 8;
+  float* my_w = acc + (long long)warp * NACC * D;
+  float* my_b = my_w + D;
+  if (warp < nwarps)
+    for (int i = lane; i < NACC * D; i += 32) my_w[i] = 0.f;
+  __syncwarp();
+  if (warp < nwarps) {
+    for (int row = blockIdx.x * nwarps + warp; row < T; row += gridDim.x * nwarps) {
+      const long long base = (long long)row * D;
+      const float rstd = rstd_in[row];
+      const float mean = (MODE == 1) ? mean_in[row] : 0.f;
+      uint4 xv[WMAXV], gv[WMAXV];
+#pragma unroll
+      for (int i = 0; i < WMAXV; ++i)
+        if (i < nv) {
+          xv[i] = *reinterpret_cast<const uint4*>(x + base + (lane + 32 * i) * 8);
+          gv[i] = *reinterpret_cast<const uint4*>(dy + base + (lane + 32 * i) * 8);
+        }
+      float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+      for (int i = 0; i < WMAXV; ++i)
+        if (i < nv) {
+          const int c = (lane + 32 * i) * 8;
+          float x8[8], d8[8], w8[8], b8[8];
+          unpack8(xv[i], x8);
+          unpack8(gv[i], d8);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) { w8[j] = 1.f; b8[j] = 0.f; }
+          if (w != nullptr) unpack8(ld16(w + c), w8);
+          if (ACT && b != nullptr) unpack8(ld16(b + c), b8);
+          float4 a0 = *reinterpret_cast<float4*>(my_w + c), a1 = *reinterpret_cast<float4*>(my_w + c + 4);
+          float aw[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+          float ab[8];
+          if (NACC == 2) {
+            float4 b0 = *reinterpret_cast<float4*>(my_b + c), b1 = *reinterpret_cast<float4*>(my_b + c + 4);
+            ab[0] = b0.x; ab[1] = b0.y; ab[2] = b0.z; ab[3] = b0.w; ab[4] = b1.x; ab[5] = b1.y; ab[6] = b1.z; ab[7] = b1.w;
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float xn = (x8[j] - mean) * rstd;
+            float dn = d8[j];
+            if (ACT) {
+              const float n = xn * w8[j] + b8[j];
+              const float sg = 1.f / (1.f + __expf(-n));
+              dn = d8[j] * x8[j] * sg * (1.f - sg);
+            }
+            aw[j] += dn * xn;
+            if (NACC == 2) ab[j] += dn;
+            const float gj = dn * w8[j];
+            s1 += gj * xn;
+            s2 += gj;
+          }
+          *reinterpret_cast<float4*>(my_w + c) = make_float4(aw[0], aw[1], aw[2], aw[3]);
+          *reinterpret_cast<float4*>(my_w + c + 4) = make_float4(aw[4], aw[5], aw[6], aw[7]);
+          if (NACC == 2) {
+            *reinterpret_cast<float4*>(my_b + c) = make_float4(ab[0], ab[1], ab[2], ab[3]);
+            *reinterpret_cast<float4*>(my_b + c + 4) = make_float4(ab[4], ab[5], ab[6], ab[7]);
+          }
+        }
+      s1 = warp_sum(s1) / D;
+      s2 = (MODE == 1) ? warp_sum(s2) / D : 0.f;
+#pragma unroll
+      for (int i = 0; i < WMAXV; ++i)
+        if (i < nv) {
+          const int c = (lane + 32 * i) * 8;
+          float x8[8], d8[8], w8[8], b8[8], o[8];
+          unpack8(xv[i], x8);
+          unpack8(gv[i], d8);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) { w8[j] = 1.f; b8[j] = 0.f; }
+          if (w != nullptr) unpack8(ld16(w + c), w8);
+          if (ACT && b != nullptr) unpack8(ld16(b + c), b8);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float xn = (x8[j] - mean) * rstd;
+            float dn = d8[j], direct = 0.f;
+            if (ACT) {
+              const float n = xn * w8[j] + b8[j];
+              const float sg = 1.f / (1.f + __expf(-n));
+              dn = d8[j] * x8[j] * sg * (1.f - sg);
+              direct = d8[j] * sg;
+            }
+            o[j] = rstd * (dn * w8[j] - xn * s1 - s2) + direct;
+          }
+          if (dres != nullptr) {
+            float r8[8];
+            unpack8(ld16(dres + base + c), r8);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] += r8[j];
+          }
+          st16(dx + base + c, pack8(o));
+        }
+    }
+  }
+  __syncthreads();
+  if (partial != nullptr) {
+    float* pw = partial + (long long)blockIdx.x * 2 * D;
+    for (int c = threadIdx.x; c < D; c += blockDim.x) {
+      float sw = 0.f, sb = 0.f;
+      for (int k = 0; k < nwarps; ++k) {
+        sw += acc[(long long)k * NACC * D + c];
+        if (NACC == 2) sb += acc[(long long)k * NACC * D + D + c];
+      }
+      pw[c] = sw;
+      pw[D + c] = sb;
+    }
+  }
+}
+
 // out[c] (+)= sum_p partial[p][which][c]: 32 columns per CTA, its 8 warps take every eighth partial row (their loads
 // are independent: one thread per column walked all of them in series), summed in a fixed order.
 __global__ void __launch_bounds__(256)
@@ -407,6 +610,11 @@ void dispatch_fwd(const FwdArgs& a) {
   else if (a.D <= 256) run_fwd<MODE, 32, 1, 4>(a);
   else if (a.D <= 512) run_fwd<MODE, 32, 2, 2>(a);
   else if (a.D <= 1024) run_fwd<MODE, 32, 4, 1>(a);
+  else if (a.D % 256 == 0 && a.D <= 4096) {
+    const int need = (a.T + 7) / 8, cap = b200::sm_count() * 8;
+    norm_fwd_warp_kernel<MODE><<<need < cap ? need : cap, 256, 0, a.st>>>(a.x, a.res, a.w, a.b, a.y, a.h, a.mean, a.rstd, a.T,
+                                                                         a.D, a.eps, a.act);
+  }
   else if (a.D <= 4096) run_fwd<MODE, 0, 2, 2>(a);
   else run_fwd<MODE, 0, 4, 2>(a);
 }
@@ -423,12 +631,35 @@ int run_bwd(const BwdArgs& a) {
 }
 
 template <int MODE, int ACT>
+int run_bwd_warp(const BwdArgs& a) {
+  constexpr int nacc = (MODE == 1 || ACT) ? 2 : 1;
+  int nwarps = (200 * 1024) / (a.D * 4 * nacc);
+  if (nwarps > 8) nwarps = 8;
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(norm_bwd_warp_kernel<MODE, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return -b200::fail(302, "norm_bwd: cannot raise shared memory: %s", cudaGetErrorString(e));
+    }
+    configured[dev & 63] = true;
+  }
+  const int grid = b200::sm_count() < a.grid ? b200::sm_count() : a.grid;
+  norm_bwd_warp_kernel<MODE, ACT><<<grid, 256, nwarps * nacc * a.D * 4, a.st>>>(a.dy, a.x, a.w, a.b, a.mean, a.rstd, a.dres, a.dx,
+                                                                                a.partial, a.T, a.D, nwarps);
+  return grid;
+}
+
+template <int MODE, int ACT>
 int dispatch_bwd(const BwdArgs& a) {
   if (a.D <= 64) return run_bwd<MODE, ACT, 8, 1, 4>(a);
   if (a.D <= 128) return run_bwd<MODE, ACT, 16, 1, 4>(a);
   if (a.D <= 256) return run_bwd<MODE, ACT, 32, 1, 4>(a);
   if (a.D <= 512) return run_bwd<MODE, ACT, 32, 2, 2>(a);
   if (a.D <= 1024) return run_bwd<MODE, ACT, 32, 4, 1>(a);
+  if (a.D % 256 == 0 && a.D <= 4096) return run_bwd_warp<MODE, ACT>(a);
   if (a.D <= 4096) return run_bwd<MODE, ACT, 0, 2, 2>(a);
   return run_bwd<MODE, ACT, 0, 2, 2, 512>(a);
 }
@@ -470,6 +701,7 @@ B200_API int b200_norm_bwd(int mode, const void* dy, const void* x, const void* 
   int parts;
   if (mode == 0) parts = act ? dispatch_bwd<0, 1>(a) : dispatch_bwd<0, 0>(a);
   else parts = act ? dispatch_bwd<1, 1>(a) : dispatch_bwd<1, 0>(a);
+  if (parts < 0) return -parts;
   b200::count_launch();
   if (int r = b200::check_launch("norm_bwd")) return r;
   if (scratch != nullptr && (dw != nullptr || db != nullptr)) {

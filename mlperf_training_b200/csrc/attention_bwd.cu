@@ -40,6 +40,7 @@ struct BwdParams {
   const float* lse;    // [B, Hq, Sq]
   const float* delta;  // [B, Hq, Sq]  rowsum(dO * O)
   int* status;
+  int bh_group;        // (batch, kv head) pairs scheduled together, longest key tiles first
 };
 
 B200_DEVICE void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
@@ -97,10 +98,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_kt = (p.Skv + BKV - 1) / BKV;
-  const int jt = blockIdx.x;  // key tile; early tiles see the most queries and are scheduled first
-  const int hk = blockIdx.y, b = blockIdx.z;
+  // early key tiles see the most queries: they are scheduled first, over all heads of a group
+  const int bh_all = p.B * p.Hkv, per_group = p.bh_group * num_kt;
+  const int grp = (int)blockIdx.x / per_group, rest = (int)blockIdx.x - grp * per_group;
+  const int gsz = min(p.bh_group, bh_all - grp * p.bh_group);
+  const int jt = rest / gsz, bh = grp * p.bh_group + rest % gsz;
+  const int b = bh / p.Hkv, hk = bh - b * p.Hkv;
   const int group = p.Hq / p.Hkv;
   const int kv0 = jt * BKV;
   const int off = p.Skv - p.Sq;
@@ -117,7 +122,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
   const int n_q = (i_hi >= i_lo) ? (i_hi - i_lo + 1) : 0;
   const int n_iter = n_q * group;
-  (void)num_kt;
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1); mbar_init(qdo_full, 1); mbar_init(qdo_empty, 1); mbar_init(sdp_full, 1);
@@ -160,60 +164,67 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0 && n_iter > 0) {
+    // The warp stays converged and one elected lane issues: operands live in uniform registers and descriptors advance by
+    // an addition (rebuilt by one lane of a divergent warp they cost more than the 64 cycles an instruction runs).
+    if (n_iter > 0) {
       const uint32_t id_kk = umma_idesc(1, 1, 0, 0, 128, 128);   // S = Q K^T, dP = dO V^T (both K-major)
       const uint32_t id_dq = umma_idesc(1, 1, 0, 1, 128, HD);    // dQ = dS (K-major) x K (MN-major)
       const uint32_t id_tt = umma_idesc(1, 1, 1, 1, 128, HD);    // dV = P^T dO, dK = dS^T Q (both MN-major)
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ), adO = smem_u32(sdO);
-      const uint32_t aP = smem_u32(sP), adS = smem_u32(sdS);
-      bool ok = mbar_wait(kv_full, 0, abort_flag, p.status, 80);
+      const uint64_t kK = umma_desc_sw128(smem_u32(sK), 16, 1024), kV = umma_desc_sw128(smem_u32(sV), 16, 1024);
+      const uint64_t kQ = umma_desc_sw128(smem_u32(sQ), 16, 1024), kdO = umma_desc_sw128(smem_u32(sdO), 16, 1024);
+      const uint64_t kdS = umma_desc_sw128(smem_u32(sdS), 16, 1024);
+      const uint64_t mK = umma_desc_sw128(smem_u32(sK), 128 * 128, 1024), mQ = umma_desc_sw128(smem_u32(sQ), 128 * 128, 1024);
+      const uint64_t mdO = umma_desc_sw128(smem_u32(sdO), 128 * 128, 1024), mP = umma_desc_sw128(smem_u32(sP), 128 * 128, 1024);
+      const uint64_t mdS = umma_desc_sw128(smem_u32(sdS), 128 * 128, 1024);
+      bool ok = mbar_wait_spin(kv_full, 0, abort_flag, p.status, 80);
       for (int it = 0; it < n_iter && ok; ++it) {
         const uint32_t ph = it & 1;
-        if (!mbar_wait(qdo_full, ph, abort_flag, p.status, 81)) { ok = false; break; }
+        if (!mbar_wait_spin(qdo_full, ph, abort_flag, p.status, 81)) { ok = false; break; }
         tc_fence_after();
         // S = Q K^T ; dP = dO V^T   (contraction over the head dim, both operands K-major)
         // dP first: its accumulator was read by the workers long ago, so these MMAs run while the workers
         // still drain dQ of the previous iteration out of the S / dQ columns
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t o = (kk / 4) * (128 * 128) + (kk % 4) * 32;
-          tc_mma_f16_ss(tm_dP, umma_desc_sw128(adO + o, 16, 1024), umma_desc_sw128(aV + o, 16, 1024), id_kk, kk > 0);
+          for (int kk = 0; kk < HD / 16; ++kk) {
+            const uint32_t o = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
+            tc_mma_f16_ss(tm_dP, kdO + o, kV + o, id_kk, kk > 0);
+          }
         }
-        if (it > 0 && !mbar_wait(dq_drained, (it - 1) & 1, abort_flag, p.status, 82)) { ok = false; break; }
+        __syncwarp();
+        if (it > 0 && !mbar_wait_spin(dq_drained, (it - 1) & 1, abort_flag, p.status, 82)) { ok = false; break; }
         tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t o = (kk / 4) * (128 * 128) + (kk % 4) * 32;
-          tc_mma_f16_ss(tm_S, umma_desc_sw128(aQ + o, 16, 1024), umma_desc_sw128(aK + o, 16, 1024), id_kk, kk > 0);
+          for (int kk = 0; kk < HD / 16; ++kk) {
+            const uint32_t o = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
+            tc_mma_f16_ss(tm_S, kQ + o, kK + o, id_kk, kk > 0);
+          }
+          tc_commit(sdp_full);
         }
-        tc_commit(sdp_full);
-        if (!mbar_wait(pds_full, ph, abort_flag, p.status, 83)) { ok = false; break; }
+        __syncwarp();
+        if (!mbar_wait_spin(pds_full, ph, abort_flag, p.status, 83)) { ok = false; break; }
         tc_fence_after();
-        // dV += P^T dO ; dK += dS^T Q : contraction over queries, both operands MN-major
+        if (elect_one()) {
+          // dV += P^T dO ; dK += dS^T Q : contraction over queries, both operands MN-major
 #pragma unroll
-        for (int kk = 0; kk < BQ / 16; ++kk) {
-          const uint32_t o = kk * (16 * 128);
-          tc_mma_f16_ss(tm_dV, umma_desc_sw128(aP + o, 128 * 128, 1024), umma_desc_sw128(adO + o, 128 * 128, 1024),
-                        id_tt, (it > 0 || kk > 0));
-        }
+          for (int kk = 0; kk < BQ / 16; ++kk)
+            tc_mma_f16_ss(tm_dV, mP + kk * 128, mdO + kk * 128, id_tt, (it > 0 || kk > 0));
 #pragma unroll
-        for (int kk = 0; kk < BQ / 16; ++kk) {
-          const uint32_t o = kk * (16 * 128);
-          tc_mma_f16_ss(tm_dK, umma_desc_sw128(adS + o, 128 * 128, 1024), umma_desc_sw128(aQ + o, 128 * 128, 1024),
-                        id_tt, (it > 0 || kk > 0));
-        }
-        tc_commit(qdo_empty);  // Q_i / dO_i may be overwritten: the next tiles load during the dQ GEMM
-        // dQ = dS K : A = dS [q][key] K-major, B = K [key][d] MN-major (contraction over keys)
+          for (int kk = 0; kk < BQ / 16; ++kk)
+            tc_mma_f16_ss(tm_dK, mdS + kk * 128, mQ + kk * 128, id_tt, (it > 0 || kk > 0));
+          tc_commit(qdo_empty);  // Q_i / dO_i may be overwritten: the next tiles load during the dQ GEMM
+          // dQ = dS K : A = dS [q][key] K-major, B = K [key][d] MN-major (contraction over keys)
 #pragma unroll
-        for (int kk = 0; kk < BKV / 16; ++kk) {
-          const uint32_t ao = (kk / 4) * (128 * 128) + (kk % 4) * 32;
-          const uint32_t bo = kk * (16 * 128);
-          tc_mma_f16_ss(tm_S, umma_desc_sw128(adS + ao, 16, 1024), umma_desc_sw128(aK + bo, 128 * 128, 1024), id_dq,
-                        kk > 0);
+          for (int kk = 0; kk < BKV / 16; ++kk) {
+            const uint32_t ao = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
+            tc_mma_f16_ss(tm_S, kdS + ao, mK + kk * 128, id_dq, kk > 0);
+          }
+          tc_commit(dq_full);    // also: P / dS shared-memory tiles are free again
+          if (it == n_iter - 1) tc_commit(acc_done);
         }
-        tc_commit(dq_full);    // also: P / dS shared-memory tiles are free again
+        __syncwarp();
       }
-      if (ok) tc_commit(acc_done);
     }
   } else {
     // ------------------------------ workers: P / dS, then dQ drain ------------------------------
@@ -355,6 +366,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (lane == 0) tma_store_wait_all<0>();
   }
 
+  __syncwarp();
   if (*abort_flag) {
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
@@ -406,8 +418,9 @@ int launch_bwd(const CUtensorMap* m, const BwdParams& p, cudaStream_t stream) {
                                             cudaGetErrorString(e));
     configured[dev & 63] = true;
   }
-  dim3 grid((p.Skv + BKV - 1) / BKV, p.Hkv, p.B);
-  attn_bwd_kernel<HD><<<grid, NTHREADS, SM::TOTAL, stream>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], p);
+  const long long grid = (long long)((p.Skv + BKV - 1) / BKV) * p.Hkv * p.B;
+  if (grid > 0x7fffffff) return b200::fail(612, "attn_bwd: %lld key tiles are too many", grid);
+  attn_bwd_kernel<HD><<<(unsigned)grid, NTHREADS, SM::TOTAL, stream>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], p);
   b200::count_launch();
   return b200::check_launch("attn_bwd");
 }
@@ -454,6 +467,11 @@ B200_API int b200_attn_bwd(const void* q, const void* k, const void* v, const vo
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.lse = lse; p.delta = delta;
   p.status = b200::status_ptr();
+  // Causal: a key tile's work falls with its position, so all heads' early tiles go first (head after head left the last
+  // head's longest CTAs running alone: 8192 x 32 / 8 heads of 128, delta and clearing included, 2370 -> 1990 us,
+  // 4096 x 64 / 8 heads 1590 -> 1130 us; groups of two heads 2070 and 1517).  Otherwise every tile costs the same and
+  // head after head keeps that head's Q and dO in L2 (8 x 512 x 24 heads 175 us, 181 the other way).
+  p.bh_group = (causal && window <= 0) ? B * Hkv : 1;
   if (HD == 128) return launch_bwd<128>(m, p, (cudaStream_t)stream);
   return launch_bwd<64>(m, p, (cudaStream_t)stream);
 }

@@ -99,7 +99,7 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_pairs = (p.max_len + 2 * BQ - 1) / (2 * BQ);
   const int pair = num_pairs - 1 - (int)blockIdx.x;  // heaviest (latest) query tiles first
   const int h = blockIdx.y, b = blockIdx.z;
@@ -170,68 +170,69 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
   } else if (warp == 9) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0 && n_max > 0) {
+    // The warp stays converged and one elected lane issues: operands live in uniform registers and descriptors advance by
+    // an addition (rebuilt by one lane of a divergent warp they cost more than the 64 cycles an instruction runs).
+    if (n_max > 0) {
       // formats: bf16 (code 1 of kind::f16) or e4m3 (code 0 of kind::f8f6f4)
       const uint32_t idesc_s = umma_idesc(F8 ? 0 : 1, F8 ? 0 : 1, 0, 0, BQ, BKV);  // Q (K-major) x K (K-major)
       const uint32_t idesc_o = umma_idesc(F8 ? 0 : 1, F8 ? 0 : 1, 0, 1, BQ, HD);   // P (TMEM)    x V (MN-major)
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.status, 50);
+      const uint64_t dQ = umma_desc_sw128(smem_u32(sQ), 16, 1024), dK = umma_desc_sw128(smem_u32(sK), 16, 1024);
+      const uint64_t dV = umma_desc_sw128(smem_u32(sV), BKV * 128, 1024);
+      bool ok = mbar_wait_spin(q_full, 0, abort_flag, p.status, 50);
       int k_ready = -1, v_ready = -1;  // last key tile index whose full barrier has been observed
       // S_t(n) = Q_t K(n)^T into the S columns of tile t
       auto issue_s = [&](int t, int n) -> bool {
         const int st = n & 1;
         if (k_ready < n) {
-          if (!mbar_wait(&k_full[st], (n >> 1) & 1, abort_flag, p.status, 51)) return false;
+          if (!mbar_wait_spin(&k_full[st], (n >> 1) & 1, abort_flag, p.status, 51)) return false;
           k_ready = n;
         }
         tc_fence_after();
-        const uint32_t qa = smem_u32(sQ + t * SM::Q_TILE), ka = smem_u32(sK + st * SM::KV_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < HD * SM::ES / 32; ++kk) {       // one MMA consumes 32 bytes of the head row
-          const uint32_t o = (kk / 4) * (BQ * 128) + (kk % 4) * 32;
-          if constexpr (F8)
-            tc_mma_f8_ss(tmem_base + t * 128, umma_desc_sw128(qa + o, 16, 1024), umma_desc_sw128(ka + o, 16, 1024),
-                         idesc_s, kk > 0 ? 1u : 0u);
-          else
-            tc_mma_f16_ss(tmem_base + t * 128, umma_desc_sw128(qa + o, 16, 1024), umma_desc_sw128(ka + o, 16, 1024),
-                          idesc_s, kk > 0 ? 1u : 0u);
-        }
-        tc_commit(&s_full[t]);
         // the last tile that reads K(n) frees its stage
         const bool last_user = (t == 1) || !(n < n_t[1]);
-        if (last_user) tc_commit(&k_empty[st]);
+        if (elect_one()) {
+          const uint64_t ad = dQ + (t * SM::Q_TILE >> 4), bd = dK + (st * SM::KV_BYTES >> 4);
+#pragma unroll
+          for (int kk = 0; kk < HD * SM::ES / 32; ++kk) {       // one MMA consumes 32 bytes of the head row
+            const uint32_t o = ((kk / 4) * (BQ * 128) + (kk % 4) * 32) >> 4;
+            if constexpr (F8) tc_mma_f8_ss(tmem_base + t * 128, ad + o, bd + o, idesc_s, kk > 0 ? 1u : 0u);
+            else tc_mma_f16_ss(tmem_base + t * 128, ad + o, bd + o, idesc_s, kk > 0 ? 1u : 0u);
+          }
+          tc_commit(&s_full[t]);
+          if (last_user) tc_commit(&k_empty[st]);
+        }
+        __syncwarp();
         return true;
       };
-      for (int t = 0; t < 2 && ok; ++t)
-        if (n_t[t] > 0) ok = issue_s(t, 0);
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+        if (ok && n_t[t] > 0) ok = issue_s(t, 0);
       for (int n = 0; n < n_max && ok; ++n) {
         const int st = n & 1;
-        for (int t = 0; t < 2 && ok; ++t) {
-          if (n >= n_t[t]) continue;
-          if (!mbar_wait(&p_full[t], n & 1, abort_flag, p.status, 53)) { ok = false; break; }
-          if (v_ready < n) {
-            if (!mbar_wait(&v_full[st], (n >> 1) & 1, abort_flag, p.status, 54)) { ok = false; break; }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (!ok || n >= n_t[t]) continue;
+          ok = mbar_wait_spin(&p_full[t], n & 1, abort_flag, p.status, 53);
+          if (ok && v_ready < n) {
+            ok = mbar_wait_spin(&v_full[st], (n >> 1) & 1, abort_flag, p.status, 54);
             v_ready = n;
           }
+          if (!ok) continue;
           tc_fence_after();
-          const uint32_t va = smem_u32(sV + st * SM::KV_BYTES);
-          if constexpr (F8) {
-#pragma unroll
-            for (int kk = 0; kk < BKV / 32; ++kk) {
-              // A = P_t in TMEM: 32 e4m3 keys = 8 columns per step; B = V: 32 key rows of 128 bytes (one block: HD = 128)
-              tc_mma_f8_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8,
-                           umma_desc_sw128(va + kk * (32 * 128), BKV * 128, 1024), idesc_o, (n > 0 || kk > 0) ? 1u : 0u);
-            }
-          } else {
-#pragma unroll
-            for (int kk = 0; kk < BKV / 16; ++kk) {
-              // A = P_t in TMEM: 16 bf16 keys = 8 columns per step; B = V: 16 key rows of 128 bytes
-              tc_mma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8,
-                            umma_desc_sw128(va + kk * (16 * 128), BKV * 128, 1024), idesc_o, (n > 0 || kk > 0) ? 1u : 0u);
-            }
-          }
-          tc_commit(&o_done[t]);
           const bool last_user = (t == 1) || !(n < n_t[1]);
-          if (last_user) tc_commit(&v_empty[st]);
+          if (elect_one()) {
+            // A = P_t in TMEM: 32 bytes of keys (8 columns) per step; B = V: that many key rows of 128 bytes
+            const uint64_t bd = dV + (st * SM::KV_BYTES >> 4);
+#pragma unroll
+            for (int kk = 0; kk < BKV * SM::ES / 32; ++kk) {
+              const uint32_t acc = (n > 0 || kk > 0) ? 1u : 0u, o = kk * (32 / SM::ES) * 128 >> 4;
+              if constexpr (F8) tc_mma_f8_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8, bd + o, idesc_o, acc);
+              else tc_mma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8, bd + o, idesc_o, acc);
+            }
+            tc_commit(&o_done[t]);
+            if (last_user) tc_commit(&v_empty[st]);
+          }
+          __syncwarp();
           if (n + 1 < n_t[t]) ok = issue_s(t, n + 1);
         }
       }
@@ -335,6 +336,7 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
   }
 
+  __syncwarp();
   if (*abort_flag) {
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);

@@ -274,6 +274,27 @@ B200_DEVICE void epilogue_drain(const CUtensorMap* tmD, const CUtensorMap* tmTai
   }
 }
 
+// Stores zeros to the rows and columns epilogue_drain would write (the tile of an expert without rows).
+template <int BN, bool WIDE>
+B200_DEVICE void zero_tile(const CUtensorMap* tmD, const EpiArgs& e, int row0, int n0, uint8_t* stg, int& buf, int lane, int row_off) {
+  static_assert(BN % 32 == 0, "grouped tiles are whole 32-column chunks");
+  if (lane == 0) tma_store_wait_read<0>();
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < STG_BYTES / 512; ++j) *reinterpret_cast<uint4*>(stg + j * 512 + lane * 16) = make_uint4(0u, 0u, 0u, 0u);
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    const int step = (!e.out_f32 && WIDE) ? 64 : 32;
+    for (int c = 0; c < BN; c += step)
+      if (n0 + c < e.N && row0 < e.M) tma_store_2d(tmD, stg, n0 + c, row0 + row_off);
+    tma_store_commit();
+    tma_store_wait_read<0>();                   // the buffer is written again by the next tile
+  }
+  __syncwarp();
+  buf = 0;
+}
+
 // Tensor map of D for epilogue_drain (ldd in elements).
 template <int BN>
 inline int make_out_tmap(CUtensorMap* tmD, CUtensorMap* tmTail, void* d, int M, int N, long long ldd, int out_f32) {
@@ -324,14 +345,16 @@ struct PairCfg {
   static_assert(BN % 16 == 0 && BN <= 256, "N of a 256-row MMA must be a multiple of 16 up to 256");
 };
 
-// Grouped (per-expert) problems on the pair kernel, MXFP8 operands:
+// Grouped (per-expert) problems on the pair kernel, MXFP8 or bf16 operands:
 //   mode 1  D[r, :] = A[r, :] * B[e(r)]^T over a row buffer whose expert segments start at multiples of
 //           256 rows; B is the experts' matrices stacked as [(E * N), K], its scale atoms were laid out
 //           with N a multiple of the N tile (a tile never straddles two experts); tiles of 256 rows whose
 //           tile_expert is negative (past the last segment) are skipped by every role
 //   mode 2  D[e] (+)= A[:, seg[e]:seg[e+1]] * B[:, seg[e]:seg[e+1]]^T - the contraction runs over the
 //           expert's rows of the (transposed, K-major) operands; D is the experts' [M, N] outputs stacked
-//           as [(E * M), N]; an expert without rows is skipped (accumulate into a zeroed D)
+//           as [(E * M), N]; the tiles of an expert without rows are left alone (accumulate) or set to zero
+// bf16: B is [(E * N), K] or, MN-major, [(E * K), N] (mode 1; the contraction of an expert ends on a whole stage);
+// mode 2 reads both operands MN-major, [rows, M] and [rows, N].
 struct GroupArgs {
   int mode;                       // 0: plain GEMM
   int E;
@@ -574,7 +597,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int mb = ti.mb;
         const int nb = ti.nb + (p.grp.mode == 1 ? ti.e * num_n : 0);   // column tile inside the stacked B
         const int m0 = mb * 256 + (int)rank * 128;          // this CTA's rows of A
-        const int n0 = ti.nb * BN + (int)rank * C::BNH + (p.grp.mode == 1 ? ti.e * p.N : 0);   // this CTA's rows of B
+        const bool b_mn = !MX && !F8 && p.b_mn_major;
+        // this CTA's rows of B, and where the expert's contraction starts in an MN-major stack
+        const int n0 = ti.nb * BN + (int)rank * C::BNH + (p.grp.mode == 1 && !b_mn ? ti.e * p.N : 0);
+        const int kb_off = (p.grp.mode == 1 && b_mn) ? ti.e * p.K : 0;
         if (p.tp.on) {
           const int c = (mb * 256) / p.tp.rows_per;             // rank block that holds this tile's rows of A
           if (!(ready & (1u << c))) {
@@ -612,11 +638,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
               for (int j = 0; j < 2; ++j) tma_load_2d_pair(a_dst + j * 8192, &tmA, bar, m0 + 64 * j, k0);
             }
-            if (MX || F8 || !p.b_mn_major) {
+            if (!b_mn) {
               tma_load_2d_pair(b_dst, &tmB, bar, k0, n0);
             } else {
 #pragma unroll
-              for (int j = 0; j < C::BNH / 64; ++j) tma_load_2d_pair(b_dst + j * 8192, &tmB, bar, n0 + 64 * j, k0);
+              for (int j = 0; j < C::BNH / 64; ++j) tma_load_2d_pair(b_dst + j * 8192, &tmB, bar, n0 + 64 * j, kb_off + k0);
             }
           }
           if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
@@ -693,7 +719,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     bool ok = true;
     for (int t = pair_id; t < num_tiles && ok; t += num_pairs) {
       const TileInfo ti = tile_info(t, num_m, num_n, num_kb, KB_ELEMS * KSUB, p);
-      if (!ti.valid) continue;
+      if (!ti.valid) {
+        if constexpr (BN % 32 == 0) {
+          if (p.grp.mode == 2 && !p.epi.accumulate)
+            zero_tile<BN, (BN % 64 == 0)>(&tmD, p.epi, ti.mb * 256 + (int)rank * 128 + q * 32, ti.nb * BN, stg, buf, lane, ti.e * p.M);
+        }
+        continue;
+      }
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
       ++it;

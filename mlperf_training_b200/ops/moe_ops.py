@@ -21,13 +21,20 @@ from . import mxfp8
 from ._lib import call, ptr, stream_ptr, use_kernels
 
 PAD = 128        # row padding of an expert segment for the bf16 grouped kernels (one 128-row tile)
-PAD_MX = 256     # ... for the block-scaled grouped kernels (one CTA pair works on 256 rows)
+PAD_MX = 256     # ... for the grouped kernels on CTA pairs (256 rows per pair): block-scaled, and bf16 where `pair_rows_ok`
 
 
 def pad_rows(precision: str) -> int:
     """Segment padding the grouped kernels of ``precision`` need."""
     from .linear import is_mx
     return PAD_MX if is_mx(precision) else PAD
+
+
+def pair_rows_ok(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor) -> bool:
+    """Whether the bf16 experts ``w1 [E, 2F, D]`` / ``w2 [E, D, F]`` run on the CTA-pair grouped kernels (segments padded to
+    ``PAD_MX`` rows): widths that are whole 64-element contraction stages.  Others keep the one-CTA kernels and ``PAD``."""
+    return (use_kernels(x) and x.dtype == torch.bfloat16 and w1.dtype == torch.bfloat16 and w2.dtype == torch.bfloat16
+            and w1.shape[2] % 64 == 0 and w2.shape[2] % 64 == 0)
 
 
 def grouped_bn(n: int) -> int:
@@ -143,6 +150,11 @@ def grouped_rows(a: torch.Tensor, b: torch.Tensor, tile_expert: torch.Tensor, se
         return out
     if out is None:
         out = torch.empty((rows, N), dtype=a.dtype, device=a.device)
+    if tile_expert.numel() * PAD_MX == rows:
+        a, b = a.contiguous(), b.contiguous()
+        call("b200_gemm_grouped_pair_rows", ptr(a), ptr(b), ptr(out), ptr(tile_expert), rows, N, Kd, E, a.stride(0), out.stride(0),
+             int(b_mn_major), 1.0, stream_ptr())
+        return out
     call("b200_gemm_grouped_rows", ptr(a.contiguous()), ptr(b.contiguous()), ptr(out), ptr(tile_expert), rows, N, Kd, E,
          a.stride(0), out.stride(0), int(b_mn_major), 0, 1.0, stream_ptr())
     # tiles past the last segment are not written: their rows are padding and are never read back
@@ -150,9 +162,17 @@ def grouped_rows(a: torch.Tensor, b: torch.Tensor, tile_expert: torch.Tensor, se
 
 
 def grouped_wgrad(dy: torch.Tensor, x: torch.Tensor, seg: torch.Tensor, n_experts: int, *,
-                  out: torch.Tensor | None = None, accumulate: bool = False, out_dtype=None) -> torch.Tensor:
-    """``d[e] (+)= dy[seg[e]:seg[e+1]]^T @ x[seg[e]:seg[e+1]]`` -> ``[E, M, N]``."""
+                  out: torch.Tensor | None = None, accumulate: bool = False, out_dtype=None, pad: int = PAD) -> torch.Tensor:
+    """``d[e] (+)= dy[seg[e]:seg[e+1]]^T @ x[seg[e]:seg[e+1]]`` -> ``[E, M, N]``.  ``pad``: what the segments are padded to."""
     M, N = dy.shape[1], x.shape[1]
+    if pad == PAD_MX and use_kernels(dy) and dy.dtype == torch.bfloat16 and M % 32 == 0:
+        if out is None:
+            # every element is written, zeros for an expert without rows
+            out, accumulate = torch.empty((n_experts, M, N), dtype=out_dtype or dy.dtype, device=dy.device), False
+        dy, x = dy.contiguous(), x.contiguous()
+        call("b200_gemm_grouped_pair_wgrad", ptr(dy), ptr(x), ptr(out), ptr(seg), dy.shape[0], M, N, n_experts, dy.stride(0),
+             x.stride(0), int(out.dtype == torch.float32), int(accumulate), 1.0, stream_ptr())
+        return out
     if out is None:
         out = torch.zeros((n_experts, M, N), dtype=out_dtype or dy.dtype, device=dy.device)
         accumulate = True if use_kernels(dy) else accumulate
@@ -262,11 +282,12 @@ class GroupedMLPFn(Function):
         gy = _zero_padding(gy.contiguous(), tile_expert)
         a = K.swiglu_fwd(gu)
         a = _zero_padding(a, tile_expert)
-        g2 = _wgrad_into(p2, gy, a, seg, E)
+        pad = gy.shape[0] // max(tile_expert.numel(), 1)
+        g2 = _wgrad_into(p2, gy, a, seg, E, pad)
         da = grouped_rows(gy, w2, tile_expert, seg, b_mn_major=True)
         dgu = K.swiglu_bwd(da, gu)
         dgu = _zero_padding(dgu, tile_expert)
-        g1 = _wgrad_into(p1, dgu, x, seg, E)
+        g1 = _wgrad_into(p1, dgu, x, seg, E, pad)
         dx = grouped_rows(dgu, w1, tile_expert, seg, b_mn_major=True, out=ctx.dx_out)
         return dx, g1, g2, None, None, None, None
 
@@ -311,18 +332,22 @@ def grouped_rows_mx(a: mxfp8.MXOperand, b: mxfp8.MXOperand, tile_expert: torch.T
     return out
 
 
-def grouped_wgrad_mx(dy_t: mxfp8.MXOperand, x_t: mxfp8.MXOperand, seg: torch.Tensor, n_experts: int, out: torch.Tensor):
+def grouped_wgrad_mx(dy_t: mxfp8.MXOperand, x_t: mxfp8.MXOperand, seg: torch.Tensor, n_experts: int, out: torch.Tensor,
+                     accumulate: bool = True):
     """``out[e] += deq(dy_t)[:, seg[e]:seg[e+1]] @ deq(x_t)[:, seg[e]:seg[e+1]]^T``; both operands are column-wise
-    copies (rows = features, contraction = the padded buffer's rows); ``out`` ``[E, M, N]`` fp32 or bf16."""
+    copies (rows = features, contraction = the padded buffer's rows); ``out`` ``[E, M, N]`` fp32 or bf16.
+    Without ``accumulate`` all of ``out`` is written (zeros for an expert without rows)."""
     M, N, T = dy_t.rows, x_t.rows, dy_t.k
     if not dy_t.is_cuda:
         A, B = mxfp8.dequantize(dy_t), mxfp8.dequantize(x_t)
         s = seg.tolist()
+        if not accumulate:
+            out.zero_()
         for e in range(n_experts):
             out[e] += (A[:, s[e]:s[e + 1]] @ B[:, s[e]:s[e + 1]].t()).to(out.dtype)
         return out
     call("b200_gemm_grouped_mx_wgrad", ptr(dy_t.q), ptr(dy_t.sf), ptr(x_t.q), ptr(x_t.sf), ptr(out), ptr(seg), T, M, N,
-         n_experts, dy_t.q.stride(0), x_t.q.stride(0), int(out.dtype == torch.float32), 1, 1.0, stream_ptr())
+         n_experts, dy_t.q.stride(0), x_t.q.stride(0), int(out.dtype == torch.float32), int(accumulate), 1.0, stream_ptr())
     return out
 
 
@@ -401,6 +426,10 @@ def _wgrad_into_mx(param, dy_t, x_t, seg, E):
     if mg is not None:
         grouped_wgrad_mx(dy_t, x_t, seg, E, mg)
         return None
+    if dy_t.is_cuda and param.dtype in (torch.bfloat16, torch.float32):
+        # rounded once from the accumulators: no fp32 copy of the expert weights to clear, add into and convert
+        out = torch.empty((E, dy_t.rows, x_t.rows), dtype=param.dtype, device=dy_t.q.device)
+        return grouped_wgrad_mx(dy_t, x_t, seg, E, out, accumulate=False)
     out = torch.zeros((E, dy_t.rows, x_t.rows), dtype=torch.float32, device=dy_t.q.device)
     return grouped_wgrad_mx(dy_t, x_t, seg, E, out).to(param.dtype)
 
@@ -428,14 +457,14 @@ def _zero_padding(t: torch.Tensor, tile_expert: torch.Tensor) -> torch.Tensor:
     return t.masked_fill(dead[:, None], 0)
 
 
-def _wgrad_into(param, dy, x, seg, E):
+def _wgrad_into(param, dy, x, seg, E, pad=PAD):
     mg = getattr(param, "main_grad", None)
     if not param.requires_grad:
         return None
     if mg is not None:
-        grouped_wgrad(dy, x, seg, E, out=mg, accumulate=True)
+        grouped_wgrad(dy, x, seg, E, out=mg, accumulate=True, pad=pad)
         return None
-    return grouped_wgrad(dy, x, seg, E, out_dtype=param.dtype)
+    return grouped_wgrad(dy, x, seg, E, out_dtype=param.dtype, pad=pad)
 
 
 def expert_precision(precision: str, w1, w2) -> str:
@@ -453,7 +482,8 @@ def moe_experts(x, idx, w, counts, w1, w2, precision: str = "bf16"):
     T, k = idx.shape
     E = w1.shape[0]
     precision = expert_precision(precision, w1, w2)
-    seg, tile_expert, dest, rows = plan(idx, counts, E, pad=pad_rows(precision))
+    pad = PAD_MX if precision == "bf16" and pair_rows_ok(x, w1, w2) else pad_rows(precision)
+    seg, tile_expert, dest, rows = plan(idx, counts, E, pad=pad)
     xp = PermuteFn.apply(x, dest, k, rows)
     yp = grouped_mlp(xp, w1, w2, seg, tile_expert, precision)
     return UnpermuteFn.apply(yp, dest, w, T, k)

@@ -114,24 +114,28 @@ B200_DEVICE float gelu_tanh_grad(float x) {
   const float th = tanhf(k * (x + 0.044715f * x * x * x));
   return 0.5f * (1.f + th) + 0.5f * x * (1.f - th * th) * k * (1.f + 3.f * 0.044715f * x * x);
 }
-__global__ void gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n8) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
+// rows x vpr vectors of 8; pitches in elements (a plain tensor is one row)
+__global__ void gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, __nv_bfloat16* __restrict__ y, long long ldy,
+                                long long total, long long vpr) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / vpr, c = (i - r * vpr) * 8;
     float a[8], o[8];
-    ld8(x + i * 8, a);
+    ld8(x + r * ldx + c, a);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = gelu_tanh(a[j]);
-    st8(y + i * 8, o);
+    st8(y + r * ldy + c, o);
   }
 }
-__global__ void gelu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                                __nv_bfloat16* __restrict__ dx, long long n8) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
+__global__ void gelu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long long ldg, const __nv_bfloat16* __restrict__ x, long long ldx,
+                                __nv_bfloat16* __restrict__ dx, long long ldd, long long total, long long vpr) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const long long r = i / vpr, c = (i - r * vpr) * 8;
     float a[8], d[8], o[8];
-    ld8(x + i * 8, a);
-    ld8(dy + i * 8, d);
+    ld8(x + r * ldx + c, a);
+    ld8(dy + r * ldg + c, d);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = d[j] * gelu_tanh_grad(a[j]);
-    st8(dx + i * 8, o);
+    st8(dx + r * ldd + c, o);
   }
 }
 
@@ -241,15 +245,15 @@ B200_API int b200_swiglu_bwd(const void* da, const void* gu, void* dgu, long lon
 B200_API int b200_gelu_fwd(const void* x, void* y, long long n, void* stream) {
   if (n % 8 != 0) return b200::fail(402, "gelu: n=%lld must be a multiple of 8", n);
   if (n == 0) return 0;
-  gelu_fwd_kernel<<<grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, n / 8);
+  gelu_fwd_kernel<<<grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, n, (__nv_bfloat16*)y, n, n / 8, n / 8);
   b200::count_launch();
   return b200::check_launch("gelu_fwd");
 }
 B200_API int b200_gelu_bwd(const void* dy, const void* x, void* dx, long long n, void* stream) {
   if (n % 8 != 0) return b200::fail(402, "gelu: n=%lld must be a multiple of 8", n);
   if (n == 0) return 0;
-  gelu_bwd_kernel<<<grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
-                                                                         (__nv_bfloat16*)dx, n / 8);
+  gelu_bwd_kernel<<<grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dy, n, (const __nv_bfloat16*)x, n,
+                                                                            (__nv_bfloat16*)dx, n, n / 8, n / 8);
   b200::count_launch();
   return b200::check_launch("gelu_bwd");
 }
@@ -285,4 +289,24 @@ B200_API int b200_accum_f32_bf16(float* acc, const void* src, long long n, void*
   accum_f32_bf16_kernel<<<grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>(acc, (const __nv_bfloat16*)src, n / 8);
   b200::count_launch();
   return b200::check_launch("accum_f32_bf16");
+}
+
+// GELU on [rows, cols] blocks of wider matrices (pitches in elements, multiples of 8 like cols).
+B200_API int b200_gelu_fwd_rows(const void* x, long long ldx, void* y, long long ldy, long long rows, long long cols, void* stream) {
+  if (cols % 8 != 0 || ldx % 8 != 0 || ldy % 8 != 0) return b200::fail(402, "gelu_rows: %lld columns, pitches %lld / %lld (x8)", cols, ldx, ldy);
+  if (rows == 0 || cols == 0) return 0;
+  gelu_fwd_kernel<<<grid_for(rows * (cols / 8), 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)y, ldy,
+                                                                                     rows * (cols / 8), cols / 8);
+  b200::count_launch();
+  return b200::check_launch("gelu_fwd_rows");
+}
+B200_API int b200_gelu_bwd_rows(const void* dy, long long ldg, const void* x, long long ldx, void* dx, long long ldd, long long rows,
+                                long long cols, void* stream) {
+  if (cols % 8 != 0 || ldg % 8 != 0 || ldx % 8 != 0 || ldd % 8 != 0)
+    return b200::fail(402, "gelu_rows: %lld columns, pitches %lld / %lld / %lld (x8)", cols, ldg, ldx, ldd);
+  if (rows == 0 || cols == 0) return 0;
+  gelu_bwd_kernel<<<grid_for(rows * (cols / 8), 256), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)dy, ldg, (const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)dx, ldd, rows * (cols / 8), cols / 8);
+  b200::count_launch();
+  return b200::check_launch("gelu_bwd_rows");
 }

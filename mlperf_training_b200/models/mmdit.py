@@ -184,18 +184,24 @@ class DoubleBlock(nn.Module):
         for s, x in (("img", img), ("txt", txt)):
             mod = getattr(self, f"{s}_mod")(vec_act).chunk(6, dim=-1)
             qkv = getattr(self, f"{s}_qkv")(_ln_modulate(x, mod[0], mod[1], B), pr)
-            S = x.shape[0] // B
-            q, k, v = qkv.view(B, S, 3, H, hd).unbind(2)
-            q, k = getattr(self, f"{s}_qknorm")(q, k)
-            parts[s] = (q, k, v, mod, S)
-        St = parts["txt"][4]
-        q = _rope(torch.cat([parts["txt"][0], parts["img"][0]], 1), cos, sin)
-        k = _rope(torch.cat([parts["txt"][1], parts["img"][1]], 1), cos, sin)
-        v = torch.cat([parts["txt"][2], parts["img"][2]], 1)
-        attn = _attention(q, k, v, self.sp)
+            parts[s] = (qkv, mod, x.shape[0] // B)
+        St, Si = parts["txt"][2], parts["img"][2]
+        streams = [(parts[s][0], getattr(self, f"{s}_qknorm").q_scale, getattr(self, f"{s}_qknorm").k_scale) for s in ("txt", "img")]
+        if F.qkv_norm_rope_ok(cos, hd, streams):
+            q, k, v = F.qkv_norm_rope(streams, cos, sin, B, H, hd)
+        else:
+            qkvs = {}
+            for s in ("txt", "img"):
+                q, k, v = parts[s][0].view(B, parts[s][2], 3, H, hd).unbind(2)
+                qkvs[s] = (*getattr(self, f"{s}_qknorm")(q, k), v)
+            q = _rope(torch.cat([qkvs["txt"][0], qkvs["img"][0]], 1), cos, sin)
+            k = _rope(torch.cat([qkvs["txt"][1], qkvs["img"][1]], 1), cos, sin)
+            v = torch.cat([qkvs["txt"][2], qkvs["img"][2]], 1)
+        # (one split: its backward is a single concatenation)
+        a_txt, a_img = _attention(q, k, v, self.sp).split([St, Si], dim=1)
         outs = {}
-        for s, x, a in (("txt", txt, attn[:, :St]), ("img", img, attn[:, St:])):
-            mod = parts[s][3]
+        for s, x, a in (("txt", txt, a_txt), ("img", img, a_img)):
+            mod = parts[s][1]
             a2 = a.reshape(-1, H * hd)
             x = _gate(x, getattr(self, f"{s}_proj")(a2, pr), mod[2], B)
             h = F.gelu(getattr(self, f"{s}_fc1")(_ln_modulate(x, mod[3], mod[4], B), pr))
@@ -220,11 +226,16 @@ class SingleBlock(nn.Module):
         shift, scale, gate = self.mod(vec_act).chunk(3, dim=-1)
         y = self.linear1(_ln_modulate(x, shift, scale, B), pr)
         S = x.shape[0] // B
-        qkv, mlp = y[:, :3 * d], y[:, 3 * d:]
-        q, k, v = qkv.reshape(B, S, 3, H, hd).unbind(2)
-        q, k = self.qknorm(q, k)
-        attn = _attention(_rope(q, cos, sin), _rope(k, cos, sin), v.contiguous(), self.sp).reshape(-1, d)
-        out = self.linear2(torch.cat([attn, F.gelu(mlp.contiguous())], dim=-1), pr)
+        if F.qkv_norm_rope_ok(cos, hd, [(y, self.qknorm.q_scale, self.qknorm.k_scale)]) and y.shape[1] % 8 == 0:
+            q, k, v, act = F.single_stream_in(y, self.qknorm.q_scale, self.qknorm.k_scale, cos, sin, B, H, hd)
+            attn = _attention(q, k, v, self.sp).reshape(-1, d)
+        else:
+            qkv, mlp = y[:, :3 * d], y[:, 3 * d:]
+            q, k, v = qkv.reshape(B, S, 3, H, hd).unbind(2)
+            q, k = self.qknorm(q, k)
+            attn = _attention(_rope(q, cos, sin), _rope(k, cos, sin), v.contiguous(), self.sp).reshape(-1, d)
+            act = F.gelu(mlp.contiguous())
+        out = self.linear2(torch.cat([attn, act], dim=-1), pr)
         return _gate(x, out, gate, B)
 
 

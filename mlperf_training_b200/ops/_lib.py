@@ -83,6 +83,10 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_ln_modulate_bwd": [P, P, P, L, P, P, P, P, P, I, I, I, P],
         "b200_gate_residual_fwd": [P, P, P, L, P, I, I, I, P],
         "b200_gate_residual_bwd": [P, P, P, L, P, P, I, I, I, P],
+        "b200_qk_norm_rope_fwd": [P, L, P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, P],
+        "b200_qk_norm_rope_bwd": [P, P, P, P, L, P, P, P, P, P, P, L, P, P, I, I, I, I, I, I, P],
+        "b200_gelu_fwd_rows": [P, L, P, L, L, L, P],
+        "b200_gelu_bwd_rows": [P, L, P, L, P, L, L, L, P],
         "b200_sort_ids": [P, P, P, L, I, P, L, P],
         "b200_unique_segments": [P, P, L, P, P, P, P, P, L, P],
         "b200_segment_sum_gather": [P, I, L, P, P, P, L, L, I, P, I, P, P],
@@ -131,6 +135,9 @@ def _declare(lib: ctypes.CDLL) -> None:
     if hasattr(lib, "b200_gemm_grouped_mx_bn"):
         lib.b200_gemm_grouped_mx_bn.argtypes = [I]
         lib.b200_gemm_grouped_mx_bn.restype = c_int
+    if hasattr(lib, "b200_qk_norm_rope_scratch_elems"):
+        lib.b200_qk_norm_rope_scratch_elems.argtypes = [I, I, I, I]
+        lib.b200_qk_norm_rope_scratch_elems.restype = c_ll
     for name in ("b200_gemm_bf16_workspace", "b200_gemm_mxfp8_workspace"):
         if hasattr(lib, name):
             getattr(lib, name).argtypes = [I, I, I]

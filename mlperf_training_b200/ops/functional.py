@@ -635,6 +635,108 @@ def rope_bshd(x, cos, sin):
     return RopeBSHDFn.apply(x, cos, sin)
 
 
+def qkv_norm_rope_ok(cos, head_dim: int, parts) -> bool:
+    """Whether ``[(qkv, q_scale, k_scale), ...]`` run on the fused kernel: bf16 rows of ``[3][H][head_dim]`` on the GPU, 16-byte
+    aligned, head dim 64 or 128, fp32 tables."""
+    return head_dim in (64, 128) and cos.dtype == torch.float32 and all(
+        use_kernels(x) and x.dtype == qs.dtype == ks.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1
+        and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and qs.data_ptr() % 16 == 0 and ks.data_ptr() % 16 == 0
+        for x, qs, ks in parts)
+
+
+def _qk_fwd(x, qs, ks, cos, sin, q, k, v, s_off, B, eps):
+    _, S, H, D = q.shape
+    if cos.shape[0] < S or cos.shape[1] * 2 != D:
+        raise ValueError(f"rotary tables {tuple(cos.shape)} for {S} tokens of head dim {D}")
+    rstd = torch.empty((x.shape[0], 2, H), dtype=torch.float32, device=x.device)
+    call("b200_qk_norm_rope_fwd", ptr(x), x.stride(0), ptr(qs), ptr(ks), ptr(cos), ptr(sin), ptr(q), ptr(k), ptr(v), ptr(rstd), B,
+         x.shape[0] // B, S, s_off, H, D, float(eps), stream_ptr())
+    return rstd
+
+
+def _qk_bwd(dq, dk, dv, x, qs, ks, cos, sin, rstd, dx, s_off, B):
+    from . import _lib
+    _, S, H, D = dq.shape
+    s_part = x.shape[0] // B
+    dscale = torch.empty((2, D), dtype=torch.float32, device=x.device)
+    scratch = torch.empty(int(_lib.load().b200_qk_norm_rope_scratch_elems(B, s_part, H, D)), dtype=torch.float32, device=x.device)
+    call("b200_qk_norm_rope_bwd", ptr(dq), ptr(dk), ptr(dv), ptr(x), x.stride(0), ptr(qs), ptr(ks), ptr(cos), ptr(sin), ptr(rstd),
+         ptr(dx), dx.stride(0), ptr(dscale), ptr(scratch), B, s_part, S, s_off, H, D, stream_ptr())
+    return dscale
+
+
+class QKVNormRopeFn(Function):
+    """Joint ``q, k, v [B, S, H, D]`` of one or several token streams from their fused projections ``[B S_i, 3 H D]``: per-head
+    RMS norm of q and k with the stream's scales, rotary embedding by joint position, concatenation along the tokens."""
+
+    @staticmethod
+    def forward(ctx, cos, sin, B, H, D, eps, *flat):
+        parts = [flat[i:i + 3] for i in range(0, len(flat), 3)]
+        cos, sin = cos.contiguous(), sin.contiguous()
+        S = sum(x.shape[0] for x, _, _ in parts) // B
+        q, k, v = (torch.empty((B, S, H, D), dtype=flat[0].dtype, device=flat[0].device) for _ in range(3))
+        off, saved = 0, []
+        for x, qs, ks in parts:
+            saved += [x, qs, ks, _qk_fwd(x, qs, ks, cos, sin, q, k, v, off, B, eps)]
+            off += x.shape[0] // B
+        ctx.save_for_backward(cos, sin, *saved)
+        ctx.B = B
+        ctx.refs = [(qs, ks) for _, qs, ks in parts]
+        return q, k, v
+
+    @staticmethod
+    def backward(ctx, dq, dk, dv):
+        cos, sin, *saved = ctx.saved_tensors
+        dq, dk, dv = dq.contiguous(), dk.contiguous(), dv.contiguous()
+        out, off = [], 0
+        for (pq, pk), i in zip(ctx.refs, range(0, len(saved), 4)):
+            x, qs, ks, rstd = saved[i:i + 4]
+            dx = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+            ds = _qk_bwd(dq, dk, dv, x, qs, ks, cos, sin, rstd, dx, off, ctx.B)
+            off += x.shape[0] // ctx.B
+            out += [dx, _vec_grad(pq, ds[0]), _vec_grad(pk, ds[1])]
+        return (None, None, None, None, None, None, *out)
+
+
+def qkv_norm_rope(parts, cos, sin, B, H, D, eps=1e-6):
+    return QKVNormRopeFn.apply(cos, sin, B, H, D, eps, *[t for p in parts for t in p])
+
+
+class SingleStreamInFn(Function):
+    """``q, k, v`` (as ``QKVNormRopeFn``) and ``gelu(mlp)`` from the fused projection ``y = [qkv | mlp]`` of a single-stream
+    block; backward fills one gradient of ``y`` instead of adding two zero-padded ones."""
+
+    @staticmethod
+    def forward(ctx, y, q_scale, k_scale, cos, sin, B, H, D, eps):
+        cos, sin = cos.contiguous(), sin.contiguous()
+        n = 3 * H * D
+        T, M = y.shape[0], y.shape[1] - n
+        q, k, v = (torch.empty((B, T // B, H, D), dtype=y.dtype, device=y.device) for _ in range(3))
+        rstd = _qk_fwd(y, q_scale, k_scale, cos, sin, q, k, v, 0, B, eps)
+        act = torch.empty((T, M), dtype=y.dtype, device=y.device)
+        call("b200_gelu_fwd_rows", ptr(y[:, n:]), y.stride(0), ptr(act), M, T, M, stream_ptr())
+        ctx.save_for_backward(y, q_scale, k_scale, cos, sin, rstd)
+        ctx.cfg = (B, n)
+        ctx.refs = (q_scale, k_scale)
+        return q, k, v, act
+
+    @staticmethod
+    def backward(ctx, dq, dk, dv, dact):
+        y, q_scale, k_scale, cos, sin, rstd = ctx.saved_tensors
+        B, n = ctx.cfg
+        dy = torch.empty(y.shape, dtype=y.dtype, device=y.device)
+        ds = _qk_bwd(dq.contiguous(), dk.contiguous(), dv.contiguous(), y, q_scale, k_scale, cos, sin, rstd, dy, 0, B)
+        if dact.stride(1) != 1 or dact.stride(0) % 8 or dact.data_ptr() % 16:
+            dact = dact.contiguous()
+        call("b200_gelu_bwd_rows", ptr(dact), dact.stride(0), ptr(y[:, n:]), y.stride(0), ptr(dy[:, n:]), dy.stride(0), y.shape[0],
+             y.shape[1] - n, stream_ptr())
+        return dy, _vec_grad(ctx.refs[0], ds[0]), _vec_grad(ctx.refs[1], ds[1]), None, None, None, None, None, None
+
+
+def single_stream_in(y, q_scale, k_scale, cos, sin, B, H, D, eps=1e-6):
+    return SingleStreamInFn.apply(y, q_scale, k_scale, cos, sin, B, H, D, eps)
+
+
 # --------------------------------------------------------------------------------------
 # MoE router projection
 # --------------------------------------------------------------------------------------

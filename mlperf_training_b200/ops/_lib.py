@@ -198,13 +198,16 @@ def use_kernels(t: torch.Tensor) -> bool:
     """Dispatch rule of every op: CUDA tensors run the sm_100a kernels (and fail loudly when
     the library is absent); CPU tensors run the eager PyTorch definition of the same op."""
     if t.is_cuda:
-        require()
+        if _lib is None:
+            require()
         return True
     return False
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Raw handle of the calling thread's current stream on its current device.  (``torch.cuda.current_stream()`` builds a
+    Stream object through several Python layers: 4 us of each launch.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t: torch.Tensor | None) -> int | None:
@@ -212,10 +215,9 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 
 def call(name: str, *args) -> None:
-    lib = load()
-    rc = getattr(lib, name)(*args)
+    rc = getattr(_lib if _lib is not None else load(), name)(*args)
     if rc != 0:
-        msg = lib.b200_last_error().decode(errors="replace")
+        msg = load().b200_last_error().decode(errors="replace")
         raise RuntimeError(f"{name} failed with code {rc}: {msg}")
 
 
@@ -228,7 +230,7 @@ def _gemm_workspace_bytes(entry: str, M: int, N: int, K: int, device: int) -> in
 def gemm_workspace(entry: str, M: int, N: int, K: int, device: torch.device) -> torch.Tensor | None:
     """Scratch for the split last wave of a GEMM (None: the problem is not split).  It comes from torch's allocator on the
     calling stream, so it is given back when the call returns and reused in stream order."""
-    n = _gemm_workspace_bytes(entry, M, N, K, device.index if device.index is not None else torch.cuda.current_device())
+    n = _gemm_workspace_bytes(entry, M, N, K, device.index if device.index is not None else torch._C._cuda_getDevice())
     return torch.empty(n, dtype=torch.uint8, device=device) if n else None
 
 

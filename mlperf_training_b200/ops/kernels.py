@@ -24,7 +24,8 @@ def _row_major(t: torch.Tensor) -> torch.Tensor:
     if t.dim() != 2:
         raise ValueError(f"expected a 2-D tensor, got shape {tuple(t.shape)}")
     esz = t.element_size()
-    if t.stride(1) != 1 or (t.stride(0) * esz) % 16 != 0 or t.data_ptr() % 16 != 0 or t.stride(0) < t.shape[1]:
+    pitch, inner = t.stride()
+    if inner != 1 or (pitch * esz) % 16 != 0 or t.data_ptr() % 16 != 0 or pitch < t.shape[1]:
         per16 = 16 // esz
         cols = (t.shape[1] + per16 - 1) // per16 * per16
         if cols == t.shape[1]:

@@ -113,8 +113,8 @@ B200_DEVICE long long run_of(const long long* __restrict__ seg, long long total,
 // partial[b][0] = sum of the long run that holds position b * SEG_CHUNK over its positions inside block b;
 // partial[b][1] = the same for the long run that holds the block's last position, when that is another run.
 __global__ void __launch_bounds__(256)
-segment_partial_kernel(RowSrc s, const long long* __restrict__ seg, const long long* __restrict__ n_seg, long long n,
-                       float* __restrict__ partial, int* status) {
+segment_partial_kernel(RowSrc s, const long long* __restrict__ seg, const long long* __restrict__ n_seg,
+                       const long long* __restrict__ inverse, long long n, float* __restrict__ partial, int* status) {
   const long long total = *n_seg;
   if (total <= 0) return;
   const int lane = threadIdx.x & 31;
@@ -122,7 +122,10 @@ segment_partial_kernel(RowSrc s, const long long* __restrict__ seg, const long l
   const long long p0 = b * SEG_CHUNK;
   if (p0 >= n) return;
   const long long p1 = p0 + SEG_CHUNK < n ? p0 + SEG_CHUNK : n;
-  const long long s0 = run_of(seg, total, p0), s1 = run_of(seg, total, p1 - 1);
+  // the runs of the block's ends: two dependent loads through the sort's inverse map, a search over the offsets without it
+  const bool mapped = inverse != nullptr && s.perm != nullptr;
+  const long long s0 = mapped ? inverse[s.perm[p0]] : run_of(seg, total, p0);
+  const long long s1 = mapped ? inverse[s.perm[p1 - 1]] : run_of(seg, total, p1 - 1);
   const int nvec = s.D / 8;
   for (int slot = 0; slot < 2; ++slot) {
     const long long run = slot == 0 ? s0 : s1;
@@ -157,11 +160,25 @@ segment_sum_gather_kernel(RowSrc s, const long long* __restrict__ seg, const lon
       if (hi - lo <= SEG_CHUNK || partial == nullptr) {
         sum_positions(acc, s, lo, hi, v, status);
       } else {
-        for (long long b = lo / SEG_CHUNK; b * SEG_CHUNK < hi; ++b) {
-          const int slot = b * SEG_CHUNK >= lo ? 0 : 1;   // the run holds the block's first position, or starts inside it
-          const float* src = partial + ((b * 2 + slot) * s.D + v * 8);
-          const float4 a = *reinterpret_cast<const float4*>(src), c = *reinterpret_cast<const float4*>(src + 4);
-          acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w; acc[4] += c.x; acc[5] += c.y; acc[6] += c.z; acc[7] += c.w;
+        // (the partial sums of the most frequent id are the longest chain of the launch: four rows of them in flight)
+        for (long long b0 = lo / SEG_CHUNK; b0 * SEG_CHUNK < hi; b0 += 4) {
+          float4 a[4], c[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const long long b = b0 + j;
+            if (b * SEG_CHUNK < hi) {
+              const int slot = b * SEG_CHUNK >= lo ? 0 : 1;   // the run holds the block's first position, or starts inside it
+              const float* src = partial + ((b * 2 + slot) * s.D + v * 8);
+              a[j] = *reinterpret_cast<const float4*>(src);
+              c[j] = *reinterpret_cast<const float4*>(src + 4);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if ((b0 + j) * SEG_CHUNK < hi) {
+              acc[0] += a[j].x; acc[1] += a[j].y; acc[2] += a[j].z; acc[3] += a[j].w;
+              acc[4] += c[j].x; acc[5] += c[j].y; acc[6] += c[j].z; acc[7] += c[j].w;
+            }
         }
       }
       if constexpr (sizeof(Out) == 2) {
@@ -245,11 +262,12 @@ B200_API long long b200_segment_sum_scratch_elems(long long n, int D) {
 
 // out[s, :] = sum of src[perm[r], :] over the sorted positions r of run s, s < *n_seg (device scalar), summed in a
 // fixed order.  src: bf16 or fp32 [src_rows, D]; perm [n] (null: identity); seg [*n_seg + 1] run offsets; out
-// [max_seg, D] bf16 or fp32; partial: b200_segment_sum_scratch_elems(n, D) floats (null: every run is summed by one
+// [max_seg, D] bf16 or fp32 (runs only: rows past *n_seg are not written); inverse [n]: run of every original position
+// (b200_unique_segments), or null; partial: b200_segment_sum_scratch_elems(n, D) floats (null: every run is summed by one
 // warp, whatever its length).
 B200_API int b200_segment_sum_gather(const void* src, int src_is_f32, long long src_rows, const long long* perm,
-                                     const long long* seg, const long long* n_seg, long long n, long long max_seg, int D,
-                                     void* out, int out_bf16, float* partial, void* stream) {
+                                     const long long* seg, const long long* n_seg, const long long* inverse, long long n,
+                                     long long max_seg, int D, void* out, int out_bf16, float* partial, void* stream) {
   if (max_seg <= 0 || n <= 0) return 0;
   if (D % 8 != 0 || ((uintptr_t)src & 15) || ((uintptr_t)out & 15) || ((uintptr_t)partial & 15))
     return b200::fail(1605, "segment_sum_gather: D=%d must be a multiple of 8 and the matrices 16-byte aligned", D);
@@ -260,7 +278,7 @@ B200_API int b200_segment_sum_gather(const void* src, int src_is_f32, long long 
   cudaStream_t st = (cudaStream_t)stream;
   if (partial != nullptr) {
     const long long blocks = (n + SEG_CHUNK - 1) / SEG_CHUNK;
-    segment_partial_kernel<<<(unsigned)((blocks + 7) / 8), 256, 0, st>>>(s, seg, n_seg, n, partial, b200::status_ptr());
+    segment_partial_kernel<<<(unsigned)((blocks + 7) / 8), 256, 0, st>>>(s, seg, n_seg, inverse, n, partial, b200::status_ptr());
     b200::count_launch();
     int rc = b200::check_launch("segment_partial");
     if (rc) return rc;

@@ -82,11 +82,12 @@ def sort_unique(ids: torch.Tensor, key_bits: int = 64) -> SortedIds:
     return SortedIds(keys, perm, uniq, seg, inverse, count)
 
 
-def segment_sum(src: torch.Tensor, s: SortedIds, out_dtype=torch.float32, max_seg: int | None = None) -> torch.Tensor:
+def segment_sum(src: torch.Tensor, s: SortedIds, out_dtype=torch.float32, max_seg: int | None = None, clear: bool = True) -> torch.Tensor:
     """``out[j] = sum of src[p] over the original positions p whose id is the j-th unique id`` (sorted
-    order inside a run).  Returns ``[n, D]`` rows (the first ``count`` are valid; the rest untouched zeros)."""
+    order inside a run).  Returns ``[n, D]`` rows (the first ``count`` are valid; the rest zeros, or
+    with ``clear=False`` whatever the allocator gave: for consumers that skip them)."""
     n, D = s.keys.numel(), src.shape[1]
-    out = torch.zeros((n if max_seg is None else max_seg, D), dtype=out_dtype, device=src.device)
+    out = (torch.zeros if clear or not use_kernels(src) else torch.empty)((n if max_seg is None else max_seg, D), dtype=out_dtype, device=src.device)
     if n == 0:
         return out
     if not use_kernels(src):
@@ -101,5 +102,5 @@ def segment_sum(src: torch.Tensor, s: SortedIds, out_dtype=torch.float32, max_se
     # partial sums of the runs that are too long for one warp (skewed ids): one fp32 row pair per 64 sorted positions
     partial = torch.empty(int(_lib.load().b200_segment_sum_scratch_elems(n, D)), dtype=torch.float32, device=src.device)
     call("b200_segment_sum_gather", ptr(src.contiguous()), int(src.dtype == torch.float32), src.shape[0], ptr(s.perm), ptr(s.seg), ptr(s.count),
-         n, out.shape[0], D, ptr(out), int(out_dtype == torch.bfloat16), ptr(partial), stream_ptr())
+         ptr(s.inverse), n, out.shape[0], D, ptr(out), int(out_dtype == torch.bfloat16), ptr(partial), stream_ptr())
     return out

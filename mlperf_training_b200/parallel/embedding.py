@@ -75,6 +75,10 @@ class ShardedEmbedding:
     def _route(self, ids: torch.Tensor):
         """Dedup + bucketise.  Returns ``(uniq_sorted_by_owner, inverse, send_counts [W], sorted)``."""
         srt = S.sort_unique(ids, S.key_bits_for(self.rows))                      # sorted ids = sorted by owner
+        if self.world == 1:
+            n_u = srt.n_unique()                                                 # the lookup's one host read
+            self._last_counts = [n_u]
+            return srt.uniq[:n_u], srt.inverse, srt.count, srt
         n = ids.numel()
         valid = torch.arange(n, device=ids.device) < srt.count
         own = torch.bucketize(srt.uniq, self.bounds[1:], right=True).clamp(max=self.world - 1)
@@ -157,7 +161,8 @@ class ShardedEmbedding:
         if grad.dtype not in (torch.bfloat16, torch.float32):
             grad = grad.float()
         # 1. duplicates of this rank: one row per unique id, summed in sorted (fixed) order, in the wire dtype
-        g_u = S.segment_sum(grad, srt, out_dtype=wire if self.world > 1 else torch.float32, max_seg=uniq.numel())
+        g_u = S.segment_sum(grad, srt, out_dtype=wire if self.world > 1 else torch.float32, max_seg=uniq.numel(),
+                            clear=self.world > 1)                 # (one rank: the update below skips entries past the runs)
         # 2. to the owners
         if self.world > 1:
             recv = torch.empty((sum(out_splits), self.dim), dtype=wire, device=grad.device)
@@ -259,9 +264,17 @@ def load_matching(state: dict, path) -> list:
 class _LookupFn(Function):
     @staticmethod
     def forward(ctx, ids, table: ShardedEmbedding, _anchor, plan=None):
-        rows_u, st = table._forward_rows(ids.reshape(-1), plan)
-        ctx.table, ctx.state = table, st
-        return rows_u[st[1]]
+        ids = ids.reshape(-1)
+        ctx.table = table
+        if plan is None and table.world == 1 and ids.is_cuda and table.weight.dtype == torch.bfloat16:
+            # one rank: nothing crosses ranks, so the rows come straight from the table in the ids' order and the number of
+            # unique ids, which sizes nothing then, stays on the device (entries of uniq past it are -1 and are skipped)
+            srt = S.sort_unique(ids, S.key_bits_for(table.rows))
+            ctx.state = (srt.uniq, srt.inverse, srt.uniq, None, None, srt)
+            return K.gather_rows(table.weight, ids)
+        rows_u, st = table._forward_rows(ids, plan)
+        ctx.state = st
+        return K.gather_rows(rows_u, st[1]) if rows_u.is_cuda and rows_u.shape[1] % 8 == 0 and rows_u.dtype == torch.bfloat16 else rows_u[st[1]]
 
     @staticmethod
     def backward(ctx, grad):

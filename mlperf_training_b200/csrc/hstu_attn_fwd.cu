@@ -24,6 +24,11 @@
 // its row layout [keys][head dim] and is consumed as an MN-major operand.  This is the forward of the
 // reference's production path (generative_recommenders/ops/flydsl/hstu_fwd.py:150, e4m3 forward).
 //
+// What bounds it: per pair of 128 x 128 tiles 2048 tensor-core cycles against 2048 of the MUFU unit (one tanh per score)
+// and the hand-overs between them (3500 cycles measured).  Scores come 64 columns per TMEM round trip, P V starts on the
+// first half of the keys, and the latest query tiles of all sequences go first.  128 users of median 512 tokens, 4 heads:
+// 728 -> 497 us; 12 users of median 700: 271 -> 204 us (rolled 32-column chunks, sequence after sequence before).
+//
 // Math oracle: generative_recommenders/ops/pytorch/pt_hstu_attention.py:33-84,130-187; the
 // reference's production kernels are generative_recommenders/ops/flydsl/hstu_fwd.py and
 // generative_recommenders/ops/triton/triton_hstu_attention.py (_hstu_attn_fwd).
@@ -61,7 +66,7 @@ B200_DEVICE uint32_t pack4_e4m3(float a, float b, float c, float d) {
 
 B200_DEVICE float tanh_approx(float x) {
   float y;
-  asm volatile("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
@@ -96,13 +101,15 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint64_t* s_full = bars + 9;      // 2 (per query tile)
   uint64_t* p_full = bars + 11;     // 2 (per query tile, 4 arrivals)
   uint64_t* o_done = bars + 13;     // 2 (per query tile)
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* p_early = bars + 15;    // 2 (per query tile, 4 arrivals): the first half of the keys of P
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_pairs = (p.max_len + 2 * BQ - 1) / (2 * BQ);
-  const int pair = num_pairs - 1 - (int)blockIdx.x;  // heaviest (latest) query tiles first
-  const int h = blockIdx.y, b = blockIdx.z;
+  // heaviest (latest) query tiles of all sequences first: a long sequence late in the batch used to run alone at the end
+  const int pair = num_pairs - 1 - (int)blockIdx.y;
+  const int h = (int)blockIdx.x % p.H, b = (int)blockIdx.x / p.H;
   const int row_base = p.offsets[b];
   const int len = p.offsets[b + 1] - row_base;
   const int q0 = pair * 2 * BQ;
@@ -130,7 +137,7 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
       mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_done[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_done[i], 1); mbar_init(&p_early[i], 4);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -212,7 +219,7 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (!ok || n >= n_t[t]) continue;
-          ok = mbar_wait_spin(&p_full[t], n & 1, abort_flag, p.status, 53);
+          ok = mbar_wait_spin(&p_early[t], n & 1, abort_flag, p.status, 53);
           if (ok && v_ready < n) {
             ok = mbar_wait_spin(&v_full[st], (n >> 1) & 1, abort_flag, p.status, 54);
             v_ready = n;
@@ -220,15 +227,25 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           if (!ok) continue;
           tc_fence_after();
           const bool last_user = (t == 1) || !(n < n_t[1]);
+          const uint64_t bd = dV + (st * SM::KV_BYTES >> 4);
+          // A = P_t in TMEM: 32 bytes of keys (8 columns) per step; B = V: that many key rows of 128 bytes
+          constexpr int STEPS = BKV * SM::ES / 32;
+          auto pv = [&](int kk) {
+            const uint32_t acc = (n > 0 || kk > 0) ? 1u : 0u, o = kk * (32 / SM::ES) * 128 >> 4;
+            if constexpr (F8) tc_mma_f8_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8, bd + o, idesc_o, acc);
+            else tc_mma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8, bd + o, idesc_o, acc);
+          };
           if (elect_one()) {
-            // A = P_t in TMEM: 32 bytes of keys (8 columns) per step; B = V: that many key rows of 128 bytes
-            const uint64_t bd = dV + (st * SM::KV_BYTES >> 4);
 #pragma unroll
-            for (int kk = 0; kk < BKV * SM::ES / 32; ++kk) {
-              const uint32_t acc = (n > 0 || kk > 0) ? 1u : 0u, o = kk * (32 / SM::ES) * 128 >> 4;
-              if constexpr (F8) tc_mma_f8_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8, bd + o, idesc_o, acc);
-              else tc_mma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8, bd + o, idesc_o, acc);
-            }
+            for (int kk = 0; kk < STEPS / 2; ++kk) pv(kk);
+          }
+          __syncwarp();
+          ok = mbar_wait_spin(&p_full[t], n & 1, abort_flag, p.status, 55);
+          if (!ok) continue;
+          tc_fence_after();
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = STEPS / 2; kk < STEPS; ++kk) pv(kk);
             tc_commit(&o_done[t]);
             if (last_user) tc_commit(&v_empty[st]);
           }
@@ -266,46 +283,56 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int last_k_id = min(max(kv0 + BKV - 1 - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
       const bool inside = (kv0 + BKV <= len) && (qt0 + BQ <= len);
       const bool need_mask = plain ? ((kv0 + BKV - 1 > qt0) || !inside) : !(inside && first_q_id > last_k_id);
-#pragma unroll 1
-      for (int c = 0; c < BKV / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(ts + c * 32, v);
+      // 64 columns at a time, unrolled: two TMEM loads in flight, and independent activations to cover each other's latency
+      // (32 columns in a rolled loop waited for one load and one chain at a time)
+      const float2 ha2 = make_float2(half_alpha, half_alpha), in2 = make_float2(inv_n, inv_n);
+#pragma unroll
+      for (int c = 0; c < BKV / 64; ++c) {
+        uint32_t v[64];
+        tmem_ld_32x32b_x32(ts + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+        tmem_ld_32x32b_x32(ts + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
         tc_wait_ld();
-        uint32_t pk[16];
-        float xf[F8 ? 32 : 1];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          // silu(a x) / N = (a x / 2)(1 + tanh(a x / 2)) / N
-          const float h0 = __uint_as_float(v[2 * i]) * half_alpha, h1 = __uint_as_float(v[2 * i + 1]) * half_alpha;
-          float x0 = h0 * (1.f + tanh_approx(h0)) * inv_n, x1 = h1 * (1.f + tanh_approx(h1)) * inv_n;
-          if (need_mask) {
-            const int kp = kv0 + c * 32 + 2 * i;
+        for (int i = 0; i < 32; ++i) {
+          // silu(a x) / N = (a x / 2) / N * (1 + tanh(a x / 2))
+          const float2 hx = fmul2(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), ha2);
+          const float2 hn = fmul2(hx, in2);
+          const float2 x = ffma2(hn, make_float2(tanh_approx(hx.x), tanh_approx(hx.y)), hn);
+          v[2 * i] = __float_as_uint(x.x);
+          v[2 * i + 1] = __float_as_uint(x.y);
+        }
+        if (need_mask) {
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int kpe = kp + e;
-              bool vis;
-              if (plain) vis = kpe <= q_pos;
-              else {
-                const int k_id = min(max(kpe - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
-                vis = (kpe == q_pos) || (q_id > k_id) || (ctx > 0 && q_id == 0 && kpe < hist_end);
-              }
-              vis = vis && kpe < len && q_pos < len;
-              if (!vis) { if (e == 0) x0 = 0.f; else x1 = 0.f; }
+          for (int i = 0; i < 64; ++i) {
+            const int kpe = kv0 + c * 64 + i;
+            bool vis;
+            if (plain) vis = kpe <= q_pos;
+            else {
+              const int k_id = min(max(kpe - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
+              vis = (kpe == q_pos) || (q_id > k_id) || (ctx > 0 && q_id == 0 && kpe < hist_end);
             }
-          }
-          if constexpr (F8) {
-            xf[2 * i] = x0; xf[2 * i + 1] = x1;
-          } else {
-            pk[i] = pack_bf16x2(x0, x1);
+            if (!(vis && kpe < len && q_pos < len)) v[i] = 0u;
           }
         }
         if constexpr (F8) {
-          uint32_t p8[8];                                  // keys 4 j .. 4 j + 3 of the chunk in column j
+          uint32_t p8[16];                                 // keys 4 j .. 4 j + 3 of the chunk in column j
 #pragma unroll
-          for (int j = 0; j < 8; ++j) p8[j] = pack4_e4m3(xf[4 * j], xf[4 * j + 1], xf[4 * j + 2], xf[4 * j + 3]);
-          tmem_st_32x32b_x8(ts + c * 8, p8);
+          for (int j = 0; j < 16; ++j)
+            p8[j] = pack4_e4m3(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]),
+                               __uint_as_float(v[4 * j + 3]));
+          tmem_st_32x32b_x16(ts + c * 16, p8);
         } else {
-          tmem_st_32x32b_x16(ts + c * 16, pk);
+          uint32_t pk[32];
+#pragma unroll
+          for (int i = 0; i < 32; ++i) pk[i] = pack_bf16x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+          tmem_st_32x32b_x32(ts + c * 32, pk);
+        }
+        if (c == 0) {
+          // the second GEMM starts on the first half of the keys
+          tc_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&p_early[t]);
         }
       }
       tc_wait_st();
@@ -358,7 +385,7 @@ int launch_hstu_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensor
     if (e != cudaSuccess) { cudaGetLastError(); return b200::fail(1201, "hstu_attn_fwd: cannot set %d bytes of shared memory: %s", SM::TOTAL, cudaGetErrorString(e)); }
     configured[dev & 63] = true;
   }
-  dim3 grid((p.max_len + 2 * BQ - 1) / (2 * BQ), p.H, B);
+  dim3 grid((unsigned)(p.H * B), (p.max_len + 2 * BQ - 1) / (2 * BQ));
   hstu_attn_fwd_kernel<HD, F8><<<grid, NTHREADS, SM::TOTAL, stream>>>(tq, tk, tv, p);
   b200::count_launch();
   return b200::check_launch("hstu_attn_fwd");

@@ -247,7 +247,7 @@ static int run_pair(const void* a, const void* b, void* d, int M, int N, int K, 
 // (gemm_core.cuh: SplitArgs); 0 where that does not pay.  The call accepts none, too.
 B200_API long long b200_gemm_bf16_workspace(int M, int N, int K) {
   using namespace gemmcore;
-  if (M <= 128 || N <= 0 || K <= 0 || !pair_enabled()) return 0;
+  if (M <= 0 || N <= 0 || K <= 0 || (M <= 128 && N <= 128) || !pair_enabled()) return 0;
   int rc = 0;
   return N > 128 ? split_bytes<256>(pair_split<KIND_BF16, 256, 1>(M, N, K, rc)) : split_bytes<128>(pair_split<KIND_BF16, 128, 1>(M, N, K, rc));
 }
@@ -261,7 +261,17 @@ B200_API int b200_gemm_bf16(const void* a, const void* b, void* d, int M, int N,
                             int accumulate, const void* bias, const void* residual, long long ldr, float alpha,
                             void* workspace, long long workspace_bytes, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return b200::fail(210, "gemm_bf16: empty problem %d x %d x %d", M, N, K);
-  const int BN = (N > 128) ? 256 : 128;
+  // At most 128 rows: bound by reading B once, so as many CTAs as there are columns for - a split along K over CTA pairs
+  // where there are few column tiles, else one CTA per 128 columns unless 256 fill the chip.  Measured, one CTA per 256
+  // columns -> now: 8 x 3072 x 18432 (MN-major B) 119 -> 40 us, 16 x 4096 x 8192 (both MN-major) 61 -> 32, 128 x 4096 x 4096
+  // 36 -> 25, 128 x 14336 x 4096 47 -> 39, 8 x 18432 x 3072 41 -> 39.
+  bool pair = M > 128;
+  if (!pair && N > 128 && workspace != nullptr) {
+    int rc = 0;
+    pair = gemmcore::pair_split<gemmcore::KIND_BF16, 256, 1>(M, N, K, rc).rem > 0;
+    if (rc) return rc;
+  }
+  const int BN = (N > 128 && (pair || (long long)N > 256ll * (b200::sm_count() - 1))) ? 256 : 128;
   gemmcore::EpiArgs epi = {};
   epi.M = M; epi.N = N;
   epi.out_f32 = out_f32 ? 1 : 0; epi.accumulate = accumulate ? 1 : 0;
@@ -269,7 +279,7 @@ B200_API int b200_gemm_bf16(const void* a, const void* b, void* d, int M, int N,
   epi.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
   epi.ldr = ldr;
   epi.alpha = alpha;
-  if (M > 128 && gemmcore::pair_enabled()) {
+  if (pair && gemmcore::pair_enabled()) {
     if (BN == 256) return run_pair<256>(a, b, d, M, N, K, lda, ldb, ldd, a_mn_major ? 1 : 0, b_mn_major ? 1 : 0, epi,
                                         workspace, workspace_bytes, (cudaStream_t)stream);
     return run_pair<128>(a, b, d, M, N, K, lda, ldb, ldd, a_mn_major ? 1 : 0, b_mn_major ? 1 : 0, epi,

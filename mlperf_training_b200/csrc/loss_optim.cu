@@ -108,12 +108,36 @@ template <typename G>
 __global__ void __launch_bounds__(256)
 sumsq_partial_kernel(const G* __restrict__ g, long long n, float* __restrict__ partial) {
   __shared__ float red[8];
-  float acc = 0.f;
-  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
-    float v;
-    if constexpr (sizeof(G) == 2) v = __bfloat162float(g[i]); else v = g[i];
-    acc += v * v;
+  // 16-byte loads, four in flight per thread (one 4-byte load at a time read 3.6 TB/s: 525 M fp32 550 -> 335 us)
+  constexpr int PER = 16 / sizeof(G);
+  const long long stride = (long long)gridDim.x * 256, first = blockIdx.x * 256ll + threadIdx.x;
+  float part[4] = {0.f, 0.f, 0.f, 0.f};
+  const long long nv = (reinterpret_cast<uintptr_t>(g) & 15) == 0 ? n / PER : 0;
+  auto add = [&](float& s, const uint4& u) {
+    if constexpr (sizeof(G) == 2) {
+      const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
+      s += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y + c.x * c.x + c.y * c.y + d.x * d.x + d.y * d.y;
+    } else {
+      const float a = __uint_as_float(u.x), b = __uint_as_float(u.y), c = __uint_as_float(u.z), d = __uint_as_float(u.w);
+      s += a * a + b * b + c * c + d * d;
+    }
+  };
+  const uint4* gv = reinterpret_cast<const uint4*>(g);
+  long long i = first;
+  for (; i + 3 * stride < nv; i += 4 * stride) {
+    uint4 u[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) u[j] = gv[i + j * stride];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) add(part[j], u[j]);
   }
+  for (; i < nv; i += stride) add(part[0], gv[i]);
+  for (long long k = nv * PER + first; k < n; k += stride) {
+    float v;
+    if constexpr (sizeof(G) == 2) v = __bfloat162float(g[k]); else v = g[k];
+    part[0] += v * v;
+  }
+  float acc = (part[0] + part[1]) + (part[2] + part[3]);
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();

@@ -68,3 +68,20 @@ def test_mxfp8(M, N, Kd, mode):
         want = want + out.double()
         _check(MX.gemm(qa, qb, out=out, accumulate=True), want, Kd)
     _lib.check_status("split gemm")
+
+
+@pytest.mark.parametrize("M", [1, 8, 16, 100, 128])
+@pytest.mark.parametrize("N,Kd", [(136, 4096), (512, 512), (3072, 9216), (4096, 4104), (38400, 64)])
+@pytest.mark.parametrize("mode", ["plain", "dgrad", "f32_accumulate"])
+def test_few_rows(M, N, Kd, mode):
+    """At most 128 rows: split over CTA pairs, 128- and 256-column tiles of one CTA."""
+    torch.manual_seed(M + N)
+    a, b, kw = _rand(M, Kd), _rand(N, Kd), {}
+    want = a.double() @ b.double().t()
+    if mode == "dgrad":
+        b, kw = b.t().contiguous(), dict(b_mn_major=True)
+    elif mode == "f32_accumulate":
+        kw = dict(out=torch.randn(M, N, device="cuda"), accumulate=True)
+        want = want + kw["out"].double()
+    _check(K.gemm(a, b, **kw), want, Kd)
+    _lib.check_status("few rows")

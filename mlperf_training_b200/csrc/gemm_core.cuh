@@ -379,7 +379,8 @@ struct SplitArgs {
 
 // Chooses S for `tiles` tiles of `num_kb` k stages of `stage_us` microseconds on P pairs; partial tiles of `tile_bytes`.
 // Estimated time of the last wave: rounds of slices, plus the partial tiles written and read once (6 TB/s, out of L2)
-// and 5 us for the second launch; the split is taken when that is 5 % less than the unsplit wave.  Measured on 74
+// and 5 us for the second launch; the split is taken when it saves 5 % of the whole launch (behind nine full waves
+// it measured 0 to 2 %, and the sums of split tiles come in another order).  Measured on 74
 // pairs, L2 flushed, without -> with the split (M x N x K):
 //   bf16   2048 x 512 x 92160 456 -> 144 us;  512 x 1536 x 92160 457 -> 112;  2048 x 3072 x 12288 131 -> 105;
 //          4011 x 4096 x 14336 341 -> 290;  256 x 3072 x 12288 68 -> 38;  2000 x 5120 x 2880 68 -> 54
@@ -389,12 +390,13 @@ inline SplitArgs split_plan(int tiles, int num_kb, double stage_us, double tile_
   SplitArgs best = {tiles, 0, 1, num_kb};
   const int first = tiles / P * P, rem = tiles - first;
   if (rem == 0) return best;
-  double best_us = num_kb * stage_us;
+  const double wave_us = num_kb * stage_us;
+  double best_us = wave_us - 0.05 * (tiles / P + 1) * wave_us;
   for (int S = 2; S <= 16 && num_kb / S >= 4; ++S) {
     const int per = (num_kb + S - 1) / S;
     if ((S - 1) * per >= num_kb) continue;             // every slice needs work: its partial tile is read
     const double us = (double)((rem * S + P - 1) / P) * per * stage_us + 2.0 * rem * S * tile_bytes / 6e6 + 5.0;
-    if (us < 0.95 * best_us) { best_us = us; best = {first, rem, S, per}; }
+    if (us < best_us) { best_us = us; best = {first, rem, S, per}; }
   }
   return best;
 }

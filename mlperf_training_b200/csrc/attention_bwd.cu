@@ -6,16 +6,21 @@
 //   dQ = dS K   (TMEM -> fp32 TMA reduce-add into a global fp32 dQ buffer)
 //   dV += P^T dO          dK += dS^T Q                  (stay in TMEM for the whole CTA)
 //
-// P and dS are written once to shared memory as [query][key] bf16 tiles and read by the tensor
-// core both key-contiguous (for dQ) and as MN-major operands (P^T, dS^T) through the UMMA
-// descriptor, so no transposed copies are made.  dK / dV leave as bf16 through TMA stores.
+// The scores are computed transposed, S^T = K Q^T and dP^T = V dO^T, so a worker thread owns a key row.  P^T goes back to
+// TMEM over its own scores (tcgen05.st) and is the TMEM operand of dV; only dS^T is written to shared memory, once, as a
+// [key][query] bf16 tile that the tensor core reads key-major for dK and, through an MN-major descriptor, transposed for
+// dQ.  The log-sum-exp and delta of the tile's queries run along the columns: they are staged in shared memory.  dK / dV
+// leave as bf16 through TMA stores.
 //
-// 320 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 workers.  Two workers share a
-// TMEM lane quarter (32 query rows): each computes P / dS for half of the 128 key columns, then
-// drains half of the dQ columns (TMEM -> registers, accumulator released, registers -> fp32 TMA
-// reduce-add while the next S / dP GEMMs run).  A quarter of the exponentials is evaluated with a
-// polynomial on the FMA pipe: 128 x 128 exp2 per tile would otherwise cost 1024 cycles of the
-// 16-per-clock special-function unit alone.  TMEM (512 columns): S/dQ | dP | dK | dV.
+// 320 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 workers.  Two workers share a TMEM lane quarter (32 key
+// rows): each takes half of the 128 query columns, then drains half of the dQ columns (TMEM -> registers, accumulator
+// released, registers -> fp32 TMA reduce-add).  A quarter of the exponentials is evaluated with a polynomial on the FMA
+// pipe.  TMEM (512 columns): S^T / P^T | dP^T, then dQ | dK | dV.  Order of the MMAs of step i, Q double-buffered:
+//     [P^T(i) written]  dV(i)   [dS^T(i) written]  dQ(i)  S(i+1)  dK(i)  [dQ(i) drained]  dP(i+1)
+// so the workers drain dQ(i) and exponentiate S(i+1) while the tensor core runs dK(i) and dP(i+1).
+// Measured with delta, clearing and launches (queries as rows, P and dS through shared memory, one Q stage -> this):
+// 8192 x 32 / 8 heads of 128 causal 1990 -> 1766 us, 4096 x 64 / 8 1130 -> 1005, 4 x 2048 607 -> 550, 2000 x 64 / 8 of 64
+// 448 -> 378, 8 x 512 x 24 full 175 -> 157.
 //
 // The reference takes this kernel from Primus-Turbo / AITER / CK (config knobs
 // llama2_sft/primus/config_MI355X_1x8x1.sh:35-39); there is no in-tree counterpart.
@@ -27,7 +32,7 @@ namespace {
 constexpr int BQ = 128;
 constexpr int BKV = 128;
 constexpr int NTHREADS = 320;
-constexpr int STG = 4096;  // dQ staging chunk: 32 rows x 32 fp32
+constexpr int STG = 4096;  // dQ staging chunk: 32 rows x 32 fp32 (one per worker)
 #ifndef B200_ATTN_BWD_POLY
 #define B200_ATTN_BWD_POLY 6
 #endif
@@ -63,10 +68,13 @@ B200_DEVICE void tma_reduce_add_4d(const CUtensorMap* map, const void* src, int 
 
 template <int HD>
 struct Smem {
-  static constexpr int T_BYTES = 128 * HD * 2;        // K, V, Q, dO tiles
-  static constexpr int PS_BYTES = BQ * BKV * 2;       // P, dS tiles
-  static constexpr int STG_BYTES = 4 * 2 * STG;
-  static constexpr int TOTAL = 4 * T_BYTES + 2 * PS_BYTES + STG_BYTES + 1024 + 256;
+  static constexpr int T_BYTES = 128 * HD * 2;        // K, V, Q (two stages), dO tiles
+  static constexpr int DS_BYTES = BQ * BKV * 2;       // dS^T tile
+  static constexpr int STG_BYTES = 8 * STG;
+  static constexpr int LD_BYTES = 2 * 2 * BQ * 4;     // log-sum-exp and delta of two query tiles
+  // The base of dynamic shared memory is 1024-byte aligned when a kernel has no static shared memory; checked at entry
+  // (at head dim 128 there is no room to align it).
+  static constexpr int TOTAL = 5 * T_BYTES + DS_BYTES + STG_BYTES + LD_BYTES + 256;
 };
 
 template <int HD>
@@ -77,26 +85,34 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 const __grid_constant__ CUtensorMap tmdV, const BwdParams p) {
   using SM = Smem<HD>;
   constexpr int NB = HD / 64;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sK = smem;
   uint8_t* sV = sK + SM::T_BYTES;
-  uint8_t* sQ = sV + SM::T_BYTES;
-  uint8_t* sdO = sQ + SM::T_BYTES;
-  uint8_t* sP = sdO + SM::T_BYTES;
-  uint8_t* sdS = sP + SM::PS_BYTES;
-  uint8_t* sStg = sdS + SM::PS_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStg + SM::STG_BYTES);
+  uint8_t* sQ = sV + SM::T_BYTES;           // two stages
+  uint8_t* sdO = sQ + 2 * SM::T_BYTES;
+  uint8_t* sdS = sdO + SM::T_BYTES;
+  uint8_t* sStg = sdS + SM::DS_BYTES;
+  float* sLD = reinterpret_cast<float*>(sStg + SM::STG_BYTES);   // [stage][lse2 | delta * scale][128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sLD + 4 * BQ);
   uint64_t* kv_full = bars + 0;     // K and V landed
-  uint64_t* qdo_full = bars + 1;    // Q_i and dO_i landed
-  uint64_t* qdo_empty = bars + 2;   // MMAs reading Q_i / dO_i / P / dS finished
-  uint64_t* sdp_full = bars + 3;    // S and dP complete in TMEM
-  uint64_t* pds_full = bars + 4;    // P and dS written to shared memory (4 arrivals)
-  uint64_t* dq_full = bars + 5;     // dQ tile complete in TMEM
-  uint64_t* dq_drained = bars + 6;  // dQ tile copied out of TMEM (4 arrivals)
-  uint64_t* acc_done = bars + 7;    // every MMA of this CTA finished
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 8);
+  uint64_t* q_full = bars + 1;      // 2: Q_i landed
+  uint64_t* q_empty = bars + 3;     // 2: MMAs reading Q_i finished
+  uint64_t* do_full = bars + 5;     // dO_i landed
+  uint64_t* do_empty = bars + 6;    // MMAs reading dO_i finished
+  uint64_t* s_full = bars + 7;      // S^T complete in TMEM
+  uint64_t* dp_full = bars + 8;     // dP^T complete in TMEM (and every MMA of the step before: dS^T is free)
+  uint64_t* p_full = bars + 9;      // P^T written to TMEM (8 arrivals)
+  uint64_t* ds_full = bars + 10;    // dS^T written to shared memory (8 arrivals)
+  uint64_t* dq_full = bars + 11;    // dQ tile complete in TMEM
+  uint64_t* dq_drained = bars + 12; // dQ tile copied out of TMEM (8 arrivals)
+  uint64_t* ld_full = bars + 13;    // 2: the step's log-sum-exp / delta are in shared memory (8 arrivals)
+  uint64_t* acc_done = bars + 15;   // every MMA of this CTA finished
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
+  if (smem_u32(smem) & 1023u) {             // (the same for every thread of the launch)
+    if (threadIdx.x == 0) b200_report(p.status, B200_ERR_BOUNDS, 94);
+    return;
+  }
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_kt = (p.Skv + BKV - 1) / BKV;
@@ -124,8 +140,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int n_iter = n_q * group;
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1); mbar_init(qdo_full, 1); mbar_init(qdo_empty, 1); mbar_init(sdp_full, 1);
-    mbar_init(pds_full, 8); mbar_init(dq_full, 1); mbar_init(dq_drained, 8); mbar_init(acc_done, 1);
+    mbar_init(kv_full, 1); mbar_init(do_full, 1); mbar_init(do_empty, 1); mbar_init(s_full, 1); mbar_init(dp_full, 1);
+    mbar_init(p_full, 8); mbar_init(ds_full, 8); mbar_init(dq_full, 1); mbar_init(dq_drained, 8); mbar_init(acc_done, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); mbar_init(&ld_full[i], 8); }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -134,8 +151,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  const uint32_t tm_S = tmem_base;          // S, later dQ (128 columns)
-  const uint32_t tm_dP = tmem_base + 128;
+  const uint32_t tm_S = tmem_base;          // S^T; P^T of queries 0-63 in columns 0-31, of 64-127 in 64-95
+  const uint32_t tm_dP = tmem_base + 128;   // dP^T, later dQ
   const uint32_t tm_dK = tmem_base + 256;
   const uint32_t tm_dV = tmem_base + 384;
 
@@ -149,17 +166,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tma_load_4d(sK + i * (BKV * 128), &tmK, kv_full, i * 64, hk, kv0, b);
         tma_load_4d(sV + i * (BKV * 128), &tmV, kv_full, i * 64, hk, kv0, b);
       }
-      bool ok = true;
-      for (int it = 0; it < n_iter && ok; ++it) {
+      for (int it = 0; it < n_iter; ++it) {
         const int h = hk * group + it / n_q;
         const int q0 = (i_lo + it % n_q) * BQ;
-        if (!mbar_wait(qdo_empty, (it & 1) ^ 1, abort_flag, p.status, 70)) { ok = false; break; }
-        mbar_expect_tx(qdo_full, 2 * SM::T_BYTES);
+        const int st = it & 1;
+        if (!mbar_wait(&q_empty[st], ((it >> 1) & 1) ^ 1, abort_flag, p.status, 70)) break;
+        mbar_expect_tx(&q_full[st], SM::T_BYTES);
 #pragma unroll
-        for (int i = 0; i < NB; ++i) {
-          tma_load_4d(sQ + i * (BQ * 128), &tmQ, qdo_full, i * 64, h, q0, b);
-          tma_load_4d(sdO + i * (BQ * 128), &tmdO, qdo_full, i * 64, h, q0, b);
-        }
+        for (int i = 0; i < NB; ++i) tma_load_4d(sQ + st * SM::T_BYTES + i * (BQ * 128), &tmQ, &q_full[st], i * 64, h, q0, b);
+        if (!mbar_wait(do_empty, (it & 1) ^ 1, abort_flag, p.status, 71)) break;
+        mbar_expect_tx(do_full, SM::T_BYTES);
+#pragma unroll
+        for (int i = 0; i < NB; ++i) tma_load_4d(sdO + i * (BQ * 128), &tmdO, do_full, i * 64, h, q0, b);
       }
     }
   } else if (warp == 1) {
@@ -167,149 +185,206 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     // The warp stays converged and one elected lane issues: operands live in uniform registers and descriptors advance by
     // an addition (rebuilt by one lane of a divergent warp they cost more than the 64 cycles an instruction runs).
     if (n_iter > 0) {
-      const uint32_t id_kk = umma_idesc(1, 1, 0, 0, 128, 128);   // S = Q K^T, dP = dO V^T (both K-major)
-      const uint32_t id_dq = umma_idesc(1, 1, 0, 1, 128, HD);    // dQ = dS (K-major) x K (MN-major)
-      const uint32_t id_tt = umma_idesc(1, 1, 1, 1, 128, HD);    // dV = P^T dO, dK = dS^T Q (both MN-major)
+      const uint32_t id_kk = umma_idesc(1, 1, 0, 0, 128, 128);   // S^T = K Q^T, dP^T = V dO^T (both K-major)
+      const uint32_t id_dv = umma_idesc(1, 1, 0, 1, 128, HD);    // dV = P^T (TMEM) x dO (MN-major)
+      const uint32_t id_dk = umma_idesc(1, 1, 0, 1, 128, HD);    // dK = dS^T (K-major) x Q (MN-major)
+      const uint32_t id_dq = umma_idesc(1, 1, 1, 1, 128, HD);    // dQ = dS (the tile read MN-major) x K (MN-major)
       const uint64_t kK = umma_desc_sw128(smem_u32(sK), 16, 1024), kV = umma_desc_sw128(smem_u32(sV), 16, 1024);
       const uint64_t kQ = umma_desc_sw128(smem_u32(sQ), 16, 1024), kdO = umma_desc_sw128(smem_u32(sdO), 16, 1024);
-      const uint64_t kdS = umma_desc_sw128(smem_u32(sdS), 16, 1024);
+      const uint64_t kdS = umma_desc_sw128(smem_u32(sdS), 16, 1024), mdS = umma_desc_sw128(smem_u32(sdS), 128 * 128, 1024);
       const uint64_t mK = umma_desc_sw128(smem_u32(sK), 128 * 128, 1024), mQ = umma_desc_sw128(smem_u32(sQ), 128 * 128, 1024);
-      const uint64_t mdO = umma_desc_sw128(smem_u32(sdO), 128 * 128, 1024), mP = umma_desc_sw128(smem_u32(sP), 128 * 128, 1024);
-      const uint64_t mdS = umma_desc_sw128(smem_u32(sdS), 128 * 128, 1024);
-      bool ok = mbar_wait_spin(kv_full, 0, abort_flag, p.status, 80);
+      const uint64_t mdO = umma_desc_sw128(smem_u32(sdO), 128 * 128, 1024);
+      auto issue_s = [&](int it) -> bool {
+        const int st = it & 1;
+        if (!mbar_wait_spin(&q_full[st], (it >> 1) & 1, abort_flag, p.status, 81)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t bd = kQ + (st * SM::T_BYTES >> 4);
+#pragma unroll
+          for (int kk = 0; kk < HD / 16; ++kk) {
+            const uint32_t o = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
+            tc_mma_f16_ss(tm_S, kK + o, bd + o, id_kk, kk > 0);
+          }
+          tc_commit(s_full);
+        }
+        __syncwarp();
+        return true;
+      };
+      auto issue_dp = [&](int it) -> bool {
+        if (!mbar_wait_spin(do_full, it & 1, abort_flag, p.status, 82)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < HD / 16; ++kk) {
+            const uint32_t o = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
+            tc_mma_f16_ss(tm_dP, kV + o, kdO + o, id_kk, kk > 0);
+          }
+          tc_commit(dp_full);
+        }
+        __syncwarp();
+        return true;
+      };
+      bool ok = mbar_wait_spin(kv_full, 0, abort_flag, p.status, 80) && issue_s(0) && issue_dp(0);
       for (int it = 0; it < n_iter && ok; ++it) {
         const uint32_t ph = it & 1;
-        if (!mbar_wait_spin(qdo_full, ph, abort_flag, p.status, 81)) { ok = false; break; }
-        tc_fence_after();
-        // S = Q K^T ; dP = dO V^T   (contraction over the head dim, both operands K-major)
-        // dP first: its accumulator was read by the workers long ago, so these MMAs run while the workers
-        // still drain dQ of the previous iteration out of the S / dQ columns
-        if (elect_one()) {
-#pragma unroll
-          for (int kk = 0; kk < HD / 16; ++kk) {
-            const uint32_t o = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
-            tc_mma_f16_ss(tm_dP, kdO + o, kV + o, id_kk, kk > 0);
-          }
-        }
-        __syncwarp();
-        if (it > 0 && !mbar_wait_spin(dq_drained, (it - 1) & 1, abort_flag, p.status, 82)) { ok = false; break; }
+        const int st = it & 1;
+        const bool last = it == n_iter - 1;
+        if (!mbar_wait_spin(p_full, ph, abort_flag, p.status, 83)) { ok = false; break; }
         tc_fence_after();
         if (elect_one()) {
-#pragma unroll
-          for (int kk = 0; kk < HD / 16; ++kk) {
-            const uint32_t o = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
-            tc_mma_f16_ss(tm_S, kQ + o, kK + o, id_kk, kk > 0);
-          }
-          tc_commit(sdp_full);
-        }
-        __syncwarp();
-        if (!mbar_wait_spin(pds_full, ph, abort_flag, p.status, 83)) { ok = false; break; }
-        tc_fence_after();
-        if (elect_one()) {
-          // dV += P^T dO ; dK += dS^T Q : contraction over queries, both operands MN-major
+          // dV += P^T dO : 16 queries = 8 TMEM columns per step, dO as 16 query rows of 128 bytes
 #pragma unroll
           for (int kk = 0; kk < BQ / 16; ++kk)
-            tc_mma_f16_ss(tm_dV, mP + kk * 128, mdO + kk * 128, id_tt, (it > 0 || kk > 0));
+            tc_mma_f16_ts(tm_dV, tm_S + (kk / 4) * 64 + (kk % 4) * 8, mdO + kk * 128, id_dv, (it > 0 || kk > 0));
+          tc_commit(do_empty);
+        }
+        __syncwarp();
+        if (!mbar_wait_spin(ds_full, ph, abort_flag, p.status, 84)) { ok = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
+          // dQ = dS K : contraction over keys, 16 key rows of the dS^T tile and of K per step
 #pragma unroll
-          for (int kk = 0; kk < BQ / 16; ++kk)
-            tc_mma_f16_ss(tm_dK, mdS + kk * 128, mQ + kk * 128, id_tt, (it > 0 || kk > 0));
-          tc_commit(qdo_empty);  // Q_i / dO_i may be overwritten: the next tiles load during the dQ GEMM
-          // dQ = dS K : A = dS [q][key] K-major, B = K [key][d] MN-major (contraction over keys)
+          for (int kk = 0; kk < BKV / 16; ++kk) tc_mma_f16_ss(tm_dP, mdS + kk * 128, mK + kk * 128, id_dq, kk > 0);
+          tc_commit(dq_full);
+        }
+        __syncwarp();
+        if (!last && !issue_s(it + 1)) { ok = false; break; }     // (P^T(i) was read by dV(i), issued before)
+        if (elect_one()) {
+          // dK += dS^T Q : contraction over queries
+          const uint64_t bd = mQ + (st * SM::T_BYTES >> 4);
 #pragma unroll
-          for (int kk = 0; kk < BKV / 16; ++kk) {
+          for (int kk = 0; kk < BQ / 16; ++kk) {
             const uint32_t ao = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
-            tc_mma_f16_ss(tm_S, kdS + ao, mK + kk * 128, id_dq, kk > 0);
+            tc_mma_f16_ss(tm_dK, kdS + ao, bd + kk * 128, id_dk, (it > 0 || kk > 0));
           }
-          tc_commit(dq_full);    // also: P / dS shared-memory tiles are free again
-          if (it == n_iter - 1) tc_commit(acc_done);
+          tc_commit(&q_empty[st]);
+          if (last) tc_commit(acc_done);
         }
         __syncwarp();
+        if (!last) ok = mbar_wait_spin(dq_drained, ph, abort_flag, p.status, 85) && issue_dp(it + 1);
       }
     }
   } else {
     // ------------------------------ workers: P / dS, then dQ drain ------------------------------
     const int q = warp & 3;                   // TMEM lane quarter
-    const int half = (warp - 2) >> 2;         // which half of the key columns / of the dQ columns
-    const int r = q * 32 + lane;
+    const int half = (warp - 2) >> 2;         // which half of the query columns / of the dQ columns
+    const int r = q * 32 + lane;              // key row of the tile (dQ drain: query row)
     const uint32_t lane_base = uint32_t(q * 32) << 16;
     uint8_t* stg = sStg + (warp - 2) * STG;   // one staging buffer per worker
     constexpr int CH = HD / 64;               // dQ chunks (32 columns) per worker
+    const int key = kv0 + r;
+    // this thread stages one value per step: the log-sum-exp (half 0) or delta (half 1) of query r of the tile
+    auto fetch = [&](int it) -> float {
+      const int q_pos = (i_lo + it % n_q) * BQ + r;
+      if (q_pos >= p.Sq) return half == 0 ? INFINITY : 0.f;      // P = exp2(s - inf) = 0 for rows that are not there
+      const long long idx = ((long long)b * p.Hq + hk * group + it / n_q) * p.Sq + q_pos;
+      if (half == 1) return p.delta[idx] * p.scale;
+      const float l = p.lse[idx];
+      return l == -INFINITY ? INFINITY : l * 1.4426950408889634f;   // a row without any visible key
+    };
     bool ok = true;
+    if (n_iter > 0) {
+      sLD[half * BQ + r] = fetch(0);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ld_full[0]);
+    }
     for (int it = 0; it < n_iter && ok; ++it) {
       const int h = hk * group + it / n_q;
       const int q0 = (i_lo + it % n_q) * BQ;
-      const int q_pos = q0 + r;
-      float lse2 = 0.f, dl = 0.f;
-      bool row_ok = q_pos < p.Sq;
-      if (row_ok) {
-        const long long idx = ((long long)b * p.Hq + h) * p.Sq + q_pos;
-        lse2 = p.lse[idx] * 1.4426950408889634f;
-        dl = p.delta[idx];
-        if (lse2 == -INFINITY) row_ok = false;  // row without any visible key
-      }
+      const float next = it + 1 < n_iter ? fetch(it + 1) : 0.f;
       const bool need_mask = (kv0 + BKV > p.Skv) || (p.causal && kv0 + BKV - 1 > q0 + off) ||
-                             (p.window > 0 && kv0 < q0 + BQ - 1 + off - p.window + 1) || (q0 + BQ > p.Sq) ||
-                             __any_sync(0xffffffffu, !row_ok);
-      const int hi = p.causal ? min(q_pos + off, p.Skv - 1) : p.Skv - 1;
-      const int lo = p.window > 0 ? q_pos + off - p.window + 1 : 0;
-      if (!mbar_wait(sdp_full, it & 1, abort_flag, p.status, 90)) { ok = false; break; }
+                             (p.window > 0 && kv0 < q0 + BQ - 1 + off - p.window + 1);
+      // visible queries of this key: columns [c_lo, c_hi)
+      int c_lo = 0, c_hi = BQ;
+      if (p.causal) c_lo = key - off - q0;
+      if (p.window > 0) c_hi = key - off - q0 + p.window;
+      if (key >= p.Skv) c_hi = c_lo = 0;
+      if (!mbar_wait(&ld_full[it & 1], (it >> 1) & 1, abort_flag, p.status, 89)) { ok = false; break; }
+      const float* ld = sLD + (it & 1) * 2 * BQ + half * 64;
+      if (!mbar_wait(s_full, it & 1, abort_flag, p.status, 90)) { ok = false; break; }
       tc_fence_after();
-      // the P / dS tiles are free: this warp waited for dq_full of the previous iteration in its drain step
-      uint8_t* prow = sP + r * 128;
-      uint8_t* drow = sdS + r * 128;
-#pragma unroll 1
-      for (int c = half * 2; c < half * 2 + 2; ++c) {
-        uint32_t s[32], d[32];
-        tmem_ld_32x32b_x32(tm_S + lane_base + c * 32, s);
-        tmem_ld_32x32b_x32(tm_dP + lane_base + c * 32, d);
+      float pr[64];
+      {
+        uint32_t s[64];
+        tmem_ld_32x32b_x32(tm_S + lane_base + half * 64, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
+        tmem_ld_32x32b_x32(tm_S + lane_base + half * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&s[32]));
         tc_wait_ld();
-        float pv[32], dv[32];
-        const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nl2 = make_float2(-lse2, -lse2);
-        const float2 s2 = make_float2(p.scale, p.scale), nd2 = make_float2(-dl * p.scale, -dl * p.scale);
+        const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float2 a = ffma2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), sc2, nl2);
-          float2 e;
-          if ((i & POLY) == POLY) e = ex2_poly2(a);
-          else e = make_float2(ex2_approx(a.x), ex2_approx(a.y));
-          float p0 = e.x, p1 = e.y;
-          if (need_mask) {
-            const int kp = kv0 + c * 32 + i;
-            if (!row_ok || kp > hi || kp < lo) p0 = 0.f;
-            if (!row_ok || kp + 1 > hi || kp + 1 < lo) p1 = 0.f;
-          }
-          const float2 t2 = ffma2(make_float2(__uint_as_float(d[i]), __uint_as_float(d[i + 1])), s2, nd2);
-          const float2 g2 = fmul2(make_float2(p0, p1), t2);
-          pv[i] = p0; pv[i + 1] = p1;
-          dv[i] = g2.x; dv[i + 1] = g2.y;
+        for (int i = 0; i < 64; i += 4) {
+          const float4 l4 = *reinterpret_cast<const float4*>(ld + i);
+          const float2 a = ffma2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), sc2, make_float2(-l4.x, -l4.y));
+          const float2 c = ffma2(make_float2(__uint_as_float(s[i + 2]), __uint_as_float(s[i + 3])), sc2, make_float2(-l4.z, -l4.w));
+          float2 e0, e1;
+          if ((i & POLY) == POLY) e0 = ex2_poly2(a);
+          else e0 = make_float2(ex2_approx(a.x), ex2_approx(a.y));
+          if (((i + 2) & POLY) == POLY) e1 = ex2_poly2(c);
+          else e1 = make_float2(ex2_approx(c.x), ex2_approx(c.y));
+          pr[i] = e0.x; pr[i + 1] = e0.y; pr[i + 2] = e1.x; pr[i + 3] = e1.y;
         }
-        uint8_t* pb = prow + (c / 2) * (BQ * 128);
-        uint8_t* db = drow + (c / 2) * (BQ * 128);
+      }
+      if (need_mask) {
+#pragma unroll
+        for (int i = 0; i < 64; ++i) {
+          const int col = half * 64 + i;
+          if (col < c_lo || col >= c_hi) pr[i] = 0.f;
+        }
+      }
+      {
+        uint32_t pk[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) pk[i] = pack_bf16x2(pr[2 * i], pr[2 * i + 1]);
+        tmem_st_32x32b_x32(tm_S + lane_base + half * 64, pk);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+      }
+      if (!mbar_wait(dp_full, it & 1, abort_flag, p.status, 91)) { ok = false; break; }
+      tc_fence_after();
+      uint8_t* drow = sdS + half * (BKV * 128) + r * 128;       // 64 queries of key r
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t d[32];
+        tmem_ld_32x32b_x32(tm_dP + lane_base + half * 64 + c * 32, d);
+        tc_wait_ld();
+        const float2 s2 = make_float2(p.scale, p.scale);
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
-          const int sw = (((c & 1) * 4 + g) ^ (r & 7)) << 4;
-          *reinterpret_cast<uint4*>(pb + sw) =
-              make_uint4(pack_bf16x2(pv[8 * g], pv[8 * g + 1]), pack_bf16x2(pv[8 * g + 2], pv[8 * g + 3]),
-                         pack_bf16x2(pv[8 * g + 4], pv[8 * g + 5]), pack_bf16x2(pv[8 * g + 6], pv[8 * g + 7]));
-          *reinterpret_cast<uint4*>(db + sw) =
-              make_uint4(pack_bf16x2(dv[8 * g], dv[8 * g + 1]), pack_bf16x2(dv[8 * g + 2], dv[8 * g + 3]),
-                         pack_bf16x2(dv[8 * g + 4], dv[8 * g + 5]), pack_bf16x2(dv[8 * g + 6], dv[8 * g + 7]));
+          const float4 d0 = *reinterpret_cast<const float4*>(ld + BQ + c * 32 + g * 8);
+          const float4 d1 = *reinterpret_cast<const float4*>(ld + BQ + c * 32 + g * 8 + 4);
+          const float dl[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+          uint32_t w[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int i = g * 8 + 2 * j;
+            const float2 t2 = ffma2(make_float2(__uint_as_float(d[i]), __uint_as_float(d[i + 1])), s2, make_float2(-dl[2 * j], -dl[2 * j + 1]));
+            const float2 g2 = fmul2(make_float2(pr[c * 32 + i], pr[c * 32 + i + 1]), t2);
+            w[j] = pack_bf16x2(g2.x, g2.y);
+          }
+          *reinterpret_cast<uint4*>(drow + (((c * 4 + g) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
       tc_fence_before();
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(pds_full);
+      if (lane == 0) mbar_arrive(ds_full);
+      // the next step's staged value: every worker has left step it - 1 (its dQ was complete), whose buffer this is
+      if (it + 1 < n_iter) {
+        sLD[((it + 1) & 1) * 2 * BQ + half * BQ + r] = next;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ld_full[(it + 1) & 1]);
+      }
       // ---- dQ drain: this worker's half of the head dim ----
       if (!mbar_wait(dq_full, it & 1, abort_flag, p.status, 95)) { ok = false; break; }
       tc_fence_after();
       uint32_t v[CH][32];
 #pragma unroll
-      for (int cc = 0; cc < CH; ++cc) tmem_ld_32x32b_x32(tm_S + lane_base + (half * CH + cc) * 32, v[cc]);
+      for (int cc = 0; cc < CH; ++cc) tmem_ld_32x32b_x32(tm_dP + lane_base + (half * CH + cc) * 32, v[cc]);
       tc_wait_ld();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(dq_drained);      // the accumulator may be overwritten by the next S
+      if (lane == 0) mbar_arrive(dq_drained);      // the accumulator may be overwritten by the next dP
 #pragma unroll
       for (int cc = 0; cc < CH; ++cc) {
         if (lane == 0) tma_store_wait_read<0>();
@@ -328,11 +403,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
     // ------------------------------ dK / dV epilogue ------------------------------
-    // workers of half 0 write dK (staged in the P tile), those of half 1 write dV (staged in the dS tile)
+    // workers of half 0 write dK (staged in the dS tile), those of half 1 write dV (staged in the first Q stage)
     if (ok && n_iter > 0) ok = mbar_wait(acc_done, 0, abort_flag, p.status, 92);
     if (ok) {
       tc_fence_after();
-      uint8_t* tile = (half == 0) ? sP : sdS;
+      uint8_t* tile = (half == 0) ? sdS : sQ;
       uint8_t* dst = tile + r * 128;
       const uint32_t src = (half == 0 ? tm_dK : tm_dV) + lane_base;
 #pragma unroll 1

@@ -1,0 +1,34 @@
+"""Attention backward at the edges of its schedule: one step, odd step counts, ragged tiles, rows without visible keys, windows,
+more keys than queries, grouped heads."""
+import pytest
+import torch
+
+from mlperf_training_b200.ops import _lib, kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,Sq,Skv,Hq,Hkv,D,causal,window,sink", [
+    (1, 1, 1, 1, 1, 128, True, 0, False), (1, 128, 128, 1, 1, 64, True, 0, False), (2, 129, 129, 3, 3, 128, True, 0, False),
+    (1, 300, 300, 8, 2, 64, True, 50, True), (1, 500, 500, 4, 1, 128, False, 0, False), (1, 130, 700, 4, 2, 128, True, 0, False),
+    (2, 200, 90, 2, 1, 64, False, 0, False), (1, 1000, 1000, 2, 2, 128, True, 128, False), (1, 383, 383, 6, 2, 64, True, 0, True)])
+def test_backward(B, Sq, Skv, Hq, Hkv, D, causal, window, sink):
+    torch.manual_seed(Sq + D)
+    q, k, v = (torch.randn(B, s, h, D, device="cuda").bfloat16() for s, h in ((Sq, Hq), (Skv, Hkv), (Skv, Hkv)))
+    do = torch.randn(B, Sq, Hq, D, device="cuda").bfloat16()
+    sk = torch.randn(Hq, device="cuda") if sink else None
+    out, lse = K.attention_fwd(q, k, v, causal=causal, window=window, sink=sk)
+    dq, dk, dv, ds = K.attention_bwd(do, q, k, v, out, lse, causal=causal, window=window, sink=sk)
+    leaves = [t.double().requires_grad_(True) for t in ((q, k, v, sk) if sink else (q, k, v))]
+    g = Hq // Hkv
+    s = torch.einsum("bqhd,bkhd->bhqk", leaves[0], leaves[1].repeat_interleave(g, 2)) * D ** -0.5
+    s = s.masked_fill(~K._attn_mask(Sq, Skv, causal, window, "cuda"), float("-inf"))
+    if sink:
+        s = torch.cat([s, leaves[3].view(1, Hq, 1, 1).expand(B, Hq, Sq, 1)], -1)
+    p = torch.softmax(s, -1)[..., :Skv]
+    want = torch.autograd.grad(torch.einsum("bhqk,bkhd->bqhd", p, leaves[2].repeat_interleave(g, 2)), leaves, do.double())
+    # bf16 P and dS (2^-9 each per term) and delta from the rounded output.  dP - delta is the difference of two fp32 sums of D
+    # products (a single visible key: exactly 0): D * 2^-24 of |dO| |v| <= 1e-5 of |dO| beside the relative part
+    for a, b in zip((dq, dk, dv, ds) if sink else (dq, dk, dv), want):
+        assert (a.double() - b).norm() <= 2 ** -7 * b.norm() + 1e-5 * do.double().norm()
+    _lib.check_status("attention_bwd")

@@ -12,15 +12,16 @@
 // dQ.  The log-sum-exp and delta of the tile's queries run along the columns: they are staged in shared memory.  dK / dV
 // leave as bf16 through TMA stores.
 //
-// 320 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 workers.  Two workers share a TMEM lane quarter (32 key
-// rows): each takes half of the 128 query columns, then drains half of the dQ columns (TMEM -> registers, accumulator
-// released, registers -> fp32 TMA reduce-add).  A quarter of the exponentials is evaluated with a polynomial on the FMA
+// 512 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 4-7 dQ drain (TMEM -> registers, accumulator released,
+// registers -> shared memory -> fp32 TMA reduce-add), warps 8-15 workers.  Two workers share a TMEM lane quarter (32 key
+// rows): each takes half of the 128 query columns.  A quarter of the exponentials is evaluated with a polynomial on the FMA
 // pipe.  TMEM (512 columns): S^T / P^T | dP^T, then dQ | dK | dV.  Order of the MMAs of step i, Q double-buffered:
 //     [P^T(i) written]  dV(i)   [dS^T(i) written]  dQ(i)  S(i+1)  dK(i)  [dQ(i) drained]  dP(i+1)
-// so the workers drain dQ(i) and exponentiate S(i+1) while the tensor core runs dK(i) and dP(i+1).
-// Measured with delta, clearing and launches (queries as rows, P and dS through shared memory, one Q stage -> this):
-// 8192 x 32 / 8 heads of 128 causal 1990 -> 1766 us, 4096 x 64 / 8 1130 -> 1005, 4 x 2048 607 -> 550, 2000 x 64 / 8 of 64
-// 448 -> 378, 8 x 512 x 24 full 175 -> 157.
+// so dQ(i) is drained and S(i+1) exponentiated while the tensor core runs dK(i) and dP(i+1).  (The drain has warps of its
+// own: staged by the workers, its 64 KB a step took 3000 of their 6700 cycles, clock64 in the roles.)
+// Measured with delta, clearing and launches: queries as rows, P and dS through shared memory, one Q stage -> transposed ->
+// drain warps: 8192 x 32 / 8 heads of 128 causal 1990 -> 1766 -> 1336 us (1.03 PFLOP/s), 4096 x 64 / 8 1130 -> 1005 -> 779,
+// 4 x 2048 607 -> 550 -> 427, 2000 x 64 / 8 of 64 448 -> 378 -> 302, 8 x 512 x 24 full 175 -> 157 -> 136.
 //
 // The reference takes this kernel from Primus-Turbo / AITER / CK (config knobs
 // llama2_sft/primus/config_MI355X_1x8x1.sh:35-39); there is no in-tree counterpart.
@@ -31,8 +32,10 @@ namespace {
 
 constexpr int BQ = 128;
 constexpr int BKV = 128;
-constexpr int NTHREADS = 320;
-constexpr int STG = 4096;  // dQ staging chunk: 32 rows x 32 fp32 (one per worker)
+constexpr int NTHREADS = 512;  // warp 0 TMA, 1 MMA (2, 3 complete the warpgroup), 4-7 dQ drain, 8-15 P / dS workers
+// 4 x 128 threads launch with 128 registers each: 88 + 88 + 2 x 168
+constexpr int REGS_OTHER = 88, REGS_WORKER = 168;
+constexpr int STG = 4096;  // dQ staging chunk: 32 rows x 32 fp32 (two per drain warp)
 #ifndef B200_ATTN_BWD_POLY
 #define B200_ATTN_BWD_POLY 6
 #endif
@@ -104,7 +107,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* p_full = bars + 9;      // P^T written to TMEM (8 arrivals)
   uint64_t* ds_full = bars + 10;    // dS^T written to shared memory (8 arrivals)
   uint64_t* dq_full = bars + 11;    // dQ tile complete in TMEM
-  uint64_t* dq_drained = bars + 12; // dQ tile copied out of TMEM (8 arrivals)
+  uint64_t* dq_drained = bars + 12; // dQ tile copied out of TMEM (4 arrivals)
   uint64_t* ld_full = bars + 13;    // 2: the step's log-sum-exp / delta are in shared memory (8 arrivals)
   uint64_t* acc_done = bars + 15;   // every MMA of this CTA finished
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 16);
@@ -141,7 +144,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1); mbar_init(do_full, 1); mbar_init(do_empty, 1); mbar_init(s_full, 1); mbar_init(dp_full, 1);
-    mbar_init(p_full, 8); mbar_init(ds_full, 8); mbar_init(dq_full, 1); mbar_init(dq_drained, 8); mbar_init(acc_done, 1);
+    mbar_init(p_full, 8); mbar_init(ds_full, 8); mbar_init(dq_full, 1); mbar_init(dq_drained, 4); mbar_init(acc_done, 1);
     for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); mbar_init(&ld_full[i], 8); }
     *abort_flag = 0;
     mbar_fence_init();
@@ -156,6 +159,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t tm_dK = tmem_base + 256;
   const uint32_t tm_dV = tmem_base + 384;
 
+  if (warp < 8) reg_dealloc<REGS_OTHER>();
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
@@ -264,34 +268,77 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (!last) ok = mbar_wait_spin(dq_drained, ph, abort_flag, p.status, 85) && issue_dp(it + 1);
       }
     }
-  } else {
-    // ------------------------------ workers: P / dS, then dQ drain ------------------------------
-    const int q = warp & 3;                   // TMEM lane quarter
-    const int half = (warp - 2) >> 2;         // which half of the query columns / of the dQ columns
-    const int r = q * 32 + lane;              // key row of the tile (dQ drain: query row)
+  } else if (warp >= 4 && warp < 8) {
+    // ------------------------------ dQ drain ------------------------------
+    const int q = warp & 3;                   // TMEM lane quarter: 32 query rows
     const uint32_t lane_base = uint32_t(q * 32) << 16;
-    uint8_t* stg = sStg + (warp - 2) * STG;   // one staging buffer per worker
-    constexpr int CH = HD / 64;               // dQ chunks (32 columns) per worker
+    uint8_t* stg = sStg + q * 2 * STG;
+    for (int it = 0; it < n_iter; ++it) {
+      const int h = hk * group + it / n_q;
+      const int q0 = (i_lo + it % n_q) * BQ;
+      if (!mbar_wait(dq_full, it & 1, abort_flag, p.status, 95)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c2 = 0; c2 < HD / 64; ++c2) {       // 64 columns at a time: two staging buffers
+        uint32_t v[64];
+        tmem_ld_32x32b_x32(tm_dP + lane_base + c2 * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+        tmem_ld_32x32b_x32(tm_dP + lane_base + c2 * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+        tc_wait_ld();
+        if (c2 == HD / 64 - 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(dq_drained);  // the accumulator may be overwritten by the next dP
+        }
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+          if (lane == 0) tma_store_wait_read<1>(); // the reduce before the last has read this buffer
+          __syncwarp();
+          uint8_t* sb = stg + cc * STG + lane * 128;
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+            *reinterpret_cast<uint4*>(sb + ((g ^ (lane & 7)) << 4)) =
+                make_uint4(v[cc * 32 + 4 * g], v[cc * 32 + 4 * g + 1], v[cc * 32 + 4 * g + 2], v[cc * 32 + 4 * g + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (q0 + q * 32 < p.Sq) tma_reduce_add_4d(&tmdQ, stg + cc * STG, c2 * 64 + cc * 32, h, q0 + q * 32, b);
+            tma_store_commit();
+          }
+        }
+      }
+    }
+    if (lane == 0) tma_store_wait_all<0>();
+  } else if (warp >= 8) {
+    // ------------------------------ workers: P / dS ------------------------------
+    reg_alloc<REGS_WORKER>();
+    const int q = warp & 3;                   // TMEM lane quarter
+    const int half = (warp - 8) >> 2;         // which half of the query columns
+    const int r = q * 32 + lane;              // key row of the tile
+    const uint32_t lane_base = uint32_t(q * 32) << 16;
     const int key = kv0 + r;
     // this thread stages one value per step: the log-sum-exp (half 0) or delta (half 1) of query r of the tile
-    auto fetch = [&](int it) -> float {
-      const int q_pos = (i_lo + it % n_q) * BQ + r;
-      if (q_pos >= p.Sq) return half == 0 ? INFINITY : 0.f;      // P = exp2(s - inf) = 0 for rows that are not there
-      const long long idx = ((long long)b * p.Hq + hk * group + it / n_q) * p.Sq + q_pos;
-      if (half == 1) return p.delta[idx] * p.scale;
-      const float l = p.lse[idx];
-      return l == -INFINITY ? INFINITY : l * 1.4426950408889634f;   // a row without any visible key
+    // (loaded a step ahead as it is and turned into what the columns need only when it is stored: used at once, it cost the
+    // step a global-memory latency)
+    auto fetch = [&](int h, int q_pos) -> float {
+      if (q_pos >= p.Sq) return half == 0 ? -INFINITY : 0.f;
+      const long long idx = ((long long)b * p.Hq + h) * p.Sq + q_pos;
+      return half == 1 ? p.delta[idx] : p.lse[idx];
     };
+    // a row that is not there or sees no key: P = exp2(s - inf) = 0
+    auto staged = [&](float x) -> float {
+      return half == 1 ? x * p.scale : (x == -INFINITY ? INFINITY : x * 1.4426950408889634f);
+    };
+    int h_next = hk * group, i_next = i_lo;
     bool ok = true;
     if (n_iter > 0) {
-      sLD[half * BQ + r] = fetch(0);
+      sLD[half * BQ + r] = staged(fetch(h_next, i_next * BQ + r));
       __syncwarp();
       if (lane == 0) mbar_arrive(&ld_full[0]);
     }
     for (int it = 0; it < n_iter && ok; ++it) {
-      const int h = hk * group + it / n_q;
-      const int q0 = (i_lo + it % n_q) * BQ;
-      const float next = it + 1 < n_iter ? fetch(it + 1) : 0.f;
+      const int q0 = i_next * BQ;
+      if (++i_next > i_hi) { i_next = i_lo; ++h_next; }
+      const float next = it + 1 < n_iter ? fetch(h_next, i_next * BQ + r) : 0.f;
       const bool need_mask = (kv0 + BKV > p.Skv) || (p.causal && kv0 + BKV - 1 > q0 + off) ||
                              (p.window > 0 && kv0 < q0 + BQ - 1 + off - p.window + 1);
       // visible queries of this key: columns [c_lo, c_hi)
@@ -369,37 +416,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_full);
-      // the next step's staged value: every worker has left step it - 1 (its dQ was complete), whose buffer this is
+      // the next step's staged value, into the buffer of step it - 1: every worker has left that step, since dP(it) was issued
+      // after all of them had written dS(it - 1)
       if (it + 1 < n_iter) {
-        sLD[((it + 1) & 1) * 2 * BQ + half * BQ + r] = next;
+        sLD[((it + 1) & 1) * 2 * BQ + half * BQ + r] = staged(next);
         __syncwarp();
         if (lane == 0) mbar_arrive(&ld_full[(it + 1) & 1]);
-      }
-      // ---- dQ drain: this worker's half of the head dim ----
-      if (!mbar_wait(dq_full, it & 1, abort_flag, p.status, 95)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t v[CH][32];
-#pragma unroll
-      for (int cc = 0; cc < CH; ++cc) tmem_ld_32x32b_x32(tm_dP + lane_base + (half * CH + cc) * 32, v[cc]);
-      tc_wait_ld();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(dq_drained);      // the accumulator may be overwritten by the next dP
-#pragma unroll
-      for (int cc = 0; cc < CH; ++cc) {
-        if (lane == 0) tma_store_wait_read<0>();
-        __syncwarp();
-        uint8_t* sb = stg + lane * 128;
-#pragma unroll
-        for (int g = 0; g < 8; ++g)
-          *reinterpret_cast<uint4*>(sb + ((g ^ (lane & 7)) << 4)) =
-              make_uint4(v[cc][4 * g], v[cc][4 * g + 1], v[cc][4 * g + 2], v[cc][4 * g + 3]);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          if (q0 + q * 32 < p.Sq) tma_reduce_add_4d(&tmdQ, stg, (half * CH + cc) * 32, h, q0 + q * 32, b);
-          tma_store_commit();
-        }
       }
     }
     // ------------------------------ dK / dV epilogue ------------------------------

@@ -3,11 +3,13 @@
 //   dV += P^T dO      dP = dO V^T      dS = dP * silu'(alpha S) * alpha / N * mask
 //   dQ  = dS K        dK += dS^T Q
 //
-// One CTA per (sequence, head, 128-key tile) loops over the query tiles that see those keys; same
-// engine as attention_bwd.cu (TMA loads, five tcgen05 GEMMs with dK / dV resident in TMEM, P and
-// dS as bf16 shared-memory tiles read both K-major and MN-major, dQ leaving through fp32 TMA
-// reduce-add).  No row statistics are needed, so nothing but Q, K, V, dO is read.
-// Mask and jagged layout as in hstu_attn_fwd.cu.
+// One CTA per (sequence, head, 128-key tile) loops over the query tiles that see those keys; the engine of
+// attention_bwd.cu: transposed scores (a worker thread owns a key row), P^T back in TMEM as the operand of dV, dS^T once in
+// shared memory for dK and dQ, Q double-buffered, warps of their own for the fp32 TMA reduce-add of dQ, and per step
+//     [P^T(i) written]  dV(i)   [dS^T(i) written]  dQ(i)  S(i+1)  dK(i)  [dQ(i) drained]  dP(i+1)
+// No row statistics are needed, so nothing but Q, K, V, dO is read.  Mask and jagged layout as in hstu_attn_fwd.cu.
+// Measured with the clearing and conversion around it, before (queries as rows, P and dS through shared memory, drained by
+// the workers) -> now: 128 users of median 512 tokens, 4 heads of 128: 1345 -> 1077 us; 12 users of median 700: 235 -> 169.
 //
 // Math oracle: autograd of generative_recommenders/ops/pytorch/pt_hstu_attention.py:130-187; the
 // reference's production kernels are generative_recommenders/ops/flydsl/hstu_bwd_dkdv.py and
@@ -19,8 +21,10 @@ namespace {
 
 constexpr int BQ = 128;
 constexpr int BKV = 128;
-constexpr int NTHREADS = 320;
-constexpr int STG = 4096;
+constexpr int NTHREADS = 512;  // warp 0 TMA, 1 MMA (2, 3 complete the warpgroup), 4-7 dQ drain, 8-15 P / dS workers
+// 4 x 128 threads launch with 128 registers each: 88 + 88 + 2 x 168
+constexpr int REGS_OTHER = 88, REGS_WORKER = 168;
+constexpr int STG = 4096;  // dQ staging chunk: 32 rows x 32 fp32 (two per drain warp)
 
 struct HstuBwdParams {
   int max_len, H, contextual;
@@ -42,10 +46,10 @@ B200_DEVICE float tanh_approx(float x) {
 
 template <int HD>
 struct Smem {
-  static constexpr int T_BYTES = 128 * HD * 2;        // K, V, Q, dO tiles
-  static constexpr int PS_BYTES = BQ * BKV * 2;       // P, dS tiles
-  static constexpr int STG_BYTES = 4 * 2 * STG;
-  static constexpr int TOTAL = 4 * T_BYTES + 2 * PS_BYTES + STG_BYTES + 1024 + 256;
+  static constexpr int T_BYTES = 128 * HD * 2;        // K, V, Q (two stages), dO tiles
+  static constexpr int DS_BYTES = BQ * BKV * 2;       // dS^T tile
+  static constexpr int STG_BYTES = 8 * STG;
+  static constexpr int TOTAL = 5 * T_BYTES + DS_BYTES + STG_BYTES + 1024 + 256;
 };
 
 template <int HD>
@@ -59,21 +63,24 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sK = smem;
   uint8_t* sV = sK + SM::T_BYTES;
-  uint8_t* sQ = sV + SM::T_BYTES;
-  uint8_t* sdO = sQ + SM::T_BYTES;
-  uint8_t* sP = sdO + SM::T_BYTES;
-  uint8_t* sdS = sP + SM::PS_BYTES;
-  uint8_t* sStg = sdS + SM::PS_BYTES;
+  uint8_t* sQ = sV + SM::T_BYTES;           // two stages
+  uint8_t* sdO = sQ + 2 * SM::T_BYTES;
+  uint8_t* sdS = sdO + SM::T_BYTES;
+  uint8_t* sStg = sdS + SM::DS_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sStg + SM::STG_BYTES);
   uint64_t* kv_full = bars + 0;     // K and V landed
-  uint64_t* qdo_full = bars + 1;    // Q_i and dO_i landed
-  uint64_t* qdo_empty = bars + 2;   // MMAs reading Q_i / dO_i / P / dS finished
-  uint64_t* sdp_full = bars + 3;    // S and dP complete in TMEM
-  uint64_t* pds_full = bars + 4;    // P and dS written to shared memory (4 arrivals)
-  uint64_t* dq_full = bars + 5;     // dQ tile complete in TMEM
-  uint64_t* dq_drained = bars + 6;  // dQ tile copied out of TMEM (4 arrivals)
-  uint64_t* acc_done = bars + 7;    // every MMA of this CTA finished
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 8);
+  uint64_t* q_full = bars + 1;      // 2: Q_i landed
+  uint64_t* q_empty = bars + 3;     // 2: MMAs reading Q_i finished
+  uint64_t* do_full = bars + 5;     // dO_i landed
+  uint64_t* do_empty = bars + 6;    // MMAs reading dO_i finished
+  uint64_t* s_full = bars + 7;      // S^T complete in TMEM
+  uint64_t* dp_full = bars + 8;     // dP^T complete in TMEM (and every MMA of the step before: dS^T is free)
+  uint64_t* p_full = bars + 9;      // P^T written to TMEM (8 arrivals)
+  uint64_t* ds_full = bars + 10;    // dS^T written to shared memory (8 arrivals)
+  uint64_t* dq_full = bars + 11;    // dQ tile complete in TMEM
+  uint64_t* dq_drained = bars + 12; // dQ tile copied out of TMEM (4 arrivals)
+  uint64_t* acc_done = bars + 13;   // every MMA of this CTA finished
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -97,8 +104,9 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   auto q_tile = [&](int it) { return (extra && it == 0) ? 0 : i_lo + it - extra; };
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1); mbar_init(qdo_full, 1); mbar_init(qdo_empty, 1); mbar_init(sdp_full, 1);
-    mbar_init(pds_full, 8); mbar_init(dq_full, 1); mbar_init(dq_drained, 8); mbar_init(acc_done, 1);
+    mbar_init(kv_full, 1); mbar_init(do_full, 1); mbar_init(do_empty, 1); mbar_init(s_full, 1); mbar_init(dp_full, 1);
+    mbar_init(p_full, 8); mbar_init(ds_full, 8); mbar_init(dq_full, 1); mbar_init(dq_drained, 4); mbar_init(acc_done, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -107,11 +115,12 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  const uint32_t tm_S = tmem_base;          // S, later dQ (128 columns)
-  const uint32_t tm_dP = tmem_base + 128;
+  const uint32_t tm_S = tmem_base;          // S^T; P^T of queries 0-63 in columns 0-31, of 64-127 in 64-95
+  const uint32_t tm_dP = tmem_base + 128;   // dP^T, later dQ
   const uint32_t tm_dK = tmem_base + 256;
   const uint32_t tm_dV = tmem_base + 384;
 
+  if (warp < 8) reg_dealloc<REGS_OTHER>();
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
@@ -122,17 +131,17 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tma_load_3d(sK + i * (BKV * 128), &tmK, kv_full, i * 64, hk, row_base + kv0);
         tma_load_3d(sV + i * (BKV * 128), &tmV, kv_full, i * 64, hk, row_base + kv0);
       }
-      bool ok = true;
-      for (int it = 0; it < n_iter && ok; ++it) {
-        const int h = hk;
+      for (int it = 0; it < n_iter; ++it) {
         const int q0 = q_tile(it) * BQ;
-        if (!mbar_wait(qdo_empty, (it & 1) ^ 1, abort_flag, p.status, 70)) { ok = false; break; }
-        mbar_expect_tx(qdo_full, 2 * SM::T_BYTES);
+        const int st = it & 1;
+        if (!mbar_wait(&q_empty[st], ((it >> 1) & 1) ^ 1, abort_flag, p.status, 70)) break;
+        mbar_expect_tx(&q_full[st], SM::T_BYTES);
 #pragma unroll
-        for (int i = 0; i < NB; ++i) {
-          tma_load_3d(sQ + i * (BQ * 128), &tmQ, qdo_full, i * 64, h, row_base + q0);
-          tma_load_3d(sdO + i * (BQ * 128), &tmdO, qdo_full, i * 64, h, row_base + q0);
-        }
+        for (int i = 0; i < NB; ++i) tma_load_3d(sQ + st * SM::T_BYTES + i * (BQ * 128), &tmQ, &q_full[st], i * 64, hk, row_base + q0);
+        if (!mbar_wait(do_empty, (it & 1) ^ 1, abort_flag, p.status, 71)) break;
+        mbar_expect_tx(do_full, SM::T_BYTES);
+#pragma unroll
+        for (int i = 0; i < NB; ++i) tma_load_3d(sdO + i * (BQ * 128), &tmdO, do_full, i * 64, hk, row_base + q0);
       }
     }
   } else if (warp == 1) {
@@ -140,166 +149,216 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // The warp stays converged and one elected lane issues: operands live in uniform registers and descriptors advance by
     // an addition (rebuilt by one lane of a divergent warp they cost more than the 64 cycles an instruction runs).
     if (n_iter > 0) {
-      const uint32_t id_kk = umma_idesc(1, 1, 0, 0, 128, 128);   // S = Q K^T, dP = dO V^T (both K-major)
-      const uint32_t id_dq = umma_idesc(1, 1, 0, 1, 128, HD);    // dQ = dS (K-major) x K (MN-major)
-      const uint32_t id_tt = umma_idesc(1, 1, 1, 1, 128, HD);    // dV = P^T dO, dK = dS^T Q (both MN-major)
+      const uint32_t id_kk = umma_idesc(1, 1, 0, 0, 128, 128);   // S^T = K Q^T, dP^T = V dO^T (both K-major)
+      const uint32_t id_dv = umma_idesc(1, 1, 0, 1, 128, HD);    // dV = P^T (TMEM) x dO (MN-major)
+      const uint32_t id_dk = umma_idesc(1, 1, 0, 1, 128, HD);    // dK = dS^T (K-major) x Q (MN-major)
+      const uint32_t id_dq = umma_idesc(1, 1, 1, 1, 128, HD);    // dQ = dS (the tile read MN-major) x K (MN-major)
       const uint64_t kK = umma_desc_sw128(smem_u32(sK), 16, 1024), kV = umma_desc_sw128(smem_u32(sV), 16, 1024);
       const uint64_t kQ = umma_desc_sw128(smem_u32(sQ), 16, 1024), kdO = umma_desc_sw128(smem_u32(sdO), 16, 1024);
-      const uint64_t kdS = umma_desc_sw128(smem_u32(sdS), 16, 1024);
+      const uint64_t kdS = umma_desc_sw128(smem_u32(sdS), 16, 1024), mdS = umma_desc_sw128(smem_u32(sdS), 128 * 128, 1024);
       const uint64_t mK = umma_desc_sw128(smem_u32(sK), 128 * 128, 1024), mQ = umma_desc_sw128(smem_u32(sQ), 128 * 128, 1024);
-      const uint64_t mdO = umma_desc_sw128(smem_u32(sdO), 128 * 128, 1024), mP = umma_desc_sw128(smem_u32(sP), 128 * 128, 1024);
-      const uint64_t mdS = umma_desc_sw128(smem_u32(sdS), 128 * 128, 1024);
-      bool ok = mbar_wait_spin(kv_full, 0, abort_flag, p.status, 80);
+      const uint64_t mdO = umma_desc_sw128(smem_u32(sdO), 128 * 128, 1024);
+      auto issue_s = [&](int it) -> bool {
+        const int st = it & 1;
+        if (!mbar_wait_spin(&q_full[st], (it >> 1) & 1, abort_flag, p.status, 81)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t bd = kQ + (st * SM::T_BYTES >> 4);
+#pragma unroll
+          for (int kk = 0; kk < HD / 16; ++kk) {
+            const uint32_t o = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
+            tc_mma_f16_ss(tm_S, kK + o, bd + o, id_kk, kk > 0);
+          }
+          tc_commit(s_full);
+        }
+        __syncwarp();
+        return true;
+      };
+      auto issue_dp = [&](int it) -> bool {
+        if (!mbar_wait_spin(do_full, it & 1, abort_flag, p.status, 82)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < HD / 16; ++kk) {
+            const uint32_t o = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
+            tc_mma_f16_ss(tm_dP, kV + o, kdO + o, id_kk, kk > 0);
+          }
+          tc_commit(dp_full);
+        }
+        __syncwarp();
+        return true;
+      };
+      bool ok = mbar_wait_spin(kv_full, 0, abort_flag, p.status, 80) && issue_s(0) && issue_dp(0);
       for (int it = 0; it < n_iter && ok; ++it) {
         const uint32_t ph = it & 1;
-        if (!mbar_wait_spin(qdo_full, ph, abort_flag, p.status, 81)) { ok = false; break; }
-        tc_fence_after();
-        // S = Q K^T ; dP = dO V^T   (contraction over the head dim, both operands K-major)
-        // dP first: its accumulator was read by the workers long ago, so these MMAs run while the workers
-        // still drain dQ of the previous iteration out of the S / dQ columns
-        if (elect_one()) {
-#pragma unroll
-          for (int kk = 0; kk < HD / 16; ++kk) {
-            const uint32_t o = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
-            tc_mma_f16_ss(tm_dP, kdO + o, kV + o, id_kk, kk > 0);
-          }
-        }
-        __syncwarp();
-        if (it > 0 && !mbar_wait_spin(dq_drained, (it - 1) & 1, abort_flag, p.status, 82)) { ok = false; break; }
+        const int st = it & 1;
+        const bool last = it == n_iter - 1;
+        if (!mbar_wait_spin(p_full, ph, abort_flag, p.status, 83)) { ok = false; break; }
         tc_fence_after();
         if (elect_one()) {
-#pragma unroll
-          for (int kk = 0; kk < HD / 16; ++kk) {
-            const uint32_t o = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
-            tc_mma_f16_ss(tm_S, kQ + o, kK + o, id_kk, kk > 0);
-          }
-          tc_commit(sdp_full);
-        }
-        __syncwarp();
-        if (!mbar_wait_spin(pds_full, ph, abort_flag, p.status, 83)) { ok = false; break; }
-        tc_fence_after();
-        if (elect_one()) {
-          // dV += P^T dO ; dK += dS^T Q : contraction over queries, both operands MN-major
+          // dV += P^T dO : 16 queries = 8 TMEM columns per step, dO as 16 query rows of 128 bytes
 #pragma unroll
           for (int kk = 0; kk < BQ / 16; ++kk)
-            tc_mma_f16_ss(tm_dV, mP + kk * 128, mdO + kk * 128, id_tt, (it > 0 || kk > 0));
+            tc_mma_f16_ts(tm_dV, tm_S + (kk / 4) * 64 + (kk % 4) * 8, mdO + kk * 128, id_dv, (it > 0 || kk > 0));
+          tc_commit(do_empty);
+        }
+        __syncwarp();
+        if (!mbar_wait_spin(ds_full, ph, abort_flag, p.status, 84)) { ok = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
+          // dQ = dS K : contraction over keys, 16 key rows of the dS^T tile and of K per step
 #pragma unroll
-          for (int kk = 0; kk < BQ / 16; ++kk)
-            tc_mma_f16_ss(tm_dK, mdS + kk * 128, mQ + kk * 128, id_tt, (it > 0 || kk > 0));
-          tc_commit(qdo_empty);  // Q_i / dO_i may be overwritten: the next tiles load during the dQ GEMM
-          // dQ = dS K : A = dS [q][key] K-major, B = K [key][d] MN-major (contraction over keys)
+          for (int kk = 0; kk < BKV / 16; ++kk) tc_mma_f16_ss(tm_dP, mdS + kk * 128, mK + kk * 128, id_dq, kk > 0);
+          tc_commit(dq_full);
+        }
+        __syncwarp();
+        if (!last && !issue_s(it + 1)) { ok = false; break; }     // (P^T(i) was read by dV(i), issued before)
+        if (elect_one()) {
+          // dK += dS^T Q : contraction over queries
+          const uint64_t bd = mQ + (st * SM::T_BYTES >> 4);
 #pragma unroll
-          for (int kk = 0; kk < BKV / 16; ++kk) {
+          for (int kk = 0; kk < BQ / 16; ++kk) {
             const uint32_t ao = ((kk / 4) * (128 * 128) + (kk % 4) * 32) >> 4;
-            tc_mma_f16_ss(tm_S, kdS + ao, mK + kk * 128, id_dq, kk > 0);
+            tc_mma_f16_ss(tm_dK, kdS + ao, bd + kk * 128, id_dk, (it > 0 || kk > 0));
           }
-          tc_commit(dq_full);    // also: P / dS shared-memory tiles are free again
-          if (it == n_iter - 1) tc_commit(acc_done);
+          tc_commit(&q_empty[st]);
+          if (last) tc_commit(acc_done);
         }
         __syncwarp();
+        if (!last) ok = mbar_wait_spin(dq_drained, ph, abort_flag, p.status, 85) && issue_dp(it + 1);
       }
     }
-  } else {
-    // ------------------------------ workers (warps 2-9): P / dS, then dQ drain ------------------------------
-    // Two workers share a TMEM lane quarter: each handles half of the key columns, then half of the
-    // dQ columns (registers, accumulator released, fp32 TMA reduce-add while the next GEMMs run).
-    const int q = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int r = q * 32 + lane;
+  } else if (warp >= 4 && warp < 8) {
+    // ------------------------------ dQ drain ------------------------------
+    const int q = warp & 3;                   // TMEM lane quarter: 32 query rows
     const uint32_t lane_base = uint32_t(q * 32) << 16;
-    uint8_t* stg = sStg + (warp - 2) * STG;
-    constexpr int CH = HD / 64;
+    uint8_t* stg = sStg + q * 2 * STG;
+    for (int it = 0; it < n_iter; ++it) {
+      const int q0 = q_tile(it) * BQ;
+      if (!mbar_wait(dq_full, it & 1, abort_flag, p.status, 95)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c2 = 0; c2 < HD / 64; ++c2) {       // 64 columns at a time: two staging buffers
+        uint32_t v[64];
+        tmem_ld_32x32b_x32(tm_dP + lane_base + c2 * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+        tmem_ld_32x32b_x32(tm_dP + lane_base + c2 * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+        tc_wait_ld();
+        if (c2 == HD / 64 - 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(dq_drained);  // the accumulator may be overwritten by the next dP
+        }
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+          if (lane == 0) tma_store_wait_read<1>(); // the reduce before the last has read this buffer
+          __syncwarp();
+          uint8_t* sb = stg + cc * STG + lane * 128;
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+            *reinterpret_cast<uint4*>(sb + ((g ^ (lane & 7)) << 4)) =
+                make_uint4(v[cc * 32 + 4 * g], v[cc * 32 + 4 * g + 1], v[cc * 32 + 4 * g + 2], v[cc * 32 + 4 * g + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (q0 + q * 32 < len) tma_reduce_add_3d(&tmdQ, stg + cc * STG, c2 * 64 + cc * 32, hk, row_base + q0 + q * 32);
+            tma_store_commit();
+          }
+        }
+      }
+    }
+    if (lane == 0) tma_store_wait_all<0>();
+  } else if (warp >= 8) {
+    // ------------------------------ workers: P / dS ------------------------------
+    reg_alloc<REGS_WORKER>();
+    const int q = warp & 3;                   // TMEM lane quarter
+    const int half = (warp - 8) >> 2;         // which half of the query columns
+    const int r = q * 32 + lane;              // key row of the tile
+    const uint32_t lane_base = uint32_t(q * 32) << 16;
+    const int kp = kv0 + r;                   // this thread's key
+    const bool plain = (n_tgt == 0 && ctx == 0);
+    const int k_id = min(max(kp - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
+    const float ha = 0.5f * p.alpha, inv_n = 1.0f / (float)p.max_len, an = p.alpha * inv_n;
     bool ok = true;
     for (int it = 0; it < n_iter && ok; ++it) {
-      const int h = hk;
       const int q0 = q_tile(it) * BQ;
-      const int q_pos = q0 + r;
-      const bool row_ok = q_pos < len;
-      const int q_id = min(max(q_pos - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
-      const bool plain = (n_tgt == 0 && ctx == 0);
       // a tile whose every (query, key) pair is visible needs no element mask: ids grow with the position, so it
       // is enough that the tile's first query is later than its last key, and that both tiles lie inside the sequence
       const int first_q_id = min(max(q0 - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
       const int last_k_id = min(max(kv0 + BKV - 1 - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
       const bool inside = (kv0 + BKV <= len) && (q0 + BQ <= len);
       const bool need_mask = plain ? ((kv0 + BKV - 1 > q0) || !inside) : !(inside && first_q_id > last_k_id);
-      if (!mbar_wait(sdp_full, it & 1, abort_flag, p.status, 90)) { ok = false; break; }
+      if (!mbar_wait(s_full, it & 1, abort_flag, p.status, 90)) { ok = false; break; }
       tc_fence_after();
-      // the P / dS tiles are free: this warp waited for dq_full of the previous iteration in its drain step
-      uint8_t* prow = sP + r * 128;
-      uint8_t* drow = sdS + r * 128;
-#pragma unroll 1
-      for (int c = half * 2; c < half * 2 + 2; ++c) {
-        uint32_t s[32], d[32];
-        tmem_ld_32x32b_x32(tm_S + lane_base + c * 32, s);
-        tmem_ld_32x32b_x32(tm_dP + lane_base + c * 32, d);
+      float f[64];                            // dS / dP of this key and the half's queries
+      {
+        uint32_t s[64];
+        tmem_ld_32x32b_x32(tm_S + lane_base + half * 64, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
+        tmem_ld_32x32b_x32(tm_S + lane_base + half * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&s[32]));
         tc_wait_ld();
-        float pv[32], dv[32];
-        const float ha = 0.5f * p.alpha, inv_n = 1.0f / (float)p.max_len, an = p.alpha * inv_n;
+        const float2 ha2 = make_float2(ha, ha), an2 = make_float2(an, an), hn2 = make_float2(inv_n, inv_n);
+        const float2 one = make_float2(1.f, 1.f), half2 = make_float2(0.5f, 0.5f), neg = make_float2(-1.f, -1.f);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
+        for (int i = 0; i < 64; i += 2) {
           // P = silu(a s) / N ; dS = dP * silu'(a s) * a / N   (sig = (1 + tanh(a s / 2)) / 2)
-          const float hx = __uint_as_float(s[i]) * ha;
-          const float sig = 0.5f * (1.f + tanh_approx(hx));
-          const float x = 2.f * hx;
-          float p0 = x * sig * inv_n;
-          float g0 = __uint_as_float(d[i]) * sig * (1.f + x * (1.f - sig)) * an;
-          if (need_mask) {
-            const int kp = kv0 + c * 32 + i;
+          const float2 hx = fmul2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), ha2);
+          const float2 sig = ffma2(make_float2(tanh_approx(hx.x), tanh_approx(hx.y)), half2, half2);
+          const float2 x = fadd2(hx, hx);
+          const float2 pv = fmul2(fmul2(x, sig), hn2);
+          const float2 fv = fmul2(fmul2(sig, ffma2(x, ffma2(sig, neg, one), one)), an2);
+          s[i] = __float_as_uint(pv.x); s[i + 1] = __float_as_uint(pv.y);
+          f[i] = fv.x; f[i + 1] = fv.y;
+        }
+        if (need_mask) {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) {
+            const int q_pos = q0 + half * 64 + i;
             bool vis;
             if (plain) vis = kp <= q_pos;
             else {
-              const int k_id = min(max(kp - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
+              const int q_id = min(max(q_pos - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
               vis = (kp == q_pos) || (q_id > k_id) || (ctx > 0 && q_id == 0 && kp < hist_end);
             }
-            if (!(vis && kp < len && row_ok)) { p0 = 0.f; g0 = 0.f; }
+            if (!(vis && kp < len && q_pos < len)) { s[i] = 0u; f[i] = 0.f; }
           }
-          pv[i] = p0;
-          dv[i] = g0;
         }
-        uint8_t* pb = prow + (c / 2) * (BQ * 128);
-        uint8_t* db = drow + (c / 2) * (BQ * 128);
+        uint32_t pk[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) pk[j] = pack_bf16x2(__uint_as_float(s[2 * j]), __uint_as_float(s[2 * j + 1]));
+        tmem_st_32x32b_x32(tm_S + lane_base + half * 64, pk);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+      }
+      if (!mbar_wait(dp_full, it & 1, abort_flag, p.status, 91)) { ok = false; break; }
+      tc_fence_after();
+      uint8_t* drow = sdS + half * (BKV * 128) + r * 128;       // 64 queries of key r
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t d[32];
+        tmem_ld_32x32b_x32(tm_dP + lane_base + half * 64 + c * 32, d);
+        tc_wait_ld();
+        if (need_mask) {
+          // (rows past the end belong to the next sequence: what it holds must not reach 0 * inf)
+#pragma unroll
+          for (int i = 0; i < 32; ++i) if (f[c * 32 + i] == 0.f) d[i] = 0u;
+        }
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
-          const int sw = (((c & 1) * 4 + g) ^ (r & 7)) << 4;
-          *reinterpret_cast<uint4*>(pb + sw) =
-              make_uint4(pack_bf16x2(pv[8 * g], pv[8 * g + 1]), pack_bf16x2(pv[8 * g + 2], pv[8 * g + 3]),
-                         pack_bf16x2(pv[8 * g + 4], pv[8 * g + 5]), pack_bf16x2(pv[8 * g + 6], pv[8 * g + 7]));
-          *reinterpret_cast<uint4*>(db + sw) =
-              make_uint4(pack_bf16x2(dv[8 * g], dv[8 * g + 1]), pack_bf16x2(dv[8 * g + 2], dv[8 * g + 3]),
-                         pack_bf16x2(dv[8 * g + 4], dv[8 * g + 5]), pack_bf16x2(dv[8 * g + 6], dv[8 * g + 7]));
+          uint32_t w[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int i = g * 8 + 2 * j;
+            const float2 g2 = fmul2(make_float2(f[c * 32 + i], f[c * 32 + i + 1]), make_float2(__uint_as_float(d[i]), __uint_as_float(d[i + 1])));
+            w[j] = pack_bf16x2(g2.x, g2.y);
+          }
+          *reinterpret_cast<uint4*>(drow + (((c * 4 + g) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
       tc_fence_before();
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(pds_full);
-      // ---- dQ drain: this worker's half of the head dim ----
-      if (!mbar_wait(dq_full, it & 1, abort_flag, p.status, 95)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t v[CH][32];
-#pragma unroll
-      for (int cc = 0; cc < CH; ++cc) tmem_ld_32x32b_x32(tm_S + lane_base + (half * CH + cc) * 32, v[cc]);
-      tc_wait_ld();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(dq_drained);
-#pragma unroll
-      for (int cc = 0; cc < CH; ++cc) {
-        if (lane == 0) tma_store_wait_read<0>();
-        __syncwarp();
-        uint8_t* sb = stg + lane * 128;
-#pragma unroll
-        for (int g = 0; g < 8; ++g)
-          *reinterpret_cast<uint4*>(sb + ((g ^ (lane & 7)) << 4)) =
-              make_uint4(v[cc][4 * g], v[cc][4 * g + 1], v[cc][4 * g + 2], v[cc][4 * g + 3]);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          if (q0 + q * 32 < len) tma_reduce_add_3d(&tmdQ, stg, (half * CH + cc) * 32, h, row_base + q0 + q * 32);
-          tma_store_commit();
-        }
-      }
+      if (lane == 0) mbar_arrive(ds_full);
     }
     // ------------------------------ dK / dV epilogue ------------------------------
     // workers of half 0 write dK, those of half 1 write dV; guarded row stores: rows past the
@@ -326,7 +385,6 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
       }
     }
-    if (lane == 0) tma_store_wait_all<0>();
   }
 
   __syncwarp();

@@ -117,31 +117,50 @@ ln_modulate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16
   }
 }
 
-// Per-sample column sums over the S rows of sample b = blockIdx.y; a thread owns 2 adjacent columns.
+// Per-sample column sums over the S rows of sample b = blockIdx.y, 128 columns per CTA: a lane owns 4 adjacent columns, a
+// warp every eighth row with four rows in flight, the warps' sums are added in order through shared memory.
 //   MODE 0 (modulation):  out_a[b, c] = sum_s dy * xhat   (xhat from x, mean, rstd),  out_b[b, c] = sum_s dy
 //   MODE 1 (gate):        out_a[b, c] = sum_s dy * x      (x is the gated branch y),  out_b unused
+// (One thread per two columns walked all S rows one load at a time: 8 samples of 512 x 3072 with the gate's row kernel 99 us,
+// now 42; 2 of 4096 x 3072 665 us, now 187.)
 template <int MODE>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
 sample_colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, float* __restrict__ out_a,
                      float* __restrict__ out_b, int D, int S) {
-  const int c = (blockIdx.x * 128 + threadIdx.x) * 2;
-  if (c >= D) return;
+  __shared__ float sm[MODE == 0 ? 2 : 1][8][128];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 128 + lane * 4;               // (D is a multiple of 256)
   const long long b = blockIdx.y;
-  float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
-  for (int s = 0; s < S; ++s) {
+  float a[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (int s = warp; s < S; s += 8) {
     const long long row = b * S + s;
-    const float2 g = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(dy + row * D + c));
-    float2 xv = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(x + row * D + c));
+    const uint2 ug = *reinterpret_cast<const uint2*>(dy + row * D + c), ux = *reinterpret_cast<const uint2*>(x + row * D + c);
+    const float2 g0 = unpack_bf16x2(ug.x), g1 = unpack_bf16x2(ug.y), x0 = unpack_bf16x2(ux.x), x1 = unpack_bf16x2(ux.y);
+    const float g[4] = {g0.x, g0.y, g1.x, g1.y};
+    float v[4] = {x0.x, x0.y, x1.x, x1.y};
     if (MODE == 0) {
       const float m = mean_in[row], r = rstd_in[row];
-      xv.x = (xv.x - m) * r; xv.y = (xv.y - m) * r;
-      b0 += g.x; b1 += g.y;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { v[j] = (v[j] - m) * r; e[j] += g[j]; }
     }
-    a0 += g.x * xv.x; a1 += g.y * xv.y;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) a[j] += g[j] * v[j];
   }
-  out_a[b * D + c] = a0; out_a[b * D + c + 1] = a1;
-  if (MODE == 0) { out_b[b * D + c] = b0; out_b[b * D + c + 1] = b1; }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    sm[0][warp][lane * 4 + j] = a[j];
+    if (MODE == 0) sm[MODE == 0 ? 1 : 0][warp][lane * 4 + j] = e[j];
+  }
+  __syncthreads();
+  const int which = threadIdx.x >> 7, col = threadIdx.x & 127;
+  if (which == 0 || MODE == 0) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += sm[MODE == 0 ? which : 0][k][col];
+    (which == 0 ? out_a : out_b)[b * D + blockIdx.x * 128 + col] = t;
+  }
 }
 
 // out = res + y * gate[b]   (BWD = 0)    |    dy = dout * gate[b]   (BWD = 1, res unused)
@@ -194,7 +213,7 @@ B200_API int b200_ln_modulate_bwd(const void* dy, const void* x, const void* sca
   if (int r = check_shapes("ln_modulate_bwd", T, D, S, ld_mod, scale, scale)) return r;
   ln_modulate_bwd_kernel<<<(T + 7) / 8, 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)scale, ld_mod, mean, rstd, (__nv_bfloat16*)dx, T, D, S);
-  sample_colsum_kernel<0><<<dim3((D / 2 + 127) / 128, T / S), 128, 0, (cudaStream_t)stream>>>(
+  sample_colsum_kernel<0><<<dim3(D / 128, T / S), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, mean, rstd, dscale, dshift, D, S);
   b200::count_launch(2);
   return b200::check_launch("ln_modulate_bwd");
@@ -220,7 +239,7 @@ B200_API int b200_gate_residual_bwd(const void* dout, const void* y, const void*
   const int grid = (int)((n8 + 255) / 256 < 148 * 16 ? (n8 + 255) / 256 : 148 * 16);
   gate_kernel<1><<<grid, 256, 0, (cudaStream_t)stream>>>(nullptr, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)gate, ld_mod,
                                                          (__nv_bfloat16*)dy, n8, D / 8, S);
-  sample_colsum_kernel<1><<<dim3((D / 2 + 127) / 128, T / S), 128, 0, (cudaStream_t)stream>>>(
+  sample_colsum_kernel<1><<<dim3(D / 128, T / S), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)dout, (const __nv_bfloat16*)y, nullptr, nullptr, dgate, nullptr, D, S);
   b200::count_launch(2);
   return b200::check_launch("gate_residual_bwd");

@@ -12,6 +12,8 @@
 // They replace chains of element-wise torch ops (LayerNorm, multiply, add, broadcast) and stand for the
 // reference's fused diffusion glue, which it obtains from per-block torch.compile and Primus fusions
 // (flux1/primus/config_common.sh:84-150).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "runtime.h"
 
@@ -117,24 +119,28 @@ ln_modulate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16
   }
 }
 
-// Per-sample column sums over the S rows of sample b = blockIdx.y, 128 columns per CTA: a lane owns 4 adjacent columns, a
-// warp every eighth row with four rows in flight, the warps' sums are added in order through shared memory.
+// Column sums over the S rows of each sample, 128 columns per CTA: a lane owns 4 adjacent columns, a warp every eighth row with
+// four rows in flight; the CTAs of a cluster take the rows in turn.  Warps and then CTAs (through their shared memory) are added
+// in order by the cluster's first CTA, so the result is the same on every run.
 //   MODE 0 (modulation):  out_a[b, c] = sum_s dy * xhat   (xhat from x, mean, rstd),  out_b[b, c] = sum_s dy
 //   MODE 1 (gate):        out_a[b, c] = sum_s dy * x      (x is the gated branch y),  out_b unused
-// (One thread per two columns walked all S rows one load at a time: 8 samples of 512 x 3072 with the gate's row kernel 99 us,
-// now 42; 2 of 4096 x 3072 665 us, now 187.)
+// (One thread per two columns walked all S rows one load at a time: gate gradient with its row kernel, 8 samples of 512 x 3072
+// 99 us, now 30; 2 of 4096 x 3072 665 us, now 58.)
 template <int MODE>
 __global__ void __launch_bounds__(256)
 sample_colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, float* __restrict__ out_a,
                      float* __restrict__ out_b, int D, int S) {
+  namespace cg = cooperative_groups;
   __shared__ float sm[MODE == 0 ? 2 : 1][8][128];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int parts = cluster.num_blocks(), part = cluster.block_rank();   // (the cluster spans y alone)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 128 + lane * 4;               // (D is a multiple of 256)
-  const long long b = blockIdx.y;
+  const long long b = blockIdx.y / parts;
   float a[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
-  for (int s = warp; s < S; s += 8) {
+  for (int s = part * 8 + warp; s < S; s += parts * 8) {
     const long long row = b * S + s;
     const uint2 ug = *reinterpret_cast<const uint2*>(dy + row * D + c), ux = *reinterpret_cast<const uint2*>(x + row * D + c);
     const float2 g0 = unpack_bf16x2(ug.x), g1 = unpack_bf16x2(ug.y), x0 = unpack_bf16x2(ux.x), x1 = unpack_bf16x2(ux.y);
@@ -155,12 +161,22 @@ sample_colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   }
   __syncthreads();
   const int which = threadIdx.x >> 7, col = threadIdx.x & 127;
-  if (which == 0 || MODE == 0) {
-    float t = 0.f;
+  const bool mine = which < (MODE == 0 ? 2 : 1);
+  float* slot = &sm[MODE == 0 ? which : 0][0][col];
+  float t = 0.f;
+  if (mine) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) t += sm[MODE == 0 ? which : 0][k][col];
-    (which == 0 ? out_a : out_b)[b * D + blockIdx.x * 128 + col] = t;
+    for (int k = 0; k < 8; ++k) t += slot[k * 128];
+    *slot = t;                                             // (read and written by this thread alone)
   }
+  if (parts > 1) {
+    cluster.sync();
+    if (part == 0 && mine)
+      for (int k = 1; k < parts; ++k) t += *cluster.map_shared_rank(slot, k);
+    cluster.sync();                                        // no CTA leaves while its sums are read
+  }
+  const int oc = blockIdx.x * 128 + col;
+  if (part == 0 && mine) (which == 0 ? out_a : out_b)[b * D + oc] = t;
 }
 
 // out = res + y * gate[b]   (BWD = 0)    |    dy = dout * gate[b]   (BWD = 1, res unused)
@@ -184,6 +200,32 @@ gate_kernel(const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restri
     }
     reinterpret_cast<uint4*>(out)[i] = make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
   }
+}
+
+// Rows of a sample are shared by a cluster of up to 8 CTAs while the grid has fewer than 4 CTAs an SM and each of their warps
+// keeps at least four rows (2 samples of 4096 x 3072: 187 us with one CTA a tile, 58 with eight; 8 of 512: 42 and 30).
+template <int MODE>
+int launch_colsum(const void* dy, const void* x, const float* mean, const float* rstd, float* out_a, float* out_b, int samples, int D,
+                  int S, cudaStream_t stream) {
+  const long long tiles = D / 128;
+  int parts = 1;
+  while (parts < 8 && tiles * samples * parts < 4 * b200::sm_count() && S >= parts * 64) parts *= 2;
+  if ((long long)samples * parts > 65535) return b200::fail(1503, "column sums: %d samples are too many", samples);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)tiles, samples * parts);
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1;
+  attr.val.clusterDim.y = parts;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, sample_colsum_kernel<MODE>, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, mean, rstd,
+                                           out_a, out_b, D, S);
+  if (e != cudaSuccess) return b200::fail(1504, "column sums: launch failed: %s", cudaGetErrorString(e));
+  return 0;
 }
 
 int check_shapes(const char* what, int T, int D, int S, long long ld_mod, const void* a, const void* b) {
@@ -213,8 +255,7 @@ B200_API int b200_ln_modulate_bwd(const void* dy, const void* x, const void* sca
   if (int r = check_shapes("ln_modulate_bwd", T, D, S, ld_mod, scale, scale)) return r;
   ln_modulate_bwd_kernel<<<(T + 7) / 8, 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)scale, ld_mod, mean, rstd, (__nv_bfloat16*)dx, T, D, S);
-  sample_colsum_kernel<0><<<dim3(D / 128, T / S), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, mean, rstd, dscale, dshift, D, S);
+  if (int r = launch_colsum<0>(dy, x, mean, rstd, dscale, dshift, T / S, D, S, (cudaStream_t)stream)) return r;
   b200::count_launch(2);
   return b200::check_launch("ln_modulate_bwd");
 }
@@ -239,8 +280,7 @@ B200_API int b200_gate_residual_bwd(const void* dout, const void* y, const void*
   const int grid = (int)((n8 + 255) / 256 < 148 * 16 ? (n8 + 255) / 256 : 148 * 16);
   gate_kernel<1><<<grid, 256, 0, (cudaStream_t)stream>>>(nullptr, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)gate, ld_mod,
                                                          (__nv_bfloat16*)dy, n8, D / 8, S);
-  sample_colsum_kernel<1><<<dim3(D / 128, T / S), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)dout, (const __nv_bfloat16*)y, nullptr, nullptr, dgate, nullptr, D, S);
+  if (int r = launch_colsum<1>(dout, y, nullptr, nullptr, dgate, nullptr, T / S, D, S, (cudaStream_t)stream)) return r;
   b200::count_launch(2);
   return b200::check_launch("gate_residual_bwd");
 }

@@ -8,7 +8,7 @@ from mlperf_training_b200.ops._lib import call, ptr, stream_ptr
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("B,S,D", [(1, 1, 256), (2, 7, 512), (3, 33, 768), (1, 8, 1280), (2, 501, 3072)])
+@pytest.mark.parametrize("B,S,D", [(1, 1, 256), (2, 7, 512), (3, 33, 768), (1, 129, 1280), (2, 501, 3072), (40, 9, 2048)])
 def test_sample_sums(B, S, D):
     torch.manual_seed(S)
     T = B * S

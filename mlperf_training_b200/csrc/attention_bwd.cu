@@ -14,8 +14,12 @@
 //
 // 512 threads: warp 0 TMA producer, warp 1 MMA issuer, warps 4-7 dQ drain (TMEM -> registers, accumulator released,
 // registers -> shared memory -> fp32 TMA reduce-add), warps 8-15 workers.  Two workers share a TMEM lane quarter (32 key
-// rows): each takes half of the 128 query columns.  A quarter of the exponentials is evaluated with a polynomial on the FMA
-// pipe.  TMEM (512 columns): S^T / P^T | dP^T, then dQ | dK | dV.  Order of the MMAs of step i, Q double-buffered:
+// rows): each takes half of the 128 query columns.  Every exponential is ex2.approx: a polynomial on the
+// FMA pipe (relative error up to 7e-4, as the forward takes for a quarter of the keys) for a quarter of the query columns was
+// neither exact nor the forward's P, and added up to 0.13 % to the errors of dQ and dK against 64 bits (6 draws of 5 shapes
+// up to 2048 x 128).  On the MUFU unit alone they are 0.02 to 0.25 % below those of the forward's own P, in the same time:
+// 8192 x 32 / 8 heads of 128 1305 (polynomial) and 1310 us, 4 x 2048 400 and 404, 8 x 512 x 24 full 136 and 133.
+// TMEM (512 columns): S^T / P^T | dP^T, then dQ | dK | dV.  Order of the MMAs of step i, Q double-buffered:
 //     [P^T(i) written]  dV(i)   [dS^T(i) written]  dQ(i)  S(i+1)  dK(i)  [dQ(i) drained]  dP(i+1)
 // so dQ(i) is drained and S(i+1) exponentiated while the tensor core runs dK(i) and dP(i+1).  (The drain has warps of its
 // own: staged by the workers, its 64 KB a step took 3000 of their 6700 cycles, clock64 in the roles.)
@@ -36,10 +40,6 @@ constexpr int NTHREADS = 512;  // warp 0 TMA, 1 MMA (2, 3 complete the warpgroup
 // 4 x 128 threads launch with 128 registers each: 88 + 88 + 2 x 168
 constexpr int REGS_OTHER = 88, REGS_WORKER = 168;
 constexpr int STG = 4096;  // dQ staging chunk: 32 rows x 32 fp32 (two per drain warp)
-#ifndef B200_ATTN_BWD_POLY
-#define B200_ATTN_BWD_POLY 6
-#endif
-constexpr int POLY = B200_ATTN_BWD_POLY;   // pairs with (i & POLY) == POLY take the FMA-pipe polynomial: 6 = a quarter, 2 = half
 
 struct BwdParams {
   int B, Hq, Hkv, Sq, Skv;
@@ -362,12 +362,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const float4 l4 = *reinterpret_cast<const float4*>(ld + i);
           const float2 a = ffma2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), sc2, make_float2(-l4.x, -l4.y));
           const float2 c = ffma2(make_float2(__uint_as_float(s[i + 2]), __uint_as_float(s[i + 3])), sc2, make_float2(-l4.z, -l4.w));
-          float2 e0, e1;
-          if ((i & POLY) == POLY) e0 = ex2_poly2(a);
-          else e0 = make_float2(ex2_approx(a.x), ex2_approx(a.y));
-          if (((i + 2) & POLY) == POLY) e1 = ex2_poly2(c);
-          else e1 = make_float2(ex2_approx(c.x), ex2_approx(c.y));
-          pr[i] = e0.x; pr[i + 1] = e0.y; pr[i + 2] = e1.x; pr[i + 3] = e1.y;
+          pr[i] = ex2_approx(a.x); pr[i + 1] = ex2_approx(a.y); pr[i + 2] = ex2_approx(c.x); pr[i + 3] = ex2_approx(c.y);
         }
       }
       if (need_mask) {

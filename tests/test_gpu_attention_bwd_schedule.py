@@ -32,3 +32,16 @@ def test_backward(B, Sq, Skv, Hq, Hkv, D, causal, window, sink):
     for a, b in zip((dq, dk, dv, ds) if sink else (dq, dk, dv), want):
         assert (a.double() - b).norm() <= 2 ** -7 * b.norm() + 1e-5 * do.double().norm()
     _lib.check_status("attention_bwd")
+
+
+@pytest.mark.parametrize("Sq,D", [(128, 128), (320, 64)])
+def test_equal_queries_have_equal_gradients(Sq, D):
+    """Probabilities must not depend on where in its tile a query stands: equal rows of q and dO give bit-equal rows of dQ (one
+    key tile, so every row is a single sum)."""
+    torch.manual_seed(D)
+    k, v = (torch.randn(1, 128, 2, D, device="cuda").bfloat16() for _ in range(2))
+    q, do = (torch.randn(1, 1, 2, D, device="cuda").bfloat16().expand(1, Sq, 2, D).contiguous() for _ in range(2))
+    out, lse = K.attention_fwd(q, k, v, causal=False)
+    dq = K.attention_bwd(do, q, k, v, out, lse, causal=False)[0]
+    assert dq.any() and torch.equal(dq, dq[:, :1].expand_as(dq))
+    _lib.check_status("attention_bwd")

@@ -200,7 +200,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint64_t mdO = umma_desc_sw128(smem_u32(sdO), 128 * 128, 1024);
       auto issue_s = [&](int it) -> bool {
         const int st = it & 1;
-        if (!mbar_wait_spin(&q_full[st], (it >> 1) & 1, abort_flag, p.status, 81)) return false;
+        if (!warp_wait_spin(&q_full[st], (it >> 1) & 1, abort_flag, p.status, 81)) return false;
         tc_fence_after();
         if (elect_one()) {
           const uint64_t bd = kQ + (st * SM::T_BYTES >> 4);
@@ -215,7 +215,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         return true;
       };
       auto issue_dp = [&](int it) -> bool {
-        if (!mbar_wait_spin(do_full, it & 1, abort_flag, p.status, 82)) return false;
+        if (!warp_wait_spin(do_full, it & 1, abort_flag, p.status, 82)) return false;
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -228,12 +228,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         __syncwarp();
         return true;
       };
-      bool ok = mbar_wait_spin(kv_full, 0, abort_flag, p.status, 80) && issue_s(0) && issue_dp(0);
+      bool ok = warp_wait_spin(kv_full, 0, abort_flag, p.status, 80) && issue_s(0) && issue_dp(0);
       for (int it = 0; it < n_iter && ok; ++it) {
         const uint32_t ph = it & 1;
         const int st = it & 1;
         const bool last = it == n_iter - 1;
-        if (!mbar_wait_spin(p_full, ph, abort_flag, p.status, 83)) { ok = false; break; }
+        if (!warp_wait_spin(p_full, ph, abort_flag, p.status, 83)) { ok = false; break; }
         tc_fence_after();
         if (elect_one()) {
           // dV += P^T dO : 16 queries = 8 TMEM columns per step, dO as 16 query rows of 128 bytes
@@ -243,7 +243,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tc_commit(do_empty);
         }
         __syncwarp();
-        if (!mbar_wait_spin(ds_full, ph, abort_flag, p.status, 84)) { ok = false; break; }
+        if (!warp_wait_spin(ds_full, ph, abort_flag, p.status, 84)) { ok = false; break; }
         tc_fence_after();
         if (elect_one()) {
           // dQ = dS K : contraction over keys, 16 key rows of the dS^T tile and of K per step
@@ -265,7 +265,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (last) tc_commit(acc_done);
         }
         __syncwarp();
-        if (!last) ok = mbar_wait_spin(dq_drained, ph, abort_flag, p.status, 85) && issue_dp(it + 1);
+        if (!last) ok = warp_wait_spin(dq_drained, ph, abort_flag, p.status, 85) && issue_dp(it + 1);
       }
     }
   } else if (warp >= 4 && warp < 8) {
@@ -276,7 +276,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     for (int it = 0; it < n_iter; ++it) {
       const int h = hk * group + it / n_q;
       const int q0 = (i_lo + it % n_q) * BQ;
-      if (!mbar_wait(dq_full, it & 1, abort_flag, p.status, 95)) break;
+      if (!warp_wait(dq_full, it & 1, abort_flag, p.status, 95)) break;
       tc_fence_after();
 #pragma unroll
       for (int c2 = 0; c2 < HD / 64; ++c2) {       // 64 columns at a time: two staging buffers
@@ -346,9 +346,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (p.causal) c_lo = key - off - q0;
       if (p.window > 0) c_hi = key - off - q0 + p.window;
       if (key >= p.Skv) c_hi = c_lo = 0;
-      if (!mbar_wait(&ld_full[it & 1], (it >> 1) & 1, abort_flag, p.status, 89)) { ok = false; break; }
+      if (!warp_wait(&ld_full[it & 1], (it >> 1) & 1, abort_flag, p.status, 89)) { ok = false; break; }
       const float* ld = sLD + (it & 1) * 2 * BQ + half * 64;
-      if (!mbar_wait(s_full, it & 1, abort_flag, p.status, 90)) { ok = false; break; }
+      if (!warp_wait(s_full, it & 1, abort_flag, p.status, 90)) { ok = false; break; }
       tc_fence_after();
       float pr[64];
       {
@@ -382,7 +382,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full);
       }
-      if (!mbar_wait(dp_full, it & 1, abort_flag, p.status, 91)) { ok = false; break; }
+      if (!warp_wait(dp_full, it & 1, abort_flag, p.status, 91)) { ok = false; break; }
       tc_fence_after();
       uint8_t* drow = sdS + half * (BKV * 128) + r * 128;       // 64 queries of key r
 #pragma unroll
@@ -421,7 +421,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     // ------------------------------ dK / dV epilogue ------------------------------
     // workers of half 0 write dK (staged in the dS tile), those of half 1 write dV (staged in the first Q stage)
-    if (ok && n_iter > 0) ok = mbar_wait(acc_done, 0, abort_flag, p.status, 92);
+    if (ok && n_iter > 0) ok = warp_wait(acc_done, 0, abort_flag, p.status, 92);
     if (ok) {
       tc_fence_after();
       uint8_t* tile = (half == 0) ? sdS : sQ;

@@ -225,7 +225,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (u >= p.items) continue;
         const Item it = make_item(u, p);
         if (it.n_max == 0) continue;
-        if (!mbar_wait_spin(q_full, nq & 1, abort_flag, p.status, 50)) { ok = false; break; }
+        if (!warp_wait_spin(q_full, nq & 1, abort_flag, p.status, 50)) { ok = false; break; }
         ++nq;
         int k_ready = -1, v_ready = -1;      // last key tile of the item whose full barrier has been observed
         int s_left = (it.hi0 - it.lo0) + (it.hi1 - it.lo1);
@@ -234,7 +234,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           const int st = (kv + n) & 1;
           while (k_ready < n) {
             ++k_ready;
-            if (!mbar_wait_spin(&k_full[(kv + k_ready) & 1], ((kv + k_ready) >> 1) & 1, abort_flag, p.status, 51)) return false;
+            if (!warp_wait_spin(&k_full[(kv + k_ready) & 1], ((kv + k_ready) >> 1) & 1, abort_flag, p.status, 51)) return false;
           }
           // the last S that reads K(n) frees its stage: S_t(n) is issued in step n - 1 (its first one before step 0)
           const int o = 1 - t;
@@ -267,12 +267,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if (!ok || n < it.lo(t) || n >= it.hi(t)) continue;
             const bool first = n == it.lo(t), last = n == it.hi(t) - 1;
             // O of the previous item has left TMEM
-            if (first && !mbar_wait_spin(&o_free[t], (no[t] & 1) ^ 1, abort_flag, p.status, 52)) { ok = false; continue; }
+            if (first && !warp_wait_spin(&o_free[t], (no[t] & 1) ^ 1, abort_flag, p.status, 52)) { ok = false; continue; }
             while (ok && v_ready < n) {
               ++v_ready;
-              ok = mbar_wait_spin(&v_full[(kv + v_ready) & 1], ((kv + v_ready) >> 1) & 1, abort_flag, p.status, 54);
+              ok = warp_wait_spin(&v_full[(kv + v_ready) & 1], ((kv + v_ready) >> 1) & 1, abort_flag, p.status, 54);
             }
-            ok = ok && mbar_wait_spin(&p_early[t], np[t] & 1, abort_flag, p.status, 53);
+            ok = ok && warp_wait_spin(&p_early[t], np[t] & 1, abort_flag, p.status, 53);
             if (!ok) continue;
             tc_fence_after();
             // A = P_t in TMEM: 16 bf16 keys = 8 columns per step; B = V: 16 key rows of 128 bytes
@@ -284,7 +284,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                               (!first || kk > 0) ? 1u : 0u);
             }
             __syncwarp();
-            ok = mbar_wait_spin(&p_full[t], np[t] & 1, abort_flag, p.status, 55);
+            ok = warp_wait_spin(&p_full[t], np[t] & 1, abort_flag, p.status, 55);
             if (!ok) continue;
             tc_fence_after();
             const bool free_v = (t == 1) || !(n >= it.lo1 && n < it.hi1);
@@ -328,7 +328,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       float m_ref = -INFINITY, l = 0.f;
       for (int n = it.lo(t); n < it.hi(t); ++n, ++ns) {
         const int kv0 = (it.j_lo + n) * BKV;
-        if (!mbar_wait(&s_full[t], ns & 1, abort_flag, p.status, 60)) { ok = false; break; }
+        if (!warp_wait(&s_full[t], ns & 1, abort_flag, p.status, 60)) { ok = false; break; }
         tc_fence_after();
         const bool need_mask = (kv0 + BKV > p.Skv) || (p.causal && kv0 + BKV - 1 > qt0 + off) ||
                                (p.window > 0 && kv0 < qt0 + BQ - 1 + off - p.window + 1);
@@ -408,7 +408,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         l += (rs2[0].x + rs2[0].y) + (rs2[1].x + rs2[1].y);
       }
       // ------------------------------ epilogue ------------------------------
-      if (!ok || !mbar_wait(&o_done[t], no & 1, abort_flag, p.status, 62)) { ok = false; break; }
+      if (!ok || !warp_wait(&o_done[t], no & 1, abort_flag, p.status, 62)) { ok = false; break; }
       ++no;
       tc_fence_after();
       if (p.sink != nullptr) {

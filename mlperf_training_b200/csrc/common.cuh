@@ -160,6 +160,38 @@ B200_DEVICE bool mbar_wait_spin(uint64_t* bar, uint32_t parity, volatile int* ab
   return true;
 }
 
+// Waits of a role that walks its schedule as a whole warp (elect.sync, tcgen05.ld / st, __syncwarp behind the wait): the warp
+// goes on when every lane has seen the phase, or gives up as one.  With a wait per lane some could see the phase at the limit
+// while others gave up, and those that went on would stand at the next warp-wide instruction for good.  Never call these from
+// one lane.
+template <bool SPIN>
+B200_DEVICE bool warp_wait_impl(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int where) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  uint64_t t0 = 0;
+  uint32_t it = 0;
+  while (!__all_sync(0xffffffffu, SPIN ? mbar_try_wait(bar, parity) : mbar_try_wait_hint(bar, parity, 20000u))) {
+    if ((++it & (SPIN ? 0xffu : 0xfu)) == 0) {
+      bool quit = *abort_flag != 0;
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      else if (!quit && now - t0 > B200_WAIT_LIMIT_NS) {
+        b200_report(status, B200_ERR_TIMEOUT_MBAR, where);
+        *abort_flag = 1;
+        __threadfence_block();
+        quit = true;
+      }
+      if (__any_sync(0xffffffffu, quit)) return false;
+    }
+  }
+  return true;
+}
+B200_DEVICE bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int where) {
+  return warp_wait_impl<false>(bar, parity, abort_flag, status, where);
+}
+B200_DEVICE bool warp_wait_spin(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int where) {
+  return warp_wait_impl<true>(bar, parity, abort_flag, status, where);
+}
+
 // Bounded acquire-wait on a 32-bit flag in global (possibly peer) memory: flag >= want.
 B200_DEVICE bool flag_wait_geq(const int* flag, int want, uint64_t limit_ns, int* status, int where) {
   uint64_t t0 = 0;

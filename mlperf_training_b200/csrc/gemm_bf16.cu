@@ -166,7 +166,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int mb, nb; tile_coords(t, num_m, num_n, p.group_m, mb, nb);
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
-      if (!mbar_wait(&tfull[acc], acc_phase, abort_flag, p.status, 30)) { ok = false; break; }
+      if (!warp_wait(&tfull[acc], acc_phase, abort_flag, p.status, 30)) { ok = false; break; }
       tc_fence_after();
       const uint32_t t_row = tmem_base + (uint32_t(q * 32) << 16) + acc * BN;
       gemmcore::epilogue_drain<BN, true>(&tmD, &tmD, p.epi, t_row, mb * BM + q * 32, nb * BN, stg, buf, lane);

@@ -675,12 +675,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
         ++it;
-        if (!mbar_wait(&tempty[acc], acc_phase ^ 1, abort_flag, p.status, 320)) { ok = false; break; }
+        if (!warp_wait(&tempty[acc], acc_phase ^ 1, abort_flag, p.status, 320)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < ti.nkb && ok; ++kb) {
-          if (!mbar_wait_spin(&full[stage], phase, abort_flag, p.status, 321)) { ok = false; break; }
-          if (MX && !mbar_wait_spin(&sfrdy[stage], phase, abort_flag, p.status, 322)) { ok = false; break; }
+          if (!warp_wait_spin(&full[stage], phase, abort_flag, p.status, 321)) { ok = false; break; }
+          if (MX && !warp_wait_spin(&sfrdy[stage], phase, abort_flag, p.status, 322)) { ok = false; break; }
           tc_fence_after();
           if (elect_one()) {
 #pragma unroll
@@ -731,7 +731,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
       ++it;
-      if (!mbar_wait(&tfull[acc], acc_phase, abort_flag, p.status, 330)) { ok = false; break; }
+      if (!warp_wait(&tfull[acc], acc_phase, abort_flag, p.status, 330)) { ok = false; break; }
       tc_fence_after();
       const uint32_t t_row = tmem_base + (uint32_t(q * 32) << 16) + acc * BN;
       if (p.rs.on) {
@@ -784,7 +784,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       for (int kb = 0; kb < ti.nkb; ++kb) {
         // the atoms of this stage have landed; its scale sets are free, because the producer loaded the
         // stage only after the MMAs of its previous use had completed
-        if (!mbar_wait_spin(&sffull[stage], phase, abort_flag, p.status, 340)) { ok = false; break; }
+        if (!warp_wait_spin(&sffull[stage], phase, abort_flag, p.status, 340)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
         for (int s = 0; s < KSUB; ++s) {

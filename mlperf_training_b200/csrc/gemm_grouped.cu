@@ -196,7 +196,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
       ++it;
-      if (!mbar_wait(&tfull[acc], acc_phase, abort_flag, p.status, 160)) { ok = false; break; }
+      if (!warp_wait(&tfull[acc], acc_phase, abort_flag, p.status, 160)) { ok = false; break; }
       tc_fence_after();
       const uint32_t t_row = tmem_base + (uint32_t(q * 32) << 16) + acc * BN;
 #pragma unroll 1

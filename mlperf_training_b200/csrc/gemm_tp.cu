@@ -275,7 +275,7 @@ gemm_tp_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const int m0 = mb * BM, n0 = nb * BN;
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
-      if (!mbar_wait(&tfull[acc], acc_phase, abort_flag, p.status, 30)) { ok = false; break; }
+      if (!warp_wait(&tfull[acc], acc_phase, abort_flag, p.status, 30)) { ok = false; break; }
       tc_fence_after();
       const uint32_t t_row = tmem_base + (uint32_t(q * 32) << 16) + acc * BN;
       // mode 3: the tile goes into the owner's staging slot of this rank through the owner's tensor map

@@ -160,7 +160,7 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const uint64_t mdO = umma_desc_sw128(smem_u32(sdO), 128 * 128, 1024);
       auto issue_s = [&](int it) -> bool {
         const int st = it & 1;
-        if (!mbar_wait_spin(&q_full[st], (it >> 1) & 1, abort_flag, p.status, 81)) return false;
+        if (!warp_wait_spin(&q_full[st], (it >> 1) & 1, abort_flag, p.status, 81)) return false;
         tc_fence_after();
         if (elect_one()) {
           const uint64_t bd = kQ + (st * SM::T_BYTES >> 4);
@@ -175,7 +175,7 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         return true;
       };
       auto issue_dp = [&](int it) -> bool {
-        if (!mbar_wait_spin(do_full, it & 1, abort_flag, p.status, 82)) return false;
+        if (!warp_wait_spin(do_full, it & 1, abort_flag, p.status, 82)) return false;
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -188,12 +188,12 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         __syncwarp();
         return true;
       };
-      bool ok = mbar_wait_spin(kv_full, 0, abort_flag, p.status, 80) && issue_s(0) && issue_dp(0);
+      bool ok = warp_wait_spin(kv_full, 0, abort_flag, p.status, 80) && issue_s(0) && issue_dp(0);
       for (int it = 0; it < n_iter && ok; ++it) {
         const uint32_t ph = it & 1;
         const int st = it & 1;
         const bool last = it == n_iter - 1;
-        if (!mbar_wait_spin(p_full, ph, abort_flag, p.status, 83)) { ok = false; break; }
+        if (!warp_wait_spin(p_full, ph, abort_flag, p.status, 83)) { ok = false; break; }
         tc_fence_after();
         if (elect_one()) {
           // dV += P^T dO : 16 queries = 8 TMEM columns per step, dO as 16 query rows of 128 bytes
@@ -203,7 +203,7 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           tc_commit(do_empty);
         }
         __syncwarp();
-        if (!mbar_wait_spin(ds_full, ph, abort_flag, p.status, 84)) { ok = false; break; }
+        if (!warp_wait_spin(ds_full, ph, abort_flag, p.status, 84)) { ok = false; break; }
         tc_fence_after();
         if (elect_one()) {
           // dQ = dS K : contraction over keys, 16 key rows of the dS^T tile and of K per step
@@ -225,7 +225,7 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           if (last) tc_commit(acc_done);
         }
         __syncwarp();
-        if (!last) ok = mbar_wait_spin(dq_drained, ph, abort_flag, p.status, 85) && issue_dp(it + 1);
+        if (!last) ok = warp_wait_spin(dq_drained, ph, abort_flag, p.status, 85) && issue_dp(it + 1);
       }
     }
   } else if (warp >= 4 && warp < 8) {
@@ -235,7 +235,7 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     uint8_t* stg = sStg + q * 2 * STG;
     for (int it = 0; it < n_iter; ++it) {
       const int q0 = q_tile(it) * BQ;
-      if (!mbar_wait(dq_full, it & 1, abort_flag, p.status, 95)) break;
+      if (!warp_wait(dq_full, it & 1, abort_flag, p.status, 95)) break;
       tc_fence_after();
 #pragma unroll
       for (int c2 = 0; c2 < HD / 64; ++c2) {       // 64 columns at a time: two staging buffers
@@ -287,7 +287,7 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int last_k_id = min(max(kv0 + BKV - 1 - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
       const bool inside = (kv0 + BKV <= len) && (q0 + BQ <= len);
       const bool need_mask = plain ? ((kv0 + BKV - 1 > q0) || !inside) : !(inside && first_q_id > last_k_id);
-      if (!mbar_wait(s_full, it & 1, abort_flag, p.status, 90)) { ok = false; break; }
+      if (!warp_wait(s_full, it & 1, abort_flag, p.status, 90)) { ok = false; break; }
       tc_fence_after();
       float f[64];                            // dS / dP of this key and the half's queries
       {
@@ -330,7 +330,7 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full);
       }
-      if (!mbar_wait(dp_full, it & 1, abort_flag, p.status, 91)) { ok = false; break; }
+      if (!warp_wait(dp_full, it & 1, abort_flag, p.status, 91)) { ok = false; break; }
       tc_fence_after();
       uint8_t* drow = sdS + half * (BKV * 128) + r * 128;       // 64 queries of key r
 #pragma unroll
@@ -363,7 +363,7 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // ------------------------------ dK / dV epilogue ------------------------------
     // workers of half 0 write dK, those of half 1 write dV; guarded row stores: rows past the
     // sequence end belong to the next sequence
-    if (ok && n_iter > 0) ok = mbar_wait(acc_done, 0, abort_flag, p.status, 92);
+    if (ok && n_iter > 0) ok = warp_wait(acc_done, 0, abort_flag, p.status, 92);
     if (ok) {
       tc_fence_after();
       const int k_pos = kv0 + r;

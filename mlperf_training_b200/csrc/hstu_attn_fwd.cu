@@ -185,13 +185,13 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const uint32_t idesc_o = umma_idesc(F8 ? 0 : 1, F8 ? 0 : 1, 0, 1, BQ, HD);   // P (TMEM)    x V (MN-major)
       const uint64_t dQ = umma_desc_sw128(smem_u32(sQ), 16, 1024), dK = umma_desc_sw128(smem_u32(sK), 16, 1024);
       const uint64_t dV = umma_desc_sw128(smem_u32(sV), BKV * 128, 1024);
-      bool ok = mbar_wait_spin(q_full, 0, abort_flag, p.status, 50);
+      bool ok = warp_wait_spin(q_full, 0, abort_flag, p.status, 50);
       int k_ready = -1, v_ready = -1;  // last key tile index whose full barrier has been observed
       // S_t(n) = Q_t K(n)^T into the S columns of tile t
       auto issue_s = [&](int t, int n) -> bool {
         const int st = n & 1;
         if (k_ready < n) {
-          if (!mbar_wait_spin(&k_full[st], (n >> 1) & 1, abort_flag, p.status, 51)) return false;
+          if (!warp_wait_spin(&k_full[st], (n >> 1) & 1, abort_flag, p.status, 51)) return false;
           k_ready = n;
         }
         tc_fence_after();
@@ -219,9 +219,9 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (!ok || n >= n_t[t]) continue;
-          ok = mbar_wait_spin(&p_early[t], n & 1, abort_flag, p.status, 53);
+          ok = warp_wait_spin(&p_early[t], n & 1, abort_flag, p.status, 53);
           if (ok && v_ready < n) {
-            ok = mbar_wait_spin(&v_full[st], (n >> 1) & 1, abort_flag, p.status, 54);
+            ok = warp_wait_spin(&v_full[st], (n >> 1) & 1, abort_flag, p.status, 54);
             v_ready = n;
           }
           if (!ok) continue;
@@ -240,7 +240,7 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             for (int kk = 0; kk < STEPS / 2; ++kk) pv(kk);
           }
           __syncwarp();
-          ok = mbar_wait_spin(&p_full[t], n & 1, abort_flag, p.status, 55);
+          ok = warp_wait_spin(&p_full[t], n & 1, abort_flag, p.status, 55);
           if (!ok) continue;
           tc_fence_after();
           if (elect_one()) {
@@ -274,7 +274,7 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     bool ok = true;
     for (int n = 0; n < my_n && ok; ++n) {
       const int kv0 = (j_lo + n) * BKV;
-      if (!mbar_wait(&s_full[t], n & 1, abort_flag, p.status, 170)) { ok = false; break; }
+      if (!warp_wait(&s_full[t], n & 1, abort_flag, p.status, 170)) { ok = false; break; }
       tc_fence_after();
       // tiles strictly below the diagonal and inside the sequence need no element mask
       // (with targets / contextual tokens: ids grow with the position, so every pair of the tile is visible when its
@@ -341,7 +341,7 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (lane == 0) mbar_arrive(&p_full[t]);
     }
     // ------------------------------ epilogue: guarded row stores (rows past the sequence end are not written)
-    if (ok && my_n > 0) ok = mbar_wait(&o_done[t], (my_n - 1) & 1, abort_flag, p.status, 171);
+    if (ok && my_n > 0) ok = warp_wait(&o_done[t], (my_n - 1) & 1, abort_flag, p.status, 171);
     if (ok && my_n > 0) {
       tc_fence_after();
       __nv_bfloat16* orow = p.out + (long long)(row_base + q_pos) * p.out_row + h * HD;

@@ -154,7 +154,7 @@ B200_DEVICE void reduce_cta(const P& p, int num_n, uint8_t* smem, uint64_t* bars
   int st = 0; uint32_t ph = 0;
   const int ctid = threadIdx.x - 32, cn = CONSUMER_WARPS * 32;
   while (true) {
-    if (!mbar_wait(&full[st], ph, abort_flag, p.status, 54)) break;
+    if (!warp_wait(&full[st], ph, abort_flag, p.status, 54)) break;
     const RedMeta m = meta[st];
     if (m.row < 0) break;
     const uint8_t* sb = smem + st * COPY_PIECE;

@@ -162,7 +162,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (warp < 8) reg_dealloc<REGS_OTHER>();
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    // (a key tile that no query sees loads nothing: nobody would wait for it, and the CTA must not leave with copies in flight)
+    if (lane == 0 && n_iter > 0) {
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
       mbar_expect_tx(kv_full, 2 * SM::T_BYTES);
 #pragma unroll

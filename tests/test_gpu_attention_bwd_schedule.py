@@ -1,17 +1,22 @@
-"""Attention backward at the edges of its schedule: one step, odd step counts, ragged tiles, rows without visible keys, windows,
+"""Attention backward at the edges of its schedule: one step, odd step counts, ragged tiles, keys that no query sees, windows,
 more keys than queries, grouped heads."""
+import re
+from pathlib import Path
+
 import pytest
 import torch
 
 from mlperf_training_b200.ops import _lib, kernels as K
 
-pytestmark = pytest.mark.gpu
+gpu = pytest.mark.gpu
 
 
+@gpu
 @pytest.mark.parametrize("B,Sq,Skv,Hq,Hkv,D,causal,window,sink", [
     (1, 1, 1, 1, 1, 128, True, 0, False), (1, 128, 128, 1, 1, 64, True, 0, False), (2, 129, 129, 3, 3, 128, True, 0, False),
     (1, 300, 300, 8, 2, 64, True, 50, True), (1, 500, 500, 4, 1, 128, False, 0, False), (1, 130, 700, 4, 2, 128, True, 0, False),
-    (2, 200, 90, 2, 1, 64, False, 0, False), (1, 1000, 1000, 2, 2, 128, True, 128, False), (1, 383, 383, 6, 2, 64, True, 0, True)])
+    (2, 200, 90, 2, 1, 64, False, 0, False), (1, 1000, 1000, 2, 2, 128, True, 128, False), (1, 383, 383, 6, 2, 64, True, 0, True),
+    (1, 200, 1500, 4, 2, 128, True, 100, False), (2, 70, 900, 2, 1, 64, True, 1, False), (1, 130, 1300, 2, 2, 128, False, 300, True)])
 def test_backward(B, Sq, Skv, Hq, Hkv, D, causal, window, sink):
     torch.manual_seed(Sq + D)
     q, k, v = (torch.randn(B, s, h, D, device="cuda").bfloat16() for s, h in ((Sq, Hq), (Skv, Hkv), (Skv, Hkv)))
@@ -31,9 +36,12 @@ def test_backward(B, Sq, Skv, Hq, Hkv, D, causal, window, sink):
     # products (a single visible key: exactly 0): D * 2^-24 of |dO| |v| <= 1e-5 of |dO| beside the relative part
     for a, b in zip((dq, dk, dv, ds) if sink else (dq, dk, dv), want):
         assert (a.double() - b).norm() <= 2 ** -7 * b.norm() + 1e-5 * do.double().norm()
+    unseen = ~K._attn_mask(Sq, Skv, causal, window, "cuda").any(0)
+    assert not dk[:, unseen].any() and not dv[:, unseen].any()
     _lib.check_status("attention_bwd")
 
 
+@gpu
 @pytest.mark.parametrize("Sq,D", [(128, 128), (320, 64)])
 def test_equal_queries_have_equal_gradients(Sq, D):
     """Probabilities must not depend on where in its tile a query stands: equal rows of q and dO give bit-equal rows of dQ (one
@@ -45,3 +53,11 @@ def test_equal_queries_have_equal_gradients(Sq, D):
     dq = K.attention_bwd(do, q, k, v, out, lse, causal=False)[0]
     assert dq.any() and torch.equal(dq, dq[:, :1].expand_as(dq))
     _lib.check_status("attention_bwd")
+
+
+def test_copies_are_issued_only_where_they_are_awaited():
+    """A key tile without queries (``n_iter == 0``) skips every wait of the kernel, so it may not start a copy either: read from
+    the source, since a CTA that leaves with copies in flight corrupts its successor's shared memory."""
+    text = (Path(__file__).resolve().parent.parent / "mlperf_training_b200/csrc/attention_bwd.cu").read_text()
+    role = text[text.index("TMA producer -"):text.index("MMA issuer -")]
+    assert role.index("n_iter > 0") < role.index("mbar_expect_tx(kv_full") and re.search(r"if \([^)]*n_iter > 0\) \{", role)

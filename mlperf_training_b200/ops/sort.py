@@ -38,17 +38,6 @@ def key_bits_for(rows: int) -> int:
     return max(int(rows - 1).bit_length(), 1)
 
 
-_scratch: dict = {}
-
-
-def _scratch_for(n: int, device) -> torch.Tensor:
-    need = int(load().b200_sort_scratch_bytes(n))
-    buf = _scratch.get(device)
-    if buf is None or buf.numel() < need:
-        buf = _scratch[device] = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=device)
-    return buf
-
-
 def sort_unique(ids: torch.Tensor, key_bits: int = 64) -> SortedIds:
     ids = ids.reshape(-1).to(torch.int64)
     n = ids.numel()
@@ -74,7 +63,8 @@ def sort_unique(ids: torch.Tensor, key_bits: int = 64) -> SortedIds:
     inverse = torch.empty_like(ids)
     count = torch.zeros(1, dtype=torch.int64, device=dev)
     if n:
-        scratch = _scratch_for(n, dev)
+        # (per call, from the caching allocator on the calling stream: sorts on other streams or threads have their own)
+        scratch = torch.empty(int(load().b200_sort_scratch_bytes(n)), dtype=torch.uint8, device=dev)
         call("b200_sort_ids", ptr(ids.contiguous()), ptr(keys), ptr(perm), n, int(min(max(key_bits, 1), 64)), ptr(scratch),
              scratch.numel(), stream_ptr())
         call("b200_unique_segments", ptr(keys), ptr(perm), n, ptr(uniq), ptr(seg), ptr(inverse), ptr(count), ptr(scratch),

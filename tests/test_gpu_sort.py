@@ -5,9 +5,10 @@ import torch
 from mlperf_training_b200.ops import _lib, sort
 from mlperf_training_b200.parallel.embedding import ShardedEmbedding
 
-pytestmark = pytest.mark.gpu
+gpu = pytest.mark.gpu
 
 
+@gpu
 @pytest.mark.parametrize("n,rows", [(1, 10), (1000, 50), (200_003, 400_000_000), (65_536, 3)])
 def test_sort_unique_and_segment_sum(n, rows):
     g = torch.Generator().manual_seed(n)
@@ -30,6 +31,7 @@ def test_sort_unique_and_segment_sum(n, rows):
     assert torch.equal(b2, sort.segment_sum(src.cuda(), d, torch.float32))                  # run twice: bit-identical
 
 
+@gpu
 def test_segment_sum_long_runs():
     """Skewed ids: runs longer than one warp's share (summed through per-block partial sums), runs that start in the
     middle of a block, a run of exactly the block size, next to ordinary short runs."""
@@ -50,6 +52,7 @@ def test_segment_sum_long_runs():
         assert torch.equal(b, sort.segment_sum(src.cuda(), d, torch.float32))               # bit-identical when repeated
 
 
+@gpu
 def test_embedding_backward_is_deterministic_and_matches_cpu():
     torch.manual_seed(0)
     ids = torch.randint(0, 500, (4000,))
@@ -64,3 +67,47 @@ def test_embedding_backward_is_deterministic_and_matches_cpu():
     torch.cuda.synchronize()
     assert torch.equal(res[1], res[2])
     assert (res[0] - res[1]).abs().max() < 1e-5
+
+
+def test_sorts_in_flight_share_no_scratch(monkeypatch):
+    """Two sorts that are in flight together (here: the second one starts inside the first one's launch) work in buffers of
+    their own."""
+    seen = []
+
+    class Lib:
+        @staticmethod
+        def b200_sort_scratch_bytes(n):
+            return 16 * n + 256
+
+    def call(name, *args):
+        seen.append((name, args[6] if name == "b200_unique_segments" else args[5]))
+        if len(seen) == 1:
+            sort.sort_unique(torch.arange(50))
+
+    monkeypatch.setattr(sort, "use_kernels", lambda t: True)
+    monkeypatch.setattr(sort, "load", lambda: Lib)
+    monkeypatch.setattr(sort, "call", call)
+    monkeypatch.setattr(sort, "stream_ptr", lambda: 0)
+    sort.sort_unique(torch.arange(100))
+    outer, inner = {seen[0][1]}, {p for _, p in seen[1:3]}
+    assert len(seen) == 4 and not outer & inner
+
+
+@gpu
+def test_sorts_on_two_streams():
+    """Sorts issued on two streams without a host read between them: each gives what it gives alone."""
+    g = torch.Generator(device="cuda").manual_seed(0)
+    ids = [torch.randint(0, 50_000, (300_000,), generator=g, device="cuda") for _ in range(8)]
+    want = [sort.sort_unique(i, 16) for i in ids]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    got = [None] * len(ids)
+    for i, t in enumerate(ids):
+        with torch.cuda.stream(streams[i % 2]):
+            got[i] = sort.sort_unique(t, 16)
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        n = int(b.count)
+        assert int(a.count) == n and torch.equal(a.keys, b.keys) and torch.equal(a.perm, b.perm)
+        assert torch.equal(a.inverse, b.inverse) and torch.equal(a.seg[:n + 1], b.seg[:n + 1]) and torch.equal(a.uniq[:n], b.uniq[:n])
+    _lib.check_status("sort")

@@ -35,6 +35,7 @@ struct HstuBwdParams {
   __nv_bfloat16* dv;
   long long dk_row, dv_row;
   int tiles_outer;          // grid order: 1 = key tile slowest, 0 = (sequence, head) slowest
+  int num_bh, num_kt;       // (sequence, head) pairs and key tiles: the grid is their product along x, which has no 65,535 limit
   int* status;
 };
 
@@ -84,8 +85,9 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int jt = p.tiles_outer ? blockIdx.y : blockIdx.x;
-  const int bh = p.tiles_outer ? blockIdx.x : blockIdx.y;
+  const int x = (int)blockIdx.x;
+  const int jt = p.tiles_outer ? x / p.num_bh : x % p.num_kt;
+  const int bh = p.tiles_outer ? x % p.num_bh : x / p.num_kt;
   const int hk = bh % p.H, b = bh / p.H;
   const int row_base = p.offsets[b];
   const int len = p.offsets[b + 1] - row_base;
@@ -398,7 +400,7 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 }
 
 template <int HD>
-int launch_hstu_bwd(const CUtensorMap* m, const HstuBwdParams& p, int B, cudaStream_t stream) {
+int launch_hstu_bwd(const CUtensorMap* m, const HstuBwdParams& p, cudaStream_t stream) {
   using SM = Smem<HD>;
   static bool configured[64] = {false};
   int dev = 0;
@@ -408,10 +410,9 @@ int launch_hstu_bwd(const CUtensorMap* m, const HstuBwdParams& p, int B, cudaStr
     if (e != cudaSuccess) { cudaGetLastError(); return b200::fail(1211, "hstu_attn_bwd: cannot set %d bytes of shared memory: %s", SM::TOTAL, cudaGetErrorString(e)); }
     configured[dev & 63] = true;
   }
-  const unsigned bh = (unsigned)(p.H * B), kt = (p.max_len + BKV - 1) / BKV;
-  if (!p.tiles_outer && bh > 65535u) return b200::fail(1212, "hstu_attn_bwd: %u sequences x heads", bh);
-  const dim3 grid = p.tiles_outer ? dim3(bh, kt) : dim3(kt, bh);
-  hstu_attn_bwd_kernel<HD><<<grid, NTHREADS, SM::TOTAL, stream>>>(m[0], m[1], m[2], m[3], m[4], p);
+  const long long grid = (long long)p.num_bh * p.num_kt;
+  if (grid > 0x7fffffff) return b200::fail(1212, "hstu_attn_bwd: %lld key tiles are too many", grid);
+  hstu_attn_bwd_kernel<HD><<<(unsigned)grid, NTHREADS, SM::TOTAL, stream>>>(m[0], m[1], m[2], m[3], m[4], p);
   b200::count_launch();
   return b200::check_launch("hstu_attn_bwd");
 }
@@ -444,7 +445,9 @@ B200_API int b200_hstu_attn_bwd(const void* q, const void* k, const void* v, con
   // Early key tiles see the most queries.  With few sequences their longest CTAs go first over all of them (4 heads: 12
   // users 271 -> 231 us, 40 users 184 -> 157); with several chips of (sequence, head) pairs one pair after the other keeps
   // its Q and dO in L2 (128 users: 1345 us, 1376 the other way).
-  p.tiles_outer = H * B <= 2 * b200::sm_count() ? 1 : 0;
-  if (HD == 128) return launch_hstu_bwd<128>(m, p, B, (cudaStream_t)stream);
-  return launch_hstu_bwd<64>(m, p, B, (cudaStream_t)stream);
+  p.num_bh = H * B;
+  p.num_kt = (max_len + BKV - 1) / BKV;
+  p.tiles_outer = p.num_bh <= 2 * b200::sm_count() ? 1 : 0;
+  if (HD == 128) return launch_hstu_bwd<128>(m, p, (cudaStream_t)stream);
+  return launch_hstu_bwd<64>(m, p, (cudaStream_t)stream);
 }

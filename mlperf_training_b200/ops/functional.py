@@ -638,16 +638,27 @@ def rope_bshd(x, cos, sin):
 def qkv_norm_rope_ok(cos, head_dim: int, parts) -> bool:
     """Whether ``[(qkv, q_scale, k_scale), ...]`` run on the fused kernel: bf16 rows of ``[3][H][head_dim]`` on the GPU, 16-byte
     aligned, head dim 64 or 128, fp32 tables."""
-    return head_dim in (64, 128) and cos.dtype == torch.float32 and all(
+    return head_dim in (64, 128) and cos.dtype == torch.float32 and cos.dim() == 2 and cos.shape[1] * 2 == head_dim and all(
         use_kernels(x) and x.dtype == qs.dtype == ks.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1
         and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and qs.data_ptr() % 16 == 0 and ks.data_ptr() % 16 == 0
         for x, qs, ks in parts)
 
 
+def _check_qkv(parts, cos, sin, B, H, D, width):
+    """The kernels index rows, heads and positions by these sizes alone."""
+    S = 0
+    for x, qs, ks in parts:
+        if B <= 0 or x.dim() != 2 or x.shape[0] % B or not width(x.shape[1]):
+            raise ValueError(f"projection {tuple(x.shape)} for {B} samples of 3 x {H} heads of {D}")
+        if qs.shape != (D,) or ks.shape != (D,) or not (qs.is_contiguous() and ks.is_contiguous()):
+            raise ValueError(f"head norm scales {tuple(qs.shape)} / {tuple(ks.shape)} for head dim {D}")
+        S += x.shape[0] // B
+    if cos.shape != sin.shape or cos.dim() != 2 or cos.shape[0] < S or cos.shape[1] * 2 != D or not cos.dtype == sin.dtype == torch.float32:
+        raise ValueError(f"rotary tables {tuple(cos.shape)} {cos.dtype} / {tuple(sin.shape)} {sin.dtype} for {S} tokens of head dim {D}")
+
+
 def _qk_fwd(x, qs, ks, cos, sin, q, k, v, s_off, B, eps):
     _, S, H, D = q.shape
-    if cos.shape[0] < S or cos.shape[1] * 2 != D:
-        raise ValueError(f"rotary tables {tuple(cos.shape)} for {S} tokens of head dim {D}")
     rstd = torch.empty((x.shape[0], 2, H), dtype=torch.float32, device=x.device)
     call("b200_qk_norm_rope_fwd", ptr(x), x.stride(0), ptr(qs), ptr(ks), ptr(cos), ptr(sin), ptr(q), ptr(k), ptr(v), ptr(rstd), B,
          x.shape[0] // B, S, s_off, H, D, float(eps), stream_ptr())
@@ -672,6 +683,7 @@ class QKVNormRopeFn(Function):
     @staticmethod
     def forward(ctx, cos, sin, B, H, D, eps, *flat):
         parts = [flat[i:i + 3] for i in range(0, len(flat), 3)]
+        _check_qkv(parts, cos, sin, B, H, D, lambda n: n == 3 * H * D)
         cos, sin = cos.contiguous(), sin.contiguous()
         S = sum(x.shape[0] for x, _, _ in parts) // B
         q, k, v = (torch.empty((B, S, H, D), dtype=flat[0].dtype, device=flat[0].device) for _ in range(3))
@@ -708,8 +720,9 @@ class SingleStreamInFn(Function):
 
     @staticmethod
     def forward(ctx, y, q_scale, k_scale, cos, sin, B, H, D, eps):
-        cos, sin = cos.contiguous(), sin.contiguous()
         n = 3 * H * D
+        _check_qkv([(y, q_scale, k_scale)], cos, sin, B, H, D, lambda w: w >= n and w % 8 == 0)
+        cos, sin = cos.contiguous(), sin.contiguous()
         T, M = y.shape[0], y.shape[1] - n
         q, k, v = (torch.empty((B, T // B, H, D), dtype=y.dtype, device=y.device) for _ in range(3))
         rstd = _qk_fwd(y, q_scale, k_scale, cos, sin, q, k, v, 0, B, eps)

@@ -5,7 +5,7 @@ import torch
 
 from mlperf_training_b200.ops import functional as F
 
-pytestmark = pytest.mark.gpu
+gpu = pytest.mark.gpu
 
 
 def _oracle(parts, cos, sin, B, H, D):
@@ -27,6 +27,7 @@ def _close(a, b):
     assert (a.double() - b).norm() <= 2 ** -8 * b.norm()
 
 
+@gpu
 @pytest.mark.parametrize("B,sizes,H,D", [(1, [1], 1, 64), (2, [5, 3], 3, 128), (3, [37], 5, 64), (2, [256, 256], 24, 128)])
 def test_streams(B, sizes, H, D):
     torch.manual_seed(sum(sizes))
@@ -49,6 +50,7 @@ def test_streams(B, sizes, H, D):
             _close(a.grad, b.grad)
 
 
+@gpu
 @pytest.mark.parametrize("B,S,H,D,m", [(2, 19, 2, 64, 72), (1, 130, 3, 128, 512)])
 def test_single_stream(B, S, H, D, m):
     torch.manual_seed(S)
@@ -67,3 +69,24 @@ def test_single_stream(B, S, H, D, m):
     torch.autograd.backward(want, [g.double() for g in gr])
     for a, b in zip([*got, y.grad, qs.grad, ks.grad], [*want, *(r.grad for r in ref)]):
         _close(a, b)
+
+
+@pytest.mark.parametrize("bad", ["narrow", "wide", "rows", "scale", "pitched_scale", "short_table", "table_width", "sin", "sin_dtype", "samples"])
+@pytest.mark.parametrize("single", [False, True])
+def test_sizes_that_do_not_fit_are_refused(monkeypatch, bad, single):
+    """What the reshapes of the separate chain refused is refused before anything is launched."""
+    monkeypatch.setattr(F, "call", lambda *a: pytest.fail("launched"))
+    B, S, H, D = 2, 6, 3, 64
+    extra = 64 if single else 0
+    n = 3 * H * D + extra
+    x = torch.zeros(B * S + (bad == "rows"), {"narrow": 3 * H * D - 8, "wide": n + (4 if single else 64)}.get(bad, n)).bfloat16()
+    qs = ks = torch.ones(D).bfloat16()
+    if bad == "scale":
+        ks = torch.ones(2 * D).bfloat16()
+    if bad == "pitched_scale":
+        qs = torch.ones(2 * D).bfloat16()[::2]
+    cos = torch.ones(S - (bad == "short_table"), D if bad == "table_width" else D // 2)
+    sin = torch.ones(S + 1, D // 2) if bad == "sin" else cos.double() if bad == "sin_dtype" else cos
+    B = 0 if bad == "samples" else B
+    with pytest.raises(ValueError):
+        F.single_stream_in(x, qs, ks, cos, sin, B, H, D) if single else F.qkv_norm_rope([(x, qs, ks)], cos, sin, B, H, D)

@@ -130,10 +130,14 @@ segment_partial_kernel(RowSrc s, const long long* __restrict__ seg, const long l
   const long long p0 = b * SEG_CHUNK;
   if (p0 >= n) return;
   const long long p1 = p0 + SEG_CHUNK < n ? p0 + SEG_CHUNK : n;
-  // the runs of the block's ends: two dependent loads through the sort's inverse map, a search over the offsets without it
-  const bool mapped = inverse != nullptr && s.perm != nullptr;
-  const long long s0 = mapped ? inverse[s.perm[p0]] : run_of(seg, total, p0);
-  const long long s1 = mapped ? inverse[s.perm[p1 - 1]] : run_of(seg, total, p1 - 1);
+  // the runs of the block's ends: two dependent loads through the sort's inverse map, a search over the offsets without it (or
+  // where an entry lies outside its range, which sum_positions reports)
+  auto run_at = [&](long long pos) -> long long {
+    const long long at = inverse != nullptr && s.perm != nullptr ? s.perm[pos] : -1;
+    const long long run = at >= 0 && at < n ? inverse[at] : -1;
+    return run >= 0 && run < total ? run : run_of(seg, total, pos);
+  };
+  const long long s0 = run_at(p0), s1 = run_at(p1 - 1);
   const int nvec = s.D / 8;
   for (int slot = 0; slot < 2; ++slot) {
     const long long run = slot == 0 ? s0 : s1;

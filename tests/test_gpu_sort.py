@@ -111,3 +111,26 @@ def test_sorts_on_two_streams():
         assert int(a.count) == n and torch.equal(a.keys, b.keys) and torch.equal(a.perm, b.perm)
         assert torch.equal(a.inverse, b.inverse) and torch.equal(a.seg[:n + 1], b.seg[:n + 1]) and torch.equal(a.uniq[:n], b.uniq[:n])
     _lib.check_status("sort")
+
+
+@gpu
+@pytest.mark.parametrize("entries", ["perm", "inverse"])
+def test_entries_outside_their_range_are_skipped(entries):
+    """Positions of the permutation outside the source (at the ends of blocks, where the partial sums look their runs up) are
+    left out of the sums; a run index outside the runs is found by search instead."""
+    ids = torch.cat([torch.full((200,), 3), torch.arange(10, 80), torch.full((100,), 5)])
+    src = torch.randn(ids.numel(), 64, generator=torch.Generator().manual_seed(1)).bfloat16()
+    d = sort.sort_unique(ids.cuda(), 7)
+    want = d.perm.cpu().clone()
+    at = torch.tensor([0, 63, 64, 127, 300, 369])
+    if entries == "perm":
+        want[at] = torch.tensor([-1, 370, 1 << 40, -(1 << 40), 371, 5000])
+        d.perm.copy_(want)
+    else:
+        d.inverse[d.perm[at.cuda()]] = torch.tensor([-1, 72, 1 << 40, -(1 << 40), 1000, 73], device="cuda")
+    out = sort.segment_sum(src.cuda(), d).cpu()
+    keys, ok = d.keys.cpu(), (want >= 0) & (want < ids.numel())
+    for j, key in enumerate(d.uniq[:int(d.count)].tolist()):
+        rows = src[want[ok & (keys == key)]].double()
+        # fp32 sums of up to 200 terms
+        assert (out[j].double() - rows.sum(0)).abs().max() <= 200 * 2 ** -24 * max(rows.abs().sum(0).max().item() if len(rows) else 0, 1e-9)

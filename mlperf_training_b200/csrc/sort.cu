@@ -156,17 +156,17 @@ segment_partial_kernel(RowSrc s, const long long* __restrict__ seg, const long l
   }
 }
 
-// one warp per run, runs taken grid-stride
+// one warp per run of [first, first + max_seg), runs taken grid-stride
 template <typename Out>
 __global__ void __launch_bounds__(256)
 segment_sum_gather_kernel(RowSrc s, const long long* __restrict__ seg, const long long* __restrict__ n_seg,
-                          const float* __restrict__ partial, Out* __restrict__ out, int* status) {
-  const long long total = *n_seg;
+                          const float* __restrict__ partial, long long first, long long max_seg, Out* __restrict__ out, int* status) {
+  const long long total = *n_seg < first + max_seg ? *n_seg : first + max_seg;
   const int lane = threadIdx.x & 31;
   const long long warp0 = (blockIdx.x * 256ll + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * 256) >> 5;
   const int nvec = s.D / 8;
-  for (long long r = warp0; r < total; r += nwarps) {
+  for (long long r = first + warp0; r < total; r += nwarps) {
     const long long lo = seg[r], hi = seg[r + 1];
     for (int v = lane; v - lane < nvec; v += 32) {
       float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -196,11 +196,11 @@ segment_sum_gather_kernel(RowSrc s, const long long* __restrict__ seg, const lon
       }
       if (v >= nvec) continue;
       if constexpr (sizeof(Out) == 2) {
-        *reinterpret_cast<uint4*>(out + r * s.D + v * 8) =
+        *reinterpret_cast<uint4*>(out + (r - first) * s.D + v * 8) =
             make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
       } else {
-        *reinterpret_cast<float4*>(out + r * s.D + v * 8) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-        *reinterpret_cast<float4*>(out + r * s.D + v * 8 + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+        *reinterpret_cast<float4*>(out + (r - first) * s.D + v * 8) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        *reinterpret_cast<float4*>(out + (r - first) * s.D + v * 8 + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
       }
     }
   }
@@ -274,15 +274,17 @@ B200_API long long b200_segment_sum_scratch_elems(long long n, int D) {
   return ((n + SEG_CHUNK - 1) / SEG_CHUNK) * 2 * (long long)D;
 }
 
-// out[s, :] = sum of src[perm[r], :] over the sorted positions r of run s, s < *n_seg (device scalar), summed in a
-// fixed order.  src: bf16 or fp32 [src_rows, D]; perm [n] (null: identity); seg [*n_seg + 1] run offsets; out
-// [max_seg, D] bf16 or fp32 (runs only: rows past *n_seg are not written); inverse [n]: run of every original position
-// (b200_unique_segments), or null; partial: b200_segment_sum_scratch_elems(n, D) floats (null: every run is summed by one
-// warp, whatever its length).
+// out[s - first, :] = sum of src[perm[r], :] over the sorted positions r of run s, for the runs s of [first, first + max_seg)
+// below *n_seg (device scalar), summed in a fixed order.  src: bf16 or fp32 [src_rows, D]; perm [n] (null: identity); seg
+// [*n_seg + 1] run offsets; out [max_seg, D] bf16 or fp32 (runs only: rows past *n_seg are not written); inverse [n]: run of
+// every original position (b200_unique_segments), or null; partial: b200_segment_sum_scratch_elems(n, D) floats (null: every
+// run is summed by one warp, whatever its length).  A call with first = 0 fills partial for all runs; calls with first > 0
+// must follow one of the same arguments and read what it left there.
 B200_API int b200_segment_sum_gather(const void* src, int src_is_f32, long long src_rows, const long long* perm,
                                      const long long* seg, const long long* n_seg, const long long* inverse, long long n,
-                                     long long max_seg, int D, void* out, int out_bf16, float* partial, void* stream) {
-  if (max_seg <= 0 || n <= 0) return 0;
+                                     long long first, long long max_seg, int D, void* out, int out_bf16, float* partial,
+                                     void* stream) {
+  if (max_seg <= 0 || n <= 0 || first < 0) return 0;
   if (D % 8 != 0 || ((uintptr_t)src & 15) || ((uintptr_t)out & 15) || ((uintptr_t)partial & 15))
     return b200::fail(1605, "segment_sum_gather: D=%d must be a multiple of 8 and the matrices 16-byte aligned", D);
   RowSrc s;
@@ -290,7 +292,7 @@ B200_API int b200_segment_sum_gather(const void* src, int src_is_f32, long long 
   s.f32 = src_is_f32 ? (const float*)src : nullptr;
   s.perm = perm; s.rows = src_rows; s.D = D;
   cudaStream_t st = (cudaStream_t)stream;
-  if (partial != nullptr) {
+  if (partial != nullptr && first == 0) {
     const long long blocks = (n + SEG_CHUNK - 1) / SEG_CHUNK;
     segment_partial_kernel<<<(unsigned)((blocks + 7) / 8), 256, 0, st>>>(s, seg, n_seg, inverse, n, partial, b200::status_ptr());
     b200::count_launch();
@@ -300,9 +302,9 @@ B200_API int b200_segment_sum_gather(const void* src, int src_is_f32, long long 
   const long long want = (max_seg + 7) / 8;            // 8 warps (runs) per CTA
   const int grid = (int)(want < 148 * 16 ? want : 148 * 16);
   if (out_bf16)
-    segment_sum_gather_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(s, seg, n_seg, partial, (__nv_bfloat16*)out, b200::status_ptr());
+    segment_sum_gather_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(s, seg, n_seg, partial, first, max_seg, (__nv_bfloat16*)out, b200::status_ptr());
   else
-    segment_sum_gather_kernel<float><<<grid, 256, 0, st>>>(s, seg, n_seg, partial, (float*)out, b200::status_ptr());
+    segment_sum_gather_kernel<float><<<grid, 256, 0, st>>>(s, seg, n_seg, partial, first, max_seg, (float*)out, b200::status_ptr());
   b200::count_launch();
   return b200::check_launch("segment_sum_gather");
 }

@@ -89,7 +89,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_gelu_bwd_rows": [P, L, P, L, P, L, L, L, P],
         "b200_sort_ids": [P, P, P, L, I, P, L, P],
         "b200_unique_segments": [P, P, L, P, P, P, P, P, L, P],
-        "b200_segment_sum_gather": [P, I, L, P, P, P, P, L, L, I, P, I, P, P],
+        "b200_segment_sum_gather": [P, I, L, P, P, P, P, L, L, L, I, P, I, P, P],
         "b200_hstu_attn_fwd": [P, P, P, P, P, P, I, L, I, I, I, I, L, L, L, L, F, P],
         "b200_hstu_gate_cat_fwd": [P, L, P, P, P, P, P, P, I, I, F, F, ctypes.c_ulonglong, P],
         "b200_hstu_gate_cat_bwd": [P, P, L, P, P, P, P, P, P, L, P, P, P, P, I, I, I, F, ctypes.c_ulonglong, P],

@@ -448,7 +448,7 @@ class ExpandRowsFn(Function):
             n_seg = torch.full((1,), B, dtype=torch.int64, device=g.device)
             n = g.shape[0]
             partial = torch.empty(int(_lib.load().b200_segment_sum_scratch_elems(n, D)), dtype=torch.float32, device=g.device)
-            call("b200_segment_sum_gather", ptr(g), int(g.dtype == torch.float32), n, None, ptr(seg), ptr(n_seg), None, n, B, D, ptr(out), 0,
+            call("b200_segment_sum_gather", ptr(g), int(g.dtype == torch.float32), n, None, ptr(seg), ptr(n_seg), None, n, 0, B, D, ptr(out), 0,
                  ptr(partial), stream_ptr())
             return out.to(ctx.dtype), None, None
         out = torch.zeros((B, D), dtype=torch.float32, device=g.device)

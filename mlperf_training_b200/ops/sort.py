@@ -72,12 +72,11 @@ def sort_unique(ids: torch.Tensor, key_bits: int = 64) -> SortedIds:
     return SortedIds(keys, perm, uniq, seg, inverse, count)
 
 
-def segment_sum(src: torch.Tensor, s: SortedIds, out_dtype=torch.float32, max_seg: int | None = None, clear: bool = True) -> torch.Tensor:
+def segment_sum(src: torch.Tensor, s: SortedIds, out_dtype=torch.float32, max_seg: int | None = None) -> torch.Tensor:
     """``out[j] = sum of src[p] over the original positions p whose id is the j-th unique id`` (sorted
-    order inside a run).  Returns ``[n, D]`` rows (the first ``count`` are valid; the rest zeros, or
-    with ``clear=False`` whatever the allocator gave: for consumers that skip them)."""
+    order inside a run).  Returns ``[n, D]`` rows (the first ``count`` are valid; the rest untouched zeros)."""
     n, D = s.keys.numel(), src.shape[1]
-    out = (torch.zeros if clear or not use_kernels(src) else torch.empty)((n if max_seg is None else max_seg, D), dtype=out_dtype, device=src.device)
+    out = torch.zeros((n if max_seg is None else max_seg, D), dtype=out_dtype, device=src.device)
     if n == 0:
         return out
     if not use_kernels(src):
@@ -88,9 +87,37 @@ def segment_sum(src: torch.Tensor, s: SortedIds, out_dtype=torch.float32, max_se
         return out
     if src.dtype not in (torch.bfloat16, torch.float32) or out_dtype not in (torch.bfloat16, torch.float32):
         raise TypeError("segment_sum: bf16 or fp32 rows")
-    from . import _lib
-    # partial sums of the runs that are too long for one warp (skewed ids): one fp32 row pair per 64 sorted positions
-    partial = torch.empty(int(_lib.load().b200_segment_sum_scratch_elems(n, D)), dtype=torch.float32, device=src.device)
-    call("b200_segment_sum_gather", ptr(src.contiguous()), int(src.dtype == torch.float32), src.shape[0], ptr(s.perm), ptr(s.seg), ptr(s.count),
-         ptr(s.inverse), n, out.shape[0], D, ptr(out), int(out_dtype == torch.bfloat16), ptr(partial), stream_ptr())
+    _sum_runs(src.contiguous(), s, 0, out, _partial_sums(n, D, src.device))
     return out
+
+
+def segment_sum_blocks(src: torch.Tensor, s: SortedIds, max_seg: int, max_bytes: int):
+    """``segment_sum`` in fp32 over at most ``max_bytes`` at a time, without a host read of the number of runs: yields
+    ``(first, rows)`` for the runs ``[first, first + len(rows))`` of the first ``max_seg``.  ``rows`` is one buffer, valid until
+    the next block is asked for; what lies past the run count is not set (entries of ``uniq`` there are -1)."""
+    n, D = s.keys.numel(), src.shape[1]
+    if n == 0 or max_seg == 0:
+        return
+    if not use_kernels(src):
+        yield 0, segment_sum(src, s, max_seg=max_seg)
+        return
+    if src.dtype not in (torch.bfloat16, torch.float32):
+        raise TypeError("segment_sum: bf16 or fp32 rows")
+    block = min(max_seg, max(max_bytes // (4 * D), 1))
+    src, partial = src.contiguous(), _partial_sums(n, D, src.device)
+    buf = torch.empty((block, D), dtype=torch.float32, device=src.device)
+    for first in range(0, max_seg, block):
+        out = buf[:min(block, max_seg - first)]
+        _sum_runs(src, s, first, out, partial)
+        yield first, out
+
+
+def _partial_sums(n: int, D: int, device) -> torch.Tensor:
+    """Of the runs that are too long for one warp (skewed ids): one fp32 row pair per 64 sorted positions."""
+    return torch.empty(int(load().b200_segment_sum_scratch_elems(n, D)), dtype=torch.float32, device=device)
+
+
+def _sum_runs(src, s: SortedIds, first: int, out, partial) -> None:
+    call("b200_segment_sum_gather", ptr(src), int(src.dtype == torch.float32), src.shape[0], ptr(s.perm), ptr(s.seg), ptr(s.count),
+         ptr(s.inverse), s.keys.numel(), first, out.shape[0], out.shape[1], ptr(out), int(out.dtype == torch.bfloat16), ptr(partial),
+         stream_ptr())

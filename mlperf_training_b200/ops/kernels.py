@@ -291,8 +291,8 @@ def gelu_bwd(dy: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
 # embedding rows
 # --------------------------------------------------------------------------------------
 def gather_rows(table: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
-    if not use_kernels(table):
-        # ids outside [0, rows) give zero rows, as in the kernel
+    if not use_kernels(table) or table.element_size() != 2:
+        # (the kernel moves rows of 2-byte elements) ids outside [0, rows) give zero rows, as in the kernel
         out = table[ids.clamp(min=0, max=table.shape[0] - 1)]
         return torch.where(((ids >= 0) & (ids < table.shape[0]))[:, None], out, torch.zeros_like(out))
     ids = ids.to(torch.int64).contiguous()

@@ -203,3 +203,13 @@ def test_rope_bshd_matches_eager_rotation():
     want = torch.cat([x1 * c - x2 * s, x2 * c + x1 * s], dim=-1)
     assert (res["cpu"][0] - want).abs().max() < 2e-2 and (res["cuda"][0] - want).abs().max() < 2e-2
     assert (res["cuda"][1] - res["cpu"][1]).abs().max() < 2e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_gather_rows_of_every_type(dtype):
+    table = torch.randn(50, 24, device="cuda").to(dtype)
+    ids = torch.tensor([3, 49, -1, 50, 0, 3], device="cuda")
+    out = kernels.gather_rows(table, ids)
+    want = table[ids.clamp(0, 49)]
+    want[2:4] = 0
+    assert out.dtype == dtype and torch.equal(out, want)

@@ -831,9 +831,6 @@ template <int BN>
 __global__ void __launch_bounds__(256)
 split_finish_kernel(const float* __restrict__ ws, SplitArgs sp, int num_m, int num_n, int group_m, EpiArgs e, void* d, long long ldd) {
   constexpr int VPR = BN / 8;
-  float alpha = e.alpha;
-  if (e.alpha_a != nullptr) alpha *= *e.alpha_a;
-  if (e.alpha_b != nullptr) alpha *= *e.alpha_b;
   const int i = blockIdx.y;
   int mb, nb;
   tile_coords(sp.first + i, num_m, num_n, group_m, mb, nb);
@@ -853,7 +850,7 @@ split_finish_kernel(const float* __restrict__ ws, SplitArgs sp, int num_m, int n
     const __nv_bfloat16* res = e.residual != nullptr ? e.residual + (long long)row * e.ldr + col : nullptr;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      v[j] *= alpha;
+      v[j] *= e.alpha;                               // (device-side factors belong to the FP8 launches, which are not split)
       if (j < n) {
         if (e.bias != nullptr) v[j] += __bfloat162float(e.bias[col + j]);
         if (res != nullptr) v[j] += __bfloat162float(res[j]);

@@ -376,7 +376,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
         const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
         // P = exp2(S * scale - m) as bf16 pairs over the first half of the S columns; every fourth
-        // pair takes the polynomial path (FMA pipe), the rest the MUFU path; -inf gives 0 on both
+        // pair takes the polynomial path (FMA pipe), the rest the MUFU path; -inf gives 2^-126 and 0
         const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
         const float2 nm2 = make_float2(-m_use, -m_use);
 #pragma unroll

@@ -429,15 +429,21 @@ B200_DEVICE float ex2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+B200_DEVICE float fmax_nan(float a, float b) {
+  float y;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
 // 2^x for a pair of values without the MUFU unit and without float<->int conversions (which also
 // run on the XU pipe): round to nearest with the 1.5 * 2^23 magic constant, a degree-3 polynomial
 // for 2^f on [-0.5, 0.5] (relative error < 7e-4, below bf16 resolution), and the integer part
 // added to the exponent field.  Used for a share of the softmax exponentials so that the
-// 16/clk/SM MUFU unit is not the only exponent engine.
+// 16/clk/SM MUFU unit is not the only exponent engine.  -inf gives 2^-126; a NaN stays non-finite (the largest float
+// from here, an infinity once it is bf16): with a maximum that drops NaN it came out as 2^-126.
 B200_DEVICE float2 ex2_poly2(float2 x) {
   const float magic = 12582912.f;
-  x.x = fmaxf(x.x, -126.f);
-  x.y = fmaxf(x.y, -126.f);
+  x.x = fmax_nan(x.x, -126.f);
+  x.y = fmax_nan(x.y, -126.f);
   const float2 t = fadd2(x, make_float2(magic, magic));
   const float2 r = fadd2(t, make_float2(-magic, -magic));
   const float2 f = fadd2(x, make_float2(-r.x, -r.y));

@@ -22,3 +22,20 @@ def test_forward(B, Sq, Skv, Hq, Hkv, D, causal, window, sink):
     assert (out.float() - ref).abs().max() <= 2 ** -7 * ref.abs().max()
     assert (lse - ref_lse).abs().max() <= 2e-3       # a quarter of the exponentials carry up to 7e-4
     _lib.check_status("attention_fwd")
+
+
+@pytest.mark.parametrize("key", [0, 6, 7, 134, 255])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_non_finite_keys_are_not_lost(key, value):
+    """A NaN or infinity in one key makes the rows that see it non-finite and leaves the others alone (keys 6 and 7 of 8 have
+    their exponentials on the FMA pipe)."""
+    torch.manual_seed(key)
+    q, k, v = (torch.randn(1, 256, 2, 64, device="cuda").bfloat16() for _ in range(3))
+    clean, _ = K.attention_fwd(q, k, v, causal=True)
+    k[0, key, 1, 5] = value
+    q[..., 5] = q[..., 5].abs() + 0.5
+    clean2, _ = K.attention_fwd(q[:, :, :1], k[:, :, :1], v[:, :, :1], causal=True)
+    out, _ = K.attention_fwd(q, k, v, causal=True)
+    assert not out[0, key:, 1].isfinite().any() and out[0, :key].isfinite().all()
+    assert torch.equal(out[:, :, :1], clean2) and clean.isfinite().all()
+    _lib.check_status("attention_fwd")

@@ -27,8 +27,9 @@
 // over, and the softmax warps hold 200 registers (all 128 scores in flight, no spills).  Items are handed out longest
 // first over all heads (head after head left 14 % of the SM cycles idle at the end of a causal launch), in snake order
 // over the rounds so that no CTA gets the longest of each.
-// Measured (causal unless noted), before -> now: 8192 x 32 heads of 128 622 -> 528 us (1.04 PFLOP/s); 4 x 2048 218 -> 181;
-// 3 x 1337 107 -> 90; 8192 x 64 heads of 64, window 128 200 -> 158; 2000 x 64 of 64 114 -> 87; 8 x 512 x 24, full 56 -> 47.
+// Measured (causal unless noted), one CTA per item -> now: 8192 x 32 heads of 128 622 -> 507 us (1.08 PFLOP/s); 4 x 2048
+// 218 -> 172; 3 x 1337 107 -> 87; 8192 x 64 heads of 64, window 128 200 -> 158; 2000 x 64 of 64 114 -> 84; 8 x 512 x 24, full
+// 56 -> 45.
 //
 // Stands in for the attention kernels the reference selects by config: Primus-Turbo / AITER /
 // CK flash attention (small_llm_pretraining/primus/conf/llama3.1_8B-pretrain-fp4.yaml:117,125)
@@ -516,10 +517,15 @@ B200_API int b200_attn_fwd(const void* q, const void* k, const void* v, void* o,
   const long long items = (long long)((Sq + 2 * BQ - 1) / (2 * BQ)) * Hq * B;
   if (items <= 0 || items > 0x3fffffff) return b200::fail(600, "attn_fwd: %lld query tile pairs", items);
   p.items = (int)items;
-  // K and V of a group of heads: half of the 126 MB L2, so that the next group's fit beside them
+  // Full attention: every item costs the same, and heads go in groups whose K and V take half of the 126 MB L2, so that the
+  // next group's fit beside them (16384 x 32 heads of 128: groups of 8 3828 us, all heads at once 4009; 2 x 4608 x 24, where
+  // the group is more than half of the heads: 505 and 504).
+  // Causal: the longest items of all heads first, whatever that does to L2.  Groups leave a tail of their own each (groups by
+  // the rule above and all at once: 16384 x 32 heads of 128 2189 and 2017 us, 2 x 8192 x 32 1159 and 1067, window 1024 383 and
+  // 365, 2 x 8192 x 64 heads of 64 1886 and 1733; single heads and groups of four lie between or above).
   const long long per_kv_head = (long long)Skv * HD * 4, fit = (64ll << 20) / per_kv_head;
   const long long group = (fit > 0 ? fit : 1) * (Hq / Hkv);
-  p.bh_group = (int)(group < (long long)B * Hq ? group : (long long)B * Hq);
+  p.bh_group = (int)(!causal && group < (long long)B * Hq ? group : (long long)B * Hq);
   if (HD == 128) return launch_fwd<128>(tq, tk, tv, to, p, (cudaStream_t)stream);
   return launch_fwd<64>(tq, tk, tv, to, p, (cudaStream_t)stream);
 }

@@ -1,5 +1,5 @@
 """Attention forward at the edges of its work schedule: odd tile counts, more and fewer items than CTAs, windows that skip
-a pair's first key tile, more keys than queries, several L2 groups' worth of head order."""
+a pair's first key tile, more keys than queries, a second, smaller L2 group of heads."""
 import pytest
 import torch
 
@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("B,Sq,Skv,Hq,Hkv,D,causal,window,sink", [
     (1, 1, 1, 1, 1, 128, True, 0, False), (1, 129, 129, 2, 1, 64, True, 1, True), (2, 257, 257, 4, 2, 128, True, 128, False),
     (1, 640, 640, 8, 8, 64, True, 200, True), (3, 384, 511, 4, 1, 128, True, 0, False), (2, 300, 1000, 6, 3, 64, False, 0, False),
-    (5, 513, 513, 8, 2, 128, True, 0, True), (1, 200, 1500, 4, 4, 128, True, 100, False)])
+    (5, 513, 513, 8, 2, 128, True, 0, True), (1, 200, 1500, 4, 4, 128, True, 100, False),
+    (3, 130, 2048, 24, 24, 128, False, 0, False)])      # 64 + 8 heads: two L2 groups
 def test_forward(B, Sq, Skv, Hq, Hkv, D, causal, window, sink):
     torch.manual_seed(Sq)
     q, k, v = (torch.randn(B, s, h, D, device="cuda").bfloat16() for s, h in ((Sq, Hq), (Skv, Hkv), (Skv, Hkv)))

@@ -17,15 +17,16 @@
 // rows): each takes half of the 128 query columns.  Every exponential is ex2.approx: a polynomial on the
 // FMA pipe (relative error up to 7e-4, as the forward takes for a quarter of the keys) for a quarter of the query columns was
 // neither exact nor the forward's P, and added up to 0.13 % to the errors of dQ and dK against 64 bits (6 draws of 5 shapes
-// up to 2048 x 128).  On the MUFU unit alone they are 0.02 to 0.25 % below those of the forward's own P, in the same time:
-// 8192 x 32 / 8 heads of 128 1305 (polynomial) and 1310 us, 4 x 2048 400 and 404, 8 x 512 x 24 full 136 and 133.
+// up to 2048 tokens).  On the MUFU unit alone the errors are 0.02 to 0.25 % below those of the forward's own P.  It costs nothing
+// at head dim 128 (8192 x 32 / 8 1293 us with the polynomial, 1297 without; 8 x 512 x 24 full 128 and 128) and 4 to 6 % at 64,
+// where the products are half as long (2000 x 64 / 8 282 and 298, 8192 x 64 / 8 with window 128 263 and 273).
 // TMEM (512 columns): S^T / P^T | dP^T, then dQ | dK | dV.  Order of the MMAs of step i, Q double-buffered:
 //     [P^T(i) written]  dV(i)   [dS^T(i) written]  dQ(i)  S(i+1)  dK(i)  [dQ(i) drained]  dP(i+1)
 // so dQ(i) is drained and S(i+1) exponentiated while the tensor core runs dK(i) and dP(i+1).  (The drain has warps of its
 // own: staged by the workers, its 64 KB a step took 3000 of their 6700 cycles, clock64 in the roles.)
 // Measured with delta, clearing and launches: queries as rows, P and dS through shared memory, one Q stage -> transposed ->
-// drain warps: 8192 x 32 / 8 heads of 128 causal 1990 -> 1766 -> 1336 us (1.03 PFLOP/s), 4096 x 64 / 8 1130 -> 1005 -> 779,
-// 4 x 2048 607 -> 550 -> 427, 2000 x 64 / 8 of 64 448 -> 378 -> 302, 8 x 512 x 24 full 175 -> 157 -> 136.
+// drain warps, as it is: 8192 x 32 / 8 heads of 128 causal 1990 -> 1766 -> 1310 us (1.05 PFLOP/s), 4096 x 64 / 8 1130 -> 1005
+// -> 765, 4 x 2048 607 -> 550 -> 408, 2000 x 64 / 8 of 64 448 -> 378 -> 298, 8 x 512 x 24 full 175 -> 157 -> 128.
 //
 // The reference takes this kernel from Primus-Turbo / AITER / CK (config knobs
 // llama2_sft/primus/config_MI355X_1x8x1.sh:35-39); there is no in-tree counterpart.
@@ -582,10 +583,11 @@ B200_API int b200_attn_bwd(const void* q, const void* k, const void* v, const vo
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.lse = lse; p.delta = delta;
   p.status = b200::status_ptr();
-  // Causal: a key tile's work falls with its position, so all heads' early tiles go first (head after head left the last
-  // head's longest CTAs running alone: 8192 x 32 / 8 heads of 128, delta and clearing included, 2370 -> 1990 us,
-  // 4096 x 64 / 8 heads 1590 -> 1130 us; groups of two heads 2070 and 1517).  Otherwise every tile costs the same and
-  // head after head keeps that head's Q and dO in L2 (8 x 512 x 24 heads 175 us, 181 the other way).
+  // Causal: a key tile's work falls with its position, so all heads' early tiles go first (head after head leaves the last
+  // head's longest CTAs running alone: 8192 x 32 / 8 heads of 128, delta and clearing included, 1512 us, this way 1310;
+  // 4096 x 64 / 8 992 and 765; 4 x 2048 480 and 408; 3 x 1337 231 and 167).  Otherwise every tile costs the same and head after
+  // head keeps that head's Q and dO in L2 (full, 8 x 512 x 24 heads 128 us, 134 the other way; 2 x 4608 x 24 1211 and 1345).
+  // With a window the two are even (8192 x 64 / 8 of 64, window 128: 269 and 269; 2 x 8192 x 32, window 1024: 920 and 925).
   p.bh_group = (causal && window <= 0) ? B * Hkv : 1;
   if (HD == 128) return launch_bwd<128>(m, p, (cudaStream_t)stream);
   return launch_bwd<64>(m, p, (cudaStream_t)stream);

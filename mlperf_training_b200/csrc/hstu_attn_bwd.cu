@@ -9,7 +9,7 @@
 //     [P^T(i) written]  dV(i)   [dS^T(i) written]  dQ(i)  S(i+1)  dK(i)  [dQ(i) drained]  dP(i+1)
 // No row statistics are needed, so nothing but Q, K, V, dO is read.  Mask and jagged layout as in hstu_attn_fwd.cu.
 // Measured with the clearing and conversion around it, before (queries as rows, P and dS through shared memory, drained by
-// the workers) -> now: 128 users of median 512 tokens, 4 heads of 128: 1345 -> 1077 us; 12 users of median 700: 235 -> 169.
+// the workers) -> now: 128 users of median 512 tokens, 4 heads of 128: 1345 -> 1018 us; 12 users of median 700: 235 -> 163.
 //
 // Math oracle: autograd of generative_recommenders/ops/pytorch/pt_hstu_attention.py:130-187; the
 // reference's production kernels are generative_recommenders/ops/flydsl/hstu_bwd_dkdv.py and
@@ -442,9 +442,11 @@ B200_API int b200_hstu_attn_bwd(const void* q, const void* k, const void* v, con
   p.offsets = offsets; p.num_targets = num_targets;
   p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.dk_row = dk_row; p.dv_row = dv_row;
   p.status = b200::status_ptr();
-  // Early key tiles see the most queries.  With few sequences their longest CTAs go first over all of them (4 heads: 12
-  // users 271 -> 231 us, 40 users 184 -> 157); with several chips of (sequence, head) pairs one pair after the other keeps
-  // its Q and dO in L2 (128 users: 1345 us, 1376 the other way).
+  // Early key tiles see the most queries.  With few sequences their longest CTAs go first over all of them (4 heads of 128,
+  // pairs slowest and tiles slowest: 12 users of median 700 171 and 163 us, 40 of median 200 165 and 144); with several chips of
+  // (sequence, head) pairs one pair after the other keeps its Q and dO in L2 (128 of median 512: 1018 and 1099).  In between
+  // the lengths decide, by 5 % at most: 45 of median 512 391 and 382, 60 493 and 517, 74 603 and 636, 74 of median 200 264 and
+  // 256; the line lies at two chips of pairs.
   p.num_bh = H * B;
   p.num_kt = (max_len + BKV - 1) / BKV;
   p.tiles_outer = p.num_bh <= 2 * b200::sm_count() ? 1 : 0;

@@ -24,10 +24,15 @@
 // its row layout [keys][head dim] and is consumed as an MN-major operand.  This is the forward of the
 // reference's production path (generative_recommenders/ops/flydsl/hstu_fwd.py:150, e4m3 forward).
 //
-// What bounds it: per pair of 128 x 128 tiles 2048 tensor-core cycles against 2048 of the MUFU unit (one tanh per score)
-// and the hand-overs between them (3500 cycles measured).  Scores come 64 columns per TMEM round trip, P V starts on the
-// first half of the keys, and the latest query tiles of all sequences go first.  128 users of median 512 tokens, 4 heads:
-// 728 -> 497 us; 12 users of median 700: 271 -> 204 us (rolled 32-column chunks, sequence after sequence before).
+// What bounds it: per pair of 128 x 128 tiles 2048 tensor-core cycles against 2048 of the MUFU unit (one tanh per score), and
+// the activation's other work.  A step of a pair takes 5600 to 6000 cycles on average (clock64 in the activation warps, 1700
+// to 1900 of them waiting for scores) and 10,900 where the element mask is applied, which a query tile that ends past its
+// sequence does on every key tile; a CTA adds 4600 cycles before its first scores and 2600 after its last.  128 users of median
+// 512 tokens, 4 heads: 1856 CTAs of 8192 have work and keep the SMs busy for 402 of 462 us.  12 users of median 700: 190 us
+// are the longest CTA, 31 masked steps in series, while the average SM works for 57 us.
+// Scores come 64 columns per TMEM round trip, P V starts on the first half of the keys, and the latest query tiles of all
+// sequences go first.  With the clearing of the output, 128 users: 728 -> 497 us; 12 users: 271 -> 203 us (rolled 32-column
+// chunks, sequence after sequence before).
 //
 // Math oracle: generative_recommenders/ops/pytorch/pt_hstu_attention.py:33-84,130-187; the
 // reference's production kernels are generative_recommenders/ops/flydsl/hstu_fwd.py and

@@ -197,7 +197,8 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // Forward of widths that are whole vectors of a warp up to 4096: a warp per row, up to 16 vectors per lane, summed lane
 // by lane in column order.  The CTA-per-row split is up to 20 % faster at 4096 (27 -> 22 us for 4011 rows), but adds the
 // squares in another order, and with block-scaled linears behind it one flipped bf16 bit in 90000 grew to 3 % of the
-// attention gradients over three quantisers.
+// attention gradients over three quantisers.  (The launch does not know what reads its result, so bf16 consumers pay for it
+// too: two norms each way of a bf16 block.)
 constexpr int WMAXV = 16;
 template <int MODE>
 __global__ void __launch_bounds__(256)

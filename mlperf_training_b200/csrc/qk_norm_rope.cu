@@ -9,8 +9,9 @@
 // zero-filled gradient per slice - moved each of q, k, v six to eight times.  Bound by HBM: D / 8 lanes own a head row, a
 // lane holds 4 columns of either half, so the rotation pairs are its own (no exchange) and the row sum is a few shuffles.
 // The normalised value and its gradient stay in fp32 between the norm and the rotation.
-// Measured for 8 samples of 512 tokens, 24 heads of 128: 27 us forward and 49 us backward a block (38 and 51 MB written and
-// read: 2.8 and 2.6 TB/s), for about 500 us of slices, clones, norms and concatenations.  MMDiT training pass of 8 samples
+// Measured for 8 samples of 512 tokens, 24 heads of 128, L2 flushed: 39 us forward (75 MB read, 75 written: 3.9 TB/s) and 77 us
+// backward with the scale gradients (126 MB read, 75 written: 2.6 TB/s), for about 500 us a block of slices, clones, norms and
+// concatenations, both directions together.  MMDiT training pass of 8 samples
 // 12.8 -> 10.9 ms, sampling pass of one 2.43 -> 2.07 ms (21 launches fewer).
 //
 // Reference: the fused norm + RoPE of the FLUX submission (flux1/primus/config_common.sh:84-150).

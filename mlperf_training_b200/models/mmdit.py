@@ -143,8 +143,12 @@ class QKNorm(nn.Module):
                 and not (self._forward_hooks or self._forward_pre_hooks or self._backward_hooks or self._backward_pre_hooks))
 
 
-def _fused_qk(norms) -> bool:
-    return all(isinstance(n, QKNorm) and n.is_plain() for n in norms) and len({n.eps for n in norms}) == 1
+def _fused_qk(*norms) -> bool:
+    """Plain norms of one eps (a fused launch takes one value)."""
+    for n in norms:
+        if type(n) is not QKNorm or not n.is_plain() or n.eps != norms[0].eps:
+            return False
+    return True
 
 
 def _ln(x2d):
@@ -200,7 +204,7 @@ class DoubleBlock(nn.Module):
             parts[s] = (qkv, mod, x.shape[0] // B)
         St, Si = parts["txt"][2], parts["img"][2]
         norms = (self.txt_qknorm, self.img_qknorm)
-        fused = _fused_qk(norms)
+        fused = _fused_qk(*norms)
         if fused:
             streams = [(parts[s][0], n.q_scale, n.k_scale) for s, n in zip(("txt", "img"), norms)]
             fused = F.qkv_norm_rope_ok(cos, hd, streams)
@@ -244,7 +248,7 @@ class SingleBlock(nn.Module):
         y = self.linear1(_ln_modulate(x, shift, scale, B), pr)
         S = x.shape[0] // B
         n = self.qknorm
-        if _fused_qk((n,)) and F.qkv_norm_rope_ok(cos, hd, [(y, n.q_scale, n.k_scale)]) and y.shape[1] % 8 == 0:
+        if _fused_qk(n) and F.qkv_norm_rope_ok(cos, hd, [(y, n.q_scale, n.k_scale)]) and y.shape[1] % 8 == 0:
             q, k, v, act = F.single_stream_in(y, n.q_scale, n.k_scale, cos, sin, B, H, hd, n.eps)
             attn = _attention(q, k, v, self.sp).reshape(-1, d)
         else:

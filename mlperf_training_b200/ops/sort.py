@@ -107,7 +107,7 @@ def segment_sum_blocks(src: torch.Tensor, s: SortedIds, max_seg: int, max_bytes:
     src, partial = src.contiguous(), _partial_sums(n, D, src.device)
     buf = torch.empty((block, D), dtype=torch.float32, device=src.device)
     for first in range(0, max_seg, block):
-        out = buf[:min(block, max_seg - first)]
+        out = buf if first + block <= max_seg else buf[:max_seg - first]
         _sum_runs(src, s, first, out, partial)
         yield first, out
 

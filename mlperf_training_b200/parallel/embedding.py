@@ -183,7 +183,7 @@ class ShardedEmbedding:
         """Sums the duplicates and updates a block of unique rows at a time.  A lookup without a plan knows only that there are
         at most as many unique rows as ids, and heavily repeated ids would otherwise hold an fp32 row for every one of them."""
         for first, g in S.segment_sum_blocks(grad, srt, rows.numel(), SUM_BLOCK_BYTES):
-            self.apply_rowwise_adagrad(rows[first:first + g.shape[0]], g)
+            self.apply_rowwise_adagrad(rows if g.shape[0] == rows.numel() else rows[first:first + g.shape[0]], g)
 
     def apply_rowwise_adagrad(self, rows: torch.Tensor, grads: torch.Tensor) -> None:
         """Row-wise Adagrad on the rows ``rows`` of the local shard (entries outside ``[0, local_rows)`` are skipped);

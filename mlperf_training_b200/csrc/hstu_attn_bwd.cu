@@ -277,18 +277,23 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int r = q * 32 + lane;              // key row of the tile
     const uint32_t lane_base = uint32_t(q * 32) << 16;
     const int kp = kv0 + r;                   // this thread's key
-    const bool plain = (n_tgt == 0 && ctx == 0);
-    const int k_id = min(max(kp - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
+    // Queries that see key kp: q >= q_begin (id(q) > id(k) is one comparison of q), q == kp, and contextual rows q < ctx_end.
+    // A key past the sequence's end belongs to the next sequence: nobody sees it.
+    constexpr int NONE = 0x3fffffff;
+    const int id_off = ctx - (ctx > 0 ? 1 : 0);
+    const int k_id = min(max(kp - id_off, 0), max_id);
+    const int q_begin = (kp < len && k_id < max_id) ? k_id + 1 + id_off : NONE;
+    const int ctx_end = (ctx > 0 && max_id >= 0 && kp < hist_end) ? (max_id == 0 ? NONE : id_off + 1) : 0;
+    const int q_self = kp < len ? kp : -1;
     const float ha = 0.5f * p.alpha, inv_n = 1.0f / (float)p.max_len, an = p.alpha * inv_n;
     bool ok = true;
     for (int it = 0; it < n_iter && ok; ++it) {
       const int q0 = q_tile(it) * BQ;
       // a tile whose every (query, key) pair is visible needs no element mask: ids grow with the position, so it
-      // is enough that the tile's first query is later than its last key, and that both tiles lie inside the sequence
-      const int first_q_id = min(max(q0 - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
-      const int last_k_id = min(max(kv0 + BKV - 1 - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
-      const bool inside = (kv0 + BKV <= len) && (q0 + BQ <= len);
-      const bool need_mask = plain ? ((kv0 + BKV - 1 > q0) || !inside) : !(inside && first_q_id > last_k_id);
+      // is enough that the tile's first query is later than its last key, and that the query tile lies inside the sequence
+      // (then its keys do)
+      const int first_q_id = min(max(q0 - id_off, 0), max_id);
+      const bool need_mask = !(q0 + BQ <= len && first_q_id > 0 && kv0 + BKV <= first_q_id + id_off);
       if (!warp_wait(s_full, it & 1, abort_flag, p.status, 90)) { ok = false; break; }
       tc_fence_after();
       float f[64];                            // dS / dP of this key and the half's queries
@@ -311,16 +316,16 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           f[i] = fv.x; f[i + 1] = fv.y;
         }
         if (need_mask) {
+          const int qc = q0 + half * 64;
+          const int beg = q_begin - qc, self = q_self - qc, end = len - qc, cend = ctx_end - qc;
+          if (ctx == 0) {
 #pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            const int q_pos = q0 + half * 64 + i;
-            bool vis;
-            if (plain) vis = kp <= q_pos;
-            else {
-              const int q_id = min(max(q_pos - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
-              vis = (kp == q_pos) || (q_id > k_id) || (ctx > 0 && q_id == 0 && kp < hist_end);
-            }
-            if (!(vis && kp < len && q_pos < len)) { s[i] = 0u; f[i] = 0.f; }
+            for (int i = 0; i < 64; ++i)
+              if ((i < beg && i != self) || i >= end) { s[i] = 0u; f[i] = 0.f; }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 64; ++i)
+              if ((i < beg && i != self && i >= cend) || i >= end) { s[i] = 0u; f[i] = 0.f; }
           }
         }
         uint32_t pk[32];

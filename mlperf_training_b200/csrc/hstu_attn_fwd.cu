@@ -26,10 +26,10 @@
 //
 // What bounds it: per pair of 128 x 128 tiles 2048 tensor-core cycles against 2048 of the MUFU unit (one tanh per score), and
 // the activation's other work.  A step of a pair takes 5600 to 6000 cycles on average (clock64 in the activation warps, 1700
-// to 1900 of them waiting for scores) and 10,900 where the element mask is applied, which a query tile that ends past its
-// sequence does on every key tile; a CTA adds 4600 cycles before its first scores and 2600 after its last.  128 users of median
-// 512 tokens, 4 heads: 1856 CTAs of 8192 have work and keep the SMs busy for 402 of 462 us.  12 users of median 700: 190 us
-// are the longest CTA, 31 masked steps in series, while the average SM works for 57 us.
+// to 1900 of them waiting for scores); a CTA adds 4600 cycles before its first scores and 2600 after its last.
+// The element mask is two comparisons a score on the tiles of the diagonal alone.  (A query tile that ends past its sequence used to
+// mask every key tile, at 10,900 cycles a step with ids recomputed for every score: 12 users of median 700 waited 190 us for the
+// longest CTA's 31 masked steps, now 60.)
 // Scores come 64 columns per TMEM round trip, P V starts on the first half of the keys, and the latest query tiles of all
 // sequences go first.  With the clearing of the output, 128 users: 728 -> 497 us; 12 users: 271 -> 203 us (rolled 32-column
 // chunks, sequence after sequence before).
@@ -270,8 +270,12 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint32_t ts = tmem_base + lane_base + t * 128;
     const uint32_t to = tmem_base + lane_base + 256 + t * 128;
     const int my_n = n_t[t];
-    const int q_id = min(max(q_pos - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
-    const bool plain = (n_tgt == 0 && ctx == 0);
+    // Keys row q sees: k < k_end, and itself.  id(k) grows with k and q's own id is at most max_id, so id(q) > id(k) is one
+    // comparison of k; a contextual row (id 0) sees the history.  Both are below len for a row inside the sequence, and a
+    // row past it is not stored: its scores may hold anything.
+    const int id_off = ctx - (ctx > 0 ? 1 : 0);
+    const int q_id = min(max(q_pos - id_off, 0), max_id);
+    const int k_end = q_id > 0 ? q_id + id_off : (ctx > 0 && q_id == 0 ? hist_end : 0);
     // 8-bit: S carries the factors of Q and K; P is stored without 1 / N (e4m3 range), O takes it with V's factor
     const float half_alpha = F8 ? 0.5f * p.alpha * (*p.inv_q) * (*p.inv_k) : 0.5f * p.alpha;
     const float inv_n = F8 ? 1.0f : 1.0f / (float)p.max_len;
@@ -281,13 +285,10 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int kv0 = (j_lo + n) * BKV;
       if (!warp_wait(&s_full[t], n & 1, abort_flag, p.status, 170)) { ok = false; break; }
       tc_fence_after();
-      // tiles strictly below the diagonal and inside the sequence need no element mask
-      // (with targets / contextual tokens: ids grow with the position, so every pair of the tile is visible when its
-      // first query is later than its last key)
-      const int first_q_id = min(max(qt0 - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
-      const int last_k_id = min(max(kv0 + BKV - 1 - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
-      const bool inside = (kv0 + BKV <= len) && (qt0 + BQ <= len);
-      const bool need_mask = plain ? ((kv0 + BKV - 1 > qt0) || !inside) : !(inside && first_q_id > last_k_id);
+      // No element mask where the tile's first row sees its last key (k_end grows with the row; rows past the sequence's end
+      // need none).  Masking every key tile of a query tile that ends past its sequence cost 10,900 cycles a step.
+      const int first_q_id = min(max(qt0 - id_off, 0), max_id);
+      const bool need_mask = !(first_q_id > 0 && kv0 + BKV <= first_q_id + id_off);
       // 64 columns at a time, unrolled: two TMEM loads in flight, and independent activations to cover each other's latency
       // (32 columns in a rolled loop waited for one load and one chain at a time)
       const float2 ha2 = make_float2(half_alpha, half_alpha), in2 = make_float2(inv_n, inv_n);
@@ -307,17 +308,10 @@ hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           v[2 * i + 1] = __float_as_uint(x.y);
         }
         if (need_mask) {
+          const int end = k_end - (kv0 + c * 64), self = q_pos - (kv0 + c * 64);
 #pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            const int kpe = kv0 + c * 64 + i;
-            bool vis;
-            if (plain) vis = kpe <= q_pos;
-            else {
-              const int k_id = min(max(kpe - ctx + (ctx > 0 ? 1 : 0), 0), max_id);
-              vis = (kpe == q_pos) || (q_id > k_id) || (ctx > 0 && q_id == 0 && kpe < hist_end);
-            }
-            if (!(vis && kpe < len && q_pos < len)) v[i] = 0u;
-          }
+          for (int i = 0; i < 64; ++i)
+            if (i >= end && i != self) v[i] = 0u;
         }
         if constexpr (F8) {
           uint32_t p8[16];                                 // keys 4 j .. 4 j + 3 of the chunk in column j

@@ -666,6 +666,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t b_kstep = (b_mn ? 16 * 128 : UMMA_K_BYTES) >> 4;
       const uint64_t ad0 = umma_desc_sw128(smem_u32(sA), a_mn ? 8192 : 16, 1024);
       const uint64_t bd0 = umma_desc_sw128(smem_u32(sB), b_mn ? 8192 : 16, 1024);
+      // An odd number of 128-byte blocks leaves nothing but padding in the second half of the last stage of two (a contraction of
+      // 2880 block-scaled elements is 22.5 blocks: 23 are multiplied, not 24).  Its operands arrive as zeros, but its scales are
+      // whatever follows in the buffer, and zero times a NaN scale is NaN: it must not be multiplied.
+      const bool odd_tail = KSUB == 2 && p.grp.mode != 2 && (num_kb128 & 1);
       int stage = 0; uint32_t phase = 0;
       int it = 0;
       bool ok = true;
@@ -685,6 +689,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (elect_one()) {
 #pragma unroll
             for (int s = 0; s < KSUB; ++s) {
+              if (s > 0 && odd_tail && ti.kb0 + kb == num_kb - 1) break;
               const uint64_t ad = ad0 + ((stage * KSUB + s) * C::A_SUB >> 4);
               const uint64_t bd = bd0 + ((stage * KSUB + s) * C::B_SUB >> 4);
               const uint32_t t_sfa = tmem_base + C::SF_COL + (uint32_t)(stage * KSUB + s) * C::SF_SET_COLS;   // MX only

@@ -76,7 +76,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
     ld8(gu + t * 2 * F + v * 8, g);
     ld8(gu + t * 2 * F + F + v * 8, u);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = g[j] / (1.f + __expf(-g[j])) * u[j];
+    for (int j = 0; j < 8; ++j) o[j] = g[j] * sigmoid(g[j]) * u[j];
     st8(a + t * F + v * 8, o);
   }
 }
@@ -94,7 +94,7 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ da, const __
     ld8(da + t * F + v * 8, d);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float sg = 1.f / (1.f + __expf(-g[j]));
+      const float sg = sigmoid(g[j]);
       const float silu = g[j] * sg;
       du[j] = d[j] * silu;
       dg[j] = d[j] * u[j] * sg * (1.f + g[j] * (1.f - sg));

@@ -58,7 +58,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_adamw": [P, I, P, P, I, P, P, L, F, F, F, F, F, I, F, P, F, I, P],
         "b200_adamw_bf16m": [P, I, P, P, I, P, P, L, F, F, F, F, F, I, F, P, F, I, P],
         "b200_attn_fwd": [P, P, P, P, P, P, I, I, I, I, I, I, L, L, L, L, L, L, L, L, F, I, I, P],
-        "b200_quant_mxfp8": [P, L, I, I, P, P, I, P, P, I, P],
+        "b200_quant_mxfp8": [P, L, I, I, P, P, I, P, P, I, P, P],
         "b200_gemm_mxfp8": [P, P, P, P, P, I, I, I, L, L, L, I, I, P, P, L, F, P, L, P],
         "b200_router_topk": [P, I, I, I, P, P, P, P],
         "b200_router_plan": [P, P, I, I, I, P, P, I, P, P],
@@ -100,8 +100,8 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_ep_route": [P, P, I, I, I, I, L, L, P, P, P, P, P, P],
         "b200_unpermute_bwd": [P, P, P, P, L, I, I, P, P, P],
         "b200_zero_dead_tiles": [P, P, I, I, P],
-        "b200_quant_swiglu_mxfp8": [P, L, I, I, P, P, I, P, P, I, P],
-        "b200_quant_swiglu_bwd_mxfp8": [P, L, P, L, I, I, P, P, I, P, P, I, P],
+        "b200_quant_swiglu_mxfp8": [P, L, I, I, P, P, I, P, P, I, P, P],
+        "b200_quant_swiglu_bwd_mxfp8": [P, L, P, L, I, I, P, P, I, P, P, I, P, P],
         "b200_flag_wait_probe": [P, I, L, P, P],
         "b200_gemm_tp_gather": [P, P, P, I, I, I, L, L, L, I, I, I, I, F, I, P, I, I, P, L, I, P, I, I, P, P],
         "b200_gemm_tp_rs": [P, P, I, I, I, L, L, I, I, F, P, P, I, I, P, P, L, P, L, I, P],

@@ -366,7 +366,8 @@ class GroupedMLPMXFn(Function):
         narrow = recipe != "mxfp8"
         if narrow:
             x = _zero_padding_mx(x, tile_expert)
-        x_row, x_col = mxfp8.quantize(x, row_tile=mxfp8.A_TILE, col_tile=grouped_bn(D), fmt=f_act, col_fmt=b_act)
+        live = seg[E:]        # rows up to the last segment's end: the quantisers skip the tiles behind it
+        x_row, x_col = mxfp8.quantize(x, row_tile=mxfp8.A_TILE, col_tile=grouped_bn(D), fmt=f_act, col_fmt=b_act, live=live)
         # rows of tiles past the last segment are never written and never contribute: the row GEMMs skip those
         # tiles and the weight-gradient contraction stops at the last segment's end
         gu = grouped_rows_mx(x_row, _stacked_weight_op(w1, False, f_w), tile_expert, E)
@@ -374,7 +375,7 @@ class GroupedMLPMXFn(Function):
             a_row, a_col = mxfp8.quantize(_zero_padding_mx(K.swiglu_fwd(gu), tile_expert), row_tile=mxfp8.A_TILE,
                                           col_tile=grouped_bn(F), fmt=f_act, col_fmt=b_act)
         else:
-            a_row, a_col = mxfp8.quantize_swiglu(gu, row_tile=mxfp8.A_TILE, col_tile=grouped_bn(F))
+            a_row, a_col = mxfp8.quantize_swiglu(gu, row_tile=mxfp8.A_TILE, col_tile=grouped_bn(F), live=live)
         y = grouped_rows_mx(a_row, _stacked_weight_op(w2, False, f_w), tile_expert, E, out=y_out)
         ctx.save_for_backward(gu, w1, w2, seg, tile_expert, x_col.q, x_col.sf, a_col.q, a_col.sf)
         ctx.refs = (w1, w2)
@@ -397,14 +398,15 @@ class GroupedMLPMXFn(Function):
         gy = gy.contiguous()
         if narrow:
             gy = _zero_padding_mx(gy, tile_expert)
-        gy_row, gy_col = mxfp8.quantize(gy, row_tile=mxfp8.A_TILE, col_tile=mxfp8.A_TILE, fmt=g_fmt, stochastic=g_sr)
+        live = seg[E:]
+        gy_row, gy_col = mxfp8.quantize(gy, row_tile=mxfp8.A_TILE, col_tile=mxfp8.A_TILE, fmt=g_fmt, stochastic=g_sr, live=live)
         g2 = _wgrad_into_mx(p2, gy_col, a_col, seg, E)
         da = grouped_rows_mx(gy_row, _stacked_weight_op(w2, True, b_w), tile_expert, E)
         if narrow:
             dgu_row, dgu_col = mxfp8.quantize(_zero_padding_mx(K.swiglu_bwd(da, gu), tile_expert), row_tile=mxfp8.A_TILE,
                                               col_tile=mxfp8.A_TILE, fmt=g_fmt, stochastic=g_sr)
         else:
-            dgu_row, dgu_col = mxfp8.quantize_swiglu_bwd(da, gu, row_tile=mxfp8.A_TILE, col_tile=mxfp8.A_TILE)
+            dgu_row, dgu_col = mxfp8.quantize_swiglu_bwd(da, gu, row_tile=mxfp8.A_TILE, col_tile=mxfp8.A_TILE, live=live)
         g1 = _wgrad_into_mx(p1, dgu_col, x_col, seg, E)
         dx = grouped_rows_mx(dgu_row, _stacked_weight_op(w1, True, b_w), tile_expert, E, out=ctx.dx_out)
         return dx, g1, g2, None, None, None, None, None

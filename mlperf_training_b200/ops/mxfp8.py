@@ -138,14 +138,16 @@ def dequantize(op: MXOperand) -> torch.Tensor:
 
 
 def quantize(x: torch.Tensor, *, row_tile: int | None = None, col_tile: int | None = None, fmt: str = "e4m3",
-             col_fmt: str | None = None, stochastic: bool = False):
+             col_fmt: str | None = None, stochastic: bool = False, live: torch.Tensor | None = None):
     """bf16 ``x`` ``[R, C]`` -> ``(row_op, col_op)``.  ``fmt`` / ``col_fmt`` (default: ``fmt``): element format of the
     row-wise / column-wise copy; anything but round-to-nearest e4m3 goes through ``quantize_rows_narrow``.
 
     ``row_op`` (when ``row_tile`` is given) has rows = R, contraction = C; ``col_op`` (when
     ``col_tile`` is given) is the transposed copy with rows = C, contraction = R.  The tile
     arguments say how the consuming GEMM tiles the operand's rows: ``A_TILE`` for an A operand,
-    ``b_tile(rows)`` for a B operand.  R must be a multiple of 128 and C of 32."""
+    ``b_tile(rows)`` for a B operand.  R must be a multiple of 128 and C of 32.  ``live``: one int32 on the device, the
+    number of leading rows (a multiple of 128) that will be used; the round-to-nearest e4m3 quantiser may leave the copies of
+    later rows unwritten."""
     R, C = x.shape
     if R % 128 or C % 32:
         raise ValueError(f"mxfp8.quantize: shape {R}x{C}: rows must be a multiple of 128, columns of 32")
@@ -169,18 +171,16 @@ def quantize(x: torch.Tensor, *, row_tile: int | None = None, col_tile: int | No
         x = x.contiguous()
     q_row, sf_row, q_col, sf_col = _alloc_ops(R, C, row_tile, col_tile, x.device)
     call("b200_quant_mxfp8", ptr(x), x.stride(0), R, C, ptr(q_row), ptr(sf_row), row_tile or 0, ptr(q_col),
-         ptr(sf_col), col_tile or 0, stream_ptr())
+         ptr(sf_col), col_tile or 0, ptr(live), stream_ptr())
     row_op = MXOperand(q_row, sf_row, R, C, row_tile) if row_tile is not None else None
     col_op = MXOperand(q_col, sf_col, C, R, col_tile) if col_tile is not None else None
     return row_op, col_op
 
 
 def _sf_buffer(rows: int, k: int, tile: int, dev) -> torch.Tensor:
-    """Scale buffer of an operand; zero-filled when the quantiser leaves padding rows of an atom unwritten."""
-    n = sf_bytes(rows, k, tile)
-    if tile % 128 or rows % 128:
-        return torch.zeros(n, dtype=torch.uint8, device=dev)
-    return torch.empty(n, dtype=torch.uint8, device=dev)
+    """Scale buffer of an operand.  Bytes of an atom's rows past the tile or the operand stay as they are: the GEMM meets
+    them only in accumulator rows and columns that it does not store."""
+    return torch.empty(sf_bytes(rows, k, tile), dtype=torch.uint8, device=dev)
 
 
 def _alloc_ops(R: int, C: int, row_tile, col_tile, dev):
@@ -194,9 +194,10 @@ def _alloc_ops(R: int, C: int, row_tile, col_tile, dev):
     return q_row, sf_row, q_col, sf_col
 
 
-def quantize_swiglu(gu: torch.Tensor, *, row_tile: int | None = None, col_tile: int | None = None):
+def quantize_swiglu(gu: torch.Tensor, *, row_tile: int | None = None, col_tile: int | None = None,
+                    live: torch.Tensor | None = None):
     """Quantised ``a = silu(gate) * up`` of ``gu [R, 2F]`` (gate columns first) without materialising
-    ``a``: same return value as ``quantize(swiglu(gu), ...)``."""
+    ``a``: same return value as ``quantize(swiglu(gu), ...)``; ``live`` as there."""
     R, F2 = gu.shape
     F = F2 // 2
     if not use_kernels(gu):
@@ -206,17 +207,18 @@ def quantize_swiglu(gu: torch.Tensor, *, row_tile: int | None = None, col_tile: 
         gu = gu.contiguous()
     q_row, sf_row, q_col, sf_col = _alloc_ops(R, F, row_tile, col_tile, gu.device)
     call("b200_quant_swiglu_mxfp8", ptr(gu), gu.stride(0), R, F, ptr(q_row), ptr(sf_row), row_tile or 0, ptr(q_col),
-         ptr(sf_col), col_tile or 0, stream_ptr())
+         ptr(sf_col), col_tile or 0, ptr(live), stream_ptr())
     return (MXOperand(q_row, sf_row, R, F, row_tile) if row_tile is not None else None,
             MXOperand(q_col, sf_col, F, R, col_tile) if col_tile is not None else None)
 
 
-def quantize_swiglu_bwd(da: torch.Tensor, gu: torch.Tensor, *, row_tile: int | None = None, col_tile: int | None = None):
+def quantize_swiglu_bwd(da: torch.Tensor, gu: torch.Tensor, *, row_tile: int | None = None, col_tile: int | None = None,
+                        live: torch.Tensor | None = None):
     """Quantised ``dgu [R, 2F]`` (d gate | d up) from ``da [R, F]`` and ``gu [R, 2F]`` without
-    materialising it: same return value as ``quantize(swiglu_bwd(da, gu), ...)``."""
+    materialising it: same return value as ``quantize(swiglu_bwd(da, gu), ...)``; ``live`` as there."""
     R, F2 = gu.shape
     F = F2 // 2
-    if not use_kernels(gu) or F % 128:      # the fused kernel's tiles must not straddle the gate | up boundary
+    if not use_kernels(gu) or F % 32:       # a 32-block must not straddle the gate | up boundary
         from . import kernels as K
         return quantize(K.swiglu_bwd(da, gu), row_tile=row_tile, col_tile=col_tile)
     da = da if (da.stride(1) == 1 and (da.stride(0) * 2) % 16 == 0 and da.data_ptr() % 16 == 0) else da.contiguous()
@@ -224,7 +226,7 @@ def quantize_swiglu_bwd(da: torch.Tensor, gu: torch.Tensor, *, row_tile: int | N
         gu = gu.contiguous()
     q_row, sf_row, q_col, sf_col = _alloc_ops(R, F2, row_tile, col_tile, gu.device)
     call("b200_quant_swiglu_bwd_mxfp8", ptr(da), da.stride(0), ptr(gu), gu.stride(0), R, F, ptr(q_row), ptr(sf_row),
-         row_tile or 0, ptr(q_col), ptr(sf_col), col_tile or 0, stream_ptr())
+         row_tile or 0, ptr(q_col), ptr(sf_col), col_tile or 0, ptr(live), stream_ptr())
     return (MXOperand(q_row, sf_row, R, F2, row_tile) if row_tile is not None else None,
             MXOperand(q_col, sf_col, F2, R, col_tile) if col_tile is not None else None)
 

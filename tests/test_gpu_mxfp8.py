@@ -46,6 +46,56 @@ def test_quantize_partial_column_tile(R, C):
     assert (mxfp8.dequantize(at_g).cpu() - mxfp8.dequantize(at_c)).abs().max() <= 0.13 * ref.abs().max()
 
 
+def test_quantize_scale_limits():
+    """Blocks whose largest magnitude sits at the ends of the scale rule: 1.75 times a power of two and its bf16 neighbours,
+    amax / 448 below the normal numbers, bf16 denormals, zero, the largest finite value."""
+    x = torch.zeros(128, 256)
+    amax = [1.75, 1.75 * (1 + 2 ** -7), 1.75 * (1 - 2 ** -7), 448.0, 450.0, 2.0 ** -118, 2.0 ** -119, 1.9 * 2.0 ** -118, 2.0 ** -126, 2.0 ** -130,
+            0.0, 3.3e38, 1.75 * 2.0 ** 100, 1.0]
+    for i, a in enumerate(amax):
+        x[i] = a * torch.linspace(-1, 1, 256)
+        x[i, ::32] = a
+    x = x.bfloat16()
+    for t, kw in ((x, dict(row_tile=128)), (x.t().contiguous(), dict(col_tile=128))):
+        for cpu, gpu in zip(mxfp8.quantize(t, **kw), mxfp8.quantize(t.cuda(), **kw)):
+            if cpu is not None:
+                assert torch.equal(mxfp8.sf_plain(gpu).cpu(), cpu.sf)
+                assert torch.equal(gpu.q.cpu(), cpu.q)
+
+
+@pytest.mark.parametrize("R,F", [(128, 128), (256, 160), (384, 2880), (128, 96)])
+def test_quantize_swiglu_bwd_equals_the_separate_kernels(R, F):
+    """d gate | d up from one tile pair: codes and scales of quantising the stand-alone kernel's output, bit for bit, at widths
+    whose halves start inside a scale word; rows past ``live`` are left alone."""
+    from mlperf_training_b200.ops import kernels as K
+    torch.manual_seed(R + F)
+    gu, da = (torch.randn(R, 2 * F, device="cuda") * 3).bfloat16(), torch.randn(R, F, device="cuda").bfloat16()
+    want = mxfp8.quantize(K.swiglu_bwd(da, gu), row_tile=128, col_tile=208)
+    got = mxfp8.quantize_swiglu_bwd(da, gu, row_tile=128, col_tile=208)
+    for a, b in zip(want, got):
+        assert torch.equal(a.q, b.q) and torch.equal(mxfp8.sf_plain(a), mxfp8.sf_plain(b))
+    assert torch.equal(want[0].sf, got[0].sf)            # (the padding of the last scale word, too)
+    for w, g in zip(mxfp8.quantize(K.swiglu_fwd(gu), row_tile=128, col_tile=192), mxfp8.quantize_swiglu(gu, row_tile=128, col_tile=192)):
+        assert torch.equal(w.q, g.q) and torch.equal(mxfp8.sf_plain(w), mxfp8.sf_plain(g))
+    live = torch.tensor([128], dtype=torch.int32, device="cuda")
+    part = mxfp8.quantize_swiglu_bwd(da, gu, row_tile=128, col_tile=208, live=live)
+    assert torch.equal(part[0].q[:128], want[0].q[:128]) and torch.equal(part[1].q[:, :128], want[1].q[:, :128])
+
+
+@pytest.mark.parametrize("K", [128, 384, 640])
+def test_gemm_does_not_read_scales_past_an_odd_contraction(K):
+    """The scales behind a contraction of an odd number of 128-blocks may be anything (here: NaN for every row tile's neighbour)."""
+    torch.manual_seed(K)
+    a, b = torch.randn(512, K, device="cuda").bfloat16(), torch.randn(416, K, device="cuda").bfloat16()
+    b = torch.cat([b, torch.zeros(96, K, device="cuda").bfloat16()])
+    qa, qb = mxfp8.quantize(a, row_tile=mxfp8.A_TILE)[0], mxfp8.quantize(b, row_tile=mxfp8.b_tile(512))[0]
+    want = mxfp8.gemm(qa, qb)
+    sf = qa.sf.clone()
+    sf.view(4, -1)[1:] = 255                             # rows 128 .. of A: not a number
+    got = mxfp8.gemm(mxfp8.MXOperand(qa.q, sf, qa.rows, qa.k, qa.tile_rows), qb)
+    assert torch.equal(got[:128], want[:128])
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 128, 128), (256, 224, 256), (384, 448, 512), (512, 1000, 384),
                                    (1024, 4096, 1024), (136, 72, 128)])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])

@@ -47,9 +47,11 @@ class LinearFn(Function):
     """y = x W^T (+ bias) (+ residual), the residual add done in the GEMM epilogue."""
 
     @staticmethod
-    def forward(ctx, x, weight, bias, residual, precision):
-        need_w = weight.requires_grad
-        y, saved = L.forward(x, weight, precision, bias=bias, residual=residual, need_wgrad=need_w)
+    def forward(ctx, x, weight, bias, residual, precision, grad=True):
+        # ``grad``: a backward may follow (inside a Function's forward the gradient mode is off in any case).  Without one the
+        # quantised copies that only a backward reads are not made.
+        y, saved = L.forward(x, weight, precision, bias=bias, residual=residual, need_wgrad=grad and weight.requires_grad,
+                             need_dgrad=grad and ctx.needs_input_grad[0])
         tensors, ctx.meta = L.Saved.pack(saved) if saved is not None else ([], None)
         ctx.save_for_backward(weight, *tensors)
         ctx.has_res = residual is not None
@@ -66,11 +68,11 @@ class LinearFn(Function):
                             need_dw=weight.requires_grad and saved is not None)
         db = _vec_grad(ctx.bias_ref, dy.sum(0, dtype=torch.float32)) if ctx.bias_ref is not None else None
         dres = dy if ctx.has_res and ctx.needs_input_grad[3] else None
-        return dx, dw, db, dres, None
+        return dx, dw, db, dres, None, None
 
 
 def linear(x, weight, bias=None, residual=None, precision="bf16"):
-    return LinearFn.apply(x, weight, bias, residual, precision)
+    return LinearFn.apply(x, weight, bias, residual, precision, torch.is_grad_enabled())
 
 
 class NormFn(Function):
@@ -111,10 +113,11 @@ class NormLinearFn(Function):
     produced by the same quantisation pass that feeds the forward GEMM, is kept instead."""
 
     @staticmethod
-    def forward(ctx, x, norm_w, norm_b, weight, bias, eps, layer_norm, precision):
+    def forward(ctx, x, norm_w, norm_b, weight, bias, eps, layer_norm, precision, grad=True):
         xn, _, mean, rstd = K.norm_fwd(x, norm_w, norm_b, eps, layer_norm=layer_norm)
-        keep = L.low_precision(precision, x.shape[0], weight.shape[0], weight.shape[1])
-        y, saved = L.forward(xn, weight, precision, bias=bias, need_wgrad=keep and weight.requires_grad)
+        grad = grad and any(ctx.needs_input_grad)
+        keep = grad and L.low_precision(precision, x.shape[0], weight.shape[0], weight.shape[1])
+        y, saved = L.forward(xn, weight, precision, bias=bias, need_wgrad=keep and weight.requires_grad, need_dgrad=grad)
         tensors, ctx.meta = L.Saved.pack(saved) if saved is not None else ([], None)
         ctx.save_for_backward(x, norm_w, norm_b, weight, mean, rstd, *tensors)
         ctx.cfg = (eps, layer_norm, precision)
@@ -137,20 +140,20 @@ class NormLinearFn(Function):
         del saved
         dx, dnw, dnb = K.norm_bwd(dxn, x, norm_w, norm_b, mean, rstd, layer_norm=layer_norm)
         db = _vec_grad(ctx.refs[2], dy.sum(0, dtype=torch.float32)) if ctx.refs[2] is not None else None
-        return dx, _vec_grad(ctx.refs[0], dnw), _vec_grad(ctx.refs[1], dnb), dw, db, None, None, None
+        return dx, _vec_grad(ctx.refs[0], dnw), _vec_grad(ctx.refs[1], dnb), dw, db, None, None, None, None
 
 
 def norm_linear(x, norm_w, weight, *, norm_b=None, bias=None, eps=1e-5, layer_norm=False, precision="bf16"):
-    return NormLinearFn.apply(x, norm_w, norm_b, weight, bias, eps, layer_norm, precision)
+    return NormLinearFn.apply(x, norm_w, norm_b, weight, bias, eps, layer_norm, precision, torch.is_grad_enabled())
 
 
 class SwiGLULinearFn(Function):
     """out = swiglu(gu) W^T + residual, saving only ``gu`` (the activation is recomputed)."""
 
     @staticmethod
-    def forward(ctx, gu, weight, residual, precision):
+    def forward(ctx, gu, weight, residual, precision, grad=True):
         a = K.swiglu_fwd(gu)
-        out, _ = L.forward(a, weight, precision, residual=residual, need_wgrad=False)
+        out, _ = L.forward(a, weight, precision, residual=residual, need_wgrad=False, need_dgrad=grad and any(ctx.needs_input_grad))
         ctx.save_for_backward(gu, weight)
         ctx.has_res = residual is not None
         ctx.precision = precision
@@ -164,11 +167,11 @@ class SwiGLULinearFn(Function):
         da, dw = L.backward(dy, a, weight, ctx.precision, need_dx=True, need_dw=weight.requires_grad)
         del a
         dgu = K.swiglu_bwd(da, gu)
-        return dgu, dw, (dy if ctx.has_res else None), None
+        return dgu, dw, (dy if ctx.has_res else None), None, None
 
 
 def swiglu_linear(gu, weight, residual=None, precision="bf16"):
-    return SwiGLULinearFn.apply(gu, weight, residual, precision)
+    return SwiGLULinearFn.apply(gu, weight, residual, precision, torch.is_grad_enabled())
 
 
 def _mx_wgrad(weight, dy_col, x_col):
@@ -198,17 +201,18 @@ class FusedMLPFn(Function):
     SwiGLU op with FP8 input store, llama2_sft/primus/patches/megatron_lm_mxfp4_recipe.patch)."""
 
     @staticmethod
-    def forward(ctx, h, norm_w, w_gu, w_down, eps, store_fp8=False):
+    def forward(ctx, h, norm_w, w_gu, w_down, eps, store_fp8=False, grad=True):
         from . import mxfp8 as MX
         D = h.shape[1]
         xn, _, mean, rstd = K.norm_fwd(h, norm_w, None, eps, layer_norm=False)
-        need1 = w_gu.requires_grad
-        w1_row, _ = L.weight_operands(w_gu, need_col=False)
+        grad = grad and any(ctx.needs_input_grad)
+        need1 = grad and w_gu.requires_grad
+        w1_row, _ = L.weight_operands(w_gu, need_col=grad)
         xn_row, xn_col = MX.quantize(xn, row_tile=MX.A_TILE, col_tile=MX.b_tile(D) if need1 else None)
         del xn
         gu = MX.gemm(xn_row, w1_row, out_dtype=h.dtype)
         a_row, _ = MX.quantize_swiglu(gu, row_tile=MX.A_TILE)
-        w2_row, _ = L.weight_operands(w_down, need_col=False)
+        w2_row, _ = L.weight_operands(w_down, need_col=grad)
         out = MX.gemm(a_row, w2_row, residual=h, out_dtype=h.dtype)
         tensors, ctx.meta = L.Saved.pack(xn_col) if xn_col is not None else ([], None)
         ctx.gu_fp8 = bool(store_fp8)
@@ -251,7 +255,7 @@ class FusedMLPFn(Function):
         dxn = MX.gemm(dgu_row, w1_col, out_dtype=dy.dtype)
         dw1 = _mx_wgrad(p_gu, dgu_col, L.Saved.unpack(tensors, ctx.meta)) if need1 else None
         dx, dnw, _ = K.norm_bwd(dxn, h, norm_w, None, mean, rstd, layer_norm=False, dres=dy)
-        return dx, _vec_grad(p_norm, dnw), dw1, dw2, None, None
+        return dx, _vec_grad(p_norm, dnw), dw1, dw2, None, None, None
 
 
 def fused_mlp_eligible(h: torch.Tensor, w_gu: torch.Tensor, w_down: torch.Tensor) -> bool:
@@ -263,7 +267,7 @@ def fused_mlp_eligible(h: torch.Tensor, w_gu: torch.Tensor, w_down: torch.Tensor
 
 def fused_mlp(h, norm_w, w_gate_up, w_down, eps=1e-5, store_fp8: bool = False):
     """``h + swiglu(rmsnorm(h) W_gu^T) W_down^T`` with MXFP8 GEMMs."""
-    return FusedMLPFn.apply(h, norm_w, w_gate_up, w_down, eps, store_fp8)
+    return FusedMLPFn.apply(h, norm_w, w_gate_up, w_down, eps, store_fp8, torch.is_grad_enabled())
 
 
 class SwiGLUFn(Function):
@@ -467,10 +471,11 @@ class LMHeadLossFn(Function):
     from dlogits without recomputing the softmax."""
 
     @staticmethod
-    def forward(ctx, x, norm_w, weight, labels, eps, loss_mask_count, precision):
+    def forward(ctx, x, norm_w, weight, labels, eps, loss_mask_count, precision, grad=True):
         xn, _, _, rstd = K.norm_fwd(x, norm_w, None, eps)
-        keep = L.low_precision(precision, x.shape[0], weight.shape[0], weight.shape[1])
-        logits, saved = L.forward(xn, weight, precision, need_wgrad=keep and weight.requires_grad)
+        grad = grad and any(ctx.needs_input_grad)
+        keep = grad and L.low_precision(precision, x.shape[0], weight.shape[0], weight.shape[1])
+        logits, saved = L.forward(xn, weight, precision, need_wgrad=keep and weight.requires_grad, need_dgrad=grad)
         del xn
         n_valid = loss_mask_count if loss_mask_count is not None else max(int(labels.numel()), 1)
         losses = K.cross_entropy_(logits, labels.view(-1), 1.0 / n_valid, write_grad=True)
@@ -499,7 +504,7 @@ class LMHeadLossFn(Function):
                              need_dw=weight.requires_grad and saved is not None)
         del saved
         dx, dnw, _ = K.norm_bwd(dxn, x, norm_w, None, None, rstd)
-        return dx, _vec_grad(ctx.refs[0], dnw), dw, None, None, None, None
+        return dx, _vec_grad(ctx.refs[0], dnw), dw, None, None, None, None, None
 
 
 def _is_one(t: torch.Tensor) -> bool:
@@ -510,7 +515,7 @@ def _is_one(t: torch.Tensor) -> bool:
 
 
 def lm_head_loss(x, norm_w, weight, labels, *, eps=1e-5, n_valid=None, precision="bf16"):
-    return LMHeadLossFn.apply(x, norm_w, weight, labels, eps, n_valid, precision)
+    return LMHeadLossFn.apply(x, norm_w, weight, labels, eps, n_valid, precision, torch.is_grad_enabled())
 
 
 # --------------------------------------------------------------------------------------

@@ -91,13 +91,18 @@ def weight_operands(weight: torch.Tensor, need_col: bool = True, fmt: str = "e4m
     cache = getattr(weight, "_mx_cache", None)
     col_fmt = col_fmt or fmt
     epoch = (_WEIGHT_EPOCH if weight.requires_grad else -1, fmt, col_fmt)
-    if cache is not None and cache[0] == epoch and (cache[2] is not None or not need_col):
-        return cache[1], cache[2]
+    row = None
+    if cache is not None and cache[0] == epoch:
+        if cache[2] is not None or not need_col:
+            return cache[1], cache[2]
+        row = cache[1]                   # (a forward that expected no backward left it: only the other copy is missing)
     N, Kd = weight.shape
     w = weight.detach()
     if w.dtype != torch.bfloat16 and w.is_cuda:
         w = w.to(torch.bfloat16)
-    row, col = MX.quantize(w, row_tile=MX.b_tile(N), col_tile=MX.b_tile(Kd) if need_col else None, fmt=fmt, col_fmt=col_fmt)
+    new_row, col = MX.quantize(w, row_tile=MX.b_tile(N) if row is None else None, col_tile=MX.b_tile(Kd) if need_col else None, fmt=fmt,
+                               col_fmt=col_fmt)
+    row = new_row if row is None else row
     weight._mx_cache = (epoch, row, col)
     return row, col
 
@@ -158,14 +163,15 @@ def low_precision(precision: str, rows: int, n_out: int, n_in: int) -> bool:
 
 
 def forward(x: torch.Tensor, weight: torch.Tensor, precision: str, *, bias=None, residual=None,
-            need_wgrad: bool = True):
+            need_wgrad: bool = True, need_dgrad: bool = False):
     """``y = x W^T (+ bias) (+ residual)``.  Returns ``(y, saved)`` where ``saved`` is what
-    ``backward`` needs of ``x`` (None when ``need_wgrad`` is False)."""
+    ``backward`` needs of ``x`` (None when ``need_wgrad`` is False).  ``need_dgrad``: the backward will ask for ``dx``, so the
+    micro-scaled copies of the weight for both directions are made in one pass over it."""
     M, Kd = x.shape
     N = weight.shape[0]
     if is_mx(precision) and mx_eligible(M, N, Kd):
         f_act, f_w, _, b_w, b_act, _, had = MX_RECIPES[precision]
-        w_row, _ = weight_operands(weight, need_col=False, fmt=f_w, col_fmt=b_w)
+        w_row, _ = weight_operands(weight, need_col=need_dgrad, fmt=f_w, col_fmt=b_w)
         if had and need_wgrad and M % had == 0:
             # the copy kept for the weight gradient passes the Hadamard transform along the tokens (its partner, the
             # output gradient, gets the same one in backward)

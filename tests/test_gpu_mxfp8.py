@@ -82,6 +82,20 @@ def test_quantize_swiglu_bwd_equals_the_separate_kernels(R, F):
     assert torch.equal(part[0].q[:128], want[0].q[:128]) and torch.equal(part[1].q[:, :128], want[1].q[:, :128])
 
 
+def test_no_column_copies_without_grad_and_weight_copies_in_one_pass():
+    from mlperf_training_b200.ops import functional as F
+    w = torch.nn.Parameter((torch.randn(256, 384, device="cuda") * 0.05).bfloat16())
+    x = torch.randn(128, 384, device="cuda").bfloat16()
+    with torch.no_grad():
+        y0 = F.linear(x, w, precision="mxfp8")
+    assert w._mx_cache[2] is None
+    row = w._mx_cache[1]
+    y1 = F.linear(x.requires_grad_(True), w, precision="mxfp8")
+    assert w._mx_cache[2] is not None and w._mx_cache[1] is row and torch.equal(y0, y1)
+    y1.float().sum().backward()
+    assert w.grad is not None and x.grad is not None
+
+
 @pytest.mark.parametrize("K", [128, 384, 640])
 def test_gemm_does_not_read_scales_past_an_odd_contraction(K):
     """The scales behind a contraction of an odd number of 128-blocks may be anything (here: NaN for every row tile's neighbour)."""

@@ -88,6 +88,29 @@ def test_gather_scatter():
     _close(g_g, g_c, 1e-5, "scatter add")
 
 
+def test_scatter_add_rows_of_an_unaligned_table():
+    torch.manual_seed(0)
+    ids = torch.randint(-1, 7, (50,))
+    dy = torch.randn(50, 16).bfloat16()
+    want = kernels.scatter_add_rows(torch.zeros(7, 16), ids, dy)
+    buf = torch.zeros(7 * 16 + 1, device="cuda")
+    got = kernels.scatter_add_rows(buf[1:].view(7, 16), ids.cuda(), dy.cuda())
+    _close(got, want, 1e-5, "scatter add")
+
+
+def test_gelu_limits():
+    """Large and infinite inputs, and the cancellation-free negative tail, against fp64."""
+    x = torch.cat([torch.linspace(-12, 12, 4091), torch.tensor([-1e30, 1e30, -200.0, 200.0, 0.0])]).bfloat16()
+    y, g = kernels.gelu_fwd(x.cuda()).cpu(), kernels.gelu_bwd(torch.ones_like(x).cuda(), x.cuda()).cpu()
+    xd = x[:4091].double().requires_grad_(True)
+    yd = xd * torch.sigmoid(2 * 0.7978845608028654 * (xd + 0.044715 * xd ** 3))      # (1 + tanh cancels in fp64, too)
+    yd.sum().backward()
+    # one bf16 rounding (2^-9) over fp32 arithmetic whose exponent of e^-2u carries |2u| 2^-23 (u up to 70 here)
+    assert ((y[:4091].double() - yd).abs() <= yd.abs() * 2 ** -8 + 1e-30).all()
+    assert ((g[:4091].double() - xd.grad).abs() <= xd.grad.abs() * 2 ** -8 + 2e-6).all()
+    assert y[4091:].tolist() == [0.0, x[4092].item(), 0.0, 200.0, 0.0]
+
+
 @pytest.mark.parametrize("V", [2048, 32000, 128256])
 def test_cross_entropy(V):
     torch.manual_seed(3)

@@ -254,6 +254,42 @@ gate_cat_reduce_kernel(const float* __restrict__ partial, int nparts, int D, flo
   *out = accumulate ? *out + s : s;
 }
 
+// Rows of [L, width] (pitch ld) that the attention does not write, set to zero: those of no sequence (before offsets[0], from
+// offsets[B] on) and those of a sequence past `cover` (the rows its grid reaches).  CTA b < B: sequence b; the others share the rest.
+// (Clearing a whole output of 105,000 x 512 took 28 us a tensor, this 2.)
+__global__ void __launch_bounds__(256)
+zero_uncovered_rows_kernel(__nv_bfloat16* __restrict__ buf, const int* __restrict__ offsets, int B, long long L, long long ld, int vpr,
+                           long long cover) {
+  long long lo, hi;
+  int part = 0, parts = 1;
+  if ((int)blockIdx.x < B) {
+    lo = offsets[blockIdx.x] + cover;
+    hi = offsets[blockIdx.x + 1];
+  } else {
+    part = (int)blockIdx.x - B;
+    parts = (int)gridDim.x - B;
+    lo = offsets[B];
+    hi = L;
+    const long long head = offsets[0];
+    for (long long i = (long long)part * 256 + threadIdx.x; i < head * vpr; i += parts * 256ll)
+      *reinterpret_cast<uint4*>(buf + i / vpr * ld + i % vpr * 8) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  for (long long i = (long long)part * 256 + threadIdx.x; i < (hi - lo) * vpr; i += parts * 256ll)
+    *reinterpret_cast<uint4*>(buf + (lo + i / vpr) * ld + i % vpr * 8) = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// dst[r, c] (bf16, pitch ld) = src[r, c] (fp32, dense rows of 8 vpr)
+template <typename I>
+__global__ void __launch_bounds__(256)
+cast_rows_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, I total, I vpr, long long ld) {
+  for (I i = blockIdx.x * (I)256 + threadIdx.x; i < total; i += (I)gridDim.x * 256) {
+    const float4 a = *reinterpret_cast<const float4*>(src + (long long)i * 8), b = *reinterpret_cast<const float4*>(src + (long long)i * 8 + 4);
+    const I r = i / vpr;
+    *reinterpret_cast<uint4*>(dst + (long long)r * ld + (long long)(i - r * vpr) * 8) =
+        make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
+  }
+}
+
 int gate_grid(int T, int rows_per_cta) {
   const int grid = (T + rows_per_cta - 1) / rows_per_cta;
   const int cap = b200::sm_count() * GATE_CTAS;
@@ -313,4 +349,30 @@ B200_API int b200_hstu_gate_cat_bwd(const void* dcat, const void* u_raw, long lo
   gate_cat_reduce_kernel<<<2 * D / 32, 256, 0, st>>>(scratch, grid, D, dw, db, accumulate);
   b200::count_launch();
   return b200::check_launch("hstu_gate_cat_reduce");
+}
+
+// Zeroes the rows of buf [L, width] bf16 (pitch ld elements) that belong to no sequence of `offsets` [B + 1], and the rows of a
+// sequence from `cover` on.
+B200_API int b200_hstu_zero_uncovered(void* buf, const int* offsets, int B, long long L, long long ld, int width, long long cover,
+                                      void* stream) {
+  if (width % 8 != 0 || ld % 8 != 0 || ((uintptr_t)buf & 15) != 0)
+    return b200::fail(903, "hstu_zero_uncovered: width %d and pitch %lld must be multiples of 8, the base 16-byte aligned", width, ld);
+  if (L <= 0 || B <= 0) return 0;
+  zero_uncovered_rows_kernel<<<B + 16, 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)buf, offsets, B, L, ld, width / 8, cover);
+  b200::count_launch();
+  return b200::check_launch("hstu_zero_uncovered");
+}
+
+// dst [rows, width] bf16 (pitch ld elements) = src [rows, width] fp32, dense.
+B200_API int b200_cast_rows(const float* src, void* dst, long long rows, int width, long long ld, void* stream) {
+  if (width % 8 != 0 || ld % 8 != 0 || (((uintptr_t)src | (uintptr_t)dst) & 15) != 0)
+    return b200::fail(904, "cast_rows: width %d and pitch %lld must be multiples of 8, pointers 16-byte aligned", width, ld);
+  const long long work = rows * (width / 8);
+  if (work <= 0) return 0;
+  const long long cap = (long long)b200::sm_count() * 16, want = (work + 255) / 256;
+  const int grid = (int)(want < cap ? want : cap);
+  if (work < (1ll << 31)) cast_rows_kernel<uint32_t><<<grid, 256, 0, (cudaStream_t)stream>>>(src, (__nv_bfloat16*)dst, (uint32_t)work, (uint32_t)(width / 8), ld);
+  else cast_rows_kernel<long long><<<grid, 256, 0, (cudaStream_t)stream>>>(src, (__nv_bfloat16*)dst, work, width / 8, ld);
+  b200::count_launch();
+  return b200::check_launch("cast_rows");
 }

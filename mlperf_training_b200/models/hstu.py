@@ -29,7 +29,7 @@ import torch.nn as nn
 import torch.nn.functional as TF
 
 from ..ops import functional as F
-from ..ops.hstu_ops import GateCatFn, gate_cat_eligible, hstu_attention
+from ..ops.hstu_ops import GateCatFn, attn_gate_cat, attn_gate_cat_eligible, gate_cat_eligible, hstu_attention
 
 
 @dataclass
@@ -253,6 +253,13 @@ class STULayer(nn.Module):
         h = cfg.heads
         uvqk = F.norm_linear(x, self.in_norm_w, self.uvqk_weight, norm_b=self.in_norm_b, bias=self.uvqk_beta,
                              eps=1e-6, layer_norm=True, precision=cfg.precision)
+        p = cfg.linear_dropout if self.training else 0.0
+        if self.fuse_glue and cfg.d_v == cfg.d_qk and attn_gate_cat_eligible(uvqk, h):
+            # attention, SiLU(u), the layer norm of the attention output, their product, the concatenation and its dropout (mask
+            # regenerated in backward from a Philox seed) over one buffer, whose gradient is one buffer too
+            cat = attn_gate_cat(uvqk, self.out_norm_w, self.out_norm_b, offsets, max_len or cfg.attn_len(), cfg.d_qk ** -0.5,
+                                num_targets, cfg.contextual, h, 1e-6, p, precision=cfg.attn_precision, owner=self)
+            return F.linear(cat, self.out_weight, None, x, cfg.precision)
         # one split (its backward is a single concatenation; four slices would each build a zero-filled
         # gradient of the whole uvqk matrix)
         u_raw, v_raw, q_raw, k_raw = torch.split(uvqk, list(self.split), dim=1)
@@ -264,8 +271,7 @@ class STULayer(nn.Module):
         if self.fuse_glue and gate_cat_eligible(u_raw, attn):
             # SiLU(u), the layer norm of the attention output, their product and the concatenation in one kernel
             # (and the dropout of the concatenation, its mask regenerated in backward from a Philox seed)
-            cat = GateCatFn.apply(u_raw, attn, self.out_norm_w, self.out_norm_b, 1e-6,
-                                  cfg.linear_dropout if self.training else 0.0)
+            cat = GateCatFn.apply(u_raw, attn, self.out_norm_w, self.out_norm_b, 1e-6, p)
         else:
             u = TF.silu(u_raw)
             y = u * F.layer_norm(attn, self.out_norm_w, self.out_norm_b, 1e-6)

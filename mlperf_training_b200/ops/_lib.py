@@ -91,6 +91,8 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_unique_segments": [P, P, L, P, P, P, P, P, L, P],
         "b200_segment_sum_gather": [P, I, L, P, P, P, P, L, L, L, I, P, I, P, P],
         "b200_hstu_attn_fwd": [P, P, P, P, P, P, I, L, I, I, I, I, L, L, L, L, F, P],
+        "b200_hstu_zero_uncovered": [P, P, I, L, L, I, L, P],
+        "b200_cast_rows": [P, P, L, I, L, P],
         "b200_hstu_gate_cat_fwd": [P, L, P, P, P, P, P, P, I, I, F, F, ctypes.c_ulonglong, P],
         "b200_hstu_gate_cat_bwd": [P, P, L, P, P, P, P, P, P, L, P, P, P, P, I, I, I, F, ctypes.c_ulonglong, P],
         "b200_hstu_attn_bwd": [P, P, P, P, P, P, P, P, P, I, L, I, I, I, I, L, L, L, L, L, L, F, P],

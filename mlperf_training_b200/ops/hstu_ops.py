@@ -84,6 +84,26 @@ def _fp8_sites(owner, device):
     return sites
 
 
+def _zero_uncovered(t: torch.Tensor, offs: torch.Tensor, max_len: int, tile: int) -> None:
+    """Zeroes the rows of ``t [L, W]`` (or ``[L, H, D]``, heads contiguous) that an attention kernel leaves alone: rows of no
+    sequence, and rows past the ``tile``-row tiles that ``max_len`` gives a sequence."""
+    call("b200_hstu_zero_uncovered", ptr(t), ptr(offs), offs.numel() - 1, t.shape[0], t.stride(0), t.numel() // max(t.shape[0], 1),
+         (max_len + tile - 1) // tile * tile, stream_ptr())
+
+
+def _hstu_attn_bwd(q, k, v, dout, offs, nt, max_len, alpha, contextual, dk, dv) -> torch.Tensor:
+    """Writes ``dk`` and ``dv`` (``[L, H, D]``, heads contiguous inside a row) and returns ``dq`` in fp32."""
+    L, H, D = q.shape
+    dout = dout if (dout.stride(2) == 1 and dout.stride(1) == D) else dout.contiguous()
+    dq = torch.zeros((L, H, D), dtype=torch.float32, device=q.device)
+    _zero_uncovered(dk, offs, int(max_len), 128)
+    _zero_uncovered(dv, offs, int(max_len), 128)
+    call("b200_hstu_attn_bwd", ptr(q), ptr(k), ptr(v), ptr(dout), ptr(dq), ptr(dk), ptr(dv), ptr(offs), ptr(nt),
+         offs.numel() - 1, L, H, D, int(max_len), int(contextual), q.stride(0), k.stride(0), v.stride(0),
+         dout.stride(0), dk.stride(0), dv.stride(0), float(alpha), stream_ptr())
+    return dq
+
+
 class HstuAttentionFn(Function):
     @staticmethod
     def forward(ctx, q, k, v, offsets, max_len, alpha, num_targets, contextual, fp8_owner=False):
@@ -100,7 +120,8 @@ class HstuAttentionFn(Function):
                 raise ValueError("hstu_attention: heads must be contiguous inside a row")
         offs = offsets.to(torch.int32).contiguous()
         nt = None if num_targets is None else num_targets.to(torch.int32).contiguous()
-        out = torch.zeros((L, H, D), dtype=q.dtype, device=q.device)
+        out = torch.empty((L, H, D), dtype=q.dtype, device=q.device)
+        _zero_uncovered(out, offs, int(max_len), 256)
         if use_fp8 and q.dtype == torch.bfloat16:
             # e4m3 forward (delayed per-tensor factors); the backward below runs on the bf16 tensors
             from . import fp8 as F8
@@ -130,14 +151,8 @@ class HstuAttentionFn(Function):
                 o = hstu_attention_reference(qf, kf, vf, offs, max_len, alpha, nt, contextual)
             dq, dk, dv = torch.autograd.grad(o, (qf, kf, vf), dout.float())
             return dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), None, None, None, None, None, None
-        L, H, D = q.shape
-        dout = dout if (dout.stride(2) == 1 and dout.stride(1) == D) else dout.contiguous()
-        dq = torch.zeros((L, H, D), dtype=torch.float32, device=q.device)
-        dk = torch.zeros((L, H, D), dtype=k.dtype, device=q.device)
-        dv = torch.zeros((L, H, D), dtype=v.dtype, device=q.device)
-        call("b200_hstu_attn_bwd", ptr(q), ptr(k), ptr(v), ptr(dout), ptr(dq), ptr(dk), ptr(dv), ptr(offs), ptr(nt),
-             offs.numel() - 1, L, H, D, int(max_len), int(contextual), q.stride(0), k.stride(0), v.stride(0),
-             dout.stride(0), dk.stride(0), dv.stride(0), float(alpha), stream_ptr())
+        dk, dv = torch.empty(k.shape, dtype=k.dtype, device=k.device), torch.empty(v.shape, dtype=v.dtype, device=v.device)
+        dq = _hstu_attn_bwd(q, k, v, dout, offs, nt, max_len, alpha, contextual, dk, dv)
         return dq.to(q.dtype), dk, dv, None, None, None, None, None, None
 
 
@@ -164,6 +179,19 @@ def gate_cat_eligible(u_raw: torch.Tensor, attn: torch.Tensor) -> bool:
     D = attn.shape[-1]
     return (use_kernels(attn) and attn.dtype == torch.bfloat16 and D in (256, 512, 768) and u_raw.stride(1) == 1
             and u_raw.stride(0) % 8 == 0 and u_raw.data_ptr() % 16 == 0)
+
+
+def _gate_cat_bwd(dcat, u_raw, attn, w, b, mean, rstd, du, drop):
+    """Writes ``du [T, D]`` (a column block is fine) and returns ``(dattn, dw, db)``; ``drop``: rate and seed of the forward."""
+    T, D = attn.shape
+    dcat = dcat.contiguous()
+    da = torch.empty_like(attn)
+    dw = torch.empty(D, dtype=torch.float32, device=attn.device)
+    db = torch.empty(D, dtype=torch.float32, device=attn.device)
+    scratch = torch.empty(_lib.load().b200_hstu_gate_cat_scratch_elems(T, D), dtype=torch.float32, device=attn.device)
+    call("b200_hstu_gate_cat_bwd", ptr(dcat), ptr(u_raw), u_raw.stride(0), ptr(attn), ptr(w), ptr(b), ptr(mean), ptr(rstd),
+         ptr(du), du.stride(0), ptr(da), ptr(dw), ptr(db), ptr(scratch), T, D, 0, drop[0], drop[1], stream_ptr())
+    return da, dw, db
 
 
 class GateCatFn(Function):
@@ -193,16 +221,69 @@ class GateCatFn(Function):
     def backward(ctx, dcat):
         from .functional import _vec_grad
         u_raw, attn, w, b, mean, rstd = ctx.saved_tensors
-        T, D = attn.shape
-        dcat = dcat.contiguous()
-        du = torch.empty((T, D), dtype=attn.dtype, device=attn.device)
-        da = torch.empty_like(attn)
-        dw = torch.empty(D, dtype=torch.float32, device=attn.device)
-        db = torch.empty(D, dtype=torch.float32, device=attn.device)
-        scratch = torch.empty(_lib.load().b200_hstu_gate_cat_scratch_elems(T, D), dtype=torch.float32, device=attn.device)
-        call("b200_hstu_gate_cat_bwd", ptr(dcat), ptr(u_raw), u_raw.stride(0), ptr(attn), ptr(w), ptr(b), ptr(mean), ptr(rstd),
-             ptr(du), du.stride(0), ptr(da), ptr(dw), ptr(db), ptr(scratch), T, D, 0, ctx.drop[0], ctx.drop[1], stream_ptr())
+        du = torch.empty(attn.shape, dtype=attn.dtype, device=attn.device)
+        da, dw, db = _gate_cat_bwd(dcat, u_raw, attn, w, b, mean, rstd, du, ctx.drop)
         return du, da, _vec_grad(ctx.refs[0], dw), _vec_grad(ctx.refs[1], db), None, None
+
+
+class AttnGateCatFn(Function):
+    """``HstuAttentionFn`` and ``GateCatFn`` over one projection ``uvqk [L, u | v | q | k]``: backward writes the four gradients into the
+    columns of one buffer, where a split's backward would concatenate them."""
+
+    @staticmethod
+    def forward(ctx, uvqk, weight, bias, offsets, max_len, alpha, num_targets, contextual, fp8_owner, heads, eps, p):
+        ctx.attn, ctx.gate = _Saver(), _Saver()
+        u, v, q, k = _uvqk_views(uvqk, heads)
+        attn = HstuAttentionFn.forward(ctx.attn, q, k, v, offsets, max_len, alpha, num_targets, contextual, fp8_owner)
+        cat = GateCatFn.forward(ctx.gate, u, attn.view(uvqk.shape[0], -1), weight, bias, eps, p)
+        offs, nt = ctx.attn.saved[3:]
+        _, a, w, b, mean, rstd = ctx.gate.saved
+        ctx.attn.saved = ctx.gate.saved = None
+        ctx.save_for_backward(uvqk, offs, nt, a, w, b, mean, rstd)
+        ctx.heads = heads
+        return cat
+
+    @staticmethod
+    def backward(ctx, dcat):
+        uvqk, offs, nt, a, w, b, mean, rstd = ctx.saved_tensors
+        u, v, q, k = _uvqk_views(uvqk, ctx.heads)
+        d = torch.empty_like(uvqk)
+        du, dv, dq, dk = _uvqk_views(d, ctx.heads)
+        da, dw, db = _gate_cat_bwd(dcat, u, a, w, b, mean, rstd, du, ctx.gate.drop)
+        max_len, alpha, contextual = ctx.attn.cfg
+        dq32 = _hstu_attn_bwd(q, k, v, da.view(q.shape), offs, nt, max_len, alpha, contextual, dk, dv)
+        call("b200_cast_rows", ptr(dq32), ptr(dq), q.shape[0], dq32.shape[1] * dq32.shape[2], d.stride(0), stream_ptr())
+        refs = ctx.gate.refs
+        from .functional import _vec_grad
+        return (d, _vec_grad(refs[0], dw), _vec_grad(refs[1], db)) + (None,) * 9
+
+
+class _Saver:
+    """Stands in for the context of a Function whose forward runs inside another one's."""
+
+    def save_for_backward(self, *tensors):
+        self.saved = tensors
+
+
+def _uvqk_views(t: torch.Tensor, heads: int):
+    """``u [L, W]`` and ``v, q, k [L, heads, D]`` of a projection of four equal blocks."""
+    W = t.shape[1] // 4
+    u, v, q, k = torch.split(t, W, dim=1)
+    return (u, *(z.unflatten(-1, (heads, W // heads)) for z in (v, q, k)))
+
+
+def attn_gate_cat_eligible(uvqk: torch.Tensor, heads: int) -> bool:
+    """One projection of four equal blocks, in memory as the kernels read and write its columns."""
+    W = uvqk.shape[1] // 4
+    return (use_kernels(uvqk) and uvqk.dtype == torch.bfloat16 and uvqk.is_contiguous() and W * 4 == uvqk.shape[1]
+            and W in (256, 512, 768) and W % heads == 0 and W // heads in (64, 128) and uvqk.data_ptr() % 16 == 0)
+
+
+def attn_gate_cat(uvqk, weight, bias, offsets, max_len: int, alpha: float, num_targets, contextual: int, heads: int,
+                  eps: float = 1e-6, p: float = 0.0, precision: str = "bf16", owner=None):
+    """``gate_cat(u, hstu_attention(q, k, v))`` of the blocks of ``uvqk`` (see ``attn_gate_cat_eligible``)."""
+    fp8_owner = owner if precision == "fp8" else False
+    return AttnGateCatFn.apply(uvqk, weight, bias, offsets, max_len, alpha, num_targets, contextual, fp8_owner, heads, eps, p)
 
 
 def gate_cat(u_raw, attn, weight, bias, eps: float = 1e-6, p: float = 0.0):

@@ -210,6 +210,55 @@ def test_stu_layer_fused_glue_matches_eager_glue():
         assert err <= 2e-2 * (a.abs().max().item() + 1e-6), f"{what}: {err}"
 
 
+def test_attention_leaves_zeros_outside_the_sequences():
+    """Rows before the first sequence, behind the last, and past the tiles of ``max_len`` are zero in the output and in dk, dv, dq."""
+    torch.manual_seed(0)
+    H, D, L = 2, 64, 900
+    offs = torch.tensor([40, 40, 300, 310, 800], dtype=torch.int32, device="cuda")
+    q, k, v = (torch.randn(L, H, D, device="cuda").bfloat16().requires_grad_(True) for _ in range(3))
+    torch.full((L, 4 * H * D), float("nan"), device="cuda", dtype=torch.bfloat16)
+    out = hstu_attention(q, k, v, offs, 500, D ** -0.5)
+    out.backward(torch.randn_like(out))
+    ref = hstu_attention_reference(q.detach().cpu(), k.detach().cpu(), v.detach().cpu(), offs.cpu(), 500, D ** -0.5)
+    for t in (out.detach(), q.grad, k.grad, v.grad):
+        assert t[:40].abs().max() == 0 and t[800:].abs().max() == 0 and not t.isnan().any()
+    assert (out.detach().float().cpu() - ref).abs().max() < 3e-2 * ref.abs().max()
+    assert all(t[40:800].abs().sum(-1).min() > 0 for t in (k.grad, v.grad))
+    short = hstu_attention(q.detach(), k.detach(), v.detach(), offs, 130, D ** -0.5)      # its grid covers 256 rows a sequence
+    assert short[310 + 256:800].abs().max() == 0 and short[311:566].abs().sum(-1).min() > 0
+
+
+@pytest.mark.parametrize("precision", ["bf16", "fp8"])
+@pytest.mark.parametrize("p", [0.0, 0.25])
+def test_attention_and_gate_over_one_buffer(precision, p):
+    """The fused form gives the split form's output and gradient bit for bit (same kernels, same seed of the mask)."""
+    from mlperf_training_b200.ops.hstu_ops import attn_gate_cat, gate_cat
+    torch.manual_seed(1)
+    H, D, L = 4, 128, 640
+    W = H * D
+    offs = torch.tensor([0, 200, 330, 600], dtype=torch.int32, device="cuda")
+    nt = torch.tensor([1, 2, 1], dtype=torch.int32, device="cuda")
+    x0, dy = torch.randn(L, 4 * W, device="cuda").bfloat16(), torch.randn(L, 3 * W, device="cuda").bfloat16()
+    w, b = (1 + 0.1 * torch.randn(W, device="cuda")).bfloat16(), (0.1 * torch.randn(W, device="cuda")).bfloat16()
+    got = []
+    for fused in (False, True):
+        x, ww, bb = (t.clone().requires_grad_(True) for t in (x0, w, b))
+        torch.manual_seed(7)
+        if fused:
+            y = attn_gate_cat(x, ww, bb, offs, 512, D ** -0.5, nt, 0, H, p=p, precision=precision)
+        else:
+            u, v, q, k = torch.split(x, W, dim=1)
+            a = hstu_attention(*(t.unflatten(-1, (H, D)) for t in (q, k, v)), offs, 512, D ** -0.5, nt, 0, precision=precision)
+            y = gate_cat(u, a.reshape(L, W), ww, bb, p=p)
+        y.backward(dy)
+        got.append((y.detach(), x.grad, ww.grad, bb.grad))
+    assert all(torch.equal(got[0][i], got[1][i]) for i in (0, 2, 3))
+    d0, d1 = got[0][1].float(), got[1][1].float()                    # (dq is summed by fp32 atomics: two runs may round apart)
+    assert torch.equal(d0[:, :2 * W], d1[:, :2 * W]) and torch.equal(d0[:, 3 * W:], d1[:, 3 * W:])
+    assert ((d0 - d1).abs() <= d0.abs() * 2 ** -7 + 1e-6 * d0.abs().max()).all()
+    _lib.check_status("attn_gate_cat")
+
+
 def test_gate_cat_dropout_mask_is_regenerated_in_backward():
     from mlperf_training_b200.ops.hstu_ops import GateCatFn
     torch.manual_seed(11)

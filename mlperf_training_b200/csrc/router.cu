@@ -98,14 +98,35 @@ __global__ void router_rank_kernel(const int* __restrict__ idx, int n, const int
   }
 }
 
-// x_perm[dest[p], :] = x[p / K, :] (rows not written stay zero: the caller clears the buffer),
-// optional per-row probability copy prob_perm[dest[p]] = w[p]
+// The rows of an expert-grouped buffer that no pair maps to, [seg[e] + counts[e], seg[e + 1]) of every expert: the first CTAs of the
+// kernels that fill such a buffer clear them, GAP_CTAS per expert.  (Clearing all of it first wrote every row twice: 40,960 rows
+// of 2880, 61 us a buffer.  Rows behind the last segment are nobody's: the grouped kernels and the quantisers skip them; cleared
+// along, by four CTAs, they took longer than the whole buffer by all.)
+constexpr int GAP_CTAS = 4;
+struct Gaps {
+  const int* seg;                  // null: the caller has cleared the buffer
+  const int* counts;
+  int E;
+};
+B200_DEVICE int gap_ctas(const Gaps& g) { return g.seg != nullptr ? g.E * GAP_CTAS : 0; }
+B200_DEVICE void clear_gap(const Gaps& g, __nv_bfloat16* out, int D) {
+  const int e = (int)blockIdx.x / GAP_CTAS, part = (int)blockIdx.x % GAP_CTAS;
+  const long long lo = (long long)g.seg[e] + g.counts[e], hi = g.seg[e + 1];
+  const long long n = (hi - lo) * (D / 8);         // the rows are contiguous
+  uint4* p = reinterpret_cast<uint4*>(out + lo * D);
+  for (long long i = part * (long long)blockDim.x + threadIdx.x; i < n; i += GAP_CTAS * (long long)blockDim.x) p[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// x_perm[dest[p], :] = x[p / K, :], optional per-row probability copy prob_perm[dest[p]] = w[p]
 __global__ void permute_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ dest, int n, int K,
                                     int D, __nv_bfloat16* __restrict__ out, const float* __restrict__ w,
-                                    float* __restrict__ w_out) {
+                                    float* __restrict__ w_out, const Gaps gaps) {
+  const int first = gap_ctas(gaps);
+  if ((int)blockIdx.x < first) { clear_gap(gaps, out, D); return; }
   const int vpr = D / 8;
   const long long total = (long long)n * vpr;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+  const long long step = (long long)((int)gridDim.x - first) * blockDim.x;
+  for (long long i = ((int)blockIdx.x - first) * (long long)blockDim.x + threadIdx.x; i < total; i += step) {
     const int p = (int)(i / vpr), v = (int)(i % vpr);
     const int d = dest[p];
     *reinterpret_cast<uint4*>(out + (long long)d * D + v * 8) =
@@ -114,9 +135,9 @@ __global__ void permute_rows_kernel(const __nv_bfloat16* __restrict__ x, const i
   }
 }
 
-// y[t, :] = sum_j scale_j * y_perm[dest[t*K + j], :]   (scale = 1 when w is null)
+// y[t, :] = sum_j scale_j * y_perm[dest[t*K + j], :] (+ res[t, :])   (scale = 1 when w is null)
 __global__ void unpermute_sum_kernel(const __nv_bfloat16* __restrict__ yp, const int* __restrict__ dest,
-                                     const float* __restrict__ w, int T, int K, int D,
+                                     const float* __restrict__ w, int T, int K, int D, const __nv_bfloat16* __restrict__ res,
                                      __nv_bfloat16* __restrict__ y) {
   const int vpr = D / 8;
   const long long total = (long long)T * vpr;
@@ -131,6 +152,11 @@ __global__ void unpermute_sum_kernel(const __nv_bfloat16* __restrict__ yp, const
       acc[0] += s * a.x; acc[1] += s * a.y; acc[2] += s * b.x; acc[3] += s * b.y;
       acc[4] += s * c.x; acc[5] += s * c.y; acc[6] += s * e.x; acc[7] += s * e.y;
     }
+    if (res != nullptr) {
+      const uint4 u = *reinterpret_cast<const uint4*>(res + (long long)t * D + v * 8);
+      const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), e = unpack_bf16x2(u.w);
+      acc[0] += a.x; acc[1] += a.y; acc[2] += b.x; acc[3] += b.y; acc[4] += c.x; acc[5] += c.y; acc[6] += e.x; acc[7] += e.y;
+    }
     *reinterpret_cast<uint4*>(y + (long long)t * D + v * 8) =
         make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]),
                    pack_bf16x2(acc[6], acc[7]));
@@ -138,12 +164,14 @@ __global__ void unpermute_sum_kernel(const __nv_bfloat16* __restrict__ yp, const
 }
 
 // Backward of unpermute_sum, one warp per (token, slot) pair p:
-//   gyp[dest[p], :] = w[p] * gy[p / K, :]        (rows no pair maps to keep their previous content)
+//   gyp[dest[p], :] = w[p] * gy[p / K, :]        (rows no pair maps to keep their previous content, or are cleared: gaps)
 //   gw[p]           = <gy[p / K, :], yp[dest[p], :]>
 __global__ void unpermute_bwd_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* __restrict__ yp,
                                      const int* __restrict__ dest, const float* __restrict__ w, long long pairs, int K,
-                                     int D, __nv_bfloat16* __restrict__ gyp, float* __restrict__ gw) {
-  const long long p = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+                                     int D, __nv_bfloat16* __restrict__ gyp, float* __restrict__ gw, const Gaps gaps) {
+  const int first = gap_ctas(gaps);
+  if ((int)blockIdx.x < first) { clear_gap(gaps, gyp, D); return; }
+  const long long p = (((long long)blockIdx.x - first) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (p >= pairs) return;
   const long long t = p / K;
@@ -179,12 +207,14 @@ __global__ void zero_dead_tiles_kernel(__nv_bfloat16* __restrict__ buf, const in
 }  // namespace
 
 B200_API int b200_unpermute_bwd(const void* gy, const void* yp, const int* dest, const float* w, long long pairs, int K,
-                                int D, void* gyp, float* gw, void* stream) {
+                                int D, void* gyp, float* gw, const int* seg, const int* counts, int E, void* stream) {
   if (D % 8 != 0) return b200::fail(904, "unpermute_bwd: D=%d must be a multiple of 8", D);
   if (pairs <= 0) return 0;
   const long long threads = pairs * 32;
-  unpermute_bwd_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)gy, (const __nv_bfloat16*)yp, dest, w, pairs, K, D, (__nv_bfloat16*)gyp, gw);
+  const Gaps gaps = {seg, counts, E};
+  const unsigned extra = seg != nullptr ? (unsigned)E * GAP_CTAS : 0u;
+  unpermute_bwd_kernel<<<extra + (unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)gy, (const __nv_bfloat16*)yp, dest, w, pairs, K, D, (__nv_bfloat16*)gyp, gw, gaps);
   b200::count_launch();
   return b200::check_launch("unpermute_bwd");
 }
@@ -215,24 +245,28 @@ B200_API int b200_router_plan(const int* counts, const int* idx, int n, int E, i
   return b200::check_launch("router_plan");
 }
 
+// seg [E + 1] / counts [E] (null: `out` is cleared by the caller): the plan whose pairs `dest` holds; the rows between its segments
+// are cleared here.  b200_unpermute_bwd: the same for gyp.
 B200_API int b200_permute_rows(const void* x, const int* dest, int n, int K, int D, void* out, const float* w,
-                               float* w_out, void* stream) {
+                               float* w_out, const int* seg, const int* counts, int E, void* stream) {
   if (D % 8 != 0) return b200::fail(902, "permute_rows: D=%d must be a multiple of 8", D);
   if (n == 0) return 0;
   long long work = (long long)n * (D / 8);
   int grid = (int)((work + 255) / 256 < (long long)b200::sm_count() * 16 ? (work + 255) / 256 : (long long)b200::sm_count() * 16);
-  permute_rows_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, dest, n, K, D, (__nv_bfloat16*)out, w, w_out);
+  const Gaps gaps = {seg, counts, E};
+  permute_rows_kernel<<<grid + (seg != nullptr ? E * GAP_CTAS : 0), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, dest, n, K, D,
+                                                                                                    (__nv_bfloat16*)out, w, w_out, gaps);
   b200::count_launch();
   return b200::check_launch("permute_rows");
 }
 
-B200_API int b200_unpermute_sum(const void* yp, const int* dest, const float* w, int T, int K, int D, void* y,
+B200_API int b200_unpermute_sum(const void* yp, const int* dest, const float* w, int T, int K, int D, const void* res, void* y,
                                 void* stream) {
   if (D % 8 != 0) return b200::fail(903, "unpermute_sum: D=%d must be a multiple of 8", D);
   if (T == 0) return 0;
   long long work = (long long)T * (D / 8);
   int grid = (int)((work + 255) / 256 < (long long)b200::sm_count() * 16 ? (work + 255) / 256 : (long long)b200::sm_count() * 16);
-  unpermute_sum_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)yp, dest, w, T, K, D, (__nv_bfloat16*)y);
+  unpermute_sum_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)yp, dest, w, T, K, D, (const __nv_bfloat16*)res, (__nv_bfloat16*)y);
   b200::count_launch();
   return b200::check_launch("unpermute_sum");
 }

@@ -47,7 +47,7 @@ class MoEMLP(nn.Module):
         idx, w, counts = M.RouterFn.apply(logits, cfg.top_k)
         prec = M.expert_precision(getattr(cfg, "precision", "bf16"), self.w1, self.w2)
         if self.dispatcher is None:
-            y = M.moe_experts(hn, idx, w, counts, self.w1, self.w2, prec)
+            return M.moe_experts(hn, idx, w, counts, self.w1, self.w2, prec, residual=h)
         elif self.ep_comm == "fused" and hn.is_cuda and hn.dtype == torch.bfloat16:
             y = self._fused_dispatcher(hn.shape[0] * cfg.top_k, hn.device, M.pad_rows(prec))(hn, idx, w, counts, self.w1,
                                                                                              self.w2, prec)

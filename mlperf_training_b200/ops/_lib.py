@@ -62,8 +62,8 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_gemm_mxfp8": [P, P, P, P, P, I, I, I, L, L, L, I, I, P, P, L, F, P, L, P],
         "b200_router_topk": [P, I, I, I, P, P, P, P],
         "b200_router_plan": [P, P, I, I, I, P, P, I, P, P],
-        "b200_permute_rows": [P, P, I, I, I, P, P, P, P],
-        "b200_unpermute_sum": [P, P, P, I, I, I, P, P],
+        "b200_permute_rows": [P, P, I, I, I, P, P, P, P, P, I, P],
+        "b200_unpermute_sum": [P, P, P, I, I, I, P, P, P],
         "b200_gemm_grouped_rows": [P, P, P, P, I, I, I, I, L, L, I, I, F, P],
         "b200_gemm_grouped_wgrad": [P, P, P, P, I, I, I, I, L, L, I, I, F, P],
         "b200_gemm_grouped_mx_rows": [P, P, P, P, P, P, I, I, I, I, L, L, L, I, F, P],
@@ -100,7 +100,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_gather_rows_from_peers": [P, P, P, L, I, P, I, L, P],
         "b200_zero_pad_rows": [P, P, P, I, I, L, P],
         "b200_ep_route": [P, P, I, I, I, I, L, L, P, P, P, P, P, P],
-        "b200_unpermute_bwd": [P, P, P, P, L, I, I, P, P, P],
+        "b200_unpermute_bwd": [P, P, P, P, L, I, I, P, P, P, P, I, P],
         "b200_zero_dead_tiles": [P, P, I, I, P],
         "b200_quant_swiglu_mxfp8": [P, L, I, I, P, P, I, P, P, I, P, P],
         "b200_quant_swiglu_bwd_mxfp8": [P, L, P, L, I, I, P, P, I, P, P, I, P, P],

@@ -108,28 +108,45 @@ def plan(idx: torch.Tensor, counts: torch.Tensor, n_experts: int, pad: int = PAD
     return seg, te, dest, rows
 
 
-def permute_rows(x: torch.Tensor, dest: torch.Tensor, k: int, rows: int) -> torch.Tensor:
-    """``out[dest[p]] = x[p // k]``; rows that no pair maps to are zero."""
+def permute_rows(x: torch.Tensor, dest: torch.Tensor, k: int, rows: int, gaps=None) -> torch.Tensor:
+    """``out[dest[p]] = x[p // k]``; rows that no pair maps to are zero.  ``gaps``: None, or ``(seg, counts)`` of a plan that
+    ``dest`` covers whole: only the rows between a segment's last pair and the next segment are cleared then, and those behind
+    the last segment may hold anything."""
     T, D = x.shape
-    out = torch.zeros((rows, D), dtype=x.dtype, device=x.device)
     if not use_kernels(x) or x.dtype != torch.bfloat16:
+        out = torch.zeros((rows, D), dtype=x.dtype, device=x.device)
         out[dest.long()] = x.repeat_interleave(k, dim=0)
         return out
-    call("b200_permute_rows", ptr(x.contiguous()), ptr(dest), dest.numel(), k, D, ptr(out), None, None, stream_ptr())
+    out = _row_buffer(rows, D, x, gaps)
+    call("b200_permute_rows", ptr(x.contiguous()), ptr(dest), dest.numel(), k, D, ptr(out), None, None, *_gap_args(gaps), stream_ptr())
     return out
 
 
-def unpermute_sum(yp: torch.Tensor, dest: torch.Tensor, w: torch.Tensor | None, T: int, k: int) -> torch.Tensor:
-    """``y[t] = sum_j w[t,j] * yp[dest[t*k + j]]`` (``w`` None = plain sum)."""
+def _row_buffer(rows: int, D: int, like: torch.Tensor, gaps) -> torch.Tensor:
+    return (torch.zeros if gaps is None else torch.empty)((rows, D), dtype=like.dtype, device=like.device)
+
+
+def _gap_args(gaps):
+    if gaps is None:
+        return None, None, 0
+    seg, counts = gaps
+    return ptr(seg), ptr(counts), counts.numel()
+
+
+def unpermute_sum(yp: torch.Tensor, dest: torch.Tensor, w: torch.Tensor | None, T: int, k: int,
+                  residual: torch.Tensor | None = None) -> torch.Tensor:
+    """``y[t] = sum_j w[t,j] * yp[dest[t*k + j]] (+ residual[t])`` (``w`` None = plain sum)."""
     D = yp.shape[1]
-    if not use_kernels(yp) or yp.dtype != torch.bfloat16:
+    if not use_kernels(yp) or yp.dtype != torch.bfloat16 or (residual is not None and residual.dtype != torch.bfloat16):
         g = yp[dest.long()].view(T, k, D).float()
         if w is not None:
             g = g * w.view(T, k, 1).float()
-        return g.sum(1).to(yp.dtype)
+        y = g.sum(1)
+        return (y if residual is None else y + residual.float()).to(yp.dtype)
     y = torch.empty((T, D), dtype=yp.dtype, device=yp.device)
     wf = None if w is None else w.float().contiguous()
-    call("b200_unpermute_sum", ptr(yp.contiguous()), ptr(dest), ptr(wf), T, k, D, ptr(y), stream_ptr())
+    call("b200_unpermute_sum", ptr(yp.contiguous()), ptr(dest), ptr(wf), T, k, D,
+         None if residual is None else ptr(residual.contiguous()), ptr(y), stream_ptr())
     return y
 
 
@@ -215,39 +232,42 @@ class RouterFn(Function):
 
 class PermuteFn(Function):
     @staticmethod
-    def forward(ctx, x, dest, k, rows):
+    def forward(ctx, x, dest, k, rows, seg=None, counts=None):
         ctx.save_for_backward(dest)
         ctx.cfg = (x.shape[0], k)
-        return permute_rows(x, dest, k, rows)
+        return permute_rows(x, dest, k, rows, None if seg is None else (seg, counts))
 
     @staticmethod
     def backward(ctx, g):
         (dest,) = ctx.saved_tensors
         T, k = ctx.cfg
-        return unpermute_sum(g.contiguous(), dest, None, T, k), None, None, None
+        return unpermute_sum(g.contiguous(), dest, None, T, k), None, None, None, None, None
 
 
 class UnpermuteFn(Function):
     @staticmethod
-    def forward(ctx, yp, dest, w, T, k):
-        ctx.save_for_backward(yp, dest, w)
+    def forward(ctx, yp, dest, w, T, k, residual=None, seg=None, counts=None):
+        ctx.save_for_backward(yp, dest, w, seg, counts)
         ctx.cfg = (T, k)
-        return unpermute_sum(yp, dest, w, T, k)
+        ctx.has_res = residual is not None
+        return unpermute_sum(yp, dest, w, T, k, residual)
 
     @staticmethod
     def backward(ctx, gy):
-        yp, dest, w = ctx.saved_tensors
+        yp, dest, w, seg, counts = ctx.saved_tensors
+        dres = gy if ctx.has_res else None
         T, k = ctx.cfg
         D = yp.shape[1]
         gy = gy.contiguous()
         if use_kernels(gy) and gy.dtype == torch.bfloat16 and yp.dtype == torch.bfloat16:
             # one pass: scaled scatter of the gradient rows and the routing-weight gradient (a dot product per pair)
-            gyp = torch.zeros_like(yp)
+            gaps = None if seg is None else (seg, counts)
+            gyp = _row_buffer(yp.shape[0], D, yp, gaps)
             gw32 = None if w is None else torch.empty(T * k, dtype=torch.float32, device=gy.device)
             wf = None if w is None else w.reshape(-1).float().contiguous()
             call("b200_unpermute_bwd", ptr(gy), ptr(yp.contiguous()), ptr(dest), ptr(wf), T * k, k, D, ptr(gyp), ptr(gw32),
-                 stream_ptr())
-            return gyp, None, (None if w is None else gw32.view(T, k).to(w.dtype)), None, None
+                 *_gap_args(gaps), stream_ptr())
+            return gyp, None, (None if w is None else gw32.view(T, k).to(w.dtype)), None, None, dres, None, None
         gyp = permute_rows(gy, dest, k, yp.shape[0])
         gw = None
         if w is not None:
@@ -256,7 +276,7 @@ class UnpermuteFn(Function):
             scale[dest.long()] = w.reshape(-1).float()
             gw = (yp[dest.long()].view(T, k, D).float() * gy.view(T, 1, D).float()).sum(-1).to(w.dtype)
             gyp = (gyp.float() * scale[:, None]).to(gyp.dtype)
-        return gyp, None, gw, None, None
+        return gyp, None, gw, None, None, dres, None, None
 
 
 class GroupedMLPFn(Function):
@@ -478,14 +498,15 @@ def expert_precision(precision: str, w1, w2) -> str:
     return "bf16"
 
 
-def moe_experts(x, idx, w, counts, w1, w2, precision: str = "bf16"):
+def moe_experts(x, idx, w, counts, w1, w2, precision: str = "bf16", residual=None):
     """Local (all experts on this rank) MoE expert stage: dispatch by permutation, grouped MLP,
-    weighted combine.  ``x`` ``[T, D]``; returns ``[T, D]``."""
+    weighted combine (+ ``residual``).  ``x`` ``[T, D]``; returns ``[T, D]``."""
     T, k = idx.shape
     E = w1.shape[0]
     precision = expert_precision(precision, w1, w2)
     pad = PAD_MX if precision == "bf16" and pair_rows_ok(x, w1, w2) else pad_rows(precision)
     seg, tile_expert, dest, rows = plan(idx, counts, E, pad=pad)
-    xp = PermuteFn.apply(x, dest, k, rows)
+    gaps = (seg, counts) if pad == PAD_MX else ()       # (the kernels on 128-row tiles want the rows behind the last segment zero)
+    xp = PermuteFn.apply(x, dest, k, rows, *gaps)
     yp = grouped_mlp(xp, w1, w2, seg, tile_expert, precision)
-    return UnpermuteFn.apply(yp, dest, w, T, k)
+    return UnpermuteFn.apply(yp, dest, w, T, k, residual, *gaps)

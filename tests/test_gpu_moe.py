@@ -33,6 +33,32 @@ def test_router_and_plan_match_cpu():
     _lib.check_status("router")
 
 
+@pytest.mark.parametrize("T,E,k,pad", [(1, 4, 1, 128), (300, 32, 4, 256), (128, 8, 1, 128)])
+def test_permutation_clears_the_gaps_only_and_adds_the_residual(T, E, k, pad):
+    """Buffers whose gap rows the kernels clear themselves (experts without rows among them) equal cleared ones."""
+    torch.manual_seed(T)
+    logits = torch.randn(T, E)
+    logits[:, 0] = -50.0
+    idx, w, cnt = M.router_topk(logits.cuda(), k)
+    seg, te, dest, rows = M.plan(idx, cnt, E, pad=pad)
+    x, res = torch.randn(T, 64, device="cuda").bfloat16(), torch.randn(T, 64, device="cuda").bfloat16()
+    live = int(seg[-1])
+    stale = torch.full((rows, 64), float("nan"), device="cuda", dtype=torch.bfloat16)
+    del stale                                            # (what the allocator hands out next)
+    xp = M.permute_rows(x, dest, k, rows, (seg, cnt))
+    assert torch.equal(xp[:live], M.permute_rows(x, dest, k, rows)[:live])
+    grads = []
+    for gaps in ((), (seg, cnt)):
+        yp, r, ww = xp.clone().requires_grad_(True), res.clone().requires_grad_(True), w.clone().requires_grad_(True)
+        y = M.UnpermuteFn.apply(yp, dest, ww, T, k, r, *gaps)
+        y.backward(x)
+        grads.append((y.detach(), yp.grad[:live], r.grad, ww.grad))
+    assert all(torch.equal(a, b) for a, b in zip(*grads)) and torch.equal(grads[0][2], x)
+    ref = M.unpermute_sum(xp.cpu(), dest.cpu(), w.cpu(), T, k, res.cpu()).float()
+    assert ((grads[0][0].float().cpu() - ref).abs() <= ref.abs() * 2 ** -7 + 1e-5).all()      # a flip of the one rounding
+    _lib.check_status("gaps")
+
+
 @pytest.mark.parametrize("T,E,k,D,Fh", [(512, 8, 2, 256, 512), (2048, 32, 4, 384, 320)])
 def test_grouped_gemms(T, E, k, D, Fh):
     torch.manual_seed(1)

@@ -64,6 +64,31 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ buf, const float* __rest
 // ---------------------------------------------------------------------------------------
 // SwiGLU: a[t, f] = silu(gu[t, f]) * gu[t, F + f]  (gate columns first, up columns second)
 // ---------------------------------------------------------------------------------------
+// One vector of SwiGLU, forward and backward (g, u: gate and up; d: gradient of the product).
+B200_DEVICE void swiglu_vec(const __nv_bfloat16* g_in, const __nv_bfloat16* u_in, __nv_bfloat16* out) {
+  float g[8], u[8], o[8];
+  ld8(g_in, g);
+  ld8(u_in, u);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) o[j] = g[j] * sigmoid(g[j]) * u[j];
+  st8(out, o);
+}
+B200_DEVICE void swiglu_grad_vec(const __nv_bfloat16* g_in, const __nv_bfloat16* u_in, const __nv_bfloat16* d_in, __nv_bfloat16* dg_out,
+                                 __nv_bfloat16* du_out) {
+  float g[8], u[8], d[8], dg[8], du[8];
+  ld8(g_in, g);
+  ld8(u_in, u);
+  ld8(d_in, d);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float sg = sigmoid(g[j]);
+    const float silu = g[j] * sg;
+    du[j] = d[j] * silu;
+    dg[j] = d[j] * u[j] * sg * (1.f + g[j] * (1.f - sg));
+  }
+  st8(dg_out, dg);
+  st8(du_out, du);
+}
 template <typename I>
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ a, I T,
                   int F) {
@@ -71,12 +96,7 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __
   for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
     const long long t = i / vpr;
     const int v = (int)(i - (I)t * vpr);
-    float g[8], u[8], o[8];
-    ld8(gu + t * 2 * F + v * 8, g);
-    ld8(gu + t * 2 * F + F + v * 8, u);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = g[j] * sigmoid(g[j]) * u[j];
-    st8(a + t * F + v * 8, o);
+    swiglu_vec(gu + t * 2 * F + v * 8, gu + t * 2 * F + F + v * 8, a + t * F + v * 8);
   }
 }
 template <typename I>
@@ -86,19 +106,26 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
   for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
     const long long t = i / vpr;
     const int v = (int)(i - (I)t * vpr);
-    float g[8], u[8], d[8], dg[8], du[8];
-    ld8(gu + t * 2 * F + v * 8, g);
-    ld8(gu + t * 2 * F + F + v * 8, u);
-    ld8(da + t * F + v * 8, d);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float sg = sigmoid(g[j]);
-      const float silu = g[j] * sg;
-      du[j] = d[j] * silu;
-      dg[j] = d[j] * u[j] * sg * (1.f + g[j] * (1.f - sg));
-    }
-    st8(dgu + t * 2 * F + v * 8, dg);
-    st8(dgu + t * 2 * F + F + v * 8, du);
+    swiglu_grad_vec(gu + t * 2 * F + v * 8, gu + t * 2 * F + F + v * 8, da + t * F + v * 8, dgu + t * 2 * F + v * 8,
+                    dgu + t * 2 * F + F + v * 8);
+  }
+}
+
+// The same over the 256-row tiles of an expert-grouped buffer: a tile's rows up to the multiple of 64 behind its expert's last one,
+// nothing in tiles of no expert.  (8000 pairs on 32 experts: 9000 of 16,192 rows, 90 / 86 / 78 -> 33 / 36 / 39 us for forward,
+// recomputed forward and backward of 2 x 2880 columns, index divisions included.)  da == nullptr: forward.
+__global__ void __launch_bounds__(256)
+swiglu_tiles_kernel(const __nv_bfloat16* __restrict__ da, const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, int F,
+                    const int* __restrict__ tile_expert, const int* __restrict__ seg, const int* __restrict__ counts) {
+  const int tile = blockIdx.y, e = tile_expert[tile];
+  if (e < 0) return;
+  const int n = min(256, (seg[e] + counts[e] - tile * 256 + 63) / 64 * 64), vpr = F / 8;
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n * vpr; i += gridDim.x * 256) {
+    const int r = i / vpr, v = (i - r * vpr) * 8;
+    const long long t = (long long)tile * 256 + r;
+    const __nv_bfloat16* g = gu + t * 2 * F + v;
+    if (da == nullptr) swiglu_vec(g, g + F, out + t * F + v);
+    else swiglu_grad_vec(g, g + F, da + t * F + v, out + t * 2 * F + v, out + t * 2 * F + F + v);
   }
 }
 
@@ -285,6 +312,17 @@ B200_API int b200_gelu_bwd(const void* dy, const void* x, void* dx, long long n,
   if (n == 0) return 0;
   run_gelu_bwd(dy, n, x, n, dx, n, n / 8, n / 8, (cudaStream_t)stream);
   return b200::check_launch("gelu_bwd");
+}
+// swiglu_tiles_kernel over n_tiles tiles of 256 rows: out [rows, F] from gu [rows, 2F], or with da [rows, F] out [rows, 2F].
+B200_API int b200_swiglu_tiles(const void* da, const void* gu, void* out, int F, const int* tile_expert, const int* seg, const int* counts,
+                               int n_tiles, void* stream) {
+  if (F % 8 != 0) return b200::fail(401, "swiglu: F=%d must be a multiple of 8", F);
+  if (n_tiles <= 0 || F <= 0) return 0;
+  if (n_tiles > 65535) return b200::fail(407, "swiglu_tiles: %d tiles are too many", n_tiles);
+  swiglu_tiles_kernel<<<dim3(32, n_tiles), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)da, (const __nv_bfloat16*)gu,
+                                                                           (__nv_bfloat16*)out, F, tile_expert, seg, counts);
+  b200::count_launch();
+  return b200::check_launch("swiglu_tiles");
 }
 B200_API int b200_gather_rows(const void* table, const long long* ids, void* out, long long T, int D, long long rows,
                               void* stream) {

@@ -360,6 +360,7 @@ struct GroupArgs {
   int E;
   const int* tile_expert;         // mode 1: [ceil(M / 256)]
   const int* seg;                 // mode 2: [E + 1], multiples of 256
+  const int* counts;              // mode 2, bf16: [E] rows of the segments that count (the rows up to the next stage are zero), null: all
 };
 
 struct TileInfo {
@@ -487,6 +488,7 @@ B200_DEVICE TileInfo tile_info(int t, int num_m, int num_n, int num_kb, int kb_e
     const int lo = p.grp.seg[ti.e], hi = p.grp.seg[ti.e + 1];
     ti.kb0 = lo / kb_elems;
     ti.nkb = (hi - lo) / kb_elems;
+    if (p.grp.counts != nullptr) ti.nkb = min(ti.nkb, (p.grp.counts[ti.e] + kb_elems - 1) / kb_elems);
     ti.valid = ti.nkb > 0;
   } else {
     tile_coords(t, num_m, num_n, p.group_m, ti.mb, ti.nb);

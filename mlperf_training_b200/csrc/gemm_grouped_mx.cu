@@ -127,8 +127,9 @@ B200_API int b200_gemm_grouped_pair_rows(const void* a, const void* b, void* d, 
 }
 
 // bf16 weight gradient: d[e] (+)= a[seg[e]:seg[e+1], :]^T b[seg[e]:seg[e+1], :]; a [rows, M], b [rows, N], d [E, M, N]
-// contiguous, bf16 or fp32; segments are multiples of 256 rows, M of 32.  accumulate as above.
-B200_API int b200_gemm_grouped_pair_wgrad(const void* a, const void* b, void* d, const int* seg, int rows, int M, int N, int E,
+// contiguous, bf16 or fp32; segments are multiples of 256 rows, M of 32.  accumulate as above.  counts [E] or null: the contraction of
+// expert e ends with its first counts[e] rows rounded up to 64 (the rows behind them are zero in a and b up to there).
+B200_API int b200_gemm_grouped_pair_wgrad(const void* a, const void* b, void* d, const int* seg, const int* counts, int rows, int M, int N, int E,
                                           long long lda, long long ldb, int out_f32, int accumulate, float alpha, void* stream) {
   if (rows <= 0 || rows % 256 != 0 || M <= 0 || M % 32 != 0 || N <= 0 || E <= 0)
     return b200::fail(833, "gemm_grouped_pair_wgrad: rows=%d (x256) M=%d (x32) N=%d E=%d", rows, M, N, E);
@@ -138,7 +139,7 @@ B200_API int b200_gemm_grouped_pair_wgrad(const void* a, const void* b, void* d,
   if ((r = b200::make_tmap_2d(&tmB, b200::DT_BF16, b, N, rows, ldb * 2, 64, 64, b200::SWZ_128))) return r;
   if ((r = make_out_tmap<256>(&tmD, &tmDt, d, E * M, N, N, out_f32))) return r;
   PairParams p = {};
-  p.grp.mode = 2; p.grp.E = E; p.grp.seg = seg;
+  p.grp.mode = 2; p.grp.E = E; p.grp.seg = seg; p.grp.counts = counts;
   p.M = M; p.N = N; p.K = rows;
   p.a_mn_major = 1; p.b_mn_major = 1;
   p.group_m = 1;

@@ -68,8 +68,9 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_gemm_grouped_wgrad": [P, P, P, P, I, I, I, I, L, L, I, I, F, P],
         "b200_gemm_grouped_mx_rows": [P, P, P, P, P, P, I, I, I, I, L, L, L, I, F, P],
         "b200_gemm_grouped_mx_wgrad": [P, P, P, P, P, P, I, I, I, I, L, L, I, I, F, P],
+        "b200_swiglu_tiles": [P, P, P, I, P, P, P, I, P],
         "b200_gemm_grouped_pair_rows": [P, P, P, P, I, I, I, I, L, L, I, F, P],
-        "b200_gemm_grouped_pair_wgrad": [P, P, P, P, I, I, I, I, L, L, I, I, F, P],
+        "b200_gemm_grouped_pair_wgrad": [P, P, P, P, P, I, I, I, I, L, L, I, I, F, P],
         "b200_zero_reduce_scatter": [P, I, I, L, L, F, P, P, P],
         "b200_zero_adamw_all_gather": [P, I, I, L, L, P, P, P, P, F, F, F, F, F, I, F, P, F, I, P],
         "b200_zero_reduce_scatter_mc": [P, L, L, F, P, I, P, P],

@@ -179,15 +179,18 @@ def grouped_rows(a: torch.Tensor, b: torch.Tensor, tile_expert: torch.Tensor, se
 
 
 def grouped_wgrad(dy: torch.Tensor, x: torch.Tensor, seg: torch.Tensor, n_experts: int, *,
-                  out: torch.Tensor | None = None, accumulate: bool = False, out_dtype=None, pad: int = PAD) -> torch.Tensor:
-    """``d[e] (+)= dy[seg[e]:seg[e+1]]^T @ x[seg[e]:seg[e+1]]`` -> ``[E, M, N]``.  ``pad``: what the segments are padded to."""
+                  out: torch.Tensor | None = None, accumulate: bool = False, out_dtype=None, pad: int = PAD,
+                  counts: torch.Tensor | None = None) -> torch.Tensor:
+    """``d[e] (+)= dy[seg[e]:seg[e+1]]^T @ x[seg[e]:seg[e+1]]`` -> ``[E, M, N]``.  ``pad``: what the segments are padded to;
+    ``counts`` (int32 ``[E]``): rows of the segments that count; the rows behind them up to the next multiple of 64 must be zero, later
+    ones are not read."""
     M, N = dy.shape[1], x.shape[1]
     if pad == PAD_MX and use_kernels(dy) and dy.dtype == torch.bfloat16 and M % 32 == 0:
         if out is None:
             # every element is written, zeros for an expert without rows
             out, accumulate = torch.empty((n_experts, M, N), dtype=out_dtype or dy.dtype, device=dy.device), False
         dy, x = dy.contiguous(), x.contiguous()
-        call("b200_gemm_grouped_pair_wgrad", ptr(dy), ptr(x), ptr(out), ptr(seg), dy.shape[0], M, N, n_experts, dy.stride(0),
+        call("b200_gemm_grouped_pair_wgrad", ptr(dy), ptr(x), ptr(out), ptr(seg), ptr(counts), dy.shape[0], M, N, n_experts, dy.stride(0),
              x.stride(0), int(out.dtype == torch.float32), int(accumulate), 1.0, stream_ptr())
         return out
     if out is None:
@@ -285,31 +288,46 @@ class GroupedMLPFn(Function):
     gradients accumulate into ``main_grad`` when the parameters carry one."""
 
     @staticmethod
-    def forward(ctx, x, w1, w2, seg, tile_expert, y_out=None, dx_out=None):
+    def forward(ctx, x, w1, w2, seg, tile_expert, y_out=None, dx_out=None, counts=None):
+        if (tile_expert.numel() * PAD_MX != x.shape[0] or not use_kernels(x) or x.dtype != torch.bfloat16
+                or w1.shape[1] % 32 or w2.shape[1] % 32):
+            counts = None                # (only the kernels on 256-row tiles leave out a segment's padding)
         gu = grouped_rows(x, w1, tile_expert, seg)
-        a = K.swiglu_fwd(gu)
+        a = _swiglu(gu, tile_expert, seg, counts)
         y = grouped_rows(a, w2, tile_expert, seg, out=y_out)
-        ctx.save_for_backward(x, gu, w1, w2, seg, tile_expert)
+        ctx.save_for_backward(x, gu, w1, w2, seg, tile_expert, counts)
         ctx.refs = (w1, w2)
         ctx.dx_out = dx_out
         return y
 
     @staticmethod
     def backward(ctx, gy):
-        x, gu, w1, w2, seg, tile_expert = ctx.saved_tensors
+        x, gu, w1, w2, seg, tile_expert, counts = ctx.saved_tensors
         p1, p2 = ctx.refs
         E = w1.shape[0]
         gy = _zero_padding(gy.contiguous(), tile_expert)
-        a = K.swiglu_fwd(gu)
+        a = _swiglu(gu, tile_expert, seg, counts)
         a = _zero_padding(a, tile_expert)
         pad = gy.shape[0] // max(tile_expert.numel(), 1)
-        g2 = _wgrad_into(p2, gy, a, seg, E, pad)
+        g2 = _wgrad_into(p2, gy, a, seg, E, pad, counts)
         da = grouped_rows(gy, w2, tile_expert, seg, b_mn_major=True)
-        dgu = K.swiglu_bwd(da, gu)
+        dgu = _swiglu(gu, tile_expert, seg, counts, da)
         dgu = _zero_padding(dgu, tile_expert)
-        g1 = _wgrad_into(p1, dgu, x, seg, E, pad)
+        g1 = _wgrad_into(p1, dgu, x, seg, E, pad, counts)
         dx = grouped_rows(dgu, w1, tile_expert, seg, b_mn_major=True, out=ctx.dx_out)
-        return dx, g1, g2, None, None, None, None
+        return dx, g1, g2, None, None, None, None, None
+
+
+def _swiglu(gu, tile_expert, seg, counts, da=None):
+    """SwiGLU of ``gu``, or with ``da`` its gradient; with ``counts`` only in each segment's rows up to the multiple of 64
+    behind its last pair (the others stay as they are: only rows of the same number depend on them, and the weight gradients stop
+    there)."""
+    if counts is None:
+        return K.swiglu_fwd(gu) if da is None else K.swiglu_bwd(da, gu)
+    F = gu.shape[1] // 2
+    out = torch.empty((gu.shape[0], F if da is None else 2 * F), dtype=gu.dtype, device=gu.device)
+    call("b200_swiglu_tiles", ptr(da), ptr(gu), ptr(out), F, ptr(tile_expert), ptr(seg), ptr(counts), tile_expert.numel(), stream_ptr())
+    return out
 
 
 # --------------------------------------------------------------------------------------
@@ -456,14 +474,15 @@ def _wgrad_into_mx(param, dy_t, x_t, seg, E):
     return grouped_wgrad_mx(dy_t, x_t, seg, E, out).to(param.dtype)
 
 
-def grouped_mlp(x, w1, w2, seg, tile_expert, precision: str = "bf16", y_out=None, dx_out=None):
+def grouped_mlp(x, w1, w2, seg, tile_expert, precision: str = "bf16", y_out=None, dx_out=None, counts=None):
     """Expert MLP over a padded row buffer whose segments are padded to ``pad_rows(precision)``.  ``y_out`` /
     ``dx_out``: buffers of the row buffer's shape that receive the output / the input gradient (peer-visible slabs
-    of the expert-parallel dispatch, filled by the last GEMM of each direction instead of by a copy)."""
+    of the expert-parallel dispatch, filled by the last GEMM of each direction instead of by a copy).  ``counts`` (int32 ``[E]``): rows
+    of each segment that are used, the others being zero in ``x`` and in the gradient; results in those others may hold anything."""
     from .linear import is_mx
     if is_mx(precision):
         return GroupedMLPMXFn.apply(x, w1, w2, seg, tile_expert, y_out, dx_out, precision)
-    return GroupedMLPFn.apply(x, w1, w2, seg, tile_expert, y_out, dx_out)
+    return GroupedMLPFn.apply(x, w1, w2, seg, tile_expert, y_out, dx_out, counts)
 
 
 def _zero_padding(t: torch.Tensor, tile_expert: torch.Tensor) -> torch.Tensor:
@@ -479,14 +498,14 @@ def _zero_padding(t: torch.Tensor, tile_expert: torch.Tensor) -> torch.Tensor:
     return t.masked_fill(dead[:, None], 0)
 
 
-def _wgrad_into(param, dy, x, seg, E, pad=PAD):
+def _wgrad_into(param, dy, x, seg, E, pad=PAD, counts=None):
     mg = getattr(param, "main_grad", None)
     if not param.requires_grad:
         return None
     if mg is not None:
-        grouped_wgrad(dy, x, seg, E, out=mg, accumulate=True, pad=pad)
+        grouped_wgrad(dy, x, seg, E, out=mg, accumulate=True, pad=pad, counts=counts)
         return None
-    return grouped_wgrad(dy, x, seg, E, out_dtype=param.dtype, pad=pad)
+    return grouped_wgrad(dy, x, seg, E, out_dtype=param.dtype, pad=pad, counts=counts)
 
 
 def expert_precision(precision: str, w1, w2) -> str:
@@ -508,5 +527,5 @@ def moe_experts(x, idx, w, counts, w1, w2, precision: str = "bf16", residual=Non
     seg, tile_expert, dest, rows = plan(idx, counts, E, pad=pad)
     gaps = (seg, counts) if pad == PAD_MX else ()       # (the kernels on 128-row tiles want the rows behind the last segment zero)
     xp = PermuteFn.apply(x, dest, k, rows, *gaps)
-    yp = grouped_mlp(xp, w1, w2, seg, tile_expert, precision)
+    yp = grouped_mlp(xp, w1, w2, seg, tile_expert, precision, counts=counts)
     return UnpermuteFn.apply(yp, dest, w, T, k, residual, *gaps)

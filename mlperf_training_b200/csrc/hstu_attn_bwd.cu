@@ -97,13 +97,13 @@ hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int ctx = p.contextual;
   const int hist_end = len - n_tgt;
   const int max_id = hist_end - (ctx > 0 ? ctx - 1 : 0);
-  // query tiles that see at least one key of this tile: the causal range, plus tile 0 when it
-  // holds contextual rows (they see every history column)
+  // query tiles that see at least one key of this tile: the causal range, plus the earlier tiles that
+  // hold contextual rows (they see every history column)
   const int i_lo = kv0 / BQ, i_hi = (len - 1) / BQ;
-  const int extra = (ctx > 0 && i_lo > 0) ? 1 : 0;
+  const int extra = min((ctx + BQ - 1) / BQ, i_lo);
   const int n_q = (i_hi - i_lo + 1) + extra;
   const int n_iter = n_q;
-  auto q_tile = [&](int it) { return (extra && it == 0) ? 0 : i_lo + it - extra; };
+  auto q_tile = [&](int it) { return it < extra ? it : i_lo + it - extra; };
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1); mbar_init(do_full, 1); mbar_init(do_empty, 1); mbar_init(s_full, 1); mbar_init(dp_full, 1);

@@ -13,9 +13,10 @@ pytestmark = pytest.mark.gpu
     ([17, 300, 1, 513], None, 0),
     ([64, 257, 130], [1, 1, 1], 0),
     ([200, 40, 384], [1, 3, 2], 8),
-    # ends around the tile and tile-pair edges, targets that fill a tile or the whole sequence
+    # ends around the tile and tile-pair edges, targets that fill a tile or the whole sequence, contextual rows past a tile
     ([127, 129, 255, 256, 257, 385], [0, 1, 2, 127, 130, 129], 0),
     ([3, 130, 260, 520], [3, 2, 4, 1], 5),
+    ([140, 300, 129, 2], [0, 1, 100, 0], 131),
 ])
 @pytest.mark.parametrize("via_uvqk", [False, True])
 def test_hstu_attention_fwd_bwd(lengths, targets, ctx, via_uvqk):

@@ -24,6 +24,7 @@ CSRC = Path(__file__).resolve().parent
 PKG = CSRC.parent
 LIB_NAME = "_b200_kernels.so"
 LIB_PATH = PKG / LIB_NAME
+HOST_LIB_NAME = "_b200_host.so"        # the CPython module of host.cpp (argument conversion, the GEMM operator)
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -52,6 +53,32 @@ def _digest(path: Path, extra: str) -> str:
 
 def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
+
+
+def build_host(force: bool = False) -> Path:
+    """Compile ``host.cpp`` against the installed torch into the in-tree module.  Returns its path."""
+    import sysconfig
+
+    import torch
+    src, out, torch_dir = CSRC / "host.cpp", PKG / HOST_LIB_NAME, Path(torch.__path__[0])
+    cuda = Path(_nvcc()).resolve().parent.parent
+    flags = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+             f"-I{sysconfig.get_paths()['include']}", f"-I{torch_dir}/include", f"-I{torch_dir}/include/torch/csrc/api/include",
+             f"-I{cuda}/include"]
+    libs = [f"-L{torch_dir}/lib", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    obj_dir = CSRC / "build"
+    obj_dir.mkdir(exist_ok=True)
+    stamp = obj_dir / f"host.{hashlib.sha256(src.read_bytes() + ' '.join(flags + libs + [torch.__version__, sys.version]).encode()).hexdigest()[:16]}.stamp"
+    if stamp.exists() and out.exists() and not force:
+        return out
+    cxx = shutil.which("g++") or "g++"
+    res = subprocess.run([cxx, *flags, str(src), "-o", str(out), *libs], capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {src.name}:\n{res.stdout}\n{res.stderr}")
+    for old in obj_dir.glob("host.*.stamp"):
+        old.unlink()
+    stamp.touch()
+    return out
 
 
 DEBUG_LIB_NAME = "_b200_kernels_dbg.so"
@@ -85,7 +112,9 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False, 
         return obj, True, res.stderr
 
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 4)) as ex:
+        host = ex.submit(build_host, force)
         results = list(ex.map(compile_one, sources()))
+        host.result()
     objs = [r[0] for r in results]
     rebuilt = any(r[1] for r in results)
     if verbose or ptxas_info:

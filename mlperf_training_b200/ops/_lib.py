@@ -23,6 +23,22 @@ _PKG = Path(__file__).resolve().parent.parent
 # B200_KERNELS_LIB selects another build of the library (the bounds-reporting debug build)
 LIB_PATH = Path(os.environ["B200_KERNELS_LIB"]) if os.environ.get("B200_KERNELS_LIB") else _PKG / "_b200_kernels.so"
 
+HOST_PATH = _PKG / "_b200_host.so"
+
+
+def _import_host():
+    """The native host module, or None before it is built (its work is then done by ctypes and Python: the same kernels)."""
+    if not HOST_PATH.exists():
+        return None
+    import importlib.machinery
+    import importlib.util
+    loader = importlib.machinery.ExtensionFileLoader("_b200_host", str(HOST_PATH))
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_b200_host", loader))
+    loader.exec_module(mod)
+    return mod
+
+
+host = _import_host()
 _lib = None
 _lock = threading.Lock()
 _load_error: str | None = None
@@ -118,12 +134,19 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_attn_delta": [P, P, P, I, I, I, I, L, L, L, L, P],
         "b200_attn_bwd": [P] * 9 + [I] * 6 + [L] * 12 + [F, I, I, P],
     }
+    codes = {P: "P", I: "I", L: "L", F: "F", ctypes.c_ulonglong: "U"}
+    table = {}
     for name, argtypes in sigs.items():
         fn = getattr(lib, name, None)
         if fn is None:
             continue
         fn.argtypes = argtypes
         fn.restype = c_int
+        table[name] = (ctypes.cast(fn, c_void_p).value, "".join(codes[t] for t in argtypes))
+    if host is not None:
+        host.bind(table, ctypes.cast(lib.b200_last_error, c_void_p).value, _call_ctypes)
+        if hasattr(lib, "b200_gemm_bf16_workspace"):
+            host.bind_gemm(table["b200_gemm_bf16"][0], ctypes.cast(lib.b200_gemm_bf16_workspace, c_void_p).value)
     lib.b200_norm_bwd_scratch_elems.argtypes = [I, I]
     lib.b200_hstu_gate_cat_scratch_elems.argtypes = [I, I]
     lib.b200_hstu_gate_cat_scratch_elems.restype = c_ll
@@ -217,11 +240,18 @@ def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
-def call(name: str, *args) -> None:
+def _call_ctypes(name: str, *args) -> None:
     rc = getattr(_lib if _lib is not None else load(), name)(*args)
     if rc != 0:
         msg = load().b200_last_error().decode(errors="replace")
         raise RuntimeError(f"{name} failed with code {rc}: {msg}")
+
+
+if host is not None:
+    host.bind({}, 0, _call_ctypes)       # until the library is loaded; then launchers are called by address
+    call = host.call
+else:
+    call = _call_ctypes
 
 
 @functools.lru_cache(maxsize=4096)

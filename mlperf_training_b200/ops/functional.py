@@ -12,11 +12,30 @@ from __future__ import annotations
 import math
 
 import torch
-from torch.autograd import Function
+from torch.autograd import Function, forward_ad
 
 from . import kernels as K
 from . import linear as L
 from ._lib import call, ptr, stream_ptr, use_kernels
+
+
+class _NoGrad:
+    """The context of a forward that no backward follows."""
+    needs_input_grad = (False,) * 32
+
+    def save_for_backward(self, *tensors):
+        pass
+
+    def set_materialize_grads(self, value):
+        pass
+
+
+def _apply(fn, *args):
+    """``fn.apply``; with the gradient mode off, no function transform and no forward-mode level under way ``fn.forward`` itself (an
+    autograd node that is thrown away costs 8 us of host time a call)."""
+    if torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0:
+        return fn.apply(*args)
+    return fn.forward(_NoGrad(), *args)
 
 
 def _wgrad(dy: torch.Tensor, x: torch.Tensor, weight: torch.Tensor):
@@ -72,7 +91,7 @@ class LinearFn(Function):
 
 
 def linear(x, weight, bias=None, residual=None, precision="bf16"):
-    return LinearFn.apply(x, weight, bias, residual, precision, torch.is_grad_enabled())
+    return _apply(LinearFn, x, weight, bias, residual, precision, torch.is_grad_enabled())
 
 
 class NormFn(Function):
@@ -95,15 +114,15 @@ class NormFn(Function):
 
 
 def rms_norm(x, weight, eps=1e-5):
-    return NormFn.apply(x, weight, None, eps, False, False)
+    return _apply(NormFn, x, weight, None, eps, False, False)
 
 
 def layer_norm(x, weight, bias, eps=1e-5):
-    return NormFn.apply(x, weight, bias, eps, True, False)
+    return _apply(NormFn, x, weight, bias, eps, True, False)
 
 
 def swish_layer_norm(x, weight, bias, eps=1e-5):
-    return NormFn.apply(x, weight, bias, eps, True, True)
+    return _apply(NormFn, x, weight, bias, eps, True, True)
 
 
 class NormLinearFn(Function):
@@ -144,7 +163,7 @@ class NormLinearFn(Function):
 
 
 def norm_linear(x, norm_w, weight, *, norm_b=None, bias=None, eps=1e-5, layer_norm=False, precision="bf16"):
-    return NormLinearFn.apply(x, norm_w, norm_b, weight, bias, eps, layer_norm, precision, torch.is_grad_enabled())
+    return _apply(NormLinearFn, x, norm_w, norm_b, weight, bias, eps, layer_norm, precision, torch.is_grad_enabled())
 
 
 class SwiGLULinearFn(Function):
@@ -171,7 +190,7 @@ class SwiGLULinearFn(Function):
 
 
 def swiglu_linear(gu, weight, residual=None, precision="bf16"):
-    return SwiGLULinearFn.apply(gu, weight, residual, precision, torch.is_grad_enabled())
+    return _apply(SwiGLULinearFn, gu, weight, residual, precision, torch.is_grad_enabled())
 
 
 def _mx_wgrad(weight, dy_col, x_col):
@@ -267,7 +286,7 @@ def fused_mlp_eligible(h: torch.Tensor, w_gu: torch.Tensor, w_down: torch.Tensor
 
 def fused_mlp(h, norm_w, w_gate_up, w_down, eps=1e-5, store_fp8: bool = False):
     """``h + swiglu(rmsnorm(h) W_gu^T) W_down^T`` with MXFP8 GEMMs."""
-    return FusedMLPFn.apply(h, norm_w, w_gate_up, w_down, eps, store_fp8, torch.is_grad_enabled())
+    return _apply(FusedMLPFn, h, norm_w, w_gate_up, w_down, eps, store_fp8, torch.is_grad_enabled())
 
 
 class SwiGLUFn(Function):
@@ -283,7 +302,7 @@ class SwiGLUFn(Function):
 
 
 def swiglu(gu):
-    return SwiGLUFn.apply(gu)
+    return _apply(SwiGLUFn, gu)
 
 
 class GeluFn(Function):
@@ -299,7 +318,7 @@ class GeluFn(Function):
 
 
 def gelu(x):
-    return GeluFn.apply(x)
+    return _apply(GeluFn, x)
 
 
 class AttentionFn(Function):
@@ -346,7 +365,7 @@ class AttentionFn(Function):
 def attention_packed(qkv, *, B, S, Hq, Hkv, D, cos=None, sin=None, sink=None, causal=True, window=0, scale=None):
     if scale is None:
         scale = 1.0 / math.sqrt(D)
-    return AttentionFn.apply(qkv, sink, cos, sin, B, S, Hq, Hkv, D, causal, window, scale)
+    return _apply(AttentionFn, qkv, sink, cos, sin, B, S, Hq, Hkv, D, causal, window, scale)
 
 
 class RopePackedFn(Function):
@@ -399,7 +418,7 @@ class AttentionBSHDFn(Function):
 def attention(q, k, v, *, causal=True, window=0, sink=None, scale=None):
     if scale is None:
         scale = 1.0 / math.sqrt(q.shape[-1])
-    return AttentionBSHDFn.apply(q, k, v, sink, causal, window, scale)
+    return _apply(AttentionBSHDFn, q, k, v, sink, causal, window, scale)
 
 
 class EmbeddingFn(Function):
@@ -574,7 +593,7 @@ class LNModulateFn(Function):
 
 
 def ln_modulate(x2d, shift, scale, B, eps=1e-6):
-    return LNModulateFn.apply(x2d, shift, scale, B, eps)
+    return _apply(LNModulateFn, x2d, shift, scale, B, eps)
 
 
 class GateResidualFn(Function):
@@ -612,7 +631,7 @@ class GateResidualFn(Function):
 
 
 def gate_residual(res2d, y2d, gate, B):
-    return GateResidualFn.apply(res2d, y2d, gate, B)
+    return _apply(GateResidualFn, res2d, y2d, gate, B)
 
 
 class RopeBSHDFn(Function):
@@ -637,7 +656,7 @@ class RopeBSHDFn(Function):
 
 
 def rope_bshd(x, cos, sin):
-    return RopeBSHDFn.apply(x, cos, sin)
+    return _apply(RopeBSHDFn, x, cos, sin)
 
 
 def qkv_norm_rope_ok(cos, head_dim: int, parts) -> bool:
@@ -716,7 +735,7 @@ class QKVNormRopeFn(Function):
 
 
 def qkv_norm_rope(parts, cos, sin, B, H, D, eps=1e-6):
-    return QKVNormRopeFn.apply(cos, sin, B, H, D, eps, *[t for p in parts for t in p])
+    return _apply(QKVNormRopeFn, cos, sin, B, H, D, eps, *[t for p in parts for t in p])
 
 
 class SingleStreamInFn(Function):
@@ -752,7 +771,7 @@ class SingleStreamInFn(Function):
 
 
 def single_stream_in(y, q_scale, k_scale, cos, sin, B, H, D, eps=1e-6):
-    return SingleStreamInFn.apply(y, q_scale, k_scale, cos, sin, B, H, D, eps)
+    return _apply(SingleStreamInFn, y, q_scale, k_scale, cos, sin, B, H, D, eps)
 
 
 # --------------------------------------------------------------------------------------
@@ -789,4 +808,4 @@ class RouterLogitsFn(Function):
 
 
 def router_logits(hn, router):
-    return RouterLogitsFn.apply(hn, router)
+    return _apply(RouterLogitsFn, hn, router)

@@ -51,6 +51,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn_major: bool = False, b_mn_maj
     ``gemm(dy, w, b_mn_major=True)`` is ``dy @ w`` (dgrad) and
     ``gemm(dy, x, a_mn_major=True, b_mn_major=True)`` is ``dy.T @ x`` (wgrad).
     """
+    if _lib.host is not None and a.is_cuda and use_kernels(a) and out_dtype in (None, BF16, torch.float32):
+        # (a result for operands that are as the kernel reads them; None leaves copies and errors to the lines below)
+        d = _lib.host.gemm(a, b, a_mn_major, b_mn_major, out, out_dtype == torch.float32, accumulate, bias, residual, alpha)
+        if d is not None:
+            return d
     M, K = (a.shape[1], a.shape[0]) if a_mn_major else (a.shape[0], a.shape[1])
     N, Kb = (b.shape[1], b.shape[0]) if b_mn_major else (b.shape[0], b.shape[1])
     if K != Kb:

@@ -61,6 +61,45 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ buf, const float* __rest
   }
 }
 
+// Gradients of the rotated projections, finished in one pass: head h < hq of a row comes from the attention backward's fp32
+// dq [T, hq, hd], the next hkv heads (k) from `buf` itself; every one of them is rotated back and stored to `buf` as bf16.  A
+// copy of dq into `buf` and the rotation in place read and wrote the q columns twice and rounded them twice (8192 tokens, 64 / 8
+// heads of 64: 82 + 22 -> 34 us; 4096, 64 / 8 of 128: 80 + 24 -> 36).
+template <typename I>
+__global__ void __launch_bounds__(256)
+rope_grad_kernel(const float* __restrict__ dq, __nv_bfloat16* __restrict__ buf, const float* __restrict__ cos_t,
+                 const float* __restrict__ sin_t, I total, int S, long long row_stride, I hq, I heads, int hd) {
+  const int half = hd / 2;
+  const I vec_per_head = half / 8, per_row = heads * vec_per_head;
+  for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    const I t = i / per_row, r = i - t * per_row, h = r / vec_per_head, v = r - h * vec_per_head;
+    const long long at = (long long)(t % (I)S) * half + v * 8;
+    __nv_bfloat16* base = buf + (long long)t * row_stride + h * hd + v * 8;
+    float x1[8], x2[8], c[8], s[8], o1[8], o2[8];
+    auto ldf = [](const float* p, float (&f)[8]) {
+      const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+      f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+    };
+    if (h < hq) {
+      const float* src = dq + ((long long)t * hq + h) * hd + v * 8;
+      ldf(src, x1);
+      ldf(src + half, x2);
+    } else {
+      ld8(base, x1);
+      ld8(base + half, x2);
+    }
+    ldf(cos_t + at, c);
+    ldf(sin_t + at, s);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      o1[j] = x1[j] * c[j] + x2[j] * s[j];
+      o2[j] = x2[j] * c[j] - x1[j] * s[j];
+    }
+    st8(base, o1);
+    st8(base + half, o2);
+  }
+}
+
 // ---------------------------------------------------------------------------------------
 // SwiGLU: a[t, f] = silu(gu[t, f]) * gu[t, F + f]  (gate columns first, up columns second)
 // ---------------------------------------------------------------------------------------
@@ -263,6 +302,22 @@ B200_API int b200_rope(void* buf, const float* cos_t, const float* sin_t, const 
                                                                      backward ? -1.f : 1.f);
   b200::count_launch();
   return b200::check_launch("rope");
+}
+// dq: fp32 [T, hq, hd] contiguous; buf: bf16 rows [hq | hkv | ...] x hd (pitch row_stride) whose k columns hold dk.
+B200_API int b200_rope_grad(const float* dq, void* buf, const float* cos_t, const float* sin_t, long long T, int S, long long row_stride,
+                            int hq, int hkv, int hd, void* stream) {
+  if (hd % 16 != 0 || row_stride % 8 != 0 || S <= 0 || (((uintptr_t)dq | (uintptr_t)buf | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15) != 0)
+    return b200::fail(406, "rope_grad: head dim %d must be a multiple of 16, the row pitch of 8, pointers 16-byte aligned", hd);
+  const long long work = T * (hq + hkv) * (hd / 16);
+  if (work == 0) return 0;
+  if (fits32(work))
+    rope_grad_kernel<uint32_t><<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
+        dq, (__nv_bfloat16*)buf, cos_t, sin_t, (uint32_t)work, S, row_stride, (uint32_t)hq, (uint32_t)(hq + hkv), hd);
+  else
+    rope_grad_kernel<long long><<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
+        dq, (__nv_bfloat16*)buf, cos_t, sin_t, work, S, row_stride, hq, hq + hkv, hd);
+  b200::count_launch();
+  return b200::check_launch("rope_grad");
 }
 B200_API int b200_swiglu_fwd(const void* gu, void* a, long long T, int F, void* stream) {
   if (F % 8 != 0) return b200::fail(401, "swiglu: F=%d must be a multiple of 8", F);

@@ -61,6 +61,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_norm_fwd": [I, P, P, P, P, P, P, P, P, I, I, F, I, P],
         "b200_norm_bwd": [I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P],
         "b200_rope": [P, P, P, P, L, I, L, I, I, I, I, P],
+        "b200_rope_grad": [P, P, P, P, L, I, L, I, I, I, P],
         "b200_swiglu_fwd": [P, P, L, I, P],
         "b200_swiglu_bwd": [P, P, P, L, I, P],
         "b200_gelu_fwd": [P, P, L, P],

@@ -354,9 +354,10 @@ class AttentionFn(Function):
         dv = d3[:, :, (Hq + Hkv) * D:].unflatten(-1, (Hkv, D))
         dq, _, _, dsink = K.attention_bwd(dout.contiguous().view(B, S, Hq, D), q, k, v, out, lse, scale=scale,
                                           causal=causal, window=window, sink=sink, dk_out=dk, dv_out=dv)
-        d3[:, :, :Hq * D].copy_(dq.reshape(B, S, Hq * D))
         if cos is not None:
-            K.rope_(dqkv, cos, sin, col0=0, n_heads=Hq + Hkv, head_dim=D, seq_len=S, backward=True)
+            K.rope_grad_(dq, dqkv, cos, sin, n_heads=Hq, n_kv_heads=Hkv, head_dim=D, seq_len=S)
+        else:
+            d3[:, :, :Hq * D].copy_(dq.reshape(B, S, Hq * D))
         if sink is not None and dsink is not None:
             dsink = dsink.to(sink.dtype)
         return dqkv, dsink, None, None, None, None, None, None, None, None, None, None

@@ -238,6 +238,21 @@ def rope_(buf: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, *, col0: int,
     return buf
 
 
+def rope_grad_(dq: torch.Tensor, dqkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, *, n_heads: int, n_kv_heads: int,
+               head_dim: int, seq_len: int) -> torch.Tensor:
+    """Writes the gradient of the unrotated q columns of ``dqkv [T, (Hq + 2 Hkv) * D]`` from ``dq`` (fp32 ``[.., Hq, D]``,
+    gradient of the rotated q) and turns its k columns back in place."""
+    T = dqkv.shape[0]
+    if not use_kernels(dqkv):
+        dqkv[:, :n_heads * head_dim].copy_(dq.reshape(T, n_heads * head_dim))
+        return rope_(dqkv, cos, sin, col0=0, n_heads=n_heads + n_kv_heads, head_dim=head_dim, seq_len=seq_len, backward=True)
+    if dqkv.stride(1) != 1:
+        raise ValueError("rope_grad_: rows must be contiguous")
+    call("b200_rope_grad", ptr(dq.contiguous()), ptr(dqkv), ptr(cos), ptr(sin), T, seq_len, dqkv.stride(0), n_heads, n_kv_heads,
+         head_dim, stream_ptr())
+    return dqkv
+
+
 # --------------------------------------------------------------------------------------
 # activations
 # --------------------------------------------------------------------------------------

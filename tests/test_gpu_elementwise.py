@@ -88,6 +88,21 @@ def test_gather_scatter():
     _close(g_g, g_c, 1e-5, "scatter add")
 
 
+@pytest.mark.parametrize("B,S,Hq,Hkv,D", [(1, 5, 2, 1, 64), (2, 33, 4, 2, 128), (3, 257, 8, 8, 32)])
+def test_rope_grad_from_fp32_dq(B, S, Hq, Hkv, D):
+    torch.manual_seed(S)
+    dq = torch.randn(B, S, Hq, D)
+    dqkv = torch.randn(B * S, (Hq + 2 * Hkv) * D).bfloat16()
+    cos, sin = kernels.rope_tables(S, D, 10000.0, "cpu")
+    ref = dqkv.float()
+    ref[:, :Hq * D] = dq.reshape(B * S, -1)
+    kernels.rope_(ref, cos, sin, col0=0, n_heads=Hq + Hkv, head_dim=D, seq_len=S, backward=True)
+    got = kernels.rope_grad_(dq.cuda(), dqkv.cuda(), cos.cuda(), sin.cuda(), n_heads=Hq, n_kv_heads=Hkv, head_dim=D, seq_len=S).cpu()
+    assert torch.equal(got[:, (Hq + Hkv) * D:], dqkv[:, (Hq + Hkv) * D:])
+    # one rounding to bf16 (2^-9 of the value) of sums whose fp32 products may be fused or not (cancellation: 2^-22 of the terms)
+    assert ((got.float() - ref).abs() <= ref.abs() * 2 ** -8 + 2 ** -20 * ref.abs().max()).all()
+
+
 def test_scatter_add_rows_of_an_unaligned_table():
     torch.manual_seed(0)
     ids = torch.randint(-1, 7, (50,))

@@ -30,6 +30,11 @@
 //
 // The reference takes this kernel from Primus-Turbo / AITER / CK (config knobs
 // llama2_sft/primus/config_MI355X_1x8x1.sh:35-39); there is no in-tree counterpart.
+#include <algorithm>
+#include <climits>
+#include <queue>
+#include <vector>
+
 #include "common.cuh"
 #include "runtime.h"
 
@@ -42,6 +47,8 @@ constexpr int NTHREADS = 512;  // warp 0 TMA, 1 MMA (2, 3 complete the warpgroup
 constexpr int REGS_OTHER = 88, REGS_WORKER = 168;
 constexpr int STG = 4096;  // dQ staging chunk: 32 rows x 32 fp32 (two per drain warp)
 
+constexpr int MAX_PARTS = 8, MAX_ENTRIES = 512;
+
 struct BwdParams {
   int B, Hq, Hkv, Sq, Skv;
   int causal, window;
@@ -50,7 +57,28 @@ struct BwdParams {
   const float* delta;  // [B, Hq, Sq]  rowsum(dO * O)
   int* status;
   int bh_group;        // (batch, kv head) pairs scheduled together, longest key tiles first
+  // Split schedule (cap > 0): no CTA takes more than cap steps of a key tile; the others of a tile take its next ones.
+  int cap, entries;    // entries: CTAs of one (batch, kv head) pair, in `order` as (key tile << 3 | part), longest first
+  int max_parts;       // most parts of a tile, at most MAX_PARTS
+  float* partial;      // fp32 [B * Hkv][key tile][max_parts][dK | dV][128][HD], of tiles with several parts
+  uint16_t order[MAX_ENTRIES];
 };
+
+// (query head, query tile) steps of key tile jt and its first query tile.
+__host__ __device__ inline int tile_steps(int jt, int Sq, int Skv, int group, int causal, int window, int& i_lo, int& i_hi) {
+  const int kv0 = jt * BKV, off = Skv - Sq;
+  i_lo = 0; i_hi = (Sq + BQ - 1) / BQ - 1;
+  if (causal) {
+    const int first_q = kv0 - off;  // first query position that sees key kv0
+    if (first_q > 0) i_lo = first_q / BQ;
+  }
+  if (window > 0) {
+    const int last_q = kv0 + BKV - 1 + window - 1 - off;  // last query that still sees the tile's last key
+    if (last_q / BQ < i_hi) i_hi = last_q / BQ;
+  }
+  return i_hi >= i_lo ? (i_hi - i_lo + 1) * group : 0;
+}
+__host__ __device__ inline int tile_parts(int steps, int cap) { return steps > cap ? (steps + cap - 1) / cap : 1; }
 
 B200_DEVICE void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
   asm volatile(
@@ -86,7 +114,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                 const __grid_constant__ CUtensorMap tmdQ, const __grid_constant__ CUtensorMap tmdK,
-                const __grid_constant__ CUtensorMap tmdV, const BwdParams p) {
+                const __grid_constant__ CUtensorMap tmdV, const __grid_constant__ BwdParams p) {
   using SM = Smem<HD>;
   constexpr int NB = HD / 64;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -121,27 +149,31 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_kt = (p.Skv + BKV - 1) / BKV;
   // early key tiles see the most queries: they are scheduled first, over all heads of a group
-  const int bh_all = p.B * p.Hkv, per_group = p.bh_group * num_kt;
-  const int grp = (int)blockIdx.x / per_group, rest = (int)blockIdx.x - grp * per_group;
-  const int gsz = min(p.bh_group, bh_all - grp * p.bh_group);
-  const int jt = rest / gsz, bh = grp * p.bh_group + rest % gsz;
+  const int bh_all = p.B * p.Hkv;
+  int jt, bh, part = 0;
+  if (p.cap > 0) {
+    const int e = (int)blockIdx.x / bh_all;
+    bh = (int)blockIdx.x - e * bh_all;
+    jt = p.order[e] >> 3;
+    part = p.order[e] & 7;
+  } else {
+    const int per_group = p.bh_group * num_kt;
+    const int grp = (int)blockIdx.x / per_group, rest = (int)blockIdx.x - grp * per_group;
+    const int gsz = min(p.bh_group, bh_all - grp * p.bh_group);
+    jt = rest / gsz;
+    bh = grp * p.bh_group + rest % gsz;
+  }
   const int b = bh / p.Hkv, hk = bh - b * p.Hkv;
   const int group = p.Hq / p.Hkv;
   const int kv0 = jt * BKV;
   const int off = p.Skv - p.Sq;
-  const int num_qt = (p.Sq + BQ - 1) / BQ;
   // query tiles that see at least one key of this tile
-  int i_lo = 0, i_hi = num_qt - 1;
-  if (p.causal) {
-    int first_q = kv0 - off;  // first query position that sees key kv0
-    if (first_q > 0) i_lo = first_q / BQ;
-  }
-  if (p.window > 0) {
-    int last_q = kv0 + BKV - 1 + p.window - 1 - off;  // last query that still sees the tile's last key
-    if (last_q / BQ < i_hi) i_hi = last_q / BQ;
-  }
-  const int n_q = (i_hi >= i_lo) ? (i_hi - i_lo + 1) : 0;
-  const int n_iter = n_q * group;
+  int i_lo, i_hi;
+  const int steps = tile_steps(jt, p.Sq, p.Skv, group, p.causal, p.window, i_lo, i_hi);
+  const int n_q = i_hi >= i_lo ? i_hi - i_lo + 1 : 0;
+  // this CTA's steps of the tile's
+  const int parts = p.cap > 0 ? tile_parts(steps, p.cap) : 1;
+  const int it0 = steps * part / parts, n_iter = steps * (part + 1) / parts - it0;
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1); mbar_init(do_full, 1); mbar_init(do_empty, 1); mbar_init(s_full, 1); mbar_init(dp_full, 1);
@@ -173,8 +205,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tma_load_4d(sV + i * (BKV * 128), &tmV, kv_full, i * 64, hk, kv0, b);
       }
       for (int it = 0; it < n_iter; ++it) {
-        const int h = hk * group + it / n_q;
-        const int q0 = (i_lo + it % n_q) * BQ;
+        const int h = hk * group + (it0 + it) / n_q;
+        const int q0 = (i_lo + (it0 + it) % n_q) * BQ;
         const int st = it & 1;
         if (!mbar_wait(&q_empty[st], ((it >> 1) & 1) ^ 1, abort_flag, p.status, 70)) break;
         mbar_expect_tx(&q_full[st], SM::T_BYTES);
@@ -276,8 +308,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t lane_base = uint32_t(q * 32) << 16;
     uint8_t* stg = sStg + q * 2 * STG;
     for (int it = 0; it < n_iter; ++it) {
-      const int h = hk * group + it / n_q;
-      const int q0 = (i_lo + it % n_q) * BQ;
+      const int h = hk * group + (it0 + it) / n_q;
+      const int q0 = (i_lo + (it0 + it) % n_q) * BQ;
       if (!warp_wait(dq_full, it & 1, abort_flag, p.status, 95)) break;
       tc_fence_after();
 #pragma unroll
@@ -330,7 +362,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     auto staged = [&](float x) -> float {
       return half == 1 ? x * p.scale : (x == -INFINITY ? INFINITY : x * 1.4426950408889634f);
     };
-    int h_next = hk * group, i_next = i_lo;
+    int h_next = hk * group + (n_iter > 0 ? it0 / n_q : 0), i_next = i_lo + (n_iter > 0 ? it0 % n_q : 0);
     bool ok = true;
     if (n_iter > 0) {
       sLD[half * BQ + r] = staged(fetch(h_next, i_next * BQ + r));
@@ -437,6 +469,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = 0u;
         }
+        if (parts > 1) {                        // fp32, as it is: attn_bwd_finish_kernel adds the parts up
+          float4* o = reinterpret_cast<float4*>(p.partial + ((((long long)bh * num_kt + jt) * p.max_parts + part) * 2 + half) * BKV * HD +
+                                                r * HD + c * 32);
+#pragma unroll
+          for (int g = 0; g < 8; ++g)
+            o[g] = make_float4(__uint_as_float(v[4 * g]), __uint_as_float(v[4 * g + 1]), __uint_as_float(v[4 * g + 2]),
+                               __uint_as_float(v[4 * g + 3]));
+          continue;
+        }
         uint8_t* blk = dst + (c / 2) * (BKV * 128);
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
@@ -450,7 +491,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0 && kv0 + q * 32 < p.Skv) {
+      if (lane == 0 && parts == 1 && kv0 + q * 32 < p.Skv) {
 #pragma unroll
         for (int i = 0; i < NB; ++i)
           tma_store_4d(half == 0 ? &tmdK : &tmdV, tile + i * (BKV * 128) + q * 32 * 128, i * 64, hk, kv0 + q * 32, b);
@@ -468,6 +509,99 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+}
+
+// dK and dV of a key tile from its parts, added in their order (no atomics: runs are bit-reproducible).
+template <int HD>
+__global__ void __launch_bounds__(256)
+attn_bwd_finish_kernel(const float* __restrict__ partial, int cap, int max_parts, int Hkv, int Sq, int Skv, int group, int causal, int window, int num_kt,
+                       __nv_bfloat16* dk, __nv_bfloat16* dv, long long dk_row, long long dv_row, long long dk_batch, long long dv_batch) {
+  constexpr int VPR = HD / 8;
+  const int bh = (int)blockIdx.x / num_kt, jt = (int)blockIdx.x - bh * num_kt;
+  int i_lo, i_hi;
+  const int parts = tile_parts(tile_steps(jt, Sq, Skv, group, causal, window, i_lo, i_hi), cap);
+  if (parts == 1) return;
+  const int b = bh / Hkv, hk = bh - b * Hkv;
+  const float* src = partial + (long long)blockIdx.x * max_parts * 2 * BKV * HD;
+  for (int i = blockIdx.y * 256 + threadIdx.x; i < 2 * BKV * VPR; i += gridDim.y * 256) {
+    const int half = i / (BKV * VPR), r = i / VPR % BKV, c = i % VPR * 8, key = jt * BKV + r;
+    if (key >= Skv) continue;
+    float v[8] = {};
+    for (int z = 0; z < parts; ++z) {
+      const float* f = src + (long long)z * 2 * BKV * HD + i * 8;
+      const float4 x = *reinterpret_cast<const float4*>(f), y = *reinterpret_cast<const float4*>(f + 4);
+      v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w; v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+    }
+    __nv_bfloat16* o = half == 0 ? dk + b * dk_batch + (long long)key * dk_row : dv + b * dv_batch + (long long)key * dv_row;
+    *reinterpret_cast<uint4*>(o + hk * HD + c) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                                                            pack_bf16x2(v[6], v[7]));
+  }
+}
+
+// (key tile << 3 | part) of every CTA of one (batch, kv head) pair, longest first; 0 if cap cuts a tile into more than MAX_PARTS or
+// there are more than MAX_ENTRIES.
+int split_order(int Sq, int Skv, int group, int causal, int window, int cap, std::vector<std::pair<int, uint16_t>>& out, int& max_parts) {
+  const int num_kt = (Skv + BKV - 1) / BKV;
+  out.clear();
+  max_parts = 1;
+  for (int jt = 0; jt < num_kt; ++jt) {
+    int lo, hi;
+    const int steps = tile_steps(jt, Sq, Skv, group, causal, window, lo, hi), parts = tile_parts(steps, cap);
+    if (parts > MAX_PARTS || (int)out.size() + parts > MAX_ENTRIES) return 0;
+    if (parts > max_parts) max_parts = parts;
+    for (int z = 0; z < parts; ++z)
+      out.push_back({steps * (z + 1) / parts - steps * z / parts + (parts > 1 ? 1 : 0), (uint16_t)(jt << 3 | z)});
+  }
+  std::stable_sort(out.begin(), out.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+  return (int)out.size();
+}
+
+// Steps until the last SM is done: CTAs are taken in their order by the SM that is free first; each costs its steps and five more
+// (set-up, first loads and the output: from the times of split and whole tiles at 2000 and 3000 tokens).
+long long makespan(const std::vector<int>& cost, long long copies, int sms) {
+  std::priority_queue<long long, std::vector<long long>, std::greater<long long>> sm;
+  for (int i = 0; i < sms; ++i) sm.push(0);
+  long long last = 0;
+  for (int c : cost)
+    for (long long i = 0; i < copies; ++i) {
+      const long long t = sm.top() + c + 5;
+      sm.pop();
+      sm.push(t);
+      if (t > last) last = t;
+    }
+  return last;
+}
+
+// Longest run of steps a CTA should take (0: whole key tiles).  One CTA takes a key tile's steps over all query heads of its
+// group in series, so with few tiles the longest outlasts the average SM (2000 tokens, 64 / 8 heads, causal: 128 steps against 59).  Caps
+// of 2/12 .. 11/12 of the longest tile are compared by the schedule they give; a split has to gain a twelfth of it.
+// Backward, whole tiles -> split: 2000 x 64 / 8 heads of 64 267 -> 171 us, 800 tokens 130 -> 68; heads of 128: 3000 x 64 / 8 532 -> 433,
+// 1024 x 32 / 8 103 -> 65, 2 x 1500 x 16 / 4 143 -> 106.  Parts of every tile alike (five at 2000 tokens) gained half as much, and cost
+// where a part is a few steps long: 4 x 512 x 12 heads 34 -> 56, so those stay whole.
+int split_cap(int B, int Sq, int Skv, int Hq, int Hkv, int causal, int window, int& max_parts) {
+  const int num_kt = (Skv + BKV - 1) / BKV, group = Hq / Hkv, P = b200::sm_count();
+  const long long copies = (long long)B * Hkv;
+  if (num_kt > MAX_ENTRIES || copies * num_kt > 8 * P) return 0;
+  std::vector<int> cost;
+  long long longest = 0;
+  for (int jt = 0; jt < num_kt; ++jt) {
+    int lo, hi;
+    cost.push_back(tile_steps(jt, Sq, Skv, group, causal, window, lo, hi));
+    if (cost.back() > longest) longest = cost.back();
+  }
+  if (longest < 4 || longest * 12 > INT_MAX) return 0;
+  long long best = makespan(cost, copies, P) * 11 / 12;
+  int cap = 0, parts;
+  std::vector<std::pair<int, uint16_t>> order;
+  for (int k = 2; k <= 11; ++k) {
+    const int c = (int)((longest * k + 11) / 12);
+    if (!split_order(Sq, Skv, group, causal, window, c, order, parts)) continue;
+    cost.clear();
+    for (const auto& e : order) cost.push_back(e.first);
+    const long long t = makespan(cost, copies, P) + 3;      // the launch that adds the parts up
+    if (t < best) { best = t; cap = c; max_parts = parts; }
+  }
+  return cap;
 }
 
 // delta[b, h, s] = sum_d O[b, s, h, d] * dO[b, s, h, d]; HD / 8 lanes per (token, head), one 16-byte load of either each (a
@@ -531,7 +665,7 @@ int launch_bwd(const CUtensorMap* m, const BwdParams& p, cudaStream_t stream) {
                                             cudaGetErrorString(e));
     configured[dev & 63] = true;
   }
-  const long long grid = (long long)((p.Skv + BKV - 1) / BKV) * p.Hkv * p.B;
+  const long long grid = (long long)(p.cap > 0 ? p.entries : (p.Skv + BKV - 1) / BKV) * p.Hkv * p.B;
   if (grid > 0x7fffffff) return b200::fail(612, "attn_bwd: %lld key tiles are too many", grid);
   attn_bwd_kernel<HD><<<(unsigned)grid, NTHREADS, SM::TOTAL, stream>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], p);
   b200::count_launch();
@@ -556,14 +690,28 @@ B200_API int b200_attn_delta(const void* o, const void* dout, float* delta, int 
   return b200::check_launch("attn_delta");
 }
 
+// plan[0]: longest run of steps a CTA should take (0: whole key tiles); plan[1]: bytes of partial sums that this needs.
+B200_API int b200_attn_bwd_plan(int B, int Sq, int Skv, int Hq, int Hkv, int HD, int causal, int window, long long* plan) {
+  plan[0] = plan[1] = 0;
+  if (B <= 0 || Sq <= 0 || Skv <= 0 || Hkv <= 0 || Hq <= 0 || Hq % Hkv != 0 || (HD != 64 && HD != 128)) return 0;
+  try {
+    int parts = 0;
+    const int cap = split_cap(B, Sq, Skv, Hq, Hkv, causal, window, parts);
+    if (cap > 0) { plan[0] = cap; plan[1] = (long long)B * Hkv * ((Skv + BKV - 1) / BKV) * parts * 2 * BKV * HD * 4; }
+  } catch (const std::exception&) {
+  }
+  return 0;
+}
+
 // dq_acc: fp32 [B, Sq, Hq, HD] contiguous, zero-initialised by the caller (reduce-add target).
-// dk / dv: bf16 [B, Skv, Hkv, HD] with their own pitches.
+// dk / dv: bf16 [B, Skv, Hkv, HD] with their own pitches.  cap, workspace: 0 and null, or b200_attn_bwd_plan's cap and as many bytes,
+// which nothing else uses until this call's work is done.
 B200_API int b200_attn_bwd(const void* q, const void* k, const void* v, const void* dout, const float* lse,
                            const float* delta, float* dq_acc, void* dk, void* dv, int B, int Sq, int Skv, int Hq,
                            int Hkv, int HD, long long q_row, long long k_row, long long v_row, long long do_row,
                            long long dk_row, long long dv_row, long long q_batch, long long k_batch,
                            long long v_batch, long long do_batch, long long dk_batch, long long dv_batch,
-                           float scale, int causal, int window, void* stream) {
+                           float scale, int causal, int window, int cap, void* workspace, long long workspace_bytes, void* stream) {
   if (HD != 64 && HD != 128) return b200::fail(610, "attn_bwd: head dim %d not supported (64 or 128)", HD);
   if (Hq % Hkv != 0) return b200::fail(610, "attn_bwd: Hq=%d not a multiple of Hkv=%d", Hq, Hkv);
   CUtensorMap m[7];
@@ -589,6 +737,24 @@ B200_API int b200_attn_bwd(const void* q, const void* k, const void* v, const vo
   // head keeps that head's Q and dO in L2 (full, 8 x 512 x 24 heads 128 us, 134 the other way; 2 x 4608 x 24 1211 and 1345).
   // With a window the two are even (8192 x 64 / 8 of 64, window 128: 269 and 269; 2 x 8192 x 32, window 1024: 920 and 925).
   p.bh_group = (causal && window <= 0) ? B * Hkv : 1;
-  if (HD == 128) return launch_bwd<128>(m, p, (cudaStream_t)stream);
-  return launch_bwd<64>(m, p, (cudaStream_t)stream);
+  const int num_kt = (Skv + BKV - 1) / BKV, group = Hq / Hkv;
+  p.cap = 0; p.entries = 0; p.max_parts = 1; p.partial = (float*)workspace;
+  if (cap > 0) {
+    try {
+      std::vector<std::pair<int, uint16_t>> order;
+      p.entries = split_order(Sq, Skv, group, causal, window, cap, order, p.max_parts);
+      if (p.entries == 0 || workspace == nullptr || workspace_bytes < (long long)B * Hkv * num_kt * p.max_parts * 2 * BKV * HD * 4)
+        return b200::fail(613, "attn_bwd: cap %d and %lld bytes are not the plan of this shape", cap, workspace_bytes);
+      for (int i = 0; i < p.entries; ++i) p.order[i] = order[i].second;
+    } catch (const std::exception& e) {
+      return b200::fail(614, "attn_bwd: %s", e.what());
+    }
+    p.cap = cap;
+  }
+  if ((r = HD == 128 ? launch_bwd<128>(m, p, (cudaStream_t)stream) : launch_bwd<64>(m, p, (cudaStream_t)stream)) || p.cap == 0) return r;
+  auto fin = HD == 128 ? attn_bwd_finish_kernel<128> : attn_bwd_finish_kernel<64>;
+  fin<<<dim3((unsigned)(B * Hkv * num_kt), HD / 16), 256, 0, (cudaStream_t)stream>>>(
+      p.partial, cap, p.max_parts, Hkv, Sq, Skv, group, causal, window, num_kt, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, dk_row, dv_row, dk_batch, dv_batch);
+  b200::count_launch();
+  return b200::check_launch("attn_bwd_finish");
 }

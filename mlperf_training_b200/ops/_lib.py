@@ -133,7 +133,8 @@ def _declare(lib: ctypes.CDLL) -> None:
         "b200_rowwise_adagrad": [P, P, P, P, L, I, F, F, L, P],
         "b200_segment_sum_rows": [P, P, L, I, P, P],
         "b200_attn_delta": [P, P, P, I, I, I, I, L, L, L, L, P],
-        "b200_attn_bwd": [P] * 9 + [I] * 6 + [L] * 12 + [F, I, I, P],
+        "b200_attn_bwd": [P] * 9 + [I] * 6 + [L] * 12 + [F, I, I, I, P, L, P],
+        "b200_attn_bwd_plan": [I] * 8 + [P],
     }
     codes = {P: "P", I: "I", L: "L", F: "F", ctypes.c_ulonglong: "U"}
     table = {}
@@ -266,6 +267,21 @@ def gemm_workspace(entry: str, M: int, N: int, K: int, device: torch.device) -> 
     calling stream, so it is given back when the call returns and reused in stream order."""
     n = _gemm_workspace_bytes(entry, M, N, K, device.index if device.index is not None else torch._C._cuda_getDevice())
     return torch.empty(n, dtype=torch.uint8, device=device) if n else None
+
+
+@functools.lru_cache(maxsize=4096)
+def _attn_bwd_plan(shape: tuple, device: int) -> tuple:
+    out = (ctypes.c_longlong * 2)()
+    with torch.cuda.device(device):
+        load().b200_attn_bwd_plan(*shape, out)
+    return int(out[0]), int(out[1])
+
+
+def attn_bwd_plan(shape: tuple, device: torch.device) -> tuple:
+    """(cap, scratch on the calling stream) of an attention backward whose longest key tiles are shared by several CTAs; (0, None):
+    they are not.  ``shape``: (B, Sq, Skv, Hq, Hkv, D, causal, window)."""
+    cap, n = _attn_bwd_plan(shape, device.index if device.index is not None else torch._C._cuda_getDevice())
+    return cap, torch.empty(n, dtype=torch.uint8, device=device) if cap else None
 
 
 def launch_count() -> int:

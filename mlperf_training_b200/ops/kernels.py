@@ -519,10 +519,11 @@ def attention_bwd(dout, q, k, v, out, lse, *, scale: float | None = None, causal
     dq = torch.zeros((B, Sq, Hq, D), dtype=torch.float32, device=q.device)
     dk = dk_out if dk_out is not None else torch.empty((B, Skv, Hkv, D), dtype=k.dtype, device=k.device)
     dv = dv_out if dv_out is not None else torch.empty((B, Skv, Hkv, D), dtype=v.dtype, device=v.device)
+    cap, ws = _lib.attn_bwd_plan((B, Sq, Skv, Hq, Hkv, D, int(causal), int(window)), q.device)
     call("b200_attn_bwd", ptr(q), ptr(k), ptr(v), ptr(dout), ptr(lse), ptr(delta), ptr(dq), ptr(dk), ptr(dv), B, Sq,
          Skv, Hq, Hkv, D, q.stride(1), k.stride(1), v.stride(1), dout.stride(1), dk.stride(1), dv.stride(1),
          q.stride(0), k.stride(0), v.stride(0), dout.stride(0), dk.stride(0), dv.stride(0), float(scale),
-         int(causal), int(window), stream_ptr())
+         int(causal), int(window), cap, ptr(ws), 0 if ws is None else ws.numel(), stream_ptr())
     dsink = None
     if sink is not None:
         # d/dsink of the extra softmax column: -sum_rows exp(sink - lse) * delta

@@ -80,3 +80,22 @@ def test_attention_packed_qkv_views():
     o_ref, _ = kernels.attention_reference(q, k, v, scale=1 / math.sqrt(D), causal=True)
     assert (o.float() - o_ref).abs().max().item() < 2e-2
     _lib.check_status("attn packed")
+
+
+@pytest.mark.parametrize("B,S,Hq,Hkv,D,causal,window", [(1, 530, 16, 2, 64, True, 0), (2, 700, 8, 1, 128, True, 0), (1, 1000, 16, 4, 64, False, 0),
+                                                        (1, 900, 16, 2, 128, True, 200), (1, 1500, 32, 8, 128, True, 0)])
+def test_attention_bwd_with_shared_key_tiles(monkeypatch, B, S, Hq, Hkv, D, causal, window):
+    """Key tiles whose steps several CTAs share (few tiles on many SMs) against one CTA per tile: the same products in another
+    order of fp32 additions."""
+    q, k, v = _mk(B, S, S, Hq, Hkv, D, S)
+    do = torch.randn(B, S, Hq, D, device="cuda").bfloat16()
+    o, lse = kernels.attention_fwd(q, k, v, causal=causal, window=window)
+    assert _lib.attn_bwd_plan((B, S, S, Hq, Hkv, D, int(causal), window), q.device)[0] > 0
+    shared = kernels.attention_bwd(do, q, k, v, o, lse, causal=causal, window=window)
+    monkeypatch.setattr(_lib, "attn_bwd_plan", lambda *a: (0, None))
+    alone = kernels.attention_bwd(do, q, k, v, o, lse, causal=causal, window=window)
+    _lib.check_status("attn bwd shared")
+    for a, b in zip(shared[:3], alone[:3]):
+        a, b = a.float(), b.float()
+        # fp32 sums of at most 16 terms of 128 products each in another order, then one rounding to bf16 (dK, dV)
+        assert ((a - b).abs() <= b.abs() * 2 ** -7 + 2 ** -15 * b.abs().max()).all()

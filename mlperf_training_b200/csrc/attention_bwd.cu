@@ -115,6 +115,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                 const __grid_constant__ CUtensorMap tmdQ, const __grid_constant__ CUtensorMap tmdK,
                 const __grid_constant__ CUtensorMap tmdV, const __grid_constant__ BwdParams p) {
+  b200::begin_kernel();
   using SM = Smem<HD>;
   constexpr int NB = HD / 64;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -516,6 +517,7 @@ template <int HD>
 __global__ void __launch_bounds__(256)
 attn_bwd_finish_kernel(const float* __restrict__ partial, int cap, int max_parts, int Hkv, int Sq, int Skv, int group, int causal, int window, int num_kt,
                        __nv_bfloat16* dk, __nv_bfloat16* dv, long long dk_row, long long dv_row, long long dk_batch, long long dv_batch) {
+  b200::begin_kernel();
   constexpr int VPR = HD / 8;
   const int bh = (int)blockIdx.x / num_kt, jt = (int)blockIdx.x - bh * num_kt;
   int i_lo, i_hi;
@@ -611,6 +613,7 @@ template <int HD, bool VEC>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout, float* __restrict__ delta, int B, int S,
                   int H, long long o_row, long long do_row, long long o_batch, long long do_batch) {
+  b200::begin_kernel();
   constexpr int LANES = HD / 8;
   const long long w = (blockIdx.x * 256ll + threadIdx.x) / LANES;
   const int l = threadIdx.x % LANES;
@@ -667,7 +670,7 @@ int launch_bwd(const CUtensorMap* m, const BwdParams& p, cudaStream_t stream) {
   }
   const long long grid = (long long)(p.cap > 0 ? p.entries : (p.Skv + BKV - 1) / BKV) * p.Hkv * p.B;
   if (grid > 0x7fffffff) return b200::fail(612, "attn_bwd: %lld key tiles are too many", grid);
-  attn_bwd_kernel<HD><<<(unsigned)grid, NTHREADS, SM::TOTAL, stream>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], p);
+  b200::launch(attn_bwd_kernel<HD>, (unsigned)grid, NTHREADS, SM::TOTAL, stream, m[0], m[1], m[2], m[3], m[4], m[5], m[6], p);
   b200::count_launch();
   return b200::check_launch("attn_bwd");
 }
@@ -684,7 +687,7 @@ B200_API int b200_attn_delta(const void* o, const void* dout, float* delta, int 
   const unsigned blocks = (unsigned)((rows * (HD / 8) + 255) / 256);
   auto fn = HD == 128 ? (vec ? attn_delta_kernel<128, true> : attn_delta_kernel<128, false>)
                       : (vec ? attn_delta_kernel<64, true> : attn_delta_kernel<64, false>);
-  fn<<<blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, S, H, o_row, do_row, o_batch,
+  b200::launch(fn, blocks, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, S, H, o_row, do_row, o_batch,
                                                do_batch);
   b200::count_launch();
   return b200::check_launch("attn_delta");
@@ -753,7 +756,7 @@ B200_API int b200_attn_bwd(const void* q, const void* k, const void* v, const vo
   }
   if ((r = HD == 128 ? launch_bwd<128>(m, p, (cudaStream_t)stream) : launch_bwd<64>(m, p, (cudaStream_t)stream)) || p.cap == 0) return r;
   auto fin = HD == 128 ? attn_bwd_finish_kernel<128> : attn_bwd_finish_kernel<64>;
-  fin<<<dim3((unsigned)(B * Hkv * num_kt), HD / 16), 256, 0, (cudaStream_t)stream>>>(
+  b200::launch(fin, dim3((unsigned)(B * Hkv * num_kt), HD / 16), 256, 0, (cudaStream_t)stream, 
       p.partial, cap, p.max_parts, Hkv, Sq, Skv, group, causal, window, num_kt, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, dk_row, dv_row, dk_batch, dv_batch);
   b200::count_launch();
   return b200::check_launch("attn_bwd_finish");

@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                 const FwdParams p) {
+  b200::begin_kernel();
   using SM = Smem<HD>;
   constexpr int NB = HD / 64;  // 64-column (128-byte) blocks per head row
   extern __shared__ uint8_t smem_raw[];
@@ -485,7 +486,7 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     configured[dev & 63] = true;
   }
   const int grid = p.items < b200::sm_count() ? p.items : b200::sm_count();
-  attn_fwd_kernel<HD><<<grid, NTHREADS, SM::TOTAL, stream>>>(tq, tk, tv, to, p);
+  b200::launch(attn_fwd_kernel<HD>, grid, NTHREADS, SM::TOTAL, stream, tq, tk, tv, to, p);
   b200::count_launch();
   return b200::check_launch("attn_fwd");
 }

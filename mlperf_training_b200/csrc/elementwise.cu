@@ -30,6 +30,7 @@ B200_DEVICE void st8(__nv_bfloat16* p, const float (&f)[8]) {
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ buf, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, const int* __restrict__ pos, long long T, int S,
                             long long row_stride, int col0, int n_heads, int hd, float sign) {
+  b200::begin_kernel();
   const int half = hd / 2;
   const int vec_per_head = half / 8;  // each work item rotates 8 pairs
   const long long total = T * n_heads * vec_per_head;
@@ -69,6 +70,7 @@ template <typename I>
 __global__ void __launch_bounds__(256)
 rope_grad_kernel(const float* __restrict__ dq, __nv_bfloat16* __restrict__ buf, const float* __restrict__ cos_t,
                  const float* __restrict__ sin_t, I total, int S, long long row_stride, I hq, I heads, int hd) {
+  b200::begin_kernel();
   const int half = hd / 2;
   const I vec_per_head = half / 8, per_row = heads * vec_per_head;
   for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
@@ -131,6 +133,7 @@ B200_DEVICE void swiglu_grad_vec(const __nv_bfloat16* g_in, const __nv_bfloat16*
 template <typename I>
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ a, I T,
                   int F) {
+  b200::begin_kernel();
   const I vpr = F / 8, total = T * vpr;
   for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
     const long long t = i / vpr;
@@ -141,6 +144,7 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __
 template <typename I>
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ da, const __nv_bfloat16* __restrict__ gu,
                                   __nv_bfloat16* __restrict__ dgu, I T, int F) {
+  b200::begin_kernel();
   const I vpr = F / 8, total = T * vpr;
   for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
     const long long t = i / vpr;
@@ -156,6 +160,7 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __
 __global__ void __launch_bounds__(256)
 swiglu_tiles_kernel(const __nv_bfloat16* __restrict__ da, const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, int F,
                     const int* __restrict__ tile_expert, const int* __restrict__ seg, const int* __restrict__ counts) {
+  b200::begin_kernel();
   const int tile = blockIdx.y, e = tile_expert[tile];
   if (e < 0) return;
   const int n = min(256, (seg[e] + counts[e] - tile * 256 + 63) / 64 * 64), vpr = F / 8;
@@ -184,6 +189,7 @@ B200_DEVICE float gelu_tanh_grad(float x) {
 template <typename I>
 __global__ void __launch_bounds__(256) gelu_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, __nv_bfloat16* __restrict__ y, long long ldy,
                                 I total, I vpr) {
+  b200::begin_kernel();
   for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
     const long long r = i / vpr, c = (long long)(i - (I)r * vpr) * 8;
     float a[8], o[8];
@@ -196,6 +202,7 @@ __global__ void __launch_bounds__(256) gelu_fwd_kernel(const __nv_bfloat16* __re
 template <typename I>
 __global__ void __launch_bounds__(256) gelu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, long long ldg, const __nv_bfloat16* __restrict__ x, long long ldx,
                                 __nv_bfloat16* __restrict__ dx, long long ldd, I total, I vpr) {
+  b200::begin_kernel();
   for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
     const long long r = i / vpr, c = (long long)(i - (I)r * vpr) * 8;
     float a[8], d[8], o[8];
@@ -212,6 +219,7 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(const __nv_bfloat16* __re
 // ---------------------------------------------------------------------------------------
 __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ table, const long long* __restrict__ ids,
                                    __nv_bfloat16* __restrict__ out, long long T, int D, long long rows, int* status) {
+  b200::begin_kernel();
   const int vpr = D / 8;
   const long long total = T * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -228,6 +236,7 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ table, cons
 // grad_table[ids[t], :] += dy[t, :]  (fp32 atomics; used for the vocabulary embedding)
 __global__ void scatter_add_rows_kernel(const __nv_bfloat16* __restrict__ dy, const long long* __restrict__ ids,
                                         float* __restrict__ grad, long long T, int D, long long rows, int* status) {
+  b200::begin_kernel();
   const int vpr = D / 8;
   const long long total = T * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -255,6 +264,7 @@ __global__ void scatter_add_rows_kernel(const __nv_bfloat16* __restrict__ dy, co
 // y = a + b (bf16)
 __global__ void add_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                                 __nv_bfloat16* __restrict__ y, long long n8) {
+  b200::begin_kernel();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
     float x[8], z[8];
     ld8(a + i * 8, x);
@@ -266,6 +276,7 @@ __global__ void add_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_
 }
 // acc(fp32) += src(bf16)
 __global__ void accum_f32_bf16_kernel(float* __restrict__ acc, const __nv_bfloat16* __restrict__ src, long long n8) {
+  b200::begin_kernel();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
     float x[8];
     ld8(src + i * 8, x);
@@ -297,7 +308,7 @@ B200_API int b200_rope(void* buf, const float* cos_t, const float* sin_t, const 
     return b200::fail(400, "rope: head dim %d must be a multiple of 16, stride/offset multiples of 8", hd);
   const long long work = T * n_heads * (hd / 16);
   if (work == 0) return 0;
-  rope_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)buf, cos_t, sin_t, pos, T, S,
+  b200::launch(rope_kernel, grid_for(work, 256), 256, 0, (cudaStream_t)stream, (__nv_bfloat16*)buf, cos_t, sin_t, pos, T, S,
                                                                      row_stride, col0, n_heads, hd,
                                                                      backward ? -1.f : 1.f);
   b200::count_launch();
@@ -311,10 +322,10 @@ B200_API int b200_rope_grad(const float* dq, void* buf, const float* cos_t, cons
   const long long work = T * (hq + hkv) * (hd / 16);
   if (work == 0) return 0;
   if (fits32(work))
-    rope_grad_kernel<uint32_t><<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
+    b200::launch(rope_grad_kernel<uint32_t>, grid_for(work, 256), 256, 0, (cudaStream_t)stream, 
         dq, (__nv_bfloat16*)buf, cos_t, sin_t, (uint32_t)work, S, row_stride, (uint32_t)hq, (uint32_t)(hq + hkv), hd);
   else
-    rope_grad_kernel<long long><<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
+    b200::launch(rope_grad_kernel<long long>, grid_for(work, 256), 256, 0, (cudaStream_t)stream, 
         dq, (__nv_bfloat16*)buf, cos_t, sin_t, work, S, row_stride, hq, hq + hkv, hd);
   b200::count_launch();
   return b200::check_launch("rope_grad");
@@ -323,8 +334,8 @@ B200_API int b200_swiglu_fwd(const void* gu, void* a, long long T, int F, void* 
   if (F % 8 != 0) return b200::fail(401, "swiglu: F=%d must be a multiple of 8", F);
   if (T == 0) return 0;
   const long long work = T * (F / 8);
-  if (fits32(work)) swiglu_fwd_kernel<uint32_t><<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)a, (uint32_t)T, F);
-  else swiglu_fwd_kernel<long long><<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)a, T, F);
+  if (fits32(work)) b200::launch(swiglu_fwd_kernel<uint32_t>, grid_for(work, 256), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)gu, (__nv_bfloat16*)a, (uint32_t)T, F);
+  else b200::launch(swiglu_fwd_kernel<long long>, grid_for(work, 256), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)gu, (__nv_bfloat16*)a, T, F);
   b200::count_launch();
   return b200::check_launch("swiglu_fwd");
 }
@@ -333,26 +344,26 @@ B200_API int b200_swiglu_bwd(const void* da, const void* gu, void* dgu, long lon
   if (T == 0) return 0;
   const long long work = T * (F / 8);
   if (fits32(work))
-    swiglu_bwd_kernel<uint32_t><<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
+    b200::launch(swiglu_bwd_kernel<uint32_t>, grid_for(work, 256), 256, 0, (cudaStream_t)stream, 
         (const __nv_bfloat16*)da, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, (uint32_t)T, F);
   else
-    swiglu_bwd_kernel<long long><<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
+    b200::launch(swiglu_bwd_kernel<long long>, grid_for(work, 256), 256, 0, (cudaStream_t)stream, 
         (const __nv_bfloat16*)da, (const __nv_bfloat16*)gu, (__nv_bfloat16*)dgu, T, F);
   b200::count_launch();
   return b200::check_launch("swiglu_bwd");
 }
 static void run_gelu_fwd(const void* x, long long ldx, void* y, long long ldy, long long work, long long vpr, cudaStream_t st) {
-  if (fits32(work)) gelu_fwd_kernel<uint32_t><<<grid_for(work, 256), 256, 0, st>>>((const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)y, ldy, (uint32_t)work, (uint32_t)vpr);
-  else gelu_fwd_kernel<long long><<<grid_for(work, 256), 256, 0, st>>>((const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)y, ldy, work, vpr);
+  if (fits32(work)) b200::launch(gelu_fwd_kernel<uint32_t>, grid_for(work, 256), 256, 0, st, (const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)y, ldy, (uint32_t)work, (uint32_t)vpr);
+  else b200::launch(gelu_fwd_kernel<long long>, grid_for(work, 256), 256, 0, st, (const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)y, ldy, work, vpr);
   b200::count_launch();
 }
 static void run_gelu_bwd(const void* dy, long long ldg, const void* x, long long ldx, void* dx, long long ldd, long long work, long long vpr,
                          cudaStream_t st) {
   if (fits32(work))
-    gelu_bwd_kernel<uint32_t><<<grid_for(work, 256), 256, 0, st>>>((const __nv_bfloat16*)dy, ldg, (const __nv_bfloat16*)x, ldx,
+    b200::launch(gelu_bwd_kernel<uint32_t>, grid_for(work, 256), 256, 0, st, (const __nv_bfloat16*)dy, ldg, (const __nv_bfloat16*)x, ldx,
                                                                    (__nv_bfloat16*)dx, ldd, (uint32_t)work, (uint32_t)vpr);
   else
-    gelu_bwd_kernel<long long><<<grid_for(work, 256), 256, 0, st>>>((const __nv_bfloat16*)dy, ldg, (const __nv_bfloat16*)x, ldx,
+    b200::launch(gelu_bwd_kernel<long long>, grid_for(work, 256), 256, 0, st, (const __nv_bfloat16*)dy, ldg, (const __nv_bfloat16*)x, ldx,
                                                                     (__nv_bfloat16*)dx, ldd, work, vpr);
   b200::count_launch();
 }
@@ -374,7 +385,7 @@ B200_API int b200_swiglu_tiles(const void* da, const void* gu, void* out, int F,
   if (F % 8 != 0) return b200::fail(401, "swiglu: F=%d must be a multiple of 8", F);
   if (n_tiles <= 0 || F <= 0) return 0;
   if (n_tiles > 65535) return b200::fail(407, "swiglu_tiles: %d tiles are too many", n_tiles);
-  swiglu_tiles_kernel<<<dim3(32, n_tiles), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)da, (const __nv_bfloat16*)gu,
+  b200::launch(swiglu_tiles_kernel, dim3(32, n_tiles), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)da, (const __nv_bfloat16*)gu,
                                                                            (__nv_bfloat16*)out, F, tile_expert, seg, counts);
   b200::count_launch();
   return b200::check_launch("swiglu_tiles");
@@ -383,7 +394,7 @@ B200_API int b200_gather_rows(const void* table, const long long* ids, void* out
                               void* stream) {
   if (D % 8 != 0) return b200::fail(403, "gather_rows: D=%d must be a multiple of 8", D);
   if (T == 0) return 0;
-  gather_rows_kernel<<<grid_for(T * (D / 8), 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)table, ids,
+  b200::launch(gather_rows_kernel, grid_for(T * (D / 8), 256), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)table, ids,
                                                                                   (__nv_bfloat16*)out, T, D, rows, b200::status_ptr());
   b200::count_launch();
   return b200::check_launch("gather_rows");
@@ -392,7 +403,7 @@ B200_API int b200_scatter_add_rows(const void* dy, const long long* ids, float* 
                                    long long rows, void* stream) {
   if (D % 8 != 0) return b200::fail(403, "scatter_add_rows: D=%d must be a multiple of 8", D);
   if (T == 0) return 0;
-  scatter_add_rows_kernel<<<grid_for(T * (D / 8), 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dy, ids,
+  b200::launch(scatter_add_rows_kernel, grid_for(T * (D / 8), 256), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)dy, ids,
                                                                                        grad, T, D, rows, b200::status_ptr());
   b200::count_launch();
   return b200::check_launch("scatter_add_rows");
@@ -400,7 +411,7 @@ B200_API int b200_scatter_add_rows(const void* dy, const long long* ids, float* 
 B200_API int b200_add_bf16(const void* a, const void* b, void* y, long long n, void* stream) {
   if (n % 8 != 0) return b200::fail(404, "add_bf16: n=%lld must be a multiple of 8", n);
   if (n == 0) return 0;
-  add_bf16_kernel<<<grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
+  b200::launch(add_bf16_kernel, grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
                                                                          (__nv_bfloat16*)y, n / 8);
   b200::count_launch();
   return b200::check_launch("add_bf16");
@@ -408,7 +419,7 @@ B200_API int b200_add_bf16(const void* a, const void* b, void* y, long long n, v
 B200_API int b200_accum_f32_bf16(float* acc, const void* src, long long n, void* stream) {
   if (n % 8 != 0) return b200::fail(405, "accum: n=%lld must be a multiple of 8", n);
   if (n == 0) return 0;
-  accum_f32_bf16_kernel<<<grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>(acc, (const __nv_bfloat16*)src, n / 8);
+  b200::launch(accum_f32_bf16_kernel, grid_for(n / 8, 256), 256, 0, (cudaStream_t)stream, acc, (const __nv_bfloat16*)src, n / 8);
   b200::count_launch();
   return b200::check_launch("accum_f32_bf16");
 }

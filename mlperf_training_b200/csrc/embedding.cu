@@ -49,6 +49,7 @@ __global__ void gather_rows_to_peers_kernel(const __nv_bfloat16* __restrict__ ta
 __global__ void rowwise_adagrad_kernel(__nv_bfloat16* __restrict__ table, float* __restrict__ state,
                                        const long long* __restrict__ ids, const float* __restrict__ grads, long long n,
                                        int D, float lr, float eps, long long rows, int* status) {
+  b200::begin_kernel();
   const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= n) return;
@@ -71,6 +72,7 @@ __global__ void rowwise_adagrad_kernel(__nv_bfloat16* __restrict__ table, float*
 // out[s, :] = sum of src[seg[s] .. seg[s+1], :] in index order (src rows sorted by key)
 __global__ void segment_sum_rows_kernel(const __nv_bfloat16* __restrict__ src, const long long* __restrict__ seg,
                                         long long n_seg, int D, float* __restrict__ out) {
+  b200::begin_kernel();
   const long long s = blockIdx.x;
   if (s >= n_seg) return;
   const long long lo = seg[s], hi = seg[s + 1];
@@ -106,7 +108,7 @@ B200_API int b200_rowwise_adagrad(void* table, float* state, const long long* id
                                   int D, float lr, float eps, long long rows, void* stream) {
   if (n <= 0) return 0;
   const long long threads = n * 32;
-  rowwise_adagrad_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+  b200::launch(rowwise_adagrad_kernel, (unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream, 
       (__nv_bfloat16*)table, state, ids, grads, n, D, lr, eps, rows, b200::status_ptr());
   b200::count_launch();
   return b200::check_launch("rowwise_adagrad");
@@ -114,7 +116,7 @@ B200_API int b200_rowwise_adagrad(void* table, float* state, const long long* id
 
 B200_API int b200_segment_sum_rows(const void* src, const long long* seg, long long n_seg, int D, float* out, void* stream) {
   if (n_seg <= 0) return 0;
-  segment_sum_rows_kernel<<<(unsigned)n_seg, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)src, seg, n_seg, D, out);
+  b200::launch(segment_sum_rows_kernel, (unsigned)n_seg, 128, 0, (cudaStream_t)stream, (const __nv_bfloat16*)src, seg, n_seg, D, out);
   b200::count_launch();
   return b200::check_launch("segment_sum_rows");
 }

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(256)
 ln_modulate_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ shift,
                        const __nv_bfloat16* __restrict__ scale, long long ld_mod, __nv_bfloat16* __restrict__ y,
                        float* __restrict__ mean_out, float* __restrict__ rstd_out, int T, int D, int S, float eps) {
+  b200::begin_kernel();
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= T) return;
   const int lane = threadIdx.x & 31;
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(256)
 ln_modulate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                        const __nv_bfloat16* __restrict__ scale, long long ld_mod, const float* __restrict__ mean_in,
                        const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx, int T, int D, int S) {
+  b200::begin_kernel();
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (row >= T) return;
   const int lane = threadIdx.x & 31;
@@ -131,6 +133,7 @@ __global__ void __launch_bounds__(256)
 sample_colsum_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, float* __restrict__ out_a,
                      float* __restrict__ out_b, int D, int S) {
+  b200::begin_kernel();
   namespace cg = cooperative_groups;
   __shared__ float sm[MODE == 0 ? 2 : 1][8][128];
   cg::cluster_group cluster = cg::this_cluster();
@@ -184,6 +187,7 @@ template <int BWD>
 __global__ void __launch_bounds__(256)
 gate_kernel(const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ gate,
             long long ld_mod, __nv_bfloat16* __restrict__ out, long long n8, int D8, int S) {
+  b200::begin_kernel();
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n8; i += (long long)gridDim.x * 256) {
     const long long row = i / D8;
     const int cv = (int)(i - row * D8);
@@ -242,7 +246,7 @@ int check_shapes(const char* what, int T, int D, int S, long long ld_mod, const 
 B200_API int b200_ln_modulate_fwd(const void* x, const void* shift, const void* scale, long long ld_mod, void* y, float* mean,
                                   float* rstd, int T, int D, int S, float eps, void* stream) {
   if (int r = check_shapes("ln_modulate_fwd", T, D, S, ld_mod, shift, scale)) return r;
-  ln_modulate_fwd_kernel<<<(T + 7) / 8, 256, 0, (cudaStream_t)stream>>>(
+  b200::launch(ln_modulate_fwd_kernel, (T + 7) / 8, 256, 0, (cudaStream_t)stream, 
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)shift, (const __nv_bfloat16*)scale, ld_mod, (__nv_bfloat16*)y, mean, rstd,
       T, D, S, eps);
   b200::count_launch();
@@ -253,7 +257,7 @@ B200_API int b200_ln_modulate_fwd(const void* x, const void* shift, const void* 
 B200_API int b200_ln_modulate_bwd(const void* dy, const void* x, const void* scale, long long ld_mod, const float* mean,
                                   const float* rstd, void* dx, float* dscale, float* dshift, int T, int D, int S, void* stream) {
   if (int r = check_shapes("ln_modulate_bwd", T, D, S, ld_mod, scale, scale)) return r;
-  ln_modulate_bwd_kernel<<<(T + 7) / 8, 256, 0, (cudaStream_t)stream>>>(
+  b200::launch(ln_modulate_bwd_kernel, (T + 7) / 8, 256, 0, (cudaStream_t)stream, 
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)scale, ld_mod, mean, rstd, (__nv_bfloat16*)dx, T, D, S);
   if (int r = launch_colsum<0>(dy, x, mean, rstd, dscale, dshift, T / S, D, S, (cudaStream_t)stream)) return r;
   b200::count_launch(2);
@@ -266,7 +270,7 @@ B200_API int b200_gate_residual_fwd(const void* res, const void* y, const void* 
   if (int r = check_shapes("gate_residual_fwd", T, D, S, ld_mod, gate, gate)) return r;
   const long long n8 = (long long)T * D / 8;
   const int grid = (int)((n8 + 255) / 256 < 148 * 16 ? (n8 + 255) / 256 : 148 * 16);
-  gate_kernel<0><<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)res, (const __nv_bfloat16*)y,
+  b200::launch(gate_kernel<0>, grid, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)res, (const __nv_bfloat16*)y,
                                                          (const __nv_bfloat16*)gate, ld_mod, (__nv_bfloat16*)out, n8, D / 8, S);
   b200::count_launch();
   return b200::check_launch("gate_residual_fwd");
@@ -278,7 +282,7 @@ B200_API int b200_gate_residual_bwd(const void* dout, const void* y, const void*
   if (int r = check_shapes("gate_residual_bwd", T, D, S, ld_mod, gate, gate)) return r;
   const long long n8 = (long long)T * D / 8;
   const int grid = (int)((n8 + 255) / 256 < 148 * 16 ? (n8 + 255) / 256 : 148 * 16);
-  gate_kernel<1><<<grid, 256, 0, (cudaStream_t)stream>>>(nullptr, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)gate, ld_mod,
+  b200::launch(gate_kernel<1>, grid, 256, 0, (cudaStream_t)stream, nullptr, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)gate, ld_mod,
                                                          (__nv_bfloat16*)dy, n8, D / 8, S);
   if (int r = launch_colsum<1>(dout, y, nullptr, nullptr, dgate, nullptr, T / S, D, S, (cudaStream_t)stream)) return r;
   b200::count_launch(2);

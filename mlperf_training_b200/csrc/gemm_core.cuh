@@ -518,6 +518,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmDt,
                  const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmWt,
                  const __grid_constant__ PairParams p, const __grid_constant__ OwnerMaps<NOWN> om) {
+  b200::begin_kernel();
   using C = PairCfg<KIND, BN, KSUB>;
   constexpr bool MX = C::MX;
   constexpr bool F8 = (KIND == KIND_FP8);
@@ -837,6 +838,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 template <int BN>
 __global__ void __launch_bounds__(256)
 split_finish_kernel(const float* __restrict__ ws, SplitArgs sp, int num_m, int num_n, int group_m, EpiArgs e, void* d, long long ldd) {
+  b200::begin_kernel();
   constexpr int VPR = BN / 8;
   const int i = blockIdx.y;
   int mb, nb;
@@ -990,9 +992,14 @@ int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMa
   const int room = max_pairs - n_aux;
   const int pairs = (units < room ? units : room) + n_aux;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   pair_launch_config<KIND, BN, KSUB>(cfg, attr, stream);
   cfg.gridDim = dim3(2 * pairs, 1, 1);
+  if (!p.tp.on && !p.rs.on) {     // a launch that waits for other GPUs is ordered as before
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
+  }
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmSFA, tmSFB, tmD, tmDt, tmW, tmWt, p, om);
   b200::count_launch();
   if (e != cudaSuccess) {
@@ -1001,7 +1008,7 @@ int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMa
   }
   if ((rc = b200::check_launch(what)) || p.split.rem == 0) return rc;
   // 256 x BN / 8 vectors per tile: enough CTAs for the whole chip whatever the number of tiles
-  split_finish_kernel<BN><<<dim3(BN / 8, p.split.rem), 256, 0, stream>>>(ws, p.split, num_m, num_n, p.group_m, p.epi, d, ldd);
+  b200::launch(split_finish_kernel<BN>, dim3(BN / 8, p.split.rem), 256, 0, stream, ws, p.split, num_m, num_n, p.group_m, p.epi, d, ldd);
   b200::count_launch();
   return b200::check_launch("split_finish");
 }

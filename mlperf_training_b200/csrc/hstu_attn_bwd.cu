@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 hstu_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                 const __grid_constant__ CUtensorMap tmdQ, const HstuBwdParams p) {
+  b200::begin_kernel();
   using SM = Smem<HD>;
   constexpr int NB = HD / 64;
   extern __shared__ uint8_t smem_raw[];
@@ -417,7 +418,7 @@ int launch_hstu_bwd(const CUtensorMap* m, const HstuBwdParams& p, cudaStream_t s
   }
   const long long grid = (long long)p.num_bh * p.num_kt;
   if (grid > 0x7fffffff) return b200::fail(1212, "hstu_attn_bwd: %lld key tiles are too many", grid);
-  hstu_attn_bwd_kernel<HD><<<(unsigned)grid, NTHREADS, SM::TOTAL, stream>>>(m[0], m[1], m[2], m[3], m[4], p);
+  b200::launch(hstu_attn_bwd_kernel<HD>, (unsigned)grid, NTHREADS, SM::TOTAL, stream, m[0], m[1], m[2], m[3], m[4], p);
   b200::count_launch();
   return b200::check_launch("hstu_attn_bwd");
 }

@@ -88,6 +88,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 hstu_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV,
                 const HstuParams p) {
+  b200::begin_kernel();
   using SM = Smem<HD, F8>;
   constexpr int EPB = 128 / SM::ES;   // elements per 128-byte block of a head row
   constexpr int NB = HD / EPB;        // 128-byte blocks per head row
@@ -385,7 +386,7 @@ int launch_hstu_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensor
     configured[dev & 63] = true;
   }
   dim3 grid((unsigned)(p.H * B), (p.max_len + 2 * BQ - 1) / (2 * BQ));
-  hstu_attn_fwd_kernel<HD, F8><<<grid, NTHREADS, SM::TOTAL, stream>>>(tq, tk, tv, p);
+  b200::launch(hstu_attn_fwd_kernel<HD, F8>, grid, NTHREADS, SM::TOTAL, stream, tq, tk, tv, p);
   b200::count_launch();
   return b200::check_launch("hstu_attn_fwd");
 }

@@ -65,6 +65,7 @@ gate_cat_fwd_kernel(const __nv_bfloat16* __restrict__ u_raw, long long ld_u, con
                     const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                     __nv_bfloat16* __restrict__ cat, float* __restrict__ mean_out, float* __restrict__ rstd_out, int T,
                     float eps, float p, unsigned thr, unsigned long long seed) {
+  b200::begin_kernel();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int D = NV * 256;
   const float inv_keep = 1.f / (1.f - p);
@@ -148,6 +149,7 @@ gate_cat_bwd_kernel(const __nv_bfloat16* __restrict__ dcat, const __nv_bfloat16*
                     const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ du_raw, long long ld_du,
                     __nv_bfloat16* __restrict__ dattn, float* __restrict__ partial, int T, float p, unsigned thr,
                     unsigned long long seed) {
+  b200::begin_kernel();
   constexpr int D = NV * 256, TEAMS = BwdShape<NV>::TEAMS;
   __shared__ float acc[TEAMS][2][D];
   __shared__ float2 red[TEAMS][2][NV];
@@ -238,6 +240,7 @@ gate_cat_bwd_kernel(const __nv_bfloat16* __restrict__ dcat, const __nv_bfloat16*
 __global__ void __launch_bounds__(256)
 gate_cat_reduce_kernel(const float* __restrict__ partial, int nparts, int D, float* __restrict__ dw, float* __restrict__ db,
                        int accumulate) {
+  b200::begin_kernel();
   __shared__ float sm[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;                    // (D is a multiple of 256)
@@ -260,6 +263,7 @@ gate_cat_reduce_kernel(const float* __restrict__ partial, int nparts, int D, flo
 __global__ void __launch_bounds__(256)
 zero_uncovered_rows_kernel(__nv_bfloat16* __restrict__ buf, const int* __restrict__ offsets, int B, long long L, long long ld, int vpr,
                            long long cover) {
+  b200::begin_kernel();
   long long lo, hi;
   int part = 0, parts = 1;
   if ((int)blockIdx.x < B) {
@@ -282,6 +286,7 @@ zero_uncovered_rows_kernel(__nv_bfloat16* __restrict__ buf, const int* __restric
 template <typename I>
 __global__ void __launch_bounds__(256)
 cast_rows_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, I total, I vpr, long long ld) {
+  b200::begin_kernel();
   for (I i = blockIdx.x * (I)256 + threadIdx.x; i < total; i += (I)gridDim.x * 256) {
     const float4 a = *reinterpret_cast<const float4*>(src + (long long)i * 8), b = *reinterpret_cast<const float4*>(src + (long long)i * 8 + 4);
     const I r = i / vpr;
@@ -318,9 +323,9 @@ B200_API int b200_hstu_gate_cat_fwd(const void* u_raw, long long ld_u, const voi
   auto B = (const __nv_bfloat16*)b; auto C = (__nv_bfloat16*)cat;
   const int grid = gate_grid(T, 8);
   cudaStream_t st = (cudaStream_t)stream;
-  if (D == 256) gate_cat_fwd_kernel<1><<<grid, 256, 0, st>>>(U, ld_u, A, W, B, C, mean, rstd, T, eps, pe, thr, seed);
-  else if (D == 512) gate_cat_fwd_kernel<2><<<grid, 256, 0, st>>>(U, ld_u, A, W, B, C, mean, rstd, T, eps, pe, thr, seed);
-  else gate_cat_fwd_kernel<3><<<grid, 256, 0, st>>>(U, ld_u, A, W, B, C, mean, rstd, T, eps, pe, thr, seed);
+  if (D == 256) b200::launch(gate_cat_fwd_kernel<1>, grid, 256, 0, st, U, ld_u, A, W, B, C, mean, rstd, T, eps, pe, thr, seed);
+  else if (D == 512) b200::launch(gate_cat_fwd_kernel<2>, grid, 256, 0, st, U, ld_u, A, W, B, C, mean, rstd, T, eps, pe, thr, seed);
+  else b200::launch(gate_cat_fwd_kernel<3>, grid, 256, 0, st, U, ld_u, A, W, B, C, mean, rstd, T, eps, pe, thr, seed);
   b200::count_launch();
   return b200::check_launch("hstu_gate_cat_fwd");
 }
@@ -341,12 +346,12 @@ B200_API int b200_hstu_gate_cat_bwd(const void* dcat, const void* u_raw, long lo
   const float pe = (float)thr / 65536.f;
   auto DC = (const __nv_bfloat16*)dcat; auto U = (const __nv_bfloat16*)u_raw; auto A = (const __nv_bfloat16*)attn;
   auto W = (const __nv_bfloat16*)w; auto B = (const __nv_bfloat16*)b; auto DU = (__nv_bfloat16*)du_raw; auto DA = (__nv_bfloat16*)dattn;
-  if (D == 256) gate_cat_bwd_kernel<1><<<grid, BwdShape<1>::THREADS, 0, st>>>(DC, U, ld_u, A, W, B, mean, rstd, DU, ld_du, DA, scratch, T, pe, thr, seed);
-  else if (D == 512) gate_cat_bwd_kernel<2><<<grid, BwdShape<2>::THREADS, 0, st>>>(DC, U, ld_u, A, W, B, mean, rstd, DU, ld_du, DA, scratch, T, pe, thr, seed);
-  else gate_cat_bwd_kernel<3><<<grid, BwdShape<3>::THREADS, 0, st>>>(DC, U, ld_u, A, W, B, mean, rstd, DU, ld_du, DA, scratch, T, pe, thr, seed);
+  if (D == 256) b200::launch(gate_cat_bwd_kernel<1>, grid, BwdShape<1>::THREADS, 0, st, DC, U, ld_u, A, W, B, mean, rstd, DU, ld_du, DA, scratch, T, pe, thr, seed);
+  else if (D == 512) b200::launch(gate_cat_bwd_kernel<2>, grid, BwdShape<2>::THREADS, 0, st, DC, U, ld_u, A, W, B, mean, rstd, DU, ld_du, DA, scratch, T, pe, thr, seed);
+  else b200::launch(gate_cat_bwd_kernel<3>, grid, BwdShape<3>::THREADS, 0, st, DC, U, ld_u, A, W, B, mean, rstd, DU, ld_du, DA, scratch, T, pe, thr, seed);
   b200::count_launch();
   if (int r = b200::check_launch("hstu_gate_cat_bwd")) return r;
-  gate_cat_reduce_kernel<<<2 * D / 32, 256, 0, st>>>(scratch, grid, D, dw, db, accumulate);
+  b200::launch(gate_cat_reduce_kernel, 2 * D / 32, 256, 0, st, scratch, grid, D, dw, db, accumulate);
   b200::count_launch();
   return b200::check_launch("hstu_gate_cat_reduce");
 }
@@ -358,7 +363,7 @@ B200_API int b200_hstu_zero_uncovered(void* buf, const int* offsets, int B, long
   if (width % 8 != 0 || ld % 8 != 0 || ((uintptr_t)buf & 15) != 0)
     return b200::fail(903, "hstu_zero_uncovered: width %d and pitch %lld must be multiples of 8, the base 16-byte aligned", width, ld);
   if (L <= 0 || B <= 0) return 0;
-  zero_uncovered_rows_kernel<<<B + 16, 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)buf, offsets, B, L, ld, width / 8, cover);
+  b200::launch(zero_uncovered_rows_kernel, B + 16, 256, 0, (cudaStream_t)stream, (__nv_bfloat16*)buf, offsets, B, L, ld, width / 8, cover);
   b200::count_launch();
   return b200::check_launch("hstu_zero_uncovered");
 }
@@ -371,8 +376,8 @@ B200_API int b200_cast_rows(const float* src, void* dst, long long rows, int wid
   if (work <= 0) return 0;
   const long long cap = (long long)b200::sm_count() * 16, want = (work + 255) / 256;
   const int grid = (int)(want < cap ? want : cap);
-  if (work < (1ll << 31)) cast_rows_kernel<uint32_t><<<grid, 256, 0, (cudaStream_t)stream>>>(src, (__nv_bfloat16*)dst, (uint32_t)work, (uint32_t)(width / 8), ld);
-  else cast_rows_kernel<long long><<<grid, 256, 0, (cudaStream_t)stream>>>(src, (__nv_bfloat16*)dst, work, width / 8, ld);
+  if (work < (1ll << 31)) b200::launch(cast_rows_kernel<uint32_t>, grid, 256, 0, (cudaStream_t)stream, src, (__nv_bfloat16*)dst, (uint32_t)work, (uint32_t)(width / 8), ld);
+  else b200::launch(cast_rows_kernel<long long>, grid, 256, 0, (cudaStream_t)stream, src, (__nv_bfloat16*)dst, work, width / 8, ld);
   b200::count_launch();
   return b200::check_launch("cast_rows");
 }

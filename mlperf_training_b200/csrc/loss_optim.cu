@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(CE_NT)
 cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels,
                      float* __restrict__ loss, float* __restrict__ lse_out, long long ld, int V, float grad_scale,
                      int write_grad, long long ignore_index) {
+  b200::begin_kernel();
   __shared__ float red_m[CE_NT / 32], red_s[CE_NT / 32];
   __shared__ float sh_m, sh_lse;
   const long long row = blockIdx.x;
@@ -107,6 +108,7 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __rest
 template <typename G>
 __global__ void __launch_bounds__(256)
 sumsq_partial_kernel(const G* __restrict__ g, long long n, float* __restrict__ partial) {
+  b200::begin_kernel();
   __shared__ float red[8];
   // 16-byte loads, four in flight per thread (one 4-byte load at a time read 3.6 TB/s: 525 M fp32 550 -> 335 us)
   constexpr int PER = 16 / sizeof(G);
@@ -149,6 +151,7 @@ sumsq_partial_kernel(const G* __restrict__ g, long long n, float* __restrict__ p
 }
 // out[0] (+)= sum(partial); one CTA
 __global__ void sumsq_final_kernel(const float* __restrict__ partial, int n, float* __restrict__ out, int accumulate) {
+  b200::begin_kernel();
   __shared__ float red[32];
   float acc = 0.f;
   for (int i = threadIdx.x; i < n; i += blockDim.x) acc += partial[i];
@@ -182,6 +185,7 @@ __global__ void __launch_bounds__(256)
 adamw_kernel(P* __restrict__ p, float* __restrict__ master, const G* __restrict__ g, M* __restrict__ m,
              M* __restrict__ v, long long n, AdamArgs a, const float* __restrict__ sumsq, int zero_grad,
              G* __restrict__ g_mut) {
+  b200::begin_kernel();
   float scale = a.grad_scale;
   if (sumsq != nullptr && a.max_norm > 0.f) {
     const float norm = sqrtf(*sumsq) * a.grad_scale;
@@ -232,6 +236,7 @@ template <typename P, typename G, typename M>
 __global__ void __launch_bounds__(256)
 adamw_vec4_kernel(P* __restrict__ p, float* __restrict__ master, G* __restrict__ g, M* __restrict__ m,
                   M* __restrict__ v, long long n4, AdamArgs a, const float* __restrict__ sumsq, int zero_grad) {
+  b200::begin_kernel();
   float scale = a.grad_scale;
   if (sumsq != nullptr && a.max_norm > 0.f) {
     const float norm = sqrtf(*sumsq) * a.grad_scale;
@@ -269,7 +274,7 @@ B200_API int b200_cross_entropy(void* logits, const long long* labels, float* lo
                                 void* stream) {
   if (V % 8 != 0 || ld % 8 != 0) return b200::fail(500, "cross_entropy: V=%d and pitch %lld must be multiples of 8", V, ld);
   if (T == 0) return 0;
-  cross_entropy_kernel<<<(unsigned)T, CE_NT, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)logits, labels, loss, lse, ld, V,
+  b200::launch(cross_entropy_kernel, (unsigned)T, CE_NT, 0, (cudaStream_t)stream, (__nv_bfloat16*)logits, labels, loss, lse, ld, V,
                                                                         grad_scale, write_grad, ignore_index);
   b200::count_launch();
   return b200::check_launch("cross_entropy");
@@ -284,9 +289,9 @@ B200_API int b200_sumsq(const void* g, long long n, int g_is_bf16, float* scratc
   int grid = b200::sm_count() * 4;
   if ((long long)grid * 256 > n) grid = (int)((n + 255) / 256);
   if (grid < 1) grid = 1;
-  if (g_is_bf16) sumsq_partial_kernel<__nv_bfloat16><<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)g, n, scratch);
-  else sumsq_partial_kernel<float><<<grid, 256, 0, (cudaStream_t)stream>>>((const float*)g, n, scratch);
-  sumsq_final_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(scratch, grid, out, accumulate);
+  if (g_is_bf16) b200::launch(sumsq_partial_kernel<__nv_bfloat16>, grid, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)g, n, scratch);
+  else b200::launch(sumsq_partial_kernel<float>, grid, 256, 0, (cudaStream_t)stream, (const float*)g, n, scratch);
+  b200::launch(sumsq_final_kernel, 1, 256, 0, (cudaStream_t)stream, scratch, grid, out, accumulate);
   b200::count_launch(2);
   return b200::check_launch("sumsq");
 }
@@ -308,19 +313,19 @@ static int launch_adamw(void* p, int p_is_bf16, float* master, void* g, int g_is
   if ((all & 15) == 0 && (n & 3) == 0) {
     const long long n4 = n / 4, g4 = (n4 + 255) / 256;
     const int grid4 = (int)(g4 < cap ? g4 : cap);
-    if (p_is_bf16 && g_is_bf16) adamw_vec4_kernel<bf, bf, M><<<grid4, 256, 0, st>>>((bf*)p, master, (bf*)g, m, v, n4, a, sumsq, zero_grad);
-    else if (p_is_bf16) adamw_vec4_kernel<bf, float, M><<<grid4, 256, 0, st>>>((bf*)p, master, (float*)g, m, v, n4, a, sumsq, zero_grad);
-    else if (g_is_bf16) adamw_vec4_kernel<float, bf, M><<<grid4, 256, 0, st>>>((float*)p, master, (bf*)g, m, v, n4, a, sumsq, zero_grad);
-    else adamw_vec4_kernel<float, float, M><<<grid4, 256, 0, st>>>((float*)p, master, (float*)g, m, v, n4, a, sumsq, zero_grad);
+    if (p_is_bf16 && g_is_bf16) b200::launch(adamw_vec4_kernel<bf, bf, M>, grid4, 256, 0, st, (bf*)p, master, (bf*)g, m, v, n4, a, sumsq, zero_grad);
+    else if (p_is_bf16) b200::launch(adamw_vec4_kernel<bf, float, M>, grid4, 256, 0, st, (bf*)p, master, (float*)g, m, v, n4, a, sumsq, zero_grad);
+    else if (g_is_bf16) b200::launch(adamw_vec4_kernel<float, bf, M>, grid4, 256, 0, st, (float*)p, master, (bf*)g, m, v, n4, a, sumsq, zero_grad);
+    else b200::launch(adamw_vec4_kernel<float, float, M>, grid4, 256, 0, st, (float*)p, master, (float*)g, m, v, n4, a, sumsq, zero_grad);
     b200::count_launch();
     return b200::check_launch("adamw");
   }
   const long long g64 = (n + 255) / 256;
   const int grid = (int)(g64 < cap ? g64 : cap);
-  if (p_is_bf16 && g_is_bf16) adamw_kernel<bf, bf, M><<<grid, 256, 0, st>>>((bf*)p, master, (const bf*)g, m, v, n, a, sumsq, zero_grad, (bf*)g);
-  else if (p_is_bf16) adamw_kernel<bf, float, M><<<grid, 256, 0, st>>>((bf*)p, master, (const float*)g, m, v, n, a, sumsq, zero_grad, (float*)g);
-  else if (g_is_bf16) adamw_kernel<float, bf, M><<<grid, 256, 0, st>>>((float*)p, master, (const bf*)g, m, v, n, a, sumsq, zero_grad, (bf*)g);
-  else adamw_kernel<float, float, M><<<grid, 256, 0, st>>>((float*)p, master, (const float*)g, m, v, n, a, sumsq, zero_grad, (float*)g);
+  if (p_is_bf16 && g_is_bf16) b200::launch(adamw_kernel<bf, bf, M>, grid, 256, 0, st, (bf*)p, master, (const bf*)g, m, v, n, a, sumsq, zero_grad, (bf*)g);
+  else if (p_is_bf16) b200::launch(adamw_kernel<bf, float, M>, grid, 256, 0, st, (bf*)p, master, (const float*)g, m, v, n, a, sumsq, zero_grad, (float*)g);
+  else if (g_is_bf16) b200::launch(adamw_kernel<float, bf, M>, grid, 256, 0, st, (float*)p, master, (const bf*)g, m, v, n, a, sumsq, zero_grad, (bf*)g);
+  else b200::launch(adamw_kernel<float, float, M>, grid, 256, 0, st, (float*)p, master, (const float*)g, m, v, n, a, sumsq, zero_grad, (float*)g);
   b200::count_launch();
   return b200::check_launch("adamw");
 }

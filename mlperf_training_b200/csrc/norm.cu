@@ -93,6 +93,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                 __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out, float* __restrict__ mean_out,
                 float* __restrict__ rstd_out, int T, int D, float eps, int act) {
+  b200::begin_kernel();
   __shared__ float red[ROWS * 16];
   const Split<G, ROWS> sp;
   const int nvec = D / 8;
@@ -206,6 +207,7 @@ norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
                      const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                      __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out, float* __restrict__ mean_out,
                      float* __restrict__ rstd_out, int T, int D, float eps, int act) {
+  b200::begin_kernel();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nv = D >> 8;  // vectors per lane
   for (int row = blockIdx.x * 8 + warp; row < T; row += gridDim.x * 8) {
@@ -284,6 +286,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
                 const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                 const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                 float* __restrict__ partial, int T, int D) {
+  b200::begin_kernel();
   constexpr int NACC = (MODE == 1 || ACT) ? 2 : 1;
   constexpr int NS = (MODE == 1) ? 2 * ROWS : ROWS;
   constexpr int TEAMS = (G == 0) ? 1 : NT / (G == 0 ? 1 : G);
@@ -443,6 +446,7 @@ norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                      const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                      float* __restrict__ partial, int T, int D, int nwarps) {
+  b200::begin_kernel();
   extern __shared__ float acc[];  // [nwarps][(MODE == 1 || ACT) ? 2 : 1][D]
   constexpr int NACC = (MODE == 1 || ACT) ? 2 : 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -560,6 +564,7 @@ norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
 __global__ void __launch_bounds__(256)
 norm_bwd_reduce_kernel(const float* __restrict__ partial, int nparts, int D, float* __restrict__ dw,
                        float* __restrict__ db, int accumulate) {
+  b200::begin_kernel();
   __shared__ float sm[8][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane, which = blockIdx.y;
@@ -601,7 +606,7 @@ template <int MODE, int G, int V, int ROWS, int MAXT = NT>
 void run_fwd(const FwdArgs& a) {
   const int per_cta = (G == 0 ? 1 : NT / (G == 0 ? 1 : G)) * ROWS;
   const int need = (a.T + per_cta - 1) / per_cta, cap = b200::sm_count() * 8;
-  norm_fwd_kernel<MODE, G, V, ROWS, MAXT><<<need < cap ? need : cap, G == 0 ? block_threads(a.D, V) : NT, 0, a.st>>>(
+  b200::launch(norm_fwd_kernel<MODE, G, V, ROWS, MAXT>, need < cap ? need : cap, G == 0 ? block_threads(a.D, V) : NT, 0, a.st, 
       a.x, a.res, a.w, a.b, a.y, a.h, a.mean, a.rstd, a.T, a.D, a.eps, a.act);
 }
 
@@ -614,7 +619,7 @@ void dispatch_fwd(const FwdArgs& a) {
   else if (a.D <= 1024) run_fwd<MODE, 32, 4, 1>(a);
   else if (a.D % 256 == 0 && a.D <= 4096) {
     const int need = (a.T + 7) / 8, cap = b200::sm_count() * 8;
-    norm_fwd_warp_kernel<MODE><<<need < cap ? need : cap, 256, 0, a.st>>>(a.x, a.res, a.w, a.b, a.y, a.h, a.mean, a.rstd, a.T,
+    b200::launch(norm_fwd_warp_kernel<MODE>, need < cap ? need : cap, 256, 0, a.st, a.x, a.res, a.w, a.b, a.y, a.h, a.mean, a.rstd, a.T,
                                                                          a.D, a.eps, a.act);
   }
   else if (a.D <= 4096) run_fwd<MODE, 0, 2, 2>(a);
@@ -627,7 +632,7 @@ int run_bwd(const BwdArgs& a) {
   const int need = (a.T + per_cta - 1) / per_cta;
   const int grid = need < a.grid ? need : a.grid;      // never more partial rows than the scratch holds
   const int smem = G == 0 ? 0 : NT / (G == 0 ? 1 : G) * a.D * 4;      // at most 32 KB
-  norm_bwd_kernel<MODE, ACT, G, V, ROWS, MAXT><<<grid, G == 0 ? block_threads(a.D, V) : NT, smem, a.st>>>(
+  b200::launch(norm_bwd_kernel<MODE, ACT, G, V, ROWS, MAXT>, grid, G == 0 ? block_threads(a.D, V) : NT, smem, a.st, 
       a.dy, a.x, a.w, a.b, a.mean, a.rstd, a.dres, a.dx, a.partial, a.T, a.D);
   return grid;
 }
@@ -649,7 +654,7 @@ int run_bwd_warp(const BwdArgs& a) {
     configured[dev & 63] = true;
   }
   const int grid = b200::sm_count() < a.grid ? b200::sm_count() : a.grid;
-  norm_bwd_warp_kernel<MODE, ACT><<<grid, 256, nwarps * nacc * a.D * 4, a.st>>>(a.dy, a.x, a.w, a.b, a.mean, a.rstd, a.dres, a.dx,
+  b200::launch(norm_bwd_warp_kernel<MODE, ACT>, grid, 256, nwarps * nacc * a.D * 4, a.st, a.dy, a.x, a.w, a.b, a.mean, a.rstd, a.dres, a.dx,
                                                                                 a.partial, a.T, a.D, nwarps);
   return grid;
 }
@@ -707,7 +712,7 @@ B200_API int b200_norm_bwd(int mode, const void* dy, const void* x, const void* 
   b200::count_launch();
   if (int r = b200::check_launch("norm_bwd")) return r;
   if (scratch != nullptr && (dw != nullptr || db != nullptr)) {
-    norm_bwd_reduce_kernel<<<dim3((D + 31) / 32, 2), 256, 0, st>>>(scratch, parts, D, dw, db, accumulate);
+    b200::launch(norm_bwd_reduce_kernel, dim3((D + 31) / 32, 2), 256, 0, st, scratch, parts, D, dw, db, accumulate);
     b200::count_launch();
     return b200::check_launch("norm_bwd_reduce");
   }

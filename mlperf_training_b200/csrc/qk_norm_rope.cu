@@ -53,6 +53,7 @@ qk_norm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat
                         const __nv_bfloat16* __restrict__ wk, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                         __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ v,
                         float* __restrict__ rstd, Shape sh, float eps) {
+  b200::begin_kernel();
   constexpr int LANES = D / 8, HALF = D / 2;
   const int l = threadIdx.x % LANES;
   const long long items = (long long)sh.B * sh.S_part * sh.H;
@@ -128,6 +129,7 @@ qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat1
                         const __nv_bfloat16* __restrict__ wq, const __nv_bfloat16* __restrict__ wk,
                         const float* __restrict__ cos_t, const float* __restrict__ sin_t, const float* __restrict__ rstd,
                         __nv_bfloat16* __restrict__ dqkv, long long ld_d, float* __restrict__ partial, Shape sh) {
+  b200::begin_kernel();
   constexpr int LANES = D / 8, HALF = D / 2, TEAMS = NT / LANES;
   __shared__ float acc[TEAMS][D];
   const int l = threadIdx.x % LANES, team = threadIdx.x / LANES;
@@ -208,6 +210,7 @@ qk_norm_rope_bwd_kernel(const __nv_bfloat16* __restrict__ dq, const __nv_bfloat1
 // out[which][c] = sum_p partial[p][which][c] in a fixed order; 32 columns per CTA, a warp takes every eighth row
 __global__ void __launch_bounds__(256)
 scale_grad_kernel(const float* __restrict__ partial, int nparts, int D, float* __restrict__ out) {
+  b200::begin_kernel();
   __shared__ float sm[8][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   float s = 0.f;
@@ -248,7 +251,7 @@ B200_API int b200_qk_norm_rope_fwd(const void* qkv, long long ld, const void* wq
   const int grid = (int)(need < cap ? need : cap);
   auto X = (const __nv_bfloat16*)qkv; auto Q = (const __nv_bfloat16*)wq; auto K = (const __nv_bfloat16*)wk;
   auto fn = D == 128 ? qk_norm_rope_fwd_kernel<128> : qk_norm_rope_fwd_kernel<64>;
-  fn<<<grid, NT, 0, (cudaStream_t)stream>>>(X, Q, K, cos_t, sin_t, (__nv_bfloat16*)q, (__nv_bfloat16*)k, (__nv_bfloat16*)v, rstd, sh, eps);
+  b200::launch(fn, grid, NT, 0, (cudaStream_t)stream, X, Q, K, cos_t, sin_t, (__nv_bfloat16*)q, (__nv_bfloat16*)k, (__nv_bfloat16*)v, rstd, sh, eps);
   b200::count_launch();
   return b200::check_launch("qk_norm_rope_fwd");
 }
@@ -274,9 +277,9 @@ B200_API int b200_qk_norm_rope_bwd(const void* dq, const void* dk, const void* d
   const Shape sh{B, S_part, S_all, s_off, H, ld};
   const int grid = bwd_grid(items, D);
   auto fn = D == 128 ? qk_norm_rope_bwd_kernel<128> : qk_norm_rope_bwd_kernel<64>;
-  fn<<<grid, NT, 0, st>>>((const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, (const __nv_bfloat16*)qkv,
+  b200::launch(fn, grid, NT, 0, st, (const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, (const __nv_bfloat16*)qkv,
                           (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, cos_t, sin_t, rstd, (__nv_bfloat16*)dqkv, ld_d, scratch, sh);
-  scale_grad_kernel<<<dim3(D / 32, 2), 256, 0, st>>>(scratch, grid, D, dscale);
+  b200::launch(scale_grad_kernel, dim3(D / 32, 2), 256, 0, st, scratch, grid, D, dscale);
   b200::count_launch(2);
   return b200::check_launch("qk_norm_rope_bwd");
 }

@@ -147,6 +147,7 @@ struct QuantArgs {
 template <int MODE>
 __global__ void __launch_bounds__(256, 4)
 quant_mxfp8_kernel(const QuantArgs p) {
+  b200::begin_kernel();
   __shared__ __align__(16) uint32_t tile[TILE_WORDS];
   __shared__ __align__(4) uint8_t sfs[2][TILE][4];     // [row pass | column pass][operand row][scale column]
   const int c0 = blockIdx.x * TILE, r0 = blockIdx.y * TILE;
@@ -228,6 +229,7 @@ quant_mxfp8_kernel(const QuantArgs p) {
 // columns past F are neither read nor stored, and the scale bytes past 2F up to a whole word are written as 0.
 __global__ void __launch_bounds__(256, 4)
 quant_swiglu_bwd_kernel(const QuantArgs p) {
+  b200::begin_kernel();
   __shared__ __align__(16) uint32_t tile[TILE_WORDS];
   __shared__ __align__(4) uint8_t sfr[TILE][4];        // row pass: scale columns of d gate (0, 1) and d up (2, 3)
   __shared__ __align__(4) uint8_t sfc[TILE][4];        // column pass
@@ -317,7 +319,7 @@ quant_swiglu_bwd_kernel(const QuantArgs p) {
 
 template <int MODE>
 int launch_quant(const QuantArgs& p, cudaStream_t stream, const char* what) {
-  quant_mxfp8_kernel<MODE><<<dim3((p.C + TILE - 1) / TILE, p.R / TILE), 256, 0, stream>>>(p);
+  b200::launch(quant_mxfp8_kernel<MODE>, dim3((p.C + TILE - 1) / TILE, p.R / TILE), 256, 0, stream, p);
   b200::count_launch();
   return b200::check_launch(what);
 }
@@ -370,7 +372,7 @@ B200_API int b200_quant_swiglu_bwd_mxfp8(const void* da, long long ldda, const v
     return b200::fail(713, "quant_swiglu_bwd: inputs must be 16-byte aligned");
   const QuantArgs p = {(const __nv_bfloat16*)gu, ldgu, (const __nv_bfloat16*)da, ldda, R, 2 * F, F, (uint8_t*)q_row,
                        (uint8_t*)sf_row, row_tile, (uint8_t*)q_col, (uint8_t*)sf_col, col_tile, live};
-  quant_swiglu_bwd_kernel<<<dim3((F + 63) / 64, R / TILE), 256, 0, (cudaStream_t)stream>>>(p);
+  b200::launch(quant_swiglu_bwd_kernel, dim3((F + 63) / 64, R / TILE), 256, 0, (cudaStream_t)stream, p);
   b200::count_launch();
   return b200::check_launch("quant_swiglu_bwd_mxfp8");
 }

@@ -14,6 +14,7 @@ constexpr int MAX_K = 8;
 // one thread per token
 __global__ void router_topk_kernel(const float* __restrict__ logits, int T, int E, int K, int* __restrict__ idx,
                                    float* __restrict__ w, int* __restrict__ counts) {
+  b200::begin_kernel();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
   const float* row = logits + (long long)t * E;
@@ -48,6 +49,7 @@ __global__ void router_topk_kernel(const float* __restrict__ logits, int T, int 
 // permuted buffer, seg[E] = total padded rows; tile_expert[i] = expert of 128-row tile i (or -1).
 __global__ void router_plan_kernel(const int* __restrict__ counts, int E, int pad, int* __restrict__ seg,
                                    int* __restrict__ tile_expert, int max_tiles) {
+  b200::begin_kernel();
   __shared__ int s_seg[MAX_E + 1];
   if (threadIdx.x == 0) {
     int acc = 0;
@@ -72,6 +74,7 @@ __global__ void router_plan_kernel(const int* __restrict__ counts, int E, int pa
 // flattened order) routed to the same expert.  One CTA per expert scans the flattened index list.
 __global__ void router_rank_kernel(const int* __restrict__ idx, int n, const int* __restrict__ seg,
                                    int* __restrict__ dest) {
+  b200::begin_kernel();
   const int e = blockIdx.x;
   __shared__ int warp_tot[32];
   __shared__ int base;
@@ -121,6 +124,7 @@ B200_DEVICE void clear_gap(const Gaps& g, __nv_bfloat16* out, int D) {
 __global__ void permute_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ dest, int n, int K,
                                     int D, __nv_bfloat16* __restrict__ out, const float* __restrict__ w,
                                     float* __restrict__ w_out, const Gaps gaps) {
+  b200::begin_kernel();
   const int first = gap_ctas(gaps);
   if ((int)blockIdx.x < first) { clear_gap(gaps, out, D); return; }
   const int vpr = D / 8;
@@ -139,6 +143,7 @@ __global__ void permute_rows_kernel(const __nv_bfloat16* __restrict__ x, const i
 __global__ void unpermute_sum_kernel(const __nv_bfloat16* __restrict__ yp, const int* __restrict__ dest,
                                      const float* __restrict__ w, int T, int K, int D, const __nv_bfloat16* __restrict__ res,
                                      __nv_bfloat16* __restrict__ y) {
+  b200::begin_kernel();
   const int vpr = D / 8;
   const long long total = (long long)T * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -169,6 +174,7 @@ __global__ void unpermute_sum_kernel(const __nv_bfloat16* __restrict__ yp, const
 __global__ void unpermute_bwd_kernel(const __nv_bfloat16* __restrict__ gy, const __nv_bfloat16* __restrict__ yp,
                                      const int* __restrict__ dest, const float* __restrict__ w, long long pairs, int K,
                                      int D, __nv_bfloat16* __restrict__ gyp, float* __restrict__ gw, const Gaps gaps) {
+  b200::begin_kernel();
   const int first = gap_ctas(gaps);
   if ((int)blockIdx.x < first) { clear_gap(gaps, gyp, D); return; }
   const long long p = (((long long)blockIdx.x - first) * blockDim.x + threadIdx.x) >> 5;
@@ -197,6 +203,7 @@ __global__ void unpermute_bwd_kernel(const __nv_bfloat16* __restrict__ gy, const
 
 // rows of tiles that belong to no expert (tile_expert < 0) are cleared; 128 rows per tile
 __global__ void zero_dead_tiles_kernel(__nv_bfloat16* __restrict__ buf, const int* __restrict__ tile_expert, int D) {
+  b200::begin_kernel();
   const int tile = blockIdx.x;
   if (tile_expert[tile] >= 0) return;
   uint4* p = reinterpret_cast<uint4*>(buf + (long long)tile * 128 * D);
@@ -213,7 +220,7 @@ B200_API int b200_unpermute_bwd(const void* gy, const void* yp, const int* dest,
   const long long threads = pairs * 32;
   const Gaps gaps = {seg, counts, E};
   const unsigned extra = seg != nullptr ? (unsigned)E * GAP_CTAS : 0u;
-  unpermute_bwd_kernel<<<extra + (unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+  b200::launch(unpermute_bwd_kernel, extra + (unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream, 
       (const __nv_bfloat16*)gy, (const __nv_bfloat16*)yp, dest, w, pairs, K, D, (__nv_bfloat16*)gyp, gw, gaps);
   b200::count_launch();
   return b200::check_launch("unpermute_bwd");
@@ -222,7 +229,7 @@ B200_API int b200_unpermute_bwd(const void* gy, const void* yp, const int* dest,
 B200_API int b200_zero_dead_tiles(void* buf, const int* tile_expert, int n_tiles, int D, void* stream) {
   if (D % 8 != 0) return b200::fail(905, "zero_dead_tiles: D=%d must be a multiple of 8", D);
   if (n_tiles <= 0) return 0;
-  zero_dead_tiles_kernel<<<n_tiles, 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)buf, tile_expert, D);
+  b200::launch(zero_dead_tiles_kernel, n_tiles, 256, 0, (cudaStream_t)stream, (__nv_bfloat16*)buf, tile_expert, D);
   b200::count_launch();
   return b200::check_launch("zero_dead_tiles");
 }
@@ -230,7 +237,7 @@ B200_API int b200_zero_dead_tiles(void* buf, const int* tile_expert, int n_tiles
 B200_API int b200_router_topk(const float* logits, int T, int E, int K, int* idx, float* w, int* counts, void* stream) {
   if (E > MAX_E || K > MAX_K || K > E) return b200::fail(900, "router_topk: E=%d (max %d), K=%d (max %d)", E, MAX_E, K, MAX_K);
   if (T == 0) return 0;
-  router_topk_kernel<<<(T + 127) / 128, 128, 0, (cudaStream_t)stream>>>(logits, T, E, K, idx, w, counts);
+  b200::launch(router_topk_kernel, (T + 127) / 128, 128, 0, (cudaStream_t)stream, logits, T, E, K, idx, w, counts);
   b200::count_launch();
   return b200::check_launch("router_topk");
 }
@@ -239,8 +246,8 @@ B200_API int b200_router_topk(const float* logits, int T, int E, int K, int* idx
 B200_API int b200_router_plan(const int* counts, const int* idx, int n, int E, int pad, int* seg, int* tile_expert,
                               int max_tiles, int* dest, void* stream) {
   if (E > MAX_E) return b200::fail(901, "router_plan: E=%d exceeds %d", E, MAX_E);
-  router_plan_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(counts, E, pad, seg, tile_expert, max_tiles);
-  router_rank_kernel<<<E, 1024, 0, (cudaStream_t)stream>>>(idx, n, seg, dest);
+  b200::launch(router_plan_kernel, 1, 256, 0, (cudaStream_t)stream, counts, E, pad, seg, tile_expert, max_tiles);
+  b200::launch(router_rank_kernel, E, 1024, 0, (cudaStream_t)stream, idx, n, seg, dest);
   b200::count_launch(2);
   return b200::check_launch("router_plan");
 }
@@ -254,7 +261,7 @@ B200_API int b200_permute_rows(const void* x, const int* dest, int n, int K, int
   long long work = (long long)n * (D / 8);
   int grid = (int)((work + 255) / 256 < (long long)b200::sm_count() * 16 ? (work + 255) / 256 : (long long)b200::sm_count() * 16);
   const Gaps gaps = {seg, counts, E};
-  permute_rows_kernel<<<grid + (seg != nullptr ? E * GAP_CTAS : 0), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, dest, n, K, D,
+  b200::launch(permute_rows_kernel, grid + (seg != nullptr ? E * GAP_CTAS : 0), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, dest, n, K, D,
                                                                                                     (__nv_bfloat16*)out, w, w_out, gaps);
   b200::count_launch();
   return b200::check_launch("permute_rows");
@@ -266,7 +273,7 @@ B200_API int b200_unpermute_sum(const void* yp, const int* dest, const float* w,
   if (T == 0) return 0;
   long long work = (long long)T * (D / 8);
   int grid = (int)((work + 255) / 256 < (long long)b200::sm_count() * 16 ? (work + 255) / 256 : (long long)b200::sm_count() * 16);
-  unpermute_sum_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)yp, dest, w, T, K, D, (const __nv_bfloat16*)res, (__nv_bfloat16*)y);
+  b200::launch(unpermute_sum_kernel, grid, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)yp, dest, w, T, K, D, (const __nv_bfloat16*)res, (__nv_bfloat16*)y);
   b200::count_launch();
   return b200::check_launch("unpermute_sum");
 }

@@ -24,10 +24,12 @@
 namespace {
 
 __global__ void iota_kernel(long long* __restrict__ p, long long n) {
+  b200::begin_kernel();
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += (long long)gridDim.x * 256) p[i] = i;
 }
 
 __global__ void head_flags_kernel(const long long* __restrict__ keys, long long n, int* __restrict__ flags) {
+  b200::begin_kernel();
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += (long long)gridDim.x * 256)
     flags[i] = (i == 0 || keys[i] != keys[i - 1]) ? 1 : 0;
 }
@@ -36,6 +38,7 @@ __global__ void head_flags_kernel(const long long* __restrict__ keys, long long 
 __global__ void runs_kernel(const long long* __restrict__ keys, const long long* __restrict__ perm,
                             const int* __restrict__ run, long long n, long long* __restrict__ uniq,
                             long long* __restrict__ seg_off, long long* __restrict__ inverse, long long* __restrict__ count) {
+  b200::begin_kernel();
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
     const int r = run[i] - 1;
     if (i == 0 || run[i] != run[i - 1]) { uniq[r] = keys[i]; seg_off[r] = i; }
@@ -123,6 +126,7 @@ B200_DEVICE long long run_of(const long long* __restrict__ seg, long long total,
 __global__ void __launch_bounds__(256)
 segment_partial_kernel(RowSrc s, const long long* __restrict__ seg, const long long* __restrict__ n_seg,
                        const long long* __restrict__ inverse, long long n, float* __restrict__ partial, int* status) {
+  b200::begin_kernel();
   const long long total = *n_seg;
   if (total <= 0) return;
   const int lane = threadIdx.x & 31;
@@ -161,6 +165,7 @@ template <typename Out>
 __global__ void __launch_bounds__(256)
 segment_sum_gather_kernel(RowSrc s, const long long* __restrict__ seg, const long long* __restrict__ n_seg,
                           const float* __restrict__ partial, long long first, long long max_seg, Out* __restrict__ out, int* status) {
+  b200::begin_kernel();
   const long long total = *n_seg < first + max_seg ? *n_seg : first + max_seg;
   const int lane = threadIdx.x & 31;
   const long long warp0 = (blockIdx.x * 256ll + threadIdx.x) >> 5;
@@ -232,7 +237,7 @@ B200_API int b200_sort_ids(const long long* keys_in, long long* keys_out, long l
   uint8_t* base = (uint8_t*)scratch;
   long long* iota = (long long*)(base + ((lib + 255) & ~size_t(255)));
   const int grid = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
-  iota_kernel<<<grid, 256, 0, st>>>(iota, n);
+  b200::launch(iota_kernel, grid, 256, 0, st, iota, n);
   cudaError_t e = cub::DeviceRadixSort::SortPairs(scratch, lib, keys_in, keys_out, iota, perm_out, (int)n, 0, end_bit, st);
   b200::count_launch(2);
   if (e != cudaSuccess) return b200::fail(1603, "sort_ids: radix sort failed: %s", cudaGetErrorString(e));
@@ -260,11 +265,11 @@ B200_API int b200_unique_segments(const long long* sorted_keys, const long long*
   int* flags = (int*)p;
   int* run = (int*)(p + (((size_t)n * 4 + 255) & ~size_t(255)));
   const int grid = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
-  head_flags_kernel<<<grid, 256, 0, st>>>(sorted_keys, n, flags);
+  b200::launch(head_flags_kernel, grid, 256, 0, st, sorted_keys, n, flags);
   size_t scan_bytes = lib;
   cudaError_t e = cub::DeviceScan::InclusiveSum(scratch, scan_bytes, flags, run, (int)n, st);
   if (e != cudaSuccess) return b200::fail(1604, "unique_segments: scan failed: %s", cudaGetErrorString(e));
-  runs_kernel<<<grid, 256, 0, st>>>(sorted_keys, perm, run, n, uniq, seg_off, inverse, count);
+  b200::launch(runs_kernel, grid, 256, 0, st, sorted_keys, perm, run, n, uniq, seg_off, inverse, count);
   b200::count_launch(3);
   return b200::check_launch("unique_segments");
 }
@@ -294,7 +299,7 @@ B200_API int b200_segment_sum_gather(const void* src, int src_is_f32, long long 
   cudaStream_t st = (cudaStream_t)stream;
   if (partial != nullptr && first == 0) {
     const long long blocks = (n + SEG_CHUNK - 1) / SEG_CHUNK;
-    segment_partial_kernel<<<(unsigned)((blocks + 7) / 8), 256, 0, st>>>(s, seg, n_seg, inverse, n, partial, b200::status_ptr());
+    b200::launch(segment_partial_kernel, (unsigned)((blocks + 7) / 8), 256, 0, st, s, seg, n_seg, inverse, n, partial, b200::status_ptr());
     b200::count_launch();
     int rc = b200::check_launch("segment_partial");
     if (rc) return rc;
@@ -302,9 +307,9 @@ B200_API int b200_segment_sum_gather(const void* src, int src_is_f32, long long 
   const long long want = (max_seg + 7) / 8;            // 8 warps (runs) per CTA
   const int grid = (int)(want < 148 * 16 ? want : 148 * 16);
   if (out_bf16)
-    segment_sum_gather_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(s, seg, n_seg, partial, first, max_seg, (__nv_bfloat16*)out, b200::status_ptr());
+    b200::launch(segment_sum_gather_kernel<__nv_bfloat16>, grid, 256, 0, st, s, seg, n_seg, partial, first, max_seg, (__nv_bfloat16*)out, b200::status_ptr());
   else
-    segment_sum_gather_kernel<float><<<grid, 256, 0, st>>>(s, seg, n_seg, partial, first, max_seg, (float*)out, b200::status_ptr());
+    b200::launch(segment_sum_gather_kernel<float>, grid, 256, 0, st, s, seg, n_seg, partial, first, max_seg, (float*)out, b200::status_ptr());
   b200::count_launch();
   return b200::check_launch("segment_sum_gather");
 }

@@ -22,6 +22,7 @@ std::mutex g_setup_mu;
 template <typename G>
 __global__ void __launch_bounds__(256)
 sumsq_static_partial_kernel(const G* __restrict__ g, long long n, float* __restrict__ partial) {
+  b200::begin_kernel();
   __shared__ float red[8];
   float acc = 0.f;
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
@@ -41,6 +42,7 @@ sumsq_static_partial_kernel(const G* __restrict__ g, long long n, float* __restr
 
 __global__ void sumsq_static_final_kernel(const float* __restrict__ partial, int n, float* __restrict__ out,
                                           int accumulate) {
+  b200::begin_kernel();
   __shared__ float red[8];
   float acc = 0.f;
   for (int i = threadIdx.x; i < n; i += 256) acc += partial[i];
@@ -90,9 +92,9 @@ extern "C" int b200_sumsq_static(const void* g, long long n, int g_is_bf16, floa
   if ((long long)grid * 256 > n) grid = (int)((n + 255) / 256);
   if (grid < 1) grid = 1;
   cudaStream_t st = (cudaStream_t)stream;
-  if (g_is_bf16) sumsq_static_partial_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)g, n, scratch);
-  else sumsq_static_partial_kernel<float><<<grid, 256, 0, st>>>((const float*)g, n, scratch);
-  sumsq_static_final_kernel<<<1, 256, 0, st>>>(scratch, grid, out, accumulate);
+  if (g_is_bf16) b200::launch(sumsq_static_partial_kernel<__nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)g, n, scratch);
+  else b200::launch(sumsq_static_partial_kernel<float>, grid, 256, 0, st, (const float*)g, n, scratch);
+  b200::launch(sumsq_static_final_kernel, 1, 256, 0, st, scratch, grid, out, accumulate);
   b200::count_launch(2);
   return b200::check_launch("sumsq_static");
 }

@@ -13,10 +13,11 @@
 //   D  > 1024   the CTA owns ROWS rows at a time: their loads are in flight together and ONE pair of
 //               barriers reduces all of them (a barrier pair per row made the kernel latency-bound).
 //   1024 < D <= 4096, a multiple of 256: a warp owns a row, for the order of its sums (reasons at norm_fwd_warp_kernel).
+// Backward without the activation, the other D > 256: the next rows' loads are in flight in a ring in shared memory
+// (norm_bwd_ring_kernel).
 // Measured (bf16 in and out, L2 flushed, launch included), one warp or CTA per row -> this split:
 //   98304 x 128   forward 276 -> 16 us   backward 722 -> 30 us
-//   92160 x 512   LayerNorm 116 -> 46 us, backward 198 -> 75 us
-//    8192 x 2880  52 -> 31 us, 149 -> 67 us;   4096 x 8192  50 -> 38 us, 163 -> 87 us
+//   92160 x 512   LayerNorm 116 -> 46 us;   8192 x 2880  52 -> 31 us;   4096 x 8192  50 -> 38 us
 // Four rows of a 512-thread CTA instead of two of a 256-thread one lost 5 to 15 % at widths 2880 and 4096; above
 // 4096 the backward takes 512 threads (with 256 its accumulators leave one CTA of 8 warps per SM: 97 us).
 //
@@ -559,6 +560,186 @@ norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   }
 }
 
+// Backward without the activation for most rows of more than 256 columns (dispatch_bwd).  Bound by memory: x and dy (and dres) are read and dx
+// written once.  A team (G = 32: a warp, G = 0: the CTA) owns whole rows, a thread the same V vectors of columns in all of them, so the
+// column sums stay in its registers.  Every thread copies its own vectors of the next S - 1 row groups into its own slots of a
+// ring in shared memory (cp.async: no registers held, no barrier).  With loads of a row that started when the row before was done,
+// column sums included: 8192 x 2880 64 us, now 46 (3.1 TB/s), 4096 x 8192 85 and 64; with a residual's gradient 89 and 50, 109 and 75;
+// LayerNorm of 46000 x 512 46 and 46, with a residual 67 and 52.
+template <int MODE, int G, int V, int R, int S, int MAXT>
+__global__ void __launch_bounds__(MAXT, MODE == 1 && V * MAXT > 512 ? 1 : 2)
+norm_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                     const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres,
+                     __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int T, int D) {
+  b200::begin_kernel();
+  constexpr int NACC = MODE == 1 ? 2 : 1, NS = R * NACC;
+  extern __shared__ uint4 ring[];                    // [S][R][x | dy | dres][V][threads]
+  __shared__ float red[2][NS][16];
+  const int nt = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  const int nvec = D / 8, nin = dres != nullptr ? 3 : 2;
+  const float inv_d = 1.f / D;
+  const int team = G == 32 ? blockIdx.x * nw + warp : blockIdx.x, teams = G == 32 ? gridDim.x * nw : gridDim.x;
+  const int first = G == 32 ? lane : tid, stride = G == 32 ? 32 : nt;
+  const int groups = (T + R - 1) / R;
+  auto slot = [&](int s, int r, int in, int i) { return ring + (((s * R + r) * nin + in) * V + i) * nt + tid; };
+  auto copy = [&](uint4* to, const __nv_bfloat16* from) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(to)), "l"(from) : "memory");
+  };
+  auto issue = [&](int g, int s) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const int row = g * R + r, vi = first + i * stride;
+        if (g < groups && row < T && vi < nvec) {
+          const long long at = (long long)row * D + vi * 8;
+          copy(slot(s, r, 0, i), x + at);
+          copy(slot(s, r, 1, i), dy + at);
+          if (nin == 3) copy(slot(s, r, 2, i), dres + at);
+        }
+      }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto stats = [&](int g, float (&rs)[R], float (&mu)[R]) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int row = g * R + r;
+      rs[r] = g < groups && row < T ? rstd_in[row] : 0.f;
+      mu[r] = MODE == 1 && g < groups && row < T ? mean_in[row] : 0.f;
+    }
+  };
+  uint4 wv[V];
+  float dw_acc[V][8], db_acc[MODE == 1 ? V : 1][8];
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int vi = first + i * stride;
+    wv[i] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);      // 1.0
+    if (w != nullptr && vi < nvec) wv[i] = ld16(w + vi * 8);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { dw_acc[i][j] = 0.f; if (MODE == 1) db_acc[MODE == 1 ? i : 0][j] = 0.f; }
+  }
+  float rs_next[R], mu_next[R];
+  stats(team, rs_next, mu_next);
+#pragma unroll
+  for (int k = 0; k < S - 1; ++k) issue(team + k * teams < groups ? team + k * teams : groups, k);
+  int cur = 0, buf = 0;
+  for (int g = team; g < groups; g += teams) {
+    // the slot that this thread read in the iteration before
+    const long long ahead = (long long)g + (long long)(S - 1) * teams;
+    issue(ahead < groups ? (int)ahead : groups, cur == 0 ? S - 1 : cur - 1);
+    float rstd[R], mean[R], s[NS];
+#pragma unroll
+    for (int r = 0; r < R; ++r) { rstd[r] = rs_next[r]; mean[r] = mu_next[r]; }
+    stats(groups - g > teams ? g + teams : groups, rs_next, mu_next);
+#pragma unroll
+    for (int r = 0; r < NS; ++r) s[r] = 0.f;
+    asm volatile("cp.async.wait_group %0;" ::"n"(S - 1) : "memory");
+    uint4 xv[R][V], gv[R][V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const bool in = first + i * stride < nvec;
+      float w8[8];
+      unpack8(wv[i], w8);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        xv[r][i] = gv[r][i] = make_uint4(0, 0, 0, 0);
+        if (in && g * R + r < T) { xv[r][i] = *slot(cur, r, 0, i); gv[r][i] = *slot(cur, r, 1, i); }
+        float x8[8], d8[8];
+        unpack8(xv[r][i], x8);
+        unpack8(gv[r][i], d8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float xn = (x8[j] - mean[r]) * rstd[r];
+          dw_acc[i][j] += d8[j] * xn;
+          if (MODE == 1) db_acc[MODE == 1 ? i : 0][j] += d8[j];
+          const float gj = d8[j] * w8[j];
+          s[r] += gj * xn;
+          if (MODE == 1) s[R * (MODE == 1) + r] += gj;
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < NS; ++k) s[k] = warp_sum(s[k]);
+    if (G == 0) {
+      if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < NS; ++k) red[buf][k][warp] = s[k];
+      __syncthreads();                               // the other buffer is free again when this is passed
+#pragma unroll
+      for (int k = 0; k < NS; ++k) s[k] = warp_sum(lane < nw ? red[buf][k][lane] : 0.f);
+      buf ^= 1;
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int vi = first + i * stride;
+      float w8[8];
+      unpack8(wv[i], w8);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (vi < nvec && g * R + r < T) {
+          const float s1 = s[r] * inv_d, s2 = MODE == 1 ? s[R * (MODE == 1) + r] * inv_d : 0.f;
+          float x8[8], d8[8], o[8];
+          unpack8(xv[r][i], x8);
+          unpack8(gv[r][i], d8);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] = rstd[r] * (d8[j] * w8[j] - (x8[j] - mean[r]) * rstd[r] * s1 - s2);
+          if (nin == 3) {
+            float r8[8];
+            unpack8(*slot(cur, r, 2, i), r8);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] += r8[j];
+          }
+          st16(dx + (long long)(g * R + r) * D + vi * 8, pack8(o));
+        }
+    }
+    cur = cur + 1 == S ? 0 : cur + 1;
+  }
+  if (partial == nullptr) return;
+  float* pw = partial + (long long)blockIdx.x * 2 * D;
+  if (G == 0) {
+    // a thread owns its columns for every row of the CTA
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int vi = first + i * stride;
+      if (vi < nvec) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float4* o = reinterpret_cast<float4*>(pw + h * D + vi * 8);
+          float v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = h == 0 ? dw_acc[i][j] : (MODE == 1 ? db_acc[MODE == 1 ? i : 0][j] : 0.f);
+          o[0] = make_float4(v[0], v[1], v[2], v[3]);
+          o[1] = make_float4(v[4], v[5], v[6], v[7]);
+        }
+      }
+    }
+    return;
+  }
+  // the warps' sums, in their order, through the ring (its copies are all done)
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  float* acc = reinterpret_cast<float*>(ring);       // [warps][D]
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (h < NACC) {
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const int vi = first + i * stride;
+        if (vi < nvec)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[warp * D + vi * 8 + j] = h == 0 ? dw_acc[i][j] : db_acc[MODE == 1 ? i : 0][j];
+      }
+      __syncthreads();
+    }
+    for (int c = tid; c < D; c += nt) {
+      float t = 0.f;
+      if (h < NACC)
+        for (int k = 0; k < nw; ++k) t += acc[k * D + c];
+      pw[h * D + c] = t;
+    }
+  }
+}
+
 // out[c] (+)= sum_p partial[p][which][c]: 32 columns per CTA, its 8 warps take every eighth partial row (their loads
 // are independent: one thread per column walked all of them in series), summed in a fixed order.
 __global__ void __launch_bounds__(256)
@@ -637,6 +818,36 @@ int run_bwd(const BwdArgs& a) {
   return grid;
 }
 
+template <int MODE, int G, int V, int R, int S, int MAXT>
+int launch_bwd_ring(const BwdArgs& a, int threads, int smem) {
+  auto kern = norm_bwd_ring_kernel<MODE, G, V, R, S, MAXT>;
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return -b200::fail(302, "norm_bwd: cannot raise shared memory: %s", cudaGetErrorString(e));
+    }
+    configured[dev & 63] = true;
+  }
+  const int per_cta = (G == 32 ? threads / 32 : 1) * R, need = (a.T + per_cta - 1) / per_cta;
+  const int grid = need < a.grid ? need : a.grid;      // never more partial rows than the scratch holds
+  b200::launch(kern, grid, threads, smem, a.st, a.dy, a.x, a.w, a.mean, a.rstd, a.dres, a.dx, a.partial, a.T, a.D);
+  return grid;
+}
+
+// As deep a ring as leaves room for two CTAs an SM: at most 4 stages and 104 KB (2 stages of 48 KB at 8192 columns and a residual).
+template <int MODE, int G, int V, int R, int MAXT>
+int run_bwd_ring(const BwdArgs& a) {
+  const int threads = G == 32 ? MAXT : block_threads(a.D, V);
+  const int stage = R * V * threads * 16 * (a.dres != nullptr ? 3 : 2);
+  if (4 * stage <= 104 * 1024) return launch_bwd_ring<MODE, G, V, R, 4, MAXT>(a, threads, 4 * stage);
+  if (3 * stage <= 104 * 1024) return launch_bwd_ring<MODE, G, V, R, 3, MAXT>(a, threads, 3 * stage);
+  return launch_bwd_ring<MODE, G, V, R, 2, MAXT>(a, threads, 2 * stage);
+}
+
 template <int MODE, int ACT>
 int run_bwd_warp(const BwdArgs& a) {
   constexpr int nacc = (MODE == 1 || ACT) ? 2 : 1;
@@ -664,11 +875,21 @@ int dispatch_bwd(const BwdArgs& a) {
   if (a.D <= 64) return run_bwd<MODE, ACT, 8, 1, 4>(a);
   if (a.D <= 128) return run_bwd<MODE, ACT, 16, 1, 4>(a);
   if (a.D <= 256) return run_bwd<MODE, ACT, 32, 1, 4>(a);
-  if (a.D <= 512) return run_bwd<MODE, ACT, 32, 2, 2>(a);
-  if (a.D <= 1024) return run_bwd<MODE, ACT, 32, 4, 1>(a);
-  if (a.D % 256 == 0 && a.D <= 4096) return run_bwd_warp<MODE, ACT>(a);
-  if (a.D <= 4096) return run_bwd<MODE, ACT, 0, 2, 2>(a);
-  return run_bwd<MODE, ACT, 0, 2, 2, 512>(a);
+  if constexpr (ACT == 0) {
+    if (a.D <= 512) return run_bwd_ring<MODE, 32, 2, 2, 256>(a);
+    if (a.D <= 1024) return run_bwd_ring<MODE, 32, 4, 1, 256>(a);
+    // The ring sums these rows in another order, which block-scaled linears behind it turn into 2.4 % of the gradients (the sums of
+    // norm_fwd_warp_kernel tell the same); 8192 x 4096: 73 us, the ring 52.
+    if (a.D % 256 == 0 && a.D <= 4096) return run_bwd_warp<MODE, ACT>(a);
+    if (a.D <= 4096) return run_bwd_ring<MODE, 0, 1, 2, 512>(a);
+    return run_bwd_ring<MODE, 0, 2, 1, 512>(a);
+  } else {
+    if (a.D <= 512) return run_bwd<MODE, ACT, 32, 2, 2>(a);
+    if (a.D <= 1024) return run_bwd<MODE, ACT, 32, 4, 1>(a);
+    if (a.D % 256 == 0 && a.D <= 4096) return run_bwd_warp<MODE, ACT>(a);
+    if (a.D <= 4096) return run_bwd<MODE, ACT, 0, 2, 2>(a);
+    return run_bwd<MODE, ACT, 0, 2, 2, 512>(a);
+  }
 }
 
 }  // namespace

@@ -29,3 +29,26 @@ def test_norm_matches_fp32(T, D, layer_norm, swish):
     for a, r in ((dw, dw_c), (db, db_c)):
         if a is not None:
             torch.testing.assert_close(a.cpu(), r, rtol=1e-4, atol=1e-4 * T ** 0.5)
+
+
+@pytest.mark.parametrize("T,D", [(5001, 512), (3001, 1016), (2501, 1032), (2500, 2880), (1301, 4096), (701, 8192)])
+@pytest.mark.parametrize("layer_norm", [False, True])
+@pytest.mark.parametrize("res", [False, True])
+def test_norm_bwd_over_many_row_groups(T, D, layer_norm, res):
+    """More rows than the ring of row groups in flight holds, with a remainder, against fp64."""
+    g = torch.Generator(device="cuda").manual_seed(D)
+    x, dy, dres = (torch.randn(T, D, device="cuda", generator=g).bfloat16() for _ in range(3))
+    w, b = (torch.randn(D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    y, h, mean, rstd = kernels.norm_fwd(x, w, b if layer_norm else None, 1e-5, layer_norm=layer_norm)
+    dx, dw, db = kernels.norm_bwd(dy, x, w, b if layer_norm else None, mean, rstd, layer_norm=layer_norm, dres=dres if res else None)
+    xd, wd = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    xc = xd - xd.mean(1, keepdim=True) if layer_norm else xd
+    (xc * (xc.square().mean(1, keepdim=True) + 1e-5).rsqrt() * wd).backward(dy.double())
+    ref = xd.grad + (dres.double() if res else 0)
+    # one rounding to bf16 (2^-9) of fp32 arithmetic on terms of the row's size
+    assert ((dx.double() - ref).abs() <= ref.abs() * 2 ** -8 + 2 ** -18 * ref.abs().max()).all()
+    # fp32 sums over T rows: each term is off by a few 2^-24, they add up like sqrt(T) at worst times the largest
+    bound = T ** 0.5 * 2 ** -20 * (dy.double() * xc.detach()).abs().max()
+    assert (dw.double() - wd.grad).abs().max() <= bound
+    if layer_norm:
+        assert (db.double() - dy.double().sum(0)).abs().max() <= T ** 0.5 * 2 ** -20 * dy.double().abs().max()

@@ -251,8 +251,8 @@ class STULayer(nn.Module):
         """``max_len``: the static length bound N of the attention (its 1 / N factor and grid); default the model's."""
         cfg = self.cfg
         h = cfg.heads
-        uvqk = F.norm_linear(x, self.in_norm_w, self.uvqk_weight, norm_b=self.in_norm_b, bias=self.uvqk_beta,
-                             eps=1e-6, layer_norm=True, precision=cfg.precision)
+        uvqk, x = F.norm_linear(x, self.in_norm_w, self.uvqk_weight, norm_b=self.in_norm_b, bias=self.uvqk_beta,
+                                eps=1e-6, layer_norm=True, precision=cfg.precision, pass_x=True)
         p = cfg.linear_dropout if self.training else 0.0
         if self.fuse_glue and cfg.d_v == cfg.d_qk and attn_gate_cat_eligible(uvqk, h):
             # attention, SiLU(u), the layer norm of the attention output, their product, the concatenation and its dropout (mask

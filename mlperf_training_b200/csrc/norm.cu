@@ -12,9 +12,9 @@
 //               threads idle and paid two barriers per 256 bytes.
 //   D  > 1024   the CTA owns ROWS rows at a time: their loads are in flight together and ONE pair of
 //               barriers reduces all of them (a barrier pair per row made the kernel latency-bound).
-//   1024 < D <= 4096, a multiple of 256: a warp owns a row, for the order of its sums (reasons at norm_fwd_warp_kernel).
-// Backward without the activation, the other D > 256: the next rows' loads are in flight in a ring in shared memory
-// (norm_bwd_ring_kernel).
+//   1024 < D <= 4096, a multiple of 256: forward and the activation's backward, a warp owns a row, for the order of its sums
+//               (reasons at norm_fwd_warp_kernel).
+// Backward without the activation, D > 256: the next rows' loads are in flight in a ring in shared memory (norm_bwd_ring_kernel).
 // Measured (bf16 in and out, L2 flushed, launch included), one warp or CTA per row -> this split:
 //   98304 x 128   forward 276 -> 16 us   backward 722 -> 30 us
 //   92160 x 512   LayerNorm 116 -> 46 us;   8192 x 2880  52 -> 31 us;   4096 x 8192  50 -> 38 us
@@ -560,12 +560,12 @@ norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   }
 }
 
-// Backward without the activation for most rows of more than 256 columns (dispatch_bwd).  Bound by memory: x and dy (and dres) are read and dx
+// Backward without the activation for rows of more than 256 columns.  Bound by memory: x and dy (and dres) are read and dx
 // written once.  A team (G = 32: a warp, G = 0: the CTA) owns whole rows, a thread the same V vectors of columns in all of them, so the
 // column sums stay in its registers.  Every thread copies its own vectors of the next S - 1 row groups into its own slots of a
 // ring in shared memory (cp.async: no registers held, no barrier).  With loads of a row that started when the row before was done,
-// column sums included: 8192 x 2880 64 us, now 46 (3.1 TB/s), 4096 x 8192 85 and 64; with a residual's gradient 89 and 50, 109 and 75;
-// LayerNorm of 46000 x 512 46 and 46, with a residual 67 and 52.
+// column sums included: 8192 x 2880 64 us, now 46 (3.1 TB/s), 8192 x 4096 73 and 52, 4096 x 8192 85 and 64; with a residual's
+// gradient 89 and 50, 114 and 58, 109 and 75; LayerNorm of 46000 x 512 46 and 46, with a residual 67 and 52.
 template <int MODE, int G, int V, int R, int S, int MAXT>
 __global__ void __launch_bounds__(MAXT, MODE == 1 && V * MAXT > 512 ? 1 : 2)
 norm_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
@@ -878,9 +878,6 @@ int dispatch_bwd(const BwdArgs& a) {
   if constexpr (ACT == 0) {
     if (a.D <= 512) return run_bwd_ring<MODE, 32, 2, 2, 256>(a);
     if (a.D <= 1024) return run_bwd_ring<MODE, 32, 4, 1, 256>(a);
-    // The ring sums these rows in another order, which block-scaled linears behind it turn into 2.4 % of the gradients (the sums of
-    // norm_fwd_warp_kernel tell the same); 8192 x 4096: 73 us, the ring 52.
-    if (a.D % 256 == 0 && a.D <= 4096) return run_bwd_warp<MODE, ACT>(a);
     if (a.D <= 4096) return run_bwd_ring<MODE, 0, 1, 2, 512>(a);
     return run_bwd_ring<MODE, 0, 2, 1, 512>(a);
   } else {

@@ -218,9 +218,12 @@ class Zero3Engine(ZeroEngine):
         b = self._by_block3.get(idx)
         if b is None:
             return
-        self._ensure(idx, need_col=False, prefetch=False)
+        # a forward that a backward may follow makes the copies of both directions (ops/linear.py: weight_operands), so copies of the
+        # forward direction alone, which an evaluation leaves, do not spare it the gather
+        need_col = torch.is_grad_enabled()
+        self._ensure(idx, need_col=need_col, prefetch=False)
         self._wait_gather(b.slot)
-        self._ensure(idx + 1, need_col=False, prefetch=True)
+        self._ensure(idx + 1, need_col=need_col, prefetch=True)
 
     def pre_backward(self, idx: int) -> None:
         b = self._by_block3.get(idx)

@@ -29,6 +29,9 @@ def main():
     if gpu:
         cfg = GPTConfig(n_layers=4, hidden=512, n_heads=4, n_kv_heads=2, head_dim=128, ffn_hidden=1024, vocab_size=2048,
                         seq_len=256, precision=precision)
+    elif precision != "bf16":
+        cfg = GPTConfig(n_layers=4, hidden=256, n_heads=4, n_kv_heads=4, head_dim=64, ffn_hidden=256, vocab_size=256,
+                        seq_len=128, dtype="fp32", precision=precision)
     else:
         cfg = GPTConfig(n_layers=4, hidden=64, n_heads=4, n_kv_heads=2, head_dim=16, ffn_hidden=128, vocab_size=128,
                         seq_len=32, dtype="fp32")
@@ -41,19 +44,25 @@ def main():
     data = synthetic_tokens(4, 2, cfg.seq_len, cfg.vocab_size, seed=1, rank=rank, pin=gpu)
     l1, l3 = [], []
     for s in range(4):
-        l1.append(t1.train_step(data[s]))
-        l3.append(t3.train_step(data[s]))
+        # An evaluation leaves weight copies of the forward direction alone; the step after it must not take the others from a
+        # window that holds another block.  (t1's step would make t3's copies stale: weights age by one count per process.)
+        for t, losses in ((t1, l1), (t3, l3)):
+            t.eval_loss(data[s].to(dev))
+            losses.append(t.train_step(data[s]))
     ev1 = float(t1.eval_loss(data[0].to(dev)))
     ev3 = float(t3.eval_loss(data[0].to(dev)))
     if gpu:
         torch.cuda.synchronize()
         from mlperf_training_b200.ops import _lib
         _lib.check_status("zero3 worker")
-    tol = 3e-2 if gpu else 2e-5
+    # (CPU, quantised linears: the engines add the same gradients in another order, and an element that then rounds to the neighbouring
+    # code is off by 2^-4; weights taken from another block's window moved the losses by 2e-2 and the weights by 0.3)
+    quantised = precision != "bf16"
+    tol = 3e-2 if gpu else (2e-3 if quantised else 2e-5)
     ok &= all(abs(a - b) < tol for a, b in zip(l1, l3)) and abs(ev1 - ev3) < tol
     # the shards, gathered, equal the replicated engine's parameter buffers
     by_key = {b.key: b for b in t1.engine.buckets}
-    worst = 0.0
+    worst, num, den = 0.0, 0.0, 0.0
     for b in sharded:
         full = e3.gather_full(b)
         mats = torch.cat([p.detach().reshape(-1) for n, p in t1.model.named_parameters()
@@ -61,12 +70,15 @@ def main():
         # same parameter order inside the bucket: weight-decayed matrices in registration order
         ref = torch.cat([p.detach().reshape(-1) for (n, p) in [(n, dict(t1.model.named_parameters())[n]) for n, _ in b.params]])
         worst = max(worst, (full[:ref.numel()].float() - ref.float()).abs().max().item())
+        num += (full[:ref.numel()].double() - ref.double()).square().sum().item()
+        den += ref.double().square().sum().item()
         del mats
-    ok &= worst < (3e-2 if gpu else 2e-5)
+    rel = (num / den) ** 0.5
+    ok &= rel < 1e-2 if quantised and not gpu else worst < (3e-2 if gpu else 2e-5)
     flag = torch.tensor([1.0 if ok else 0.0], device=dev)
     dist.all_reduce(flag, op=dist.ReduceOp.MIN)
     if rank == 0:
-        print(f"zero1 {l1} eval {ev1:.5f}\nzero3 {l3} eval {ev3:.5f}\nworst param diff {worst:.3g} nvls={e3.nvls} "
+        print(f"zero1 {l1} eval {ev1:.5f}\nzero3 {l3} eval {ev3:.5f}\nworst param diff {worst:.3g} rel {rel:.3g} nvls={e3.nvls} "
               f"state MB z1 {t1.engine.state_bytes() / 2**20:.1f} z3 {e3.state_bytes() / 2**20:.1f}", flush=True)
     print(f"RESULT rank {rank} ok={bool(flag.item())}", flush=True)
     dist.barrier()

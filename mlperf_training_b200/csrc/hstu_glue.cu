@@ -258,7 +258,8 @@ gate_cat_reduce_kernel(const float* __restrict__ partial, int nparts, int D, flo
 }
 
 // Rows of [L, width] (pitch ld) that the attention does not write, set to zero: those of no sequence (before offsets[0], from
-// offsets[B] on) and those of a sequence past `cover` (the rows its grid reaches).  CTA b < B: sequence b; the others share the rest.
+// offsets[B] on; with no sequence, B = 0, all of them) and those of a sequence past `cover` (the rows its grid reaches).  CTA b < B:
+// sequence b; the others share the rest.
 // (Clearing a whole output of 105,000 x 512 took 28 us a tensor, this 2.)
 __global__ void __launch_bounds__(256)
 zero_uncovered_rows_kernel(__nv_bfloat16* __restrict__ buf, const int* __restrict__ offsets, int B, long long L, long long ld, int vpr,
@@ -362,7 +363,7 @@ B200_API int b200_hstu_zero_uncovered(void* buf, const int* offsets, int B, long
                                       void* stream) {
   if (width % 8 != 0 || ld % 8 != 0 || ((uintptr_t)buf & 15) != 0)
     return b200::fail(903, "hstu_zero_uncovered: width %d and pitch %lld must be multiples of 8, the base 16-byte aligned", width, ld);
-  if (L <= 0 || B <= 0) return 0;
+  if (L <= 0 || B < 0) return 0;          // (B < 0 is for the attention's launcher to refuse)
   b200::launch(zero_uncovered_rows_kernel, B + 16, 256, 0, (cudaStream_t)stream, (__nv_bfloat16*)buf, offsets, B, L, ld, width / 8, cover);
   b200::count_launch();
   return b200::check_launch("hstu_zero_uncovered");

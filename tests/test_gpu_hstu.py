@@ -230,6 +230,31 @@ def test_attention_leaves_zeros_outside_the_sequences():
 
 
 @pytest.mark.parametrize("precision", ["bf16", "fp8"])
+@pytest.mark.parametrize("first", [0, 17])
+def test_attention_of_no_sequence_is_zero(precision, first):
+    """A batch without sequences, padding rows only: zeros in the output and in every gradient, whatever the allocator hands out."""
+    from mlperf_training_b200.ops.hstu_ops import attn_gate_cat
+    torch.manual_seed(0)
+    H, D, L = 4, 128, 300
+    W = H * D
+    offs = torch.tensor([first], dtype=torch.int32, device="cuda")
+    x = torch.randn(L, 4 * W, device="cuda").bfloat16().requires_grad_(True)
+    w, b = (torch.randn(W, device="cuda").bfloat16().requires_grad_(True) for _ in range(2))
+    junk = [torch.full((L, n * W), float("nan"), device="cuda", dtype=torch.bfloat16) for n in (1, 1, 1, 3, 4)]
+    q, k, v = (t.detach().unflatten(-1, (H, D)).requires_grad_(True) for t in torch.split(x.detach(), W, dim=1)[1:])
+    del junk
+    out = hstu_attention(q, k, v, offs, 256, D ** -0.5, precision=precision)
+    out.backward(torch.randn_like(out))
+    assert all((t == 0).all() for t in (out.detach(), q.grad, k.grad, v.grad))
+    junk = [torch.full((L, n * W), float("nan"), device="cuda", dtype=torch.bfloat16) for n in (1, 1, 1, 3, 4)]
+    del junk
+    y = attn_gate_cat(x, w, b, offs, 256, D ** -0.5, None, 0, H, precision=precision)
+    y.backward(torch.randn_like(y))
+    assert y.isfinite().all() and (x.grad[:, W:] == 0).all() and x.grad.isfinite().all()
+    _lib.check_status("no sequence")
+
+
+@pytest.mark.parametrize("precision", ["bf16", "fp8"])
 @pytest.mark.parametrize("p", [0.0, 0.25])
 def test_attention_and_gate_over_one_buffer(precision, p):
     """The fused form gives the split form's output and gradient bit for bit (same kernels, same seed of the mask)."""

@@ -114,7 +114,12 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False, 
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 4)) as ex:
         host = ex.submit(build_host, force)
         results = list(ex.map(compile_one, sources()))
+    try:
         host.result()
+    except Exception as e:  # noqa: BLE001 - another processor, no C++ compiler, a torch without CUDA headers
+        # the kernels do not need the module (ops/_lib.py then calls them through ctypes); one of an older build must not stay beside them
+        (PKG / HOST_LIB_NAME).unlink(missing_ok=True)
+        print(f"warning: {HOST_LIB_NAME} was not built, launches go through ctypes: {e}", file=sys.stderr)
     objs = [r[0] for r in results]
     rebuilt = any(r[1] for r in results)
     if verbose or ptxas_info:

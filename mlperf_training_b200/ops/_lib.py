@@ -15,6 +15,7 @@ import ctypes
 import functools
 import os
 import threading
+import warnings
 from pathlib import Path
 
 import torch
@@ -27,14 +28,19 @@ HOST_PATH = _PKG / "_b200_host.so"
 
 
 def _import_host():
-    """The native host module, or None before it is built (its work is then done by ctypes and Python: the same kernels)."""
+    """The native host module, or None before it is built or where it does not load, as one of another torch or Python (its work
+    is then done by ctypes and Python: the same kernels)."""
     if not HOST_PATH.exists():
         return None
     import importlib.machinery
     import importlib.util
     loader = importlib.machinery.ExtensionFileLoader("_b200_host", str(HOST_PATH))
-    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_b200_host", loader))
-    loader.exec_module(mod)
+    try:
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_b200_host", loader))
+        loader.exec_module(mod)
+    except ImportError as e:
+        warnings.warn(f"{HOST_PATH.name} does not load, launches go through ctypes: {e}", RuntimeWarning, stacklevel=2)
+        return None
     return mod
 
 

@@ -136,8 +136,10 @@ def _gap_args(gaps):
 def unpermute_sum(yp: torch.Tensor, dest: torch.Tensor, w: torch.Tensor | None, T: int, k: int,
                   residual: torch.Tensor | None = None) -> torch.Tensor:
     """``y[t] = sum_j w[t,j] * yp[dest[t*k + j]] (+ residual[t])`` (``w`` None = plain sum)."""
+    if residual is not None and (residual.dtype != yp.dtype or yp.dtype == torch.float64):
+        return residual + unpermute_sum(yp, dest, w, T, k)      # in the promoted type
     D = yp.shape[1]
-    if not use_kernels(yp) or yp.dtype != torch.bfloat16 or (residual is not None and residual.dtype != torch.bfloat16):
+    if not use_kernels(yp) or yp.dtype != torch.bfloat16:
         g = yp[dest.long()].view(T, k, D).float()
         if w is not None:
             g = g * w.view(T, k, 1).float()
@@ -261,7 +263,7 @@ class UnpermuteFn(Function):
         dres = gy if ctx.has_res else None
         T, k = ctx.cfg
         D = yp.shape[1]
-        gy = gy.contiguous()
+        gy = gy.to(yp.dtype).contiguous()
         if use_kernels(gy) and gy.dtype == torch.bfloat16 and yp.dtype == torch.bfloat16:
             # one pass: scaled scatter of the gradient rows and the routing-weight gradient (a dot product per pair)
             gaps = None if seg is None else (seg, counts)

@@ -242,3 +242,21 @@ def test_grouped_mlp_block_scaled_emulation_close_to_bf16():
     e4 = [((u - v).norm() / u.norm()).item() for u, v in zip(ref, run("mxfp4"))]
     assert all(a < b * 1.3 for a, b in zip(e8, e6)) and all(a < b for a, b in zip(e6, e4)) and max(e4) < 0.6
     assert w1.grad[2].abs().max() == 0 and w1._mx_stack[0][2] == "e2m1"
+
+
+@pytest.mark.parametrize("rows,res", [(torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16), (torch.float64, torch.float64)])
+def test_expert_sum_keeps_the_bits_of_its_residual(rows, res):
+    """The combine of another type than its residual stream gives what the sum of the two gives: the promoted type, unrounded."""
+    from mlperf_training_b200.ops import moe_ops as M
+    torch.manual_seed(0)
+    T, k, D = 5, 2, 16
+    yp, w = torch.randn(T * k, D).to(rows).requires_grad_(True), torch.rand(T, k).requires_grad_(True)
+    r = torch.randn(T, D, dtype=torch.float64).to(res).requires_grad_(True)
+    dest = torch.randperm(T * k).int()
+    want = r + M.UnpermuteFn.apply(yp, dest, w, T, k)
+    gy = torch.randn(T, D, dtype=torch.float64).to(want.dtype)
+    grads = torch.autograd.grad(want, (yp, w, r), gy)
+    got = M.UnpermuteFn.apply(yp, dest, w, T, k, r)
+    assert got.dtype == want.dtype and torch.equal(got, want)
+    for a, b in zip(torch.autograd.grad(got, (yp, w, r), gy), grads):
+        assert a.dtype == b.dtype and torch.equal(a, b)

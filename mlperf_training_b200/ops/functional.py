@@ -31,9 +31,11 @@ class _NoGrad:
 
 
 def _apply(fn, *args):
-    """``fn.apply``; with the gradient mode off, no function transform and no forward-mode level under way ``fn.forward`` itself (an
-    autograd node that is thrown away costs 8 us of host time a call)."""
-    if torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0:
+    """``fn.apply``; with the gradient mode off, no function transform, no forward-mode level and no trace under way ``fn.forward``
+    itself (an autograd node that is thrown away costs 8 us of host time a call).  A trace records the operator by its node: of a
+    forward whose kernels are launched past torch it would keep the allocation of the result and nothing that fills it."""
+    if (torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0
+            or torch._C._get_tracing_state() is not None):
         return fn.apply(*args)
     return fn.forward(_NoGrad(), *args)
 

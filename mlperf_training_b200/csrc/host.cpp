@@ -84,8 +84,7 @@ PyObject* py_call(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     } else if (o == Py_None && c == 'P') {
       a[na++] = 0;
     } else if (PyLong_Check(o)) {                    // (bool is one)
-      if (c == 'L') a[na] = PyLong_AsLongLong(o);
-      else a[na] = (long long)PyLong_AsUnsignedLongLongMask(o);      // wraps, as ctypes does
+      a[na] = (long long)PyLong_AsUnsignedLongLongMask(o);           // wraps, as ctypes does
       if (c == 'I') a[na] = (int)a[na];
       if (a[na] == -1 && PyErr_Occurred()) return nullptr;
       ++na;
@@ -151,6 +150,7 @@ PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const at::Tensor &a = THPVariable_Unpack(args[0]), &b = THPVariable_Unpack(args[1]);
   const bool a_mn = PyObject_IsTrue(args[2]) == 1, b_mn = PyObject_IsTrue(args[3]) == 1, acc = PyObject_IsTrue(args[6]) == 1;
   bool f32 = PyObject_IsTrue(args[5]) == 1;
+  if (PyErr_Occurred()) return nullptr;
   if (!a.is_cuda() || !b.is_cuda() || a.scalar_type() != at::kBFloat16 || b.scalar_type() != at::kBFloat16 || !plain(a) || !plain(b) ||
       a.device() != b.device())
     Py_RETURN_NONE;

@@ -59,9 +59,16 @@ struct BwdParams {
   int bh_group;        // (batch, kv head) pairs scheduled together, longest key tiles first
   // Split schedule (cap > 0): no CTA takes more than cap steps of a key tile; the others of a tile take its next ones.
   int cap, entries;    // entries: CTAs of one (batch, kv head) pair, in `order` as (key tile << 3 | part), longest first
-  int max_parts;       // most parts of a tile, at most MAX_PARTS
-  float* partial;      // fp32 [B * Hkv][key tile][max_parts][dK | dV][128][HD], of tiles with several parts
+  int slots;           // parts of the tiles that are cut, and where in them each entry's is
+  float* partial;      // fp32 [B * Hkv][slots][dK | dV][128][HD]
   uint16_t order[MAX_ENTRIES];
+  uint16_t slot[MAX_ENTRIES];
+};
+
+// The key tiles that are cut, and the first slot of each.
+struct CutTiles {
+  int n;
+  uint16_t tile[MAX_ENTRIES / 2], slot[MAX_ENTRIES / 2];
 };
 
 // (query head, query tile) steps of key tile jt and its first query tile.
@@ -151,9 +158,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int num_kt = (p.Skv + BKV - 1) / BKV;
   // early key tiles see the most queries: they are scheduled first, over all heads of a group
   const int bh_all = p.B * p.Hkv;
-  int jt, bh, part = 0;
+  int jt, bh, part = 0, e = 0;
   if (p.cap > 0) {
-    const int e = (int)blockIdx.x / bh_all;
+    e = (int)blockIdx.x / bh_all;
     bh = (int)blockIdx.x - e * bh_all;
     jt = p.order[e] >> 3;
     part = p.order[e] & 7;
@@ -471,8 +478,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           for (int i = 0; i < 32; ++i) v[i] = 0u;
         }
         if (parts > 1) {                        // fp32, as it is: attn_bwd_finish_kernel adds the parts up
-          float4* o = reinterpret_cast<float4*>(p.partial + ((((long long)bh * num_kt + jt) * p.max_parts + part) * 2 + half) * BKV * HD +
-                                                r * HD + c * 32);
+          float4* o = reinterpret_cast<float4*>(p.partial + (((long long)bh * p.slots + p.slot[e]) * 2 + half) * BKV * HD + r * HD +
+                                                c * 32);
 #pragma unroll
           for (int g = 0; g < 8; ++g)
             o[g] = make_float4(__uint_as_float(v[4 * g]), __uint_as_float(v[4 * g + 1]), __uint_as_float(v[4 * g + 2]),
@@ -512,19 +519,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
-// dK and dV of a key tile from its parts, added in their order (no atomics: runs are bit-reproducible).
+// dK and dV of a key tile that is cut from its parts, added in their order (no atomics: runs are bit-reproducible).
 template <int HD>
 __global__ void __launch_bounds__(256)
-attn_bwd_finish_kernel(const float* __restrict__ partial, int cap, int max_parts, int Hkv, int Sq, int Skv, int group, int causal, int window, int num_kt,
-                       __nv_bfloat16* dk, __nv_bfloat16* dv, long long dk_row, long long dv_row, long long dk_batch, long long dv_batch) {
+attn_bwd_finish_kernel(const float* __restrict__ partial, int cap, int slots, int Hkv, int Sq, int Skv, int group, int causal, int window,
+                       const __grid_constant__ CutTiles cut, __nv_bfloat16* dk, __nv_bfloat16* dv, long long dk_row, long long dv_row,
+                       long long dk_batch, long long dv_batch) {
   b200::begin_kernel();
   constexpr int VPR = HD / 8;
-  const int bh = (int)blockIdx.x / num_kt, jt = (int)blockIdx.x - bh * num_kt;
+  const int bh = (int)blockIdx.x / cut.n, t = (int)blockIdx.x - bh * cut.n, jt = cut.tile[t];
   int i_lo, i_hi;
   const int parts = tile_parts(tile_steps(jt, Sq, Skv, group, causal, window, i_lo, i_hi), cap);
-  if (parts == 1) return;
   const int b = bh / Hkv, hk = bh - b * Hkv;
-  const float* src = partial + (long long)blockIdx.x * max_parts * 2 * BKV * HD;
+  const float* src = partial + ((long long)bh * slots + cut.slot[t]) * 2 * BKV * HD;
   for (int i = blockIdx.y * 256 + threadIdx.x; i < 2 * BKV * VPR; i += gridDim.y * 256) {
     const int half = i / (BKV * VPR), r = i / VPR % BKV, c = i % VPR * 8, key = jt * BKV + r;
     if (key >= Skv) continue;
@@ -540,23 +547,40 @@ attn_bwd_finish_kernel(const float* __restrict__ partial, int cap, int max_parts
   }
 }
 
-// (key tile << 3 | part) of every CTA of one (batch, kv head) pair, longest first; 0 if cap cuts a tile into more than MAX_PARTS or
+// A CTA of one (batch, kv head) pair: a part of a key tile (tile << 3 | part), its cost in steps, and the slot of its sums.
+struct Entry {
+  int cost;
+  uint16_t id, slot;
+};
+
+// The CTAs of one (batch, kv head) pair, longest first, and the tiles that are cut; 0 if cap cuts a tile into more than MAX_PARTS or
 // there are more than MAX_ENTRIES.
-int split_order(int Sq, int Skv, int group, int causal, int window, int cap, std::vector<std::pair<int, uint16_t>>& out, int& max_parts) {
+int split_order(int Sq, int Skv, int group, int causal, int window, int cap, std::vector<Entry>& out, CutTiles& cut, int& slots) {
   const int num_kt = (Skv + BKV - 1) / BKV;
   out.clear();
-  max_parts = 1;
+  cut.n = slots = 0;
   for (int jt = 0; jt < num_kt; ++jt) {
     int lo, hi;
     const int steps = tile_steps(jt, Sq, Skv, group, causal, window, lo, hi), parts = tile_parts(steps, cap);
     if (parts > MAX_PARTS || (int)out.size() + parts > MAX_ENTRIES) return 0;
-    if (parts > max_parts) max_parts = parts;
+    if (parts > 1) {
+      cut.tile[cut.n] = (uint16_t)jt;
+      cut.slot[cut.n++] = (uint16_t)slots;
+    }
     for (int z = 0; z < parts; ++z)
-      out.push_back({steps * (z + 1) / parts - steps * z / parts + (parts > 1 ? 1 : 0), (uint16_t)(jt << 3 | z)});
+      out.push_back({steps * (z + 1) / parts - steps * z / parts + (parts > 1 ? 1 : 0), (uint16_t)(jt << 3 | z),
+                     (uint16_t)(parts > 1 ? slots++ : 0)});
   }
-  std::stable_sort(out.begin(), out.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+  std::stable_sort(out.begin(), out.end(), [](const Entry& a, const Entry& b) { return a.cost > b.cost; });
   return (int)out.size();
 }
+
+// Bytes of the sums of the parts, and how many a plan may take: four times the bf16 dK and dV (two fp32 parts of every tile), or 32 MB.
+// (Unbounded, a fuller chip was bought with any amount: 7168 tokens, 64 / 8 heads of 128, not causal, took 336 MB beside 28 MB of dK
+// and dV for 4300 us, now 112 MB for the same 4300; 256 / 16 heads 672 MB, now none.  The shapes of split_cap's times take 6 to 24 MB,
+// half of what slots for every tile took, in the same times.)
+long long split_bytes(long long copies, int slots, int HD) { return copies * slots * 2 * BKV * HD * 4; }
+long long split_bytes_limit(long long copies, int Skv, int HD) { return std::max(32ll << 20, 4 * copies * Skv * HD * 2 * 2); }
 
 // Steps until the last SM is done: CTAs are taken in their order by the SM that is free first; each costs its steps and five more
 // (set-up, first loads and the output: from the times of split and whole tiles at 2000 and 3000 tokens).
@@ -580,7 +604,7 @@ long long makespan(const std::vector<int>& cost, long long copies, int sms) {
 // Backward, whole tiles -> split: 2000 x 64 / 8 heads of 64 267 -> 171 us, 800 tokens 130 -> 68; heads of 128: 3000 x 64 / 8 532 -> 433,
 // 1024 x 32 / 8 103 -> 65, 2 x 1500 x 16 / 4 143 -> 106.  Parts of every tile alike (five at 2000 tokens) gained half as much, and cost
 // where a part is a few steps long: 4 x 512 x 12 heads 34 -> 56, so those stay whole.
-int split_cap(int B, int Sq, int Skv, int Hq, int Hkv, int causal, int window, int& max_parts) {
+int split_cap(int B, int Sq, int Skv, int Hq, int Hkv, int HD, int causal, int window, int& slots) {
   const int num_kt = (Skv + BKV - 1) / BKV, group = Hq / Hkv, P = b200::sm_count();
   const long long copies = (long long)B * Hkv;
   if (num_kt > MAX_ENTRIES || copies * num_kt > 8 * P) return 0;
@@ -593,15 +617,17 @@ int split_cap(int B, int Sq, int Skv, int Hq, int Hkv, int causal, int window, i
   }
   if (longest < 4 || longest * 12 > INT_MAX) return 0;
   long long best = makespan(cost, copies, P) * 11 / 12;
-  int cap = 0, parts;
-  std::vector<std::pair<int, uint16_t>> order;
+  int cap = 0, n;
+  std::vector<Entry> order;
+  CutTiles cut;
   for (int k = 2; k <= 11; ++k) {
     const int c = (int)((longest * k + 11) / 12);
-    if (!split_order(Sq, Skv, group, causal, window, c, order, parts)) continue;
+    if (!split_order(Sq, Skv, group, causal, window, c, order, cut, n)) continue;
+    if (split_bytes(copies, n, HD) > split_bytes_limit(copies, Skv, HD)) continue;
     cost.clear();
-    for (const auto& e : order) cost.push_back(e.first);
+    for (const auto& e : order) cost.push_back(e.cost);
     const long long t = makespan(cost, copies, P) + 3;      // the launch that adds the parts up
-    if (t < best) { best = t; cap = c; max_parts = parts; }
+    if (t < best) { best = t; cap = c; slots = n; }
   }
   return cap;
 }
@@ -698,9 +724,9 @@ B200_API int b200_attn_bwd_plan(int B, int Sq, int Skv, int Hq, int Hkv, int HD,
   plan[0] = plan[1] = 0;
   if (B <= 0 || Sq <= 0 || Skv <= 0 || Hkv <= 0 || Hq <= 0 || Hq % Hkv != 0 || (HD != 64 && HD != 128)) return 0;
   try {
-    int parts = 0;
-    const int cap = split_cap(B, Sq, Skv, Hq, Hkv, causal, window, parts);
-    if (cap > 0) { plan[0] = cap; plan[1] = (long long)B * Hkv * ((Skv + BKV - 1) / BKV) * parts * 2 * BKV * HD * 4; }
+    int slots = 0;
+    const int cap = split_cap(B, Sq, Skv, Hq, Hkv, HD, causal, window, slots);
+    if (cap > 0) { plan[0] = cap; plan[1] = split_bytes((long long)B * Hkv, slots, HD); }
   } catch (const std::exception&) {
   }
   return 0;
@@ -740,24 +766,29 @@ B200_API int b200_attn_bwd(const void* q, const void* k, const void* v, const vo
   // head keeps that head's Q and dO in L2 (full, 8 x 512 x 24 heads 128 us, 134 the other way; 2 x 4608 x 24 1211 and 1345).
   // With a window the two are even (8192 x 64 / 8 of 64, window 128: 269 and 269; 2 x 8192 x 32, window 1024: 920 and 925).
   p.bh_group = (causal && window <= 0) ? B * Hkv : 1;
-  const int num_kt = (Skv + BKV - 1) / BKV, group = Hq / Hkv;
-  p.cap = 0; p.entries = 0; p.max_parts = 1; p.partial = (float*)workspace;
+  const int group = Hq / Hkv;
+  p.cap = 0; p.entries = 0; p.slots = 0; p.partial = (float*)workspace;
+  CutTiles cut;
+  cut.n = 0;
   if (cap > 0) {
     try {
-      std::vector<std::pair<int, uint16_t>> order;
-      p.entries = split_order(Sq, Skv, group, causal, window, cap, order, p.max_parts);
-      if (p.entries == 0 || workspace == nullptr || workspace_bytes < (long long)B * Hkv * num_kt * p.max_parts * 2 * BKV * HD * 4)
+      std::vector<Entry> order;
+      p.entries = split_order(Sq, Skv, group, causal, window, cap, order, cut, p.slots);
+      if (p.entries == 0 || workspace == nullptr || workspace_bytes < split_bytes((long long)B * Hkv, p.slots, HD))
         return b200::fail(613, "attn_bwd: cap %d and %lld bytes are not the plan of this shape", cap, workspace_bytes);
-      for (int i = 0; i < p.entries; ++i) p.order[i] = order[i].second;
+      for (int i = 0; i < p.entries; ++i) {
+        p.order[i] = order[i].id;
+        p.slot[i] = order[i].slot;
+      }
     } catch (const std::exception& e) {
       return b200::fail(614, "attn_bwd: %s", e.what());
     }
     p.cap = cap;
   }
-  if ((r = HD == 128 ? launch_bwd<128>(m, p, (cudaStream_t)stream) : launch_bwd<64>(m, p, (cudaStream_t)stream)) || p.cap == 0) return r;
+  if ((r = HD == 128 ? launch_bwd<128>(m, p, (cudaStream_t)stream) : launch_bwd<64>(m, p, (cudaStream_t)stream)) || cut.n == 0) return r;
   auto fin = HD == 128 ? attn_bwd_finish_kernel<128> : attn_bwd_finish_kernel<64>;
-  b200::launch(fin, dim3((unsigned)(B * Hkv * num_kt), HD / 16), 256, 0, (cudaStream_t)stream, 
-      p.partial, cap, p.max_parts, Hkv, Sq, Skv, group, causal, window, num_kt, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, dk_row, dv_row, dk_batch, dv_batch);
+  b200::launch(fin, dim3((unsigned)(B * Hkv * cut.n), HD / 16), 256, 0, (cudaStream_t)stream, (const float*)p.partial, cap, p.slots, Hkv, Sq, Skv,
+               group, causal, window, cut, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, dk_row, dv_row, dk_batch, dv_batch);
   b200::count_launch();
   return b200::check_launch("attn_bwd_finish");
 }

@@ -1,5 +1,6 @@
 """Attention backward at the edges of its schedule: one step, odd step counts, ragged tiles, keys that no query sees, windows,
 more keys than queries, grouped heads."""
+import ctypes
 import re
 from pathlib import Path
 
@@ -61,3 +62,23 @@ def test_copies_are_issued_only_where_they_are_awaited():
     text = (Path(__file__).resolve().parent.parent / "mlperf_training_b200/csrc/attention_bwd.cu").read_text()
     role = text[text.index("TMA producer -"):text.index("MMA issuer -")]
     assert role.index("n_iter > 0") < role.index("mbar_expect_tx(kv_full") and re.search(r"if \([^)]*n_iter > 0\) \{", role)
+
+
+def test_scratch_of_cut_key_tiles_is_bounded():
+    """The planner's scratch stays below four times the bf16 dK and dV, or 32 MB, over sizes, groups, head dims and masks; the
+    sizes whose times are known keep their cut."""
+    out = (ctypes.c_longlong * 2)()
+    plan = _lib.load().b200_attn_bwd_plan
+    cut = 0
+    for S in (200, 777, 2000, 4096, 7168, 9000):
+        for Hq, Hkv in ((2, 2), (16, 2), (64, 8), (256, 16), (32, 1)):
+            for D in (64, 128):
+                for B, causal, window in ((1, 1, 0), (1, 0, 0), (3, 0, 0), (1, 1, 300)):
+                    plan(B, S, S, Hq, Hkv, D, causal, window, out)
+                    assert out[1] <= max(32 << 20, 4 * 2 * B * S * Hkv * D * 2), (S, Hq, Hkv, D, B, causal, window, out[1])
+                    assert (out[0] > 0) == (out[1] > 0)
+                    cut += out[0] > 0
+    assert cut > 20
+    for shape in ((1, 2000, 2000, 64, 8, 64, 1, 0), (1, 3000, 3000, 64, 8, 128, 1, 0), (1, 1024, 1024, 32, 8, 128, 1, 0)):
+        plan(*shape, out)
+        assert 0 < out[0] and out[1] < 26 << 20

@@ -183,7 +183,8 @@ B200_DEVICE float gelu_tanh(float x) {
 B200_DEVICE float gelu_tanh_grad(float x) {
   const float k2 = 2.f * 0.7978845608028654f;
   const float s = sigmoid(k2 * (x + 0.044715f * x * x * x));
-  return s + x * s * (1.f - s) * k2 * (1.f + 3.f * 0.044715f * x * x);
+  const float c = fminf(fmaxf(x, -16.f), 16.f);      // beyond, s (1 - s) is 0 and the factor beside it must not overflow
+  return s + c * s * (1.f - s) * k2 * (1.f + 3.f * 0.044715f * c * c);
 }
 // rows x vpr vectors of 8; pitches in elements (a plain tensor is one row)
 template <typename I>

@@ -115,7 +115,9 @@ def test_scatter_add_rows_of_an_unaligned_table():
 
 def test_gelu_limits():
     """Large and infinite inputs, and the cancellation-free negative tail, against fp64."""
-    x = torch.cat([torch.linspace(-12, 12, 4091), torch.tensor([-1e30, 1e30, -200.0, 200.0, 0.0])]).bfloat16()
+    inf = float("inf")
+    x = torch.cat([torch.linspace(-12, 12, 4091), torch.tensor([-1e30, 1e30, -200.0, 200.0, 0.0, -3.3e38, 3.3e38, inf, -inf, float("nan"),
+                                                                -16.0, 16.0, -17.0])]).bfloat16()
     y, g = kernels.gelu_fwd(x.cuda()).cpu(), kernels.gelu_bwd(torch.ones_like(x).cuda(), x.cuda()).cpu()
     xd = x[:4091].double().requires_grad_(True)
     yd = xd * torch.sigmoid(2 * 0.7978845608028654 * (xd + 0.044715 * xd ** 3))      # (1 + tanh cancels in fp64, too)
@@ -123,7 +125,11 @@ def test_gelu_limits():
     # one bf16 rounding (2^-9) over fp32 arithmetic whose exponent of e^-2u carries |2u| 2^-23 (u up to 70 here)
     assert ((y[:4091].double() - yd).abs() <= yd.abs() * 2 ** -8 + 1e-30).all()
     assert ((g[:4091].double() - xd.grad).abs() <= xd.grad.abs() * 2 ** -8 + 2e-6).all()
-    assert y[4091:].tolist() == [0.0, x[4092].item(), 0.0, 200.0, 0.0]
+    big = x[4091:]
+    assert y[4091:4099].tolist() == [0.0, big[1].item(), 0.0, 200.0, 0.0, 0.0, big[6].item(), inf]
+    assert y[4099:4101].isnan().all() and y[4101:].tolist() == [0.0, 16.0, 0.0]      # (-inf times 0, as x sigmoid(2 u) has it)
+    assert g[4091:4100].tolist() == [0.0, 1.0, 0.0, 1.0, 0.5, 0.0, 1.0, 1.0, 0.0] and g[4100].isnan()
+    assert g[4101:].tolist() == [0.0, 1.0, 0.0]
 
 
 @pytest.mark.parametrize("V", [2048, 32000, 128256])

@@ -92,3 +92,71 @@ def test_gemm_deterministic():
     d2 = kernels.gemm(a, b)
     torch.cuda.synchronize()
     assert torch.equal(d1, d2)
+
+
+def _forms():
+    """Operands as callers hand them over: (name, arguments) of gemm, whose operands the native operator takes or leaves to the
+    general path."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    out = []
+    for M, N, K in ((1, 136, 64), (5, 72, 136), (129, 264, 136), (256, 2880, 320), (300, 520, 1000)):
+        for a_mn in (False, True):
+            for b_mn in (False, True):
+                def ab(pad=0, off=0):
+                    def t(r, c):
+                        return rnd(r, c + pad + off)[:, off:off + c]
+                    return (t(K, M) if a_mn else t(M, K)), (t(K, N) if b_mn else t(N, K))
+                lay = dict(a_mn_major=a_mn, b_mn_major=b_mn)
+                tag = f"{M}x{N}x{K} {int(a_mn)}{int(b_mn)}"
+                a, b = ab()
+                out.append((tag, a, b, lay))
+                out.append((tag + " padded rows", *ab(pad=8), lay))
+                out.append((tag + " odd pitch", *ab(pad=3), lay))
+                out.append((tag + " off 16 bytes", *ab(pad=7, off=1), lay))
+                out.append((tag + " fp32 out, alpha", a, b, dict(lay, out_dtype=torch.float32, alpha=0.5)))
+                out.append((tag + " bias", a, b, dict(lay, bias=rnd(N))))
+                out.append((tag + " fp32 strided bias", a, b, dict(lay, bias=rnd(2 * N).float()[::2])))
+                out.append((tag + " residual of wider rows", a, b, dict(lay, residual=rnd(M, N + 8)[:, :N], bias=rnd(N))))
+                out.append((tag + " fp32 residual", a, b, dict(lay, residual=rnd(M, N).float())))
+                out.append((tag + " transposed residual", a, b, dict(lay, residual=rnd(N, M).t())))
+                out.append((tag + " into wider rows", a, b, dict(lay, out=rnd(M, N + 16)[:, :N])))
+                out.append((tag + " added to fp32", a, b, dict(lay, out=rnd(M, N).float(), accumulate=True)))
+    a, b = rnd(16, 64), rnd(24, 64)
+    out += [("expanded", rnd(1, 64).expand(16, 64), b, {}), ("one row", a[3:4], b, {}), ("transposed", rnd(64, 16).t(), b, {}),
+            ("empty", a[:0], b, {}), ("widths", a, rnd(24, 72), {}), ("odd columns", a, b[:5], {}), ("fp32", a.float(), b, {}),
+            ("fp16 out", a, b, dict(out_dtype=torch.float16)), ("nothing to add to", a, b, dict(accumulate=True)),
+            ("other rows", a, b, dict(out=rnd(15, 24))), ("out in columns", a, b, dict(out=rnd(24, 16).t())),
+            ("out off 16 bytes", a, b, dict(out=rnd(16, 32)[:, 1:25]))]
+    return out
+
+
+def test_native_operator_equals_the_general_path(monkeypatch):
+    """Same results, bit for bit, and the same refusals, over the layouts, pitches, types and options of the operands."""
+    if _lib.host is None:
+        pytest.skip("no native operator in this build")
+
+    def run(a, b, kw):
+        if "out" in kw:
+            base = kw["out"]
+            kw = dict(kw, out=base.clone() if base.is_contiguous() else base._base.clone().as_strided(base.shape, base.stride(),
+                                                                                                     base.storage_offset()))
+        try:
+            d = kernels.gemm(a, b, **kw)
+            assert kw.get("out") is None or d is kw["out"]
+            return d
+        except (ValueError, TypeError, RuntimeError) as e:
+            return type(e), str(e)
+    forms = _forms()
+    native = [run(a, b, kw) for _, a, b, kw in forms]
+    monkeypatch.setattr(_lib, "host", None)
+    refused = 0
+    for (name, a, b, kw), got in zip(forms, native):
+        want = run(a, b, kw)
+        if isinstance(want, tuple):
+            assert got == want, name
+            refused += 1
+        else:
+            assert got.dtype == want.dtype and got.stride() == want.stride() and torch.equal(got, want), name
+    assert refused >= 6
+    _lib.check_status("native gemm")

@@ -66,7 +66,7 @@ def test_quantize_scale_limits():
 @pytest.mark.parametrize("R,F", [(128, 128), (256, 160), (384, 2880), (128, 96)])
 def test_quantize_swiglu_bwd_equals_the_separate_kernels(R, F):
     """d gate | d up from one tile pair: codes and scales of quantising the stand-alone kernel's output, bit for bit, at widths
-    whose halves start inside a scale word; rows past ``live`` are left alone."""
+    whose halves start inside a scale word; with ``live`` the rows before it are the same."""
     from mlperf_training_b200.ops import kernels as K
     torch.manual_seed(R + F)
     gu, da = (torch.randn(R, 2 * F, device="cuda") * 3).bfloat16(), torch.randn(R, F, device="cuda").bfloat16()
@@ -80,6 +80,34 @@ def test_quantize_swiglu_bwd_equals_the_separate_kernels(R, F):
     live = torch.tensor([128], dtype=torch.int32, device="cuda")
     part = mxfp8.quantize_swiglu_bwd(da, gu, row_tile=128, col_tile=208, live=live)
     assert torch.equal(part[0].q[:128], want[0].q[:128]) and torch.equal(part[1].q[:, :128], want[1].q[:, :128])
+
+
+@pytest.mark.parametrize("live", [0, 128, 256, 384])
+@pytest.mark.parametrize("F", [128, 160])
+def test_quantisers_leave_rows_past_live_alone(live, F):
+    """Codes and scales of the 128-row tiles behind ``live`` keep what the buffers held, those before it are the full run's."""
+    from mlperf_training_b200.ops import _lib
+    torch.manual_seed(live + F)
+    R = 384
+    gu, da = torch.randn(R, 2 * F, device="cuda").bfloat16(), torch.randn(R, F, device="cuda").bfloat16()
+    n = torch.tensor([live], dtype=torch.int32, device="cuda")
+    p, st = _lib.ptr, _lib.stream_ptr()
+    for name, args, C in (("b200_quant_mxfp8", (p(gu), 2 * F, R, 2 * F), 2 * F), ("b200_quant_swiglu_mxfp8", (p(gu), 2 * F, R, F), F),
+                          ("b200_quant_swiglu_bwd_mxfp8", (p(da), F, p(gu), 2 * F, R, F), 2 * F)):
+        runs = []
+        for fill, lv in ((0x5A, None), (0x5A, n)):
+            size = (R * C, mxfp8.sf_bytes(R, C, 128), C * R, mxfp8.sf_bytes(C, R, 128))
+            q_row, sf_row, q_col, sf_col = (torch.full((k,), fill, dtype=torch.uint8, device="cuda") for k in size)
+            _lib.call(name, *args, p(q_row), p(sf_row), 128, p(q_col), p(sf_col), 128, p(lv), st)
+            # rows tile by tile; the transposed copy's contraction in groups of 128 rows of the source
+            runs.append((q_row.view(R // 128, -1), sf_row.view(R // 128, -1), q_col.view(C, R // 128, 128).transpose(0, 1),
+                         sf_col.view(-1, R // 128, 512).transpose(0, 1)))
+        for full, part in zip(*runs):
+            assert torch.equal(part[:live // 128], full[:live // 128])
+            assert (part[live // 128:] == 0x5A).all()
+            if live < R:
+                assert (full[live // 128:] != 0x5A).any()
+    _lib.check_status("live")
 
 
 def test_no_column_copies_without_grad_and_weight_copies_in_one_pass():

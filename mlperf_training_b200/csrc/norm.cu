@@ -437,10 +437,10 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
   }
 }
 
-// Backward of the same widths, with the row sums in the same lane order (dx of the CTA-per-row split differs in the last
-// bit of 4 elements in a million; that split took 50 instead of 62 us for 4011 x 4096): dx per row; dw / db accumulated per warp in shared memory (fixed lane -> column mapping, no
+// Backward of the same widths with the activation: a warp per row, summed lane by lane in column order as in the forward, so that the
+// activation is recomputed over the same split.  dw / db accumulated per warp in shared memory (fixed lane -> column mapping, no
 // atomics), summed over the CTA's warps in order and written as one partial row per CTA.
-template <int MODE, int ACT>
+template <int MODE>
 __global__ void __launch_bounds__(256)
 norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                      const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
@@ -448,14 +448,13 @@ norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
                      const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                      float* __restrict__ partial, int T, int D, int nwarps) {
   b200::begin_kernel();
-  extern __shared__ float acc[];  // [nwarps][(MODE == 1 || ACT) ? 2 : 1][D]
-  constexpr int NACC = (MODE == 1 || ACT) ? 2 : 1;
+  extern __shared__ float acc[];  // [nwarps][dw | db][D]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nv = D >> 8;
-  float* my_w = acc + (long long)warp * NACC * D;
+  float* my_w = acc + (long long)warp * 2 * D;
   float* my_b = my_w + D;
   if (warp < nwarps)
-    for (int i = lane; i < NACC * D; i += 32) my_w[i] = 0.f;
+    for (int i = lane; i < 2 * D; i += 32) my_w[i] = 0.f;
   __syncwarp();
   if (warp < nwarps) {
     for (int row = blockIdx.x * nwarps + warp; row < T; row += gridDim.x * nwarps) {
@@ -480,35 +479,27 @@ norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
 #pragma unroll
           for (int j = 0; j < 8; ++j) { w8[j] = 1.f; b8[j] = 0.f; }
           if (w != nullptr) unpack8(ld16(w + c), w8);
-          if (ACT && b != nullptr) unpack8(ld16(b + c), b8);
+          if (b != nullptr) unpack8(ld16(b + c), b8);
           float4 a0 = *reinterpret_cast<float4*>(my_w + c), a1 = *reinterpret_cast<float4*>(my_w + c + 4);
           float aw[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-          float ab[8];
-          if (NACC == 2) {
-            float4 b0 = *reinterpret_cast<float4*>(my_b + c), b1 = *reinterpret_cast<float4*>(my_b + c + 4);
-            ab[0] = b0.x; ab[1] = b0.y; ab[2] = b0.z; ab[3] = b0.w; ab[4] = b1.x; ab[5] = b1.y; ab[6] = b1.z; ab[7] = b1.w;
-          }
+          float4 b0 = *reinterpret_cast<float4*>(my_b + c), b1 = *reinterpret_cast<float4*>(my_b + c + 4);
+          float ab[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float xn = (x8[j] - mean) * rstd;
-            float dn = d8[j];
-            if (ACT) {
-              const float n = xn * w8[j] + b8[j];
-              const float sg = 1.f / (1.f + __expf(-n));
-              dn = d8[j] * x8[j] * sg * (1.f - sg);
-            }
+            const float n = xn * w8[j] + b8[j];
+            const float sg = 1.f / (1.f + __expf(-n));
+            const float dn = d8[j] * x8[j] * sg * (1.f - sg);
             aw[j] += dn * xn;
-            if (NACC == 2) ab[j] += dn;
+            ab[j] += dn;
             const float gj = dn * w8[j];
             s1 += gj * xn;
             s2 += gj;
           }
           *reinterpret_cast<float4*>(my_w + c) = make_float4(aw[0], aw[1], aw[2], aw[3]);
           *reinterpret_cast<float4*>(my_w + c + 4) = make_float4(aw[4], aw[5], aw[6], aw[7]);
-          if (NACC == 2) {
-            *reinterpret_cast<float4*>(my_b + c) = make_float4(ab[0], ab[1], ab[2], ab[3]);
-            *reinterpret_cast<float4*>(my_b + c + 4) = make_float4(ab[4], ab[5], ab[6], ab[7]);
-          }
+          *reinterpret_cast<float4*>(my_b + c) = make_float4(ab[0], ab[1], ab[2], ab[3]);
+          *reinterpret_cast<float4*>(my_b + c + 4) = make_float4(ab[4], ab[5], ab[6], ab[7]);
         }
       s1 = warp_sum(s1) / D;
       s2 = (MODE == 1) ? warp_sum(s2) / D : 0.f;
@@ -522,18 +513,14 @@ norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
 #pragma unroll
           for (int j = 0; j < 8; ++j) { w8[j] = 1.f; b8[j] = 0.f; }
           if (w != nullptr) unpack8(ld16(w + c), w8);
-          if (ACT && b != nullptr) unpack8(ld16(b + c), b8);
+          if (b != nullptr) unpack8(ld16(b + c), b8);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float xn = (x8[j] - mean) * rstd;
-            float dn = d8[j], direct = 0.f;
-            if (ACT) {
-              const float n = xn * w8[j] + b8[j];
-              const float sg = 1.f / (1.f + __expf(-n));
-              dn = d8[j] * x8[j] * sg * (1.f - sg);
-              direct = d8[j] * sg;
-            }
-            o[j] = rstd * (dn * w8[j] - xn * s1 - s2) + direct;
+            const float n = xn * w8[j] + b8[j];
+            const float sg = 1.f / (1.f + __expf(-n));
+            const float dn = d8[j] * x8[j] * sg * (1.f - sg);
+            o[j] = rstd * (dn * w8[j] - xn * s1 - s2) + d8[j] * sg;
           }
           if (dres != nullptr) {
             float r8[8];
@@ -551,8 +538,8 @@ norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
     for (int c = threadIdx.x; c < D; c += blockDim.x) {
       float sw = 0.f, sb = 0.f;
       for (int k = 0; k < nwarps; ++k) {
-        sw += acc[(long long)k * NACC * D + c];
-        if (NACC == 2) sb += acc[(long long)k * NACC * D + D + c];
+        sw += acc[(long long)k * 2 * D + c];
+        sb += acc[(long long)k * 2 * D + D + c];
       }
       pw[c] = sw;
       pw[D + c] = sb;
@@ -848,16 +835,15 @@ int run_bwd_ring(const BwdArgs& a) {
   return launch_bwd_ring<MODE, G, V, R, 2, MAXT>(a, threads, 2 * stage);
 }
 
-template <int MODE, int ACT>
+template <int MODE>
 int run_bwd_warp(const BwdArgs& a) {
-  constexpr int nacc = (MODE == 1 || ACT) ? 2 : 1;
-  int nwarps = (200 * 1024) / (a.D * 4 * nacc);
+  int nwarps = (200 * 1024) / (a.D * 4 * 2);
   if (nwarps > 8) nwarps = 8;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!configured[dev & 63]) {
-    cudaError_t e = cudaFuncSetAttribute(norm_bwd_warp_kernel<MODE, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(norm_bwd_warp_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return -b200::fail(302, "norm_bwd: cannot raise shared memory: %s", cudaGetErrorString(e));
@@ -865,8 +851,8 @@ int run_bwd_warp(const BwdArgs& a) {
     configured[dev & 63] = true;
   }
   const int grid = b200::sm_count() < a.grid ? b200::sm_count() : a.grid;
-  b200::launch(norm_bwd_warp_kernel<MODE, ACT>, grid, 256, nwarps * nacc * a.D * 4, a.st, a.dy, a.x, a.w, a.b, a.mean, a.rstd, a.dres, a.dx,
-                                                                                a.partial, a.T, a.D, nwarps);
+  b200::launch(norm_bwd_warp_kernel<MODE>, grid, 256, nwarps * 2 * a.D * 4, a.st, a.dy, a.x, a.w, a.b, a.mean, a.rstd, a.dres, a.dx,
+               a.partial, a.T, a.D, nwarps);
   return grid;
 }
 
@@ -883,7 +869,7 @@ int dispatch_bwd(const BwdArgs& a) {
   } else {
     if (a.D <= 512) return run_bwd<MODE, ACT, 32, 2, 2>(a);
     if (a.D <= 1024) return run_bwd<MODE, ACT, 32, 4, 1>(a);
-    if (a.D % 256 == 0 && a.D <= 4096) return run_bwd_warp<MODE, ACT>(a);
+    if (a.D % 256 == 0 && a.D <= 4096) return run_bwd_warp<MODE>(a);
     if (a.D <= 4096) return run_bwd<MODE, ACT, 0, 2, 2>(a);
     return run_bwd<MODE, ACT, 0, 2, 2, 512>(a);
   }

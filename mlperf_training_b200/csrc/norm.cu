@@ -197,10 +197,10 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 }
 
 // Forward of widths that are whole vectors of a warp up to 4096: a warp per row, up to 16 vectors per lane, summed lane
-// by lane in column order.  The CTA-per-row split is up to 20 % faster at 4096 (27 -> 22 us for 4011 rows), but adds the
-// squares in another order, and with block-scaled linears behind it one flipped bf16 bit in 90000 grew to 3 % of the
-// attention gradients over three quantisers.  (The launch does not know what reads its result, so bf16 consumers pay for it
-// too: two norms each way of a bf16 block.)
+// by lane in column order.  The CTA-per-row split is up to 20 % faster at 4096 (27 -> 22 us for 4011 rows) and no less exact.  It is not
+// taken here yet: it adds the squares in another order, one bf16 bit in 90000 flips, and block-scaled linears behind it turn that
+// into 3 % of the attention gradients over three quantisers, at the same error against 64 bits.  (The backward has taken the ring's
+// order, which does the same to a step's gradients, for 73 -> 52 us at 8192 x 4096.)
 constexpr int WMAXV = 16;
 template <int MODE>
 __global__ void __launch_bounds__(256)
@@ -547,12 +547,15 @@ norm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   }
 }
 
-// Backward without the activation for rows of more than 256 columns.  Bound by memory: x and dy (and dres) are read and dx
+// Backward without the activation for rows of more than 256 columns: x and dy (and dres) are read and dx
 // written once.  A team (G = 32: a warp, G = 0: the CTA) owns whole rows, a thread the same V vectors of columns in all of them, so the
 // column sums stay in its registers.  Every thread copies its own vectors of the next S - 1 row groups into its own slots of a
 // ring in shared memory (cp.async: no registers held, no barrier).  With loads of a row that started when the row before was done,
-// column sums included: 8192 x 2880 64 us, now 46 (3.1 TB/s), 8192 x 4096 73 and 52, 4096 x 8192 85 and 64; with a residual's
+// column sums included: 8192 x 2880 64 us, now 46, 8192 x 4096 73 and 52, 4096 x 8192 85 and 64; with a residual's
 // gradient 89 and 50, 114 and 58, 109 and 75; LayerNorm of 46000 x 512 46 and 46, with a residual 67 and 52.
+// Bound by instructions before memory: alone it takes 34 us for 8192 x 2880 (4.1 TB/s, 0.63 of the measured copy rate) and 42 for
+// 8192 x 4096 (4.8 TB/s), with 68 and 73 % of the issue slots taken by the 23 and 29 warps that 64 registers a thread leave on an SM;
+// the rest waits for barriers and shared memory.  The sum over the CTAs' partial rows and the launches are the other 10 us.
 template <int MODE, int G, int V, int R, int S, int MAXT>
 __global__ void __launch_bounds__(MAXT, MODE == 1 && V * MAXT > 512 ? 1 : 2)
 norm_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
